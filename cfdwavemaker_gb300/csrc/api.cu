@@ -211,44 +211,17 @@ __global__ void k_clamp_z(long n, const double *z, double depth, double *zc) {
     if (p < n) zc[p] = fmax(-depth, z[p]);
 }
 
-// Irregular wave types 1 and 5 finish here: out rows
-// 0 SurfElev, 1 VeloX, 2 VeloY, 3 VeloZ, 4 DynPres, 5 nhPres.  sgp: the
-// s-grid holds the dynamic pressure (row 4 of its query).
-// The API rows of the model outputs: out[6][n] (eta, u, v, w, dp, nhpres;
-// or null) and/or the wave_Kinematics records kin[n][4] (eta, u, v, w; or
-// null), written in one pass.  Without a ramp the factor is not applied: FP64
-// multiplies run at a small fraction of the FP32 rate on this GPU.
-__global__ void k_finish(long n, int wavetype, int sgp, RampDev r, double rho, double g, const double *x,
-                         const double *y, const double *t, const double *f, const double *fe,
-                         double *out, double *kin) {
+// The Smit theory finishes here (the other waves write their rows in their
+// own last kernel): the API rows of f[5][n] = eta, u, v, w, dp.  Without a
+// ramp the factor is not applied: FP64 multiplies run at a small fraction of
+// the FP32 rate on this GPU.
+__global__ void k_finish(long n, const double *f, ApiRows a) {
     long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (p >= n) return;
-    const bool ramped = r.init;
-    const double rr = ramped ? d_ramp(r, t[p], x[p], y[p]) : 1.0;
     double v[6];
-    if (wavetype == WT_IRREGULAR) {
-        // f = [5][n] eta, u, v, w, dp of Irregular::*
-        for (int q = 0; q < 5; q++) v[q] = f[q * n + p];
-        v[5] = f[4 * n + p] - rho * g * f[0 * n + p];
-    } else {
-        // WT_IRR_SGRID (regular waves write their rows in their own kernel)
-        // f = [4][n] query at the clamped z (sgp: [5][n] with the pressure),
-        // fe = [4][n] query at z = 0.  Without a pressure field the
-        // reference's 0.0 (CFDwavemaker.cpp:1808-1812, 1815-1891); with one,
-        // the irregular sea's forms (:1807-1808, 1826-1830) on the grid.
-        v[0] = fe[0 * n + p];
-        v[1] = f[1 * n + p];
-        v[2] = f[2 * n + p];
-        v[3] = f[3 * n + p];
-        v[4] = sgp ? f[4 * n + p] : 0.0;
-        v[5] = sgp ? f[4 * n + p] - rho * g * f[0 * n + p] : 0.0;
-    }
-    if (ramped)
-        for (int q = 0; q < 6; q++) v[q] *= rr;
-    if (out)
-        for (int q = 0; q < 6; q++) out[q * n + p] = v[q];
-    if (kin)
-        for (int q = 0; q < 4; q++) kin[4 * p + q] = v[q];
+    for (int q = 0; q < 5; q++) v[q] = f[q * n + p];
+    v[5] = v[4] - a.rho * a.g * v[0];
+    api_store(a, p, v);
 }
 
 // wave_VFrac (CFDwavemaker.cpp:1990-2009) from the ramped elevation.
@@ -278,61 +251,61 @@ RampDev ramp_dev(const RampCfg &r) {
     return d;
 }
 
-// The device pipeline: out[6][n] of the reference's wave_* functions for
-// the points (x, y, z, t), all device pointers.  want: bit q = output q.
+// The rows of one call: row[q][n] of wave_SurfElev .. wave_nhPres (null: not
+// wanted) and the wave_Kinematics records.
+struct OutRows {
+    double *row[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    double *kin = nullptr;
+};
+
+// The device pipeline: the rows of the reference's wave_* functions for the
+// points (x, y, z, t), all addresses the kernels can use.  want: bit q =
+// output q.
 int eval_api(long n, const double *x, const double *y, const double *z, const double *t, int want,
-             double *out, cudaStream_t s, double *kin = nullptr) {
+             const OutRows &out, cudaStream_t s) {
     Model &M = g_model;
     if (!M.init) return E_NOT_INITIALIZED;
     if (n <= 0) return OK;
     int wt = M.cfg.wavetype;
-    RampDev rd = ramp_dev(M.cfg.ramp);
+    ApiRows ar{};
+    ar.ramp = ramp_dev(M.cfg.ramp);
+    ar.rho = M.cfg.rho; ar.g = M.cfg.gravity;
+    ar.x = x; ar.y = y; ar.t = t;
+    for (int q = 0; q < 6; q++) ar.row[q] = out.row[q];
+    ar.kin = out.kin;
     // regular waves: one kernel clamps z, evaluates, applies the ramp and
     // writes the rows and records
-    if (wt == WT_REGULAR) return regular_eval(M.reg, M.cfg, n, x, y, z, t, rd, out, kin, s);
+    if (wt == WT_REGULAR) return regular_eval(M.reg, M.cfg, n, z, ar, s);
+    // the s-grid query likewise (one pass instead of a clamp, a query and a
+    // finishing pass)
+    if (wt == WT_IRR_SGRID) return grid_query(M.grid, n, z, ar, s);
+    if (wt != WT_IRREGULAR) return E_UNSUPPORTED;
     Workspace &ws = t_ctx.ws;
     int mask = 0;
-    if (wt == WT_IRREGULAR) {
-        if (want & (1 | 32)) mask |= 1;
-        if (want & 2) mask |= 2;
-        if (want & 4) mask |= 4;
-        if (want & 8) mask |= 8;
-        if (want & (16 | 32)) mask |= 16;
-        // irregular waves: the seabed clamp in the height pass and the API
-        // rows written by the combining pass (no clamp or finishing pass),
-        // except where the Smit theory's kernels write the velocity rows
-        if ((out || kin) && !(M.sea.smit && (mask & 30))) {
-            const ApiRows ar{rd, M.cfg.rho, M.cfg.gravity, x, y, t, out, kin};
-            return irregular_eval(M.sea, n, x, y, z, t, mask, nullptr, ws, s, &ar);
-        }
-    }
-    // scratch: clamped z [n], model outputs [5][n] and [4][n]
-    size_t need = sizeof(double) * (size_t)n * 10;
+    if (want & (1 | 32)) mask |= 1;
+    if (want & 2) mask |= 2;
+    if (want & 4) mask |= 4;
+    if (want & 8) mask |= 8;
+    if (want & (16 | 32)) mask |= 16;
+    // irregular waves: the seabed clamp in the height pass and the API
+    // rows written by the combining pass (no clamp or finishing pass),
+    // except where the Smit theory's kernels write the velocity rows
+    if (ar.any() && !(M.sea.smit && (mask & 30)))
+        return irregular_eval(M.sea, n, x, y, z, t, mask, nullptr, ws, s, &ar);
+    // scratch: clamped z [n], model outputs [5][n]
+    size_t need = sizeof(double) * (size_t)n * 6;
     // irregular_eval uses the same thread workspace; keep a separate buffer
     Workspace &api_ws = t_ctx.api_ws;
     int rc = workspace_reserve(api_ws, need);
     if (rc) return rc;
-    double *zc = (double *)api_ws.base, *f = zc + n, *fe = f + 5 * n;
+    double *zc = (double *)api_ws.base, *f = zc + n;
     k_clamp_z<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, z, M.cfg.depth, zc);
     note_launch();
     CKR(cudaGetLastError());
-    if (wt == WT_IRREGULAR) {
-        CKR(cudaMemsetAsync(f, 0, sizeof(double) * 5 * n, s));
-        rc = irregular_eval(M.sea, n, x, y, zc, t, mask, f, ws, s);
-        if (rc) return rc;
-    } else if (wt == WT_IRR_SGRID) {
-        // get_kinematics_at_point forms eta before it looks at z
-        // (lsgrid_spline.cpp:505-571), so one query serves wave_SurfElev
-        // (queried at z = 0) and the velocities (queried at the clamped z)
-        rc = grid_query(M.grid, n, x, y, zc, t, f, s);
-        if (rc) return rc;
-        fe = f;
-    } else {
-        return E_UNSUPPORTED;
-    }
-    const int sgp = (wt == WT_IRR_SGRID && M.grid.nf == 4) ? 1 : 0;
-    k_finish<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(n, wt, sgp, rd, M.cfg.rho, M.cfg.gravity, x, y, t,
-                                                         f, fe, out, kin);
+    CKR(cudaMemsetAsync(f, 0, sizeof(double) * 5 * n, s));
+    rc = irregular_eval(M.sea, n, x, y, zc, t, mask, f, ws, s);
+    if (rc) return rc;
+    k_finish<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(n, f, ar);
     note_launch();
     CKR(cudaGetLastError());
     return OK;
@@ -359,6 +332,36 @@ static void host_copy(double *dst, const double *src, long n) {
     for (auto &t : th) t.join();
 }
 
+// Whether the evaluation's last kernel may write the caller's rows itself
+// with the result that a scratch block and a copy per row would give: every
+// row aligned for FP64 stores, in this device's memory (or host memory it
+// addresses), and overlapping no input and no other row except where it is
+// that same array (each thread reads its point's inputs before it writes that
+// point's rows, in row order, and no other thread reads them).
+bool rows_in_place(double *const outs[6], const double *const ins[4], long n) {
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    auto apart = [n](const double *a, const double *b) {
+        return a == b || (const char *)a + sizeof(double) * n <= (const char *)b ||
+               (const char *)b + sizeof(double) * n <= (const char *)a;
+    };
+    for (int q = 0; q < 6; q++) {
+        if (!outs[q]) continue;
+        if (((uintptr_t)outs[q] & 7) != 0) return false;
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, outs[q]) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type == cudaMemoryTypeDevice && at.device != dev) return false;
+        for (int i = 0; i < 4; i++)
+            if (!apart(outs[q], ins[i])) return false;
+        for (int r = 0; r < q; r++)
+            if (outs[r] && !apart(outs[q], outs[r])) return false;
+    }
+    return true;
+}
+
 // Runs eval_api on user arrays, staging host memory as needed.  outs[q]
 // receives row q of the pipeline output (NULL: not wanted).  For VFrac the
 // caller post-processes row 0.
@@ -382,31 +385,37 @@ int run_batch(const double *x, const double *y, const double *z, const double *t
     // 3.73e8 points/s).
     const bool direct = !dev && n <= (1L << 22) && direct_host_access();
     if (dev || direct) {
-        double *out = nullptr;
-        Workspace &ws = t_ctx.ws;
-        (void)ws;
-        static thread_local Workspace dev_out;
-        int rc = workspace_reserve(dev_out, sizeof(double) * 6 * (size_t)n);
-        if (rc) return rc;
-        out = (double *)dev_out.base;
         const double *zz = z ? z : t;   // z unused for SurfElev only
-        bool rows = vf_out != nullptr;
-        for (int q = 0; q < 6; q++) rows = rows || outs[q] != nullptr;
-        // the Kinematics records come straight from the finishing pass
-        rc = eval_api(n, x, y, zz, t, want, rows ? out : nullptr, s, kin_out);
+        const double *ins[4] = {x, y, zz, t};
+        // the caller's arrays are written by the evaluation's last kernel;
+        // where that could give another result (rows_in_place), through a
+        // scratch block and a copy per row
+        const bool place = rows_in_place(outs, ins, n);
+        OutRows o;
+        o.kin = kin_out;
+        double *scratch = nullptr;
+        static thread_local Workspace dev_out;
+        if (vf_out || !place) {
+            int rc = workspace_reserve(dev_out, sizeof(double) * 6 * (size_t)n);
+            if (rc) return rc;
+            scratch = (double *)dev_out.base;
+        }
+        for (int q = 0; q < 6; q++) o.row[q] = !outs[q] ? nullptr : place ? outs[q] : scratch + (long)q * n;
+        if (vf_out) o.row[0] = scratch;
+        int rc = eval_api(n, x, y, zz, t, want, o, s);
         if (rc) return rc;
-        for (int q = 0; q < 6; q++) {
+        for (int q = 0; q < 6 && !place; q++) {
             if (!outs[q]) continue;
             if (direct) {
-                k_copy_row<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, out + (long)q * n, outs[q]);
+                k_copy_row<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, scratch + (long)q * n, outs[q]);
                 note_launch();
                 CKR(cudaGetLastError());
             } else {
-                CKR(cudaMemcpyAsync(outs[q], out + (long)q * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+                CKR(cudaMemcpyAsync(outs[q], scratch + (long)q * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
             }
         }
         if (vf_out) {
-            k_vfrac<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, z, out, vf_dcell, vf_out);
+            k_vfrac<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, z, scratch, vf_dcell, vf_out);
             note_launch();
             CKR(cudaGetLastError());
         }
@@ -431,7 +440,10 @@ int run_batch(const double *x, const double *y, const double *z, const double *t
                                     cudaMemcpyHostToDevice, s));
             }
         }
-        rc = eval_api(m, din, din + m, din + 2 * m, din + 3 * m, want, dout, s);
+        OutRows o;
+        for (int q = 0; q < 6; q++)
+            if (outs[q] || (q == 0 && vf_out) || (q < 4 && kin_out)) o.row[q] = dout + (long)q * m;
+        rc = eval_api(m, din, din + m, din + 2 * m, din + 3 * m, want, o, s);
         if (rc) return rc;
         if (vf_out) {
             k_vfrac<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(m, din + 2 * m, dout, vf_dcell, dout + 5 * m);
@@ -549,13 +561,15 @@ int initialize_from_text(const std::string &text) {
 }
 
 // The one-point pipeline of quantity q on the thread's pinned point buffer:
-// eval_api reads x, y, z, t from its first four elements and writes the six
-// API rows of the point (one value each) into the next six, where row q is
-// read back (q = 6: the eta, u, v, w record of wave_Kinematics there).
+// eval_api reads x, y, z, t from its first four elements and writes row q of
+// the point into element 4 + q (q = 6: the eta, u, v, w record of
+// wave_Kinematics from element 4).
 int scalar_pipeline(int q, cudaStream_t s) {
     double *in = t_ctx.h_pt;
-    if (q == 6) return eval_api(1, in, in + 1, in + 2, in + 3, 15, nullptr, s, in + 4);
-    return eval_api(1, in, in + 1, in + 2, in + 3, 1 << q, in + 4, s);
+    OutRows o;
+    if (q == 6) o.kin = in + 4;
+    else o.row[q] = in + 4 + q;
+    return eval_api(1, in, in + 1, in + 2, in + 3, q == 6 ? 15 : 1 << q, o, s);
 }
 
 // Scalar calls replay a graph of scalar_pipeline.  The graph is captured

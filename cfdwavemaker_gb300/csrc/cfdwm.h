@@ -211,7 +211,8 @@ void workspace_free(Workspace &ws);
 // clamp): the reference's Irregular::eta/u/v/w/dp.
 struct ApiRows;
 // api: when given (and the sea is not on the Smit theory), the combining pass
-// writes the API rows and records of api instead of out (which may be null).
+// writes the API rows and records of api instead of out (which may be null),
+// with the seabed clamp of the wave_* calls.
 int irregular_eval(const DevSea &sea, long n, const double *x, const double *y,
                    const double *z, const double *t, int mask, double *out,
                    Workspace &ws, void *stream, const ApiRows *api = nullptr);
@@ -238,7 +239,8 @@ struct DevGrid {
     float *Uy[4] = {nullptr, nullptr, nullptr, nullptr};
     float *Us[4] = {nullptr, nullptr, nullptr, nullptr};
     int *IGNORE = nullptr;
-    float *QIMG = nullptr;       // query image of the two slots a query reads ([2][nodes][5][4] floats)
+    float *QIMG = nullptr;       // query image of the two slots a query reads ([2][nodes] records, sgrid.cu)
+    float *EIMG = nullptr;       // its elevation records ([2][columns][4] floats)
     float *zlev = nullptr;       // scratch: level heights of the slot being written
     double *colpts = nullptr;    // scratch: column x, y, t (FP64)
     double *first = nullptr;     // scratch: eta1, gx, gy, gz per column
@@ -260,9 +262,8 @@ void grid_free(DevGrid &g);
 int grid_initialize(DevGrid &g, const DevSea &sea, Workspace &ws, void *stream);
 int grid_update(DevGrid &g, const DevSea &sea, Workspace &ws, void *stream);
 bool grid_check_time(const DevGrid &g, double t);
-// out [1 + nf][n] FP64: eta, u, v, w (and p when nf = 4), no ramp
-int grid_query(const DevGrid &g, long n, const double *x, const double *y, const double *z,
-               const double *t, double *out, void *stream);
+// the API rows of the spline query at n points (z clamped at the seabed)
+int grid_query(const DevGrid &g, long n, const double *z, const ApiRows &rows, void *stream);
 int grid_download(const DevGrid &g, int which, double *dst, long cap, void *stream);
 // .vtu export of the ring's base slot (last: the slot after it), as
 // lsGridSpline::export_vtu (lsgrid_spline.cpp:1222-1403) writes it, to `path`.
@@ -333,14 +334,10 @@ struct DevRegular {
 };
 int regular_build(const Config &cfg, DevRegular &r, void *stream);
 void regular_free(DevRegular &r);
-// out [5][n] FP64: eta, u, v, w, nhpres (no ramp); z is used as given.
-struct RampDev;
-// The API rows ([6][n]: wave_SurfElev .. wave_nhPres) and/or the
-// wave_Kinematics records ([n][4]) of regular waves in one pass: z clamped at
-// the seabed, the ramp applied.
-int regular_eval(const DevRegular &r, const Config &cfg, long n, const double *x,
-                 const double *y, const double *z, const double *t, const RampDev &ramp, double *rows,
-                 double *kin, void *stream);
+// The API rows and/or wave_Kinematics records of regular waves in one pass: z
+// clamped at the seabed, the ramp applied.
+int regular_eval(const DevRegular &r, const Config &cfg, long n, const double *z, const ApiRows &rows,
+                 void *stream);
 int regular_solution(const DevRegular &r, double *dst, int cap, void *stream);
 
 // ---------------------------------------------------------------------------

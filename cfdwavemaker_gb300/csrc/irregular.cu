@@ -1172,8 +1172,8 @@ __global__ void k_prep_z(long n, const double *z, double swl, int order, int cla
 
 // Irregular::eta/u/v/w/dp assembled from the pieces (Irregular.cpp:9-157).
 // out has row stride ldo (the full batch length).
-// With api.rows or api.kin set, the API rows and records are written here
-// (the finishing pass folded in) instead of out.
+// With any row or record of api set, the API rows and records are written
+// here (the finishing pass folded in) instead of out.
 __global__ void k_combine(long n, long ldo, int order, double swl, const double *z,
                           const double *first, const float *sec, const float *eta2, int mask,
                           double *out, ApiRows api) {
@@ -1186,20 +1186,13 @@ __global__ void k_combine(long n, long ldo, int order, double swl, const double 
     if (mask & 4) v[2] = (double)sec[1 * n + p] + first[2 * n + p] * za;
     if (mask & 8) v[3] = (double)sec[2 * n + p] + first[3 * n + p] * za;
     if (mask & 16) v[4] = (double)sec[3 * n + p] + first[4 * n + p] * za;
-    if (!api.rows && !api.kin) {
+    if (!api.any()) {
         for (int q = 0; q < 5; q++)
             if (mask & (1 << q)) out[q * ldo + p] = v[q];
         return;
     }
     v[5] = v[4] - api.rho * api.g * v[0];
-    if (api.ramp.init) {
-        const double rr = d_ramp(api.ramp, api.t[p], api.x[p], api.y[p]);
-        for (int q = 0; q < 6; q++) v[q] *= rr;
-    }
-    if (api.rows)
-        for (int q = 0; q < 6; q++) api.rows[q * ldo + p] = v[q];
-    if (api.kin)
-        for (int q = 0; q < 4; q++) api.kin[4 * p + q] = v[q];
+    api_store(api, p, v);
 }
 
 }  // namespace
@@ -1579,7 +1572,7 @@ int irregular_eval(const DevSea &sea, long n, const double *x, const double *y, 
         if (api && !smit) {
             ar = *api;
             ar.x = api->x + b; ar.y = api->y + b; ar.t = api->t + b;
-            ar.rows = api->rows ? api->rows + b : nullptr;
+            for (int q = 0; q < 6; q++) ar.row[q] = api->row[q] ? api->row[q] + b : nullptr;
             ar.kin = api->kin ? api->kin + 4 * b : nullptr;
         }
         k_combine<<<(unsigned)((m + 255) / 256), 256, 0, stream>>>(m, n, sea.order, sea.swl, z + b,

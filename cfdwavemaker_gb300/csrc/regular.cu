@@ -352,10 +352,8 @@ __global__ void __launch_bounds__(128) k_fenton_solve(RegIn in, double *sol, dou
 // ----------------------------- evaluation --------------------------------
 struct EvalArgs {
     long n;
-    const double *x, *y, *z, *t;
-    double *rows;       // [6][n] API rows (wave_SurfElev .. wave_nhPres), or null
-    double *kin;        // [n][4] wave_Kinematics records, or null
-    RampDev ramp;
+    const double *z;
+    ApiRows api;        // x, y, t of the points and the rows and records to write
     float2 nd;          // -depth as a float pair (the z clamp)
     const float *cf;    // [4][MAXN]: U, W, E, Q harmonic coefficients in FP32
     int N, finite;
@@ -379,67 +377,78 @@ __device__ __forceinline__ float reg_exp(float x) {
     return y;
 }
 
+// NEED: 1 the elevation sum, 2 the velocity sums, 3 both: a call pays for its
+// rows only, and with both the harmonics' recurrence runs once.  The
+// coefficients of a harmonic are one 16-byte broadcast read.  4e6 points of a
+// Fenton wave of order 24, a wave_VeloXYZ_batch call: 193 us with both sums,
+// six scratch rows and three row copies; 117 us with the velocity sums and the
+// caller's rows (issue-bound: about 16 instructions a harmonic; 56 B a point).
+template <int NEED>
 __global__ void __launch_bounds__(128) k_regular_eval(EvalArgs a) {
-    __shared__ float cU[MAXN], cW[MAXN], cE[MAXN], cQ[MAXN];
-    for (int j = threadIdx.x; j < MAXN; j += blockDim.x) {
-        cU[j] = a.cf[j];
-        cW[j] = a.cf[MAXN + j];
-        cE[j] = a.cf[2 * MAXN + j];
-        cQ[j] = a.cf[3 * MAXN + j];
-    }
+    __shared__ float4 s_c[MAXN];      // U, W, E, Q of a harmonic
+    const int N = a.N;
+    for (int j = threadIdx.x; j < N; j += blockDim.x)
+        s_c[j] = make_float4(a.cf[j], a.cf[MAXN + j], a.cf[2 * MAXN + j], a.cf[3 * MAXN + j]);
     __syncthreads();
     long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (p >= a.n) return;
     // kx = k (cos th (X - x0) + sin th (Y - y0) - c (t - t0)) in float-float
-    const float2 dx = ff_add(ff_from_double(a.x[p]), a.P[3]);
-    const float2 dy = ff_add(ff_from_double(a.y[p]), a.P[4]);
-    const float2 dt = ff_add(ff_from_double(a.t[p]), a.P[5]);
+    const float2 dx = ff_add(ff_from_double(a.api.x[p]), a.P[3]);
+    const float2 dy = ff_add(ff_from_double(a.api.y[p]), a.P[4]);
+    const float2 dt = ff_add(ff_from_double(a.api.t[p]), a.P[5]);
     float2 kx = ff_add(ff_mul(a.P[0].x, a.P[0].y, dx.x, dx.y), ff_mul(a.P[1].x, a.P[1].y, dy.x, dy.y));
     kx = ff_add(kx, ff_mul(a.P[2].x, a.P[2].y, dt.x, dt.y));
     float s1, c1;
     ff_sincos_poly(ff_reduce_2pi(kx), s1, c1);
-    const int N = a.N;
-    // elevation: sum_j E_j cos(j kx)
-    float cj = c1, sj = s1, eta = 0.f;
-    for (int j = 0; j < N; j++) {
-        eta = fmaf(cE[j], cj, eta);
-        float cn = cj * c1 - sj * s1, sn = sj * c1 + cj * s1;
-        cj = cn; sj = sn;
-    }
-    const float etao = eta + a.F[6];
-    // velocity sums with depth ratios, z clamped at the seabed (max(-d, z))
-    float2 zf = ff_from_double(a.z[p]);
-    if (zf.x < a.nd.x || (zf.x == a.nd.x && zf.y < a.nd.y)) zf = a.nd;
-    float su = 0.f, sw = 0.f;
-    if (a.finite) {
-        const float kd = a.F[3];
-        const float ky = a.F[0] * ((zf.x + a.F[4]) + zf.y);
-        const float e1 = reg_exp(ky - kd), e2 = reg_exp(-2.f * ky);
-        float p1 = 1.f, p2 = 1.f;
-        cj = c1; sj = s1;
+    float cj = c1, sj = s1;
+    // elevation sum_j E_j cos(j kx); velocity sums with depth ratios, z
+    // clamped at the seabed (max(-d, z))
+    float eta = 0.f, su = 0.f, sw = 0.f;
+    if (NEED == 1) {
+#pragma unroll 4
         for (int j = 0; j < N; j++) {
-            p1 *= e1; p2 *= e2;
-            // cosh(j ky)/cosh(j kd) = e^{j(ky-kd)} (1 + e^{-2 j ky}) q_j, q_j = 1/(1+e^{-2 j kd})
-            float ch = p1 * (1.f + p2) * cQ[j];
-            float shh = p1 * (1.f - p2) * cQ[j];
-            su = fmaf(cU[j] * ch, cj, su);
-            sw = fmaf(cW[j] * shh, sj, sw);
+            eta = fmaf(s_c[j].z, cj, eta);
             float cn = cj * c1 - sj * s1, sn = sj * c1 + cj * s1;
             cj = cn; sj = sn;
         }
     } else {
-        const float ky = a.F[0] * ((zf.x + a.F[5]) + zf.y);
-        const float e1 = reg_exp(ky);
-        float p1 = 1.f;
-        cj = c1; sj = s1;
-        for (int j = 0; j < N; j++) {
-            p1 *= e1;
-            su = fmaf(cU[j] * p1, cj, su);
-            sw = fmaf(cW[j] * p1, sj, sw);
-            float cn = cj * c1 - sj * s1, sn = sj * c1 + cj * s1;
-            cj = cn; sj = sn;
+        float2 zf = ff_from_double(a.z[p]);
+        if (zf.x < a.nd.x || (zf.x == a.nd.x && zf.y < a.nd.y)) zf = a.nd;
+        if (a.finite) {
+            const float kd = a.F[3];
+            const float ky = a.F[0] * ((zf.x + a.F[4]) + zf.y);
+            const float e1 = reg_exp(ky - kd), e2 = reg_exp(-2.f * ky);
+            float p1 = 1.f, p2 = 1.f;
+#pragma unroll 4
+            for (int j = 0; j < N; j++) {
+                const float4 k = s_c[j];
+                p1 *= e1; p2 *= e2;
+                // cosh(j ky)/cosh(j kd) = e^{j(ky-kd)} (1 + e^{-2 j ky}) q_j, q_j = 1/(1+e^{-2 j kd})
+                float ch = p1 * (1.f + p2) * k.w;
+                float shh = p1 * (1.f - p2) * k.w;
+                su = fmaf(k.x * ch, cj, su);
+                sw = fmaf(k.y * shh, sj, sw);
+                if (NEED & 1) eta = fmaf(k.z, cj, eta);
+                float cn = cj * c1 - sj * s1, sn = sj * c1 + cj * s1;
+                cj = cn; sj = sn;
+            }
+        } else {
+            const float ky = a.F[0] * ((zf.x + a.F[5]) + zf.y);
+            const float e1 = reg_exp(ky);
+            float p1 = 1.f;
+#pragma unroll 4
+            for (int j = 0; j < N; j++) {
+                const float4 k = s_c[j];
+                p1 *= e1;
+                su = fmaf(k.x * p1, cj, su);
+                sw = fmaf(k.y * p1, sj, sw);
+                if (NEED & 1) eta = fmaf(k.z, cj, eta);
+                float cn = cj * c1 - sj * s1, sn = sj * c1 + cj * s1;
+                cj = cn; sj = sn;
+            }
         }
     }
+    const float etao = eta + a.F[6];
     const float U = a.F[7] + su;
     // p_nh = rho (R - g (eta + d - z0) - q'^2 / 2), q'^2 = (U_osc - ubar)^2 + w^2;
     // F[8] = R - g (d - z0), and the elevation includes z0
@@ -450,14 +459,7 @@ __global__ void __launch_bounds__(128) k_regular_eval(EvalArgs a) {
     // (FP64 multiplies only then: the FP64 rate is a small fraction of FP32's)
     double v[6] = {d_from_float(etao), d_from_float(a.F[1] * U), d_from_float(a.F[2] * U), d_from_float(sw), 0.0,
                    d_from_float(a.F[11] * (fmaf(-a.F[10], etao, a.F[8]) - 0.5f * q2))};
-    if (a.ramp.init) {
-        const double rr = d_ramp(a.ramp, a.t[p], a.x[p], a.y[p]);
-        for (int q = 0; q < 6; q++) v[q] *= rr;
-    }
-    if (a.rows)
-        for (int q = 0; q < 6; q++) a.rows[q * a.n + p] = v[q];
-    if (a.kin)
-        for (int q = 0; q < 4; q++) a.kin[4 * p + q] = v[q];
+    api_store(a.api, p, v);
 }
 
 // ----------------------------- host side ---------------------------------
@@ -523,17 +525,18 @@ void regular_free(DevRegular &r) {
     r.d_cf = nullptr;
 }
 
-int regular_eval(const DevRegular &r, const Config &cfg, long n, const double *x, const double *y,
-                 const double *z, const double *t, const RampDev &ramp, double *rows, double *kin,
+int regular_eval(const DevRegular &r, const Config &cfg, long n, const double *z, const ApiRows &rows,
                  void *stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
     if (n <= 0) return OK;
     if (!r.d_cf) return E_NOT_INITIALIZED;
     EvalArgs a;
-    a.n = n; a.x = x; a.y = y; a.z = z; a.t = t; a.rows = rows; a.kin = kin; a.cf = r.d_cf;
-    a.ramp = ramp;
+    a.n = n; a.z = z; a.api = rows; a.cf = r.d_cf;
     ff_split(-cfg.depth, a.nd.x, a.nd.y);
     a.N = r.N;
+    // elevation: rows 0 and 5; velocities: rows 1-3 and 5; both for the records
+    const bool el = rows.row[0] || rows.row[5] || rows.kin;
+    const bool ve = rows.row[1] || rows.row[2] || rows.row[3] || rows.row[5] || rows.kin;
     a.finite = (cfg.depth > 0.0 && cfg.depth < 1e8) ? 1 : 0;
     const double k = r.head[0], c = r.head[1], cth = r.head[8], sth = r.head[9];
     const double pv[6] = {k * cth, k * sth, -k * c, -cfg.x_pos, -cfg.y_pos, -cfg.tofmax};
@@ -542,7 +545,10 @@ int regular_eval(const DevRegular &r, const Config &cfg, long n, const double *x
                            r.soff[0], r.soff[1], r.soff[2], r.soff[3], cfg.gravity, cfg.rho};
     for (int q = 0; q < 12; q++) a.F[q] = (float)fv[q];
     prof_begin(PK_REGULAR, stream);
-    k_regular_eval<<<(unsigned)((n + 127) / 128), 128, 0, stream>>>(a);
+    const unsigned nb = (unsigned)((n + 127) / 128);
+    if (el && ve) k_regular_eval<3><<<nb, 128, 0, stream>>>(a);
+    else if (ve) k_regular_eval<2><<<nb, 128, 0, stream>>>(a);
+    else k_regular_eval<1><<<nb, 128, 0, stream>>>(a);
     note_launch();
     prof_end(PK_REGULAR, stream);
     CK(cudaGetLastError());

@@ -19,6 +19,7 @@
 #include "cfdwm.h"
 #include "sgrid_geom.cuh"
 #include "ffmath.cuh"
+#include "ramp.cuh"
 
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -115,63 +116,111 @@ __global__ void k_scatter_levels(GridGeom g, long nact, const int *act, const do
     }
 }
 
-// All finite differences of lsgrid_spline.cpp:124-366 in one pass over the
-// nodes: x/y/s gradients of slots (tstep+1)%4, (tstep+2)%4 into gradient
-// slots 0/1 and the time gradient of the slot(s) the reference writes.
+// Floats of a query-image record: U, U_t, U_x, U_y, U_s of a node, each over
+// the fields; 15 values in 64 bytes with three fields, 20 in 80 with the
+// pressure.
+template <int NF> struct QRec { static constexpr int F = NF == 3 ? 16 : 20, F4 = F / 4; };
+
+// All finite differences of lsgrid_spline.cpp:124-366 and the query image in
+// one pass over the nodes: x/y/s gradients of slots (tstep+1)%4, (tstep+2)%4
+// into gradient slots 0/1, the time gradient of the slot(s) the reference
+// writes, and, per node of those two slots, the record that the queries read
+// (per column the elevation's: eta, eta_t, eta_x, eta_y).  The records are
+// staged in shared memory so that they are written whole and coalesced; the
+// image kernel that came after this one read all the gradients back (256 x 256
+// x 16 ring: 49 + 61 us as two kernels).
 struct GradArgs {
     GridGeom g;
     int tstep;
     const float *F[5];      // ETA, UX, UY, UZ (and the pressure)
     float *Fx[5], *Fy[5], *Fs[5], *Ft[5];
     float rdx, rdy, rds, rdt;   // reciprocal spacings
+    float4 *img;            // [2][nodes] records
+    float4 *eimg;           // [2][columns] elevation records
 };
 
-__global__ void k_gradients(GradArgs a) {
+constexpr int GRAD_B = 128;
+
+// FP32 differences of the FP32 node values times the reciprocal spacings
+// (one-sided at the boundaries, central inside)
+__device__ __forceinline__ float fd(const float *d, long e, long s, int i, int n, float r) {
+    if (n == 1) return 0.f;
+    if (i == 0) return (d[e + s] - d[e]) * r;
+    if (i == n - 1) return (d[e] - d[e - s]) * r;
+    return (d[e + s] - d[e - s]) * (0.5f * r);
+}
+
+// time gradients of element e of one field (stride S between slots); returns
+// those of the two slots the image holds
+__device__ __forceinline__ float2 fd_time(const GradArgs &a, const float *D, float *T, long S, long e) {
+    if (a.tstep > 0) {
+        const int tid = (a.tstep + 2) % 4, tid1 = (a.tstep + 3) % 4, tid0 = (a.tstep + 1) % 4;
+        const float v = (D[tid1 * S + e] - D[tid0 * S + e]) * (0.5f * a.rdt);
+        T[tid * S + e] = v;
+        return make_float2(T[tid0 * S + e], v);
+    }
+    const float v1 = (D[2 * S + e] - D[1 * S + e]) * a.rdt;
+    const float v2 = (D[3 * S + e] - D[1 * S + e]) * (0.5f * a.rdt);
+    T[1 * S + e] = v1;
+    T[2 * S + e] = v2;
+    return make_float2(v1, v2);
+}
+
+template <int NF>
+__global__ void __launch_bounds__(GRAD_B) k_gradients(GradArgs a) {
+    constexpr int RF = QRec<NF>::F, R4 = QRec<NF>::F4;
+    __shared__ float s_rec[GRAD_B][RF + 1];
     const GridGeom &g = a.g;
-    long nodes = (long)g.nx * g.ny * g.nl, cols = (long)g.nx * g.ny;
-    long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    int field = blockIdx.y;                  // 0 ETA (column nodes), 1..3 U, V, W, 4 P
-    int nl = field == 0 ? 1 : g.nl;
-    long S = field == 0 ? cols : nodes;
-    if (e >= S) return;
-    int m = (int)(e % nl);
-    long c = e / nl;
-    int i = (int)(c / g.ny), j = (int)(c % g.ny);
-    const float *D = a.F[field];
-    int tids[2] = {(a.tstep + 1) % 4, (a.tstep + 2) % 4};
-    long sx = (long)g.ny * nl, sy = nl;
-    // FP32 differences of the FP32 node values times the reciprocal spacings
-    // (one-sided at the boundaries, central inside)
-    const float rdx = a.rdx, rdy = a.rdy, rds = a.rds, rdt = a.rdt;
-    for (int q = 0; q < 2; q++) {
-        const float *d = D + tids[q] * S;
-        float gx, gy;
-        if (g.nx == 1) gx = 0.f;
-        else if (i == 0) gx = (d[e + sx] - d[e]) * rdx;
-        else if (i == g.nx - 1) gx = (d[e] - d[e - sx]) * rdx;
-        else gx = (d[e + sx] - d[e - sx]) * (0.5f * rdx);
-        if (g.ny == 1) gy = 0.f;
-        else if (j == 0) gy = (d[e + sy] - d[e]) * rdy;
-        else if (j == g.ny - 1) gy = (d[e] - d[e - sy]) * rdy;
-        else gy = (d[e + sy] - d[e - sy]) * (0.5f * rdy);
-        a.Fx[field][q * S + e] = gx;
-        a.Fy[field][q * S + e] = gy;
-        if (field > 0) {
-            float gs;
-            if (nl == 1) gs = 0.f;
-            else if (m == 0) gs = (d[e + 1] - d[e]) * rds;
-            else if (m == nl - 1) gs = (d[e] - d[e - 1]) * rds;
-            else gs = (d[e + 1] - d[e - 1]) * (0.5f * rds);
-            a.Fs[field][q * S + e] = gs;
+    const long S = (long)g.nx * g.ny * g.nl, cols = (long)g.nx * g.ny;
+    const long e0 = blockIdx.x * (long)GRAD_B, e = e0 + threadIdx.x;
+    const bool on = e < S;
+    const long ec = on ? e : 0;
+    const int m = (int)(ec % g.nl);
+    const long c = ec / g.nl;
+    const int i = (int)(c / g.ny), j = (int)(c % g.ny);
+    const long sx = (long)g.ny * g.nl, sy = g.nl;
+    const int slot[2] = {(a.tstep + 1) % 4, (a.tstep + 2) % 4};
+    if (on && m == 0) {
+        const float2 t = fd_time(a, a.F[0], a.Ft[0], cols, c);
+        for (int q = 0; q < 2; q++) {
+            const float *d = a.F[0] + slot[q] * cols;
+            const float gx = fd(d, c, g.ny, i, g.nx, a.rdx), gy = fd(d, c, 1, j, g.ny, a.rdy);
+            a.Fx[0][q * cols + c] = gx;
+            a.Fy[0][q * cols + c] = gy;
+            a.eimg[q * cols + c] = make_float4(d[c], q == 0 ? t.x : t.y, gx, gy);
         }
     }
-    float *T = a.Ft[field];
-    if (a.tstep > 0) {
-        int tid = (a.tstep + 2) % 4, tid1 = (a.tstep + 3) % 4, tid0 = (a.tstep + 1) % 4;
-        T[tid * S + e] = (D[tid1 * S + e] - D[tid0 * S + e]) * (0.5f * rdt);
-    } else {
-        T[1 * S + e] = (D[2 * S + e] - D[1 * S + e]) * rdt;
-        T[2 * S + e] = (D[3 * S + e] - D[1 * S + e]) * (0.5f * rdt);
+    float2 t[NF];
+    if (on)
+#pragma unroll
+        for (int f = 0; f < NF; f++) t[f] = fd_time(a, a.F[f + 1], a.Ft[f + 1], S, e);
+    for (int q = 0; q < 2; q++) {
+        if (on) {
+            float *r = s_rec[threadIdx.x];
+#pragma unroll
+            for (int f = 0; f < NF; f++) {
+                const float *d = a.F[f + 1] + slot[q] * S;
+                const float gx = fd(d, e, sx, i, g.nx, a.rdx), gy = fd(d, e, sy, j, g.ny, a.rdy);
+                const float gs = fd(d, e, 1, m, g.nl, a.rds);
+                a.Fx[f + 1][q * S + e] = gx;
+                a.Fy[f + 1][q * S + e] = gy;
+                a.Fs[f + 1][q * S + e] = gs;
+                r[f] = d[e];
+                r[NF + f] = q == 0 ? t[f].x : t[f].y;
+                r[2 * NF + f] = gx;
+                r[3 * NF + f] = gy;
+                r[4 * NF + f] = gs;
+            }
+            if (NF == 3) r[15] = 0.f;
+        }
+        __syncthreads();
+        const long nrec = S - e0 < GRAD_B ? S - e0 : GRAD_B;
+        float4 *o = a.img + ((long)q * S + e0) * R4;
+        for (int k = threadIdx.x; k < nrec * R4; k += GRAD_B) {
+            const float *r = s_rec[k / R4] + 4 * (k % R4);
+            o[k] = make_float4(r[0], r[1], r[2], r[3]);
+        }
+        __syncthreads();
     }
 }
 
@@ -180,14 +229,12 @@ __global__ void k_gradients(GradArgs a) {
 // ---------------------------------------------------------------------------
 struct QueryArgs {
     GridGeom g;
-    int tid1, tid2;
     double t0;
-    const float *ETA, *ETAdt, *ETAdx, *ETAdy;
-    const float4 *img;      // query image: [2][nodes][5] (U, U_t, U_x, U_y, U_s over the fields)
-    int nf;
+    const float4 *eimg;     // [2][columns]: eta, eta_t, eta_x, eta_y
+    const float4 *img;      // [2][nodes] records (QRec)
     long n;
-    const double *x, *y, *z, *t;
-    double *out;    // [1 + nf][n]
+    const double *z;
+    ApiRows api;    // x, y, t of the queries and the rows and records to write
     double inv_dx, inv_dy, inv_dt;   // reciprocals of the spacings (host-computed)
     float tanab;                     // tan(a)^b of the stretching
 };
@@ -212,58 +259,42 @@ __device__ __forceinline__ float cart2sigmaS(const GridGeom &g, float tanab, flo
 
 __device__ __forceinline__ int iclamp(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
-__device__ __forceinline__ float4 herm4(float4 f0, float4 f1, float4 d0, float4 d1, float h, float r) {
-    return make_float4(herm(f0.x, f1.x, d0.x, d1.x, h, r), herm(f0.y, f1.y, d0.y, d1.y, h, r),
-                       herm(f0.z, f1.z, d0.z, d1.z, h, r), herm(f0.w, f1.w, d0.w, d1.w, h, r));
+__device__ __forceinline__ void q_cp16(void *smem, const void *gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ float4 lin4(float4 f0, float4 f1, float r) {
-    return make_float4(lin(f0.x, f1.x, r), lin(f0.y, f1.y, r), lin(f0.z, f1.z, r), lin(f0.w, f1.w, r));
-}
-
-// spline_interp_velo (lsgrid_spline.cpp:386-502) of every velocity field at
-// once: the eight corners of each of the two bracketing slots are read as
-// records of the query image, and the reductions x -> y -> s -> t run on the
-// fields as float4 lanes (the reference's order, per field).
-__device__ float4 spline_velo4(const QueryArgs &a, int xp, int yp, int s0, int s1, float xd, float yd, float sd0,
-                               float sd1, float td) {
-    const GridGeom &g = a.g;
-    const long nn = (long)g.nx * g.ny * g.nl;
-    const int x1 = iclamp(xp + 1, 0, g.nx - 1), y1 = iclamp(yp + 1, 0, g.ny - 1);
-    const int ls[2] = {s0, s1};
-    const float dx = (float)g.dx, dy = (float)g.dy, ds = (float)g.ds;
-    float4 red[2], redt[2];
-    for (int q = 0; q < 2; q++) {            // q = 0: slot (tstep+1)%4 at s0; q = 1: slot (tstep+2)%4 at s1
-        const int l0 = ls[q], l1 = iclamp(ls[q] + 1, 0, g.nl - 1);
-        const float4 *base = a.img + (long)q * nn * 5;
-        // corners: x-pairs (xp, x1) at (yp, l0), (y1, l0), (yp, l1), (y1, l1)
-        const int ys[4] = {yp, y1, yp, y1}, zs[4] = {l0, l0, l1, l1};
-        float4 v[4], yv[4], tv[4], sv[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const float4 *ra = base + (((long)xp * g.ny + ys[k]) * g.nl + zs[k]) * 5;
-            const float4 *rb = base + (((long)x1 * g.ny + ys[k]) * g.nl + zs[k]) * 5;
-            const float4 aU = __ldg(ra), aT = __ldg(ra + 1), aX = __ldg(ra + 2), aY = __ldg(ra + 3), aS = __ldg(ra + 4);
-            const float4 bU = __ldg(rb), bT = __ldg(rb + 1), bX = __ldg(rb + 2), bY = __ldg(rb + 3), bS = __ldg(rb + 4);
-            v[k] = herm4(aU, bU, aX, bX, dx, xd);
-            yv[k] = lin4(aY, bY, xd);
-            tv[k] = lin4(aT, bT, xd);
-            sv[k] = lin4(aS, bS, xd);
-        }
-        const float4 c0 = herm4(v[0], v[1], yv[0], yv[1], dy, yd), c1 = herm4(v[2], v[3], yv[2], yv[3], dy, yd);
-        const float4 c0s = lin4(sv[0], sv[1], yd), c1s = lin4(sv[2], sv[3], yd);
-        const float4 c0t = lin4(tv[0], tv[1], yd), c1t = lin4(tv[2], tv[3], yd);
-        const float sd = q == 0 ? sd0 : sd1;
-        red[q] = herm4(c0, c1, c0s, c1s, ds, sd);
-        redt[q] = lin4(c0t, c1t, sd);
-    }
-    return herm4(red[0], red[1], redt[0], redt[1], (float)g.dt, td);
+__device__ __forceinline__ void q_cp_wait() {
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }
 
-__global__ void __launch_bounds__(128) k_query(QueryArgs a) {
-    long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (p >= a.n) return;
+// A query reads, in each of the two bracketing slots and at each of the four
+// columns around it, the records of two neighbouring levels: 128 (with the
+// pressure 160) contiguous bytes.  A warp fetches these blocks for its 32
+// queries together, 16 bytes a lane and neighbouring lanes on neighbouring
+// addresses, into shared memory, two columns (the x pair) at a time; each
+// lane then reads its own from there.  With every lane loading its own
+// records 16 bytes at a time each load instruction touched 32 cache lines, and
+// the L1's line lookups were the bound (88 % busy).  1e6 random queries of the
+// 256 x 256 x 16 ring, the whole wave_Kinematics call: 0.35 ms then, 0.19 ms
+// with the warp's fetch and 64-byte records (and the seabed clamp, the ramp
+// and the rows in this kernel).  Registers are held to four blocks an SM: 0.20
+// ms without the limit (144 registers), 0.22 with five, 0.28 with six.
+constexpr int QB = 128;      // threads of a query block
+template <int NF> struct QStage {
+    static constexpr int PAIR = 4 * QRec<NF>::F4;     // float4 of the x pair's two blocks
+    static constexpr int STRIDE = PAIR + 1;           // per query: lanes' 16-byte reads fall on distinct banks
+};
+
+template <int NF>
+__global__ void __launch_bounds__(QB, NF == 3 ? 4 : 3) k_query(QueryArgs a) {
+    constexpr int RF = QRec<NF>::F, R4 = QRec<NF>::F4, PAIR = QStage<NF>::PAIR, STRIDE = QStage<NF>::STRIDE;
+    extern __shared__ float4 s_q[];
+    const int lane = threadIdx.x & 31;
+    float4 *sw = s_q + (threadIdx.x >> 5) * 32 * STRIDE;     // this warp's stage
+    const long p0 = blockIdx.x * (long)QB + threadIdx.x;
+    const long p = p0 < a.n ? p0 : a.n - 1;                  // (idle lanes help with the loads)
     const GridGeom &g = a.g;
-    const double xpt = a.x[p], ypt = a.y[p], zpt = a.z[p], tpt = a.t[p];
+    const double xpt = a.api.x[p], ypt = a.api.y[p], tpt = a.api.t[p];
     // std::modf with a float* argument selects the float overload in the
     // reference (lsgrid_spline.cpp:515-520): the fractions are float.
     float xi, yi;
@@ -275,71 +306,103 @@ __global__ void __launch_bounds__(128) k_query(QueryArgs a) {
     int xp = (int)xi, yp = (int)yi;
     const long nc = (long)g.nx * g.ny;
     const int x1 = iclamp(xp + 1, 0, g.nx - 1), y1 = iclamp(yp + 1, 0, g.ny - 1);
-    long cid[4] = {(long)xp * g.ny + yp, (long)xp * g.ny + y1, (long)x1 * g.ny + yp, (long)x1 * g.ny + y1};
-    float C[4], D[4], Ct[4], Dt[4], Cx[4], Dx[4], Cy[4], Dy[4];
+    const long cid[4] = {(long)xp * g.ny + yp, (long)xp * g.ny + y1, (long)x1 * g.ny + yp, (long)x1 * g.ny + y1};
+    float4 C[4], D[4];       // eta, eta_t, eta_x, eta_y of the two slots
+#pragma unroll
     for (int k = 0; k < 4; k++) {
-        C[k] = __ldg(a.ETA + a.tid1 * nc + cid[k]);
-        D[k] = __ldg(a.ETA + a.tid2 * nc + cid[k]);
-        Ct[k] = __ldg(a.ETAdt + a.tid1 * nc + cid[k]);
-        Dt[k] = __ldg(a.ETAdt + a.tid2 * nc + cid[k]);
-        Cx[k] = __ldg(a.ETAdx + cid[k]);
-        Dx[k] = __ldg(a.ETAdx + nc + cid[k]);
-        Cy[k] = __ldg(a.ETAdy + cid[k]);
-        Dy[k] = __ldg(a.ETAdy + nc + cid[k]);
+        C[k] = __ldg(a.eimg + cid[k]);
+        D[k] = __ldg(a.eimg + nc + cid[k]);
     }
     const float dx = (float)g.dx, dy = (float)g.dy;
-    float C0 = herm(C[0], C[2], Cx[0], Cx[2], dx, xd), C1 = herm(C[1], C[3], Cx[1], Cx[3], dx, xd);
-    float D0 = herm(D[0], D[2], Dx[0], Dx[2], dx, xd), D1 = herm(D[1], D[3], Dx[1], Dx[3], dx, xd);
-    float C0y = lin(Cy[0], Cy[2], xd), C1y = lin(Cy[1], Cy[3], xd);
-    float D0y = lin(Dy[0], Dy[2], xd), D1y = lin(Dy[1], Dy[3], xd);
-    float C0t = lin(Ct[0], Ct[2], xd), C1t = lin(Ct[1], Ct[3], xd);
-    float D0t = lin(Dt[0], Dt[2], xd), D1t = lin(Dt[1], Dt[3], xd);
+    float C0 = herm(C[0].x, C[2].x, C[0].z, C[2].z, dx, xd), C1 = herm(C[1].x, C[3].x, C[1].z, C[3].z, dx, xd);
+    float D0 = herm(D[0].x, D[2].x, D[0].z, D[2].z, dx, xd), D1 = herm(D[1].x, D[3].x, D[1].z, D[3].z, dx, xd);
+    float C0y = lin(C[0].w, C[2].w, xd), C1y = lin(C[1].w, C[3].w, xd);
+    float D0y = lin(D[0].w, D[2].w, xd), D1y = lin(D[1].w, D[3].w, xd);
+    float C0t = lin(C[0].y, C[2].y, xd), C1t = lin(C[1].y, C[3].y, xd);
+    float D0t = lin(D[0].y, D[2].y, xd), D1t = lin(D[1].y, D[3].y, xd);
     float e0 = herm(C0, C1, C0y, C1y, dy, yd), e1 = herm(D0, D1, D0y, D1y, dy, yd);
     float CCt = lin(C0t, C1t, yd), DDt = lin(D0t, D1t, yd);
     float eta = herm(e0, e1, CCt, DDt, (float)g.dt, td);
-    const float tanab = a.tanab;
-    float n0 = cart2sigmaS(g, tanab, (float)zpt, e0) / (float)g.ds;
-    float n1 = cart2sigmaS(g, tanab, (float)zpt, e1) / (float)g.ds;
-    float s0i, s1i;
-    float sd0 = modff(n0, &s0i), sd1 = modff(n1, &s1i);
-    int s0 = iclamp((int)s0i, 0, g.nl - 1), s1 = iclamp((int)s1i, 0, g.nl - 1);
-    a.out[p] = d_from_float(eta);
-    const float4 u = spline_velo4(a, xp, yp, s0, s1, xd, yd, sd0, sd1, td);
-    a.out[1 * a.n + p] = d_from_float(u.x);
-    a.out[2 * a.n + p] = d_from_float(u.y);
-    a.out[3 * a.n + p] = d_from_float(u.z);
-    if (a.nf == 4) a.out[4 * a.n + p] = d_from_float(u.w);
-}
-
-// The query image of the two slots the queries read, (tstep+1)%4 and
-// (tstep+2)%4: per node one record of five float4, U, U_t, U_x, U_y, U_s, each
-// over the velocity fields (and the pressure; lane 3 is 0 without it).  A
-// query corner is then one 80-byte record instead of 5 nf separate loads.
-struct QImgArgs {
-    const float *U[4], *Ut[4], *Ux[4], *Uy[4], *Us[4];
-    int nf, tstep;
-    long nodes;
-    float4 *img;
-};
-__global__ void k_query_image(QImgArgs a) {
-    const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (e >= a.nodes) return;
-    const int q = blockIdx.y;
-    const long S = a.nodes;
-    const long ts = (long)((a.tstep + 1 + q) % 4) * S + e, gs = (long)q * S + e;
-    float r[5][4];
+    // get_kinematics_at_point forms eta before it looks at z
+    // (lsgrid_spline.cpp:505-571): one query serves wave_SurfElev (queried at
+    // z = 0) and the velocities (queried at z clamped to the seabed).  Without
+    // a pressure field rows 4 and 5 are the reference's 0.0
+    // (CFDwavemaker.cpp:1808-1812, 1815-1891); with one, the irregular sea's
+    // forms (:1807-1808, 1826-1830) on the grid.
+    const ApiRows &A = a.api;
+    double v[6] = {d_from_float(eta), 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (A.row[1] || A.row[2] || A.row[3] || A.kin || (NF == 4 && (A.row[4] || A.row[5]))) {
+        // spline_interp_velo (lsgrid_spline.cpp:386-502) of every field, the
+        // reductions x -> y -> s -> t in the reference's order
+        const float zpt = (float)fmax(-g.depth, a.z[p]);
+        float s0i, s1i;
+        const float sd0 = modff(cart2sigmaS(g, a.tanab, zpt, e0) / (float)g.ds, &s0i);
+        const float sd1 = modff(cart2sigmaS(g, a.tanab, zpt, e1) / (float)g.ds, &s1i);
+        const int ls[2] = {iclamp((int)s0i, 0, g.nl - 1), iclamp((int)s1i, 0, g.nl - 1)};
+        const unsigned nn = (unsigned)(nc * g.nl);
+        const float ds = (float)g.ds;
+        float red[2][NF], redt[2][NF];
 #pragma unroll
-    for (int f = 0; f < 4; f++) {
-        const bool on = f < a.nf;
-        r[0][f] = on ? a.U[f][ts] : 0.f;
-        r[1][f] = on ? a.Ut[f][ts] : 0.f;
-        r[2][f] = on ? a.Ux[f][gs] : 0.f;
-        r[3][f] = on ? a.Uy[f][gs] : 0.f;
-        r[4][f] = on ? a.Us[f][gs] : 0.f;
+        for (int q = 0; q < 2; q++) {        // q = 0: slot (tstep+1)%4 at s0; q = 1: slot (tstep+2)%4 at s1
+            // the block's first level, and the two levels' records within it
+            const int lb = g.nl > 1 ? min(ls[q], g.nl - 2) : 0;
+            const int i0 = ls[q] - lb, i1 = iclamp(ls[q] + 1, 0, g.nl - 1) - lb;
+            const float4 *img = a.img + (long)q * nn * R4;
+            float vv[2][NF], yv[2][NF], tv[2][NF], sv[2][NF];    // [level]: at yp, then reduced in y
+#pragma unroll
+            for (int yy = 0; yy < 2; yy++) {
+                const unsigned nb0 = (unsigned)(cid[yy] * g.nl) + lb, nb1 = (unsigned)(cid[2 + yy] * g.nl) + lb;
+                __syncwarp();                                    // the stage has been read
+#pragma unroll
+                for (int it = 0; it < PAIR; it++) {
+                    const int e = it * 32 + lane, qq = e / PAIR, r = e % PAIR;
+                    const unsigned a0 = __shfl_sync(0xffffffffu, nb0, qq), a1 = __shfl_sync(0xffffffffu, nb1, qq);
+                    int k = r < PAIR / 2 ? r : r - PAIR / 2;
+                    if (g.nl == 1 && k >= R4) k -= R4;           // one level: its record twice
+                    q_cp16(sw + qq * STRIDE + r, img + (long)(r < PAIR / 2 ? a0 : a1) * R4 + k);
+                }
+                q_cp_wait();
+                __syncwarp();
+                const float4 *mine = sw + lane * STRIDE;
+#pragma unroll
+                for (int l = 0; l < 2; l++) {
+                    const float4 *ra = mine + (l == 0 ? i0 : i1) * R4, *rb = ra + PAIR / 2;
+                    float fa[RF], fb[RF];
+#pragma unroll
+                    for (int k = 0; k < R4; k++) {
+                        const float4 u = ra[k], w = rb[k];
+                        fa[4 * k] = u.x; fa[4 * k + 1] = u.y; fa[4 * k + 2] = u.z; fa[4 * k + 3] = u.w;
+                        fb[4 * k] = w.x; fb[4 * k + 1] = w.y; fb[4 * k + 2] = w.z; fb[4 * k + 3] = w.w;
+                    }
+#pragma unroll
+                    for (int f = 0; f < NF; f++) {
+                        const float hv = herm(fa[f], fb[f], fa[2 * NF + f], fb[2 * NF + f], dx, xd);
+                        const float ht = lin(fa[NF + f], fb[NF + f], xd);
+                        const float hy = lin(fa[3 * NF + f], fb[3 * NF + f], xd);
+                        const float hs = lin(fa[4 * NF + f], fb[4 * NF + f], xd);
+                        if (yy == 0) {
+                            vv[l][f] = hv; tv[l][f] = ht; yv[l][f] = hy; sv[l][f] = hs;
+                        } else {
+                            vv[l][f] = herm(vv[l][f], hv, yv[l][f], hy, dy, yd);
+                            sv[l][f] = lin(sv[l][f], hs, yd);
+                            tv[l][f] = lin(tv[l][f], ht, yd);
+                        }
+                    }
+                }
+            }
+            const float sd = q == 0 ? sd0 : sd1;
+#pragma unroll
+            for (int f = 0; f < NF; f++) {
+                red[q][f] = herm(vv[0][f], vv[1][f], sv[0][f], sv[1][f], ds, sd);
+                redt[q][f] = lin(tv[0][f], tv[1][f], sd);
+            }
+        }
+#pragma unroll
+        for (int f = 0; f < NF; f++)
+            v[1 + f] = d_from_float(herm(red[0][f], red[1][f], redt[0][f], redt[1][f], (float)g.dt, td));
+        if (NF == 4 && A.row[5]) v[5] = v[4] - A.rho * A.g * v[0];
     }
-    float4 *o = a.img + ((long)q * S + e) * 5;
-#pragma unroll
-    for (int k = 0; k < 5; k++) o[k] = make_float4(r[k][0], r[k][1], r[k][2], r[k][3]);
+    if (p0 < a.n) api_store(A, p, v);
 }
 
 // ---------------------------------------------------------------------------
@@ -444,6 +507,7 @@ int grid_create(const Config &cfg, DevGrid &g, void *stream_) {
     x->split_cap = column_pairs_split_floats(g.nl);
     CK(cudaMalloc(&x->split, sizeof(float) * x->split_cap));
     CK(cudaMalloc(&g.QIMG, sizeof(float4) * 10 * v));
+    CK(cudaMalloc(&g.EIMG, sizeof(float4) * 2 * c));
     CK(cudaStreamSynchronize(stream));
     return OK;
 }
@@ -459,9 +523,11 @@ void grid_free(DevGrid &g) {
     g.nf = 3;
     if (g.IGNORE) cudaFree(g.IGNORE);
     if (g.QIMG) cudaFree(g.QIMG);
+    if (g.EIMG) cudaFree(g.EIMG);
     g.ETA = g.ETAdx = g.ETAdy = g.ETAdt = nullptr;
     g.IGNORE = nullptr;
     g.QIMG = nullptr;
+    g.EIMG = nullptr;
     for (auto it = g_extra.begin(); it != g_extra.end(); ++it)
         if (it->first == &g) {
             GridExtra &x = it->second;
@@ -590,18 +656,13 @@ static int gradients(DevGrid &g, cudaStream_t stream) {
         a.F[f + 1] = g.U[f]; a.Fx[f + 1] = g.Ux[f]; a.Fy[f + 1] = g.Uy[f];
         a.Fs[f + 1] = g.Us[f]; a.Ft[f + 1] = g.Ut[f];
     }
-    long nodes = (long)g.nx * g.ny * g.nl;
-    dim3 grid((unsigned)((nodes + 255) / 256), (unsigned)(1 + g.nf));
+    a.img = reinterpret_cast<float4 *>(g.QIMG);
+    a.eimg = reinterpret_cast<float4 *>(g.EIMG);
+    const long nodes = (long)g.nx * g.ny * g.nl;
+    const unsigned nb = (unsigned)((nodes + GRAD_B - 1) / GRAD_B);
     prof_begin(PK_GRADIENTS, stream);
-    k_gradients<<<grid, 256, 0, stream>>>(a);
-    note_launch();
-    CK(cudaGetLastError());
-    QImgArgs qa;
-    for (int f = 0; f < 4; f++) {
-        qa.U[f] = g.U[f]; qa.Ut[f] = g.Ut[f]; qa.Ux[f] = g.Ux[f]; qa.Uy[f] = g.Uy[f]; qa.Us[f] = g.Us[f];
-    }
-    qa.nf = g.nf; qa.tstep = g.tstep; qa.nodes = nodes; qa.img = reinterpret_cast<float4 *>(g.QIMG);
-    k_query_image<<<dim3((unsigned)((nodes + 255) / 256), 2), 256, 0, stream>>>(qa);
+    if (g.nf == 4) k_gradients<4><<<nb, GRAD_B, 0, stream>>>(a);
+    else k_gradients<3><<<nb, GRAD_B, 0, stream>>>(a);
     note_launch();
     prof_end(PK_GRADIENTS, stream);
     CK(cudaGetLastError());
@@ -742,21 +803,23 @@ int grid_block_copy(DevGrid &g, int f, int i0, int i1, float *buf, bool into_gri
     return OK;
 }
 
-int grid_query(const DevGrid &g, long n, const double *x, const double *y, const double *z,
-               const double *t, double *out, void *stream_) {
+int grid_query(const DevGrid &g, long n, const double *z, const ApiRows &rows, void *stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
     if (n <= 0) return OK;
     QueryArgs a;
     a.g = geom(g);
-    a.tid1 = (g.tstep + 1) % 4; a.tid2 = (g.tstep + 2) % 4; a.t0 = g.t0;
-    a.ETA = g.ETA; a.ETAdt = g.ETAdt; a.ETAdx = g.ETAdx; a.ETAdy = g.ETAdy;
+    a.t0 = g.t0;
+    a.eimg = reinterpret_cast<const float4 *>(g.EIMG);
     a.img = reinterpret_cast<const float4 *>(g.QIMG);
-    a.nf = g.nf;
-    a.n = n; a.x = x; a.y = y; a.z = z; a.t = t; a.out = out;
+    a.n = n; a.z = z; a.api = rows;
     a.inv_dx = 1.0 / a.g.dx; a.inv_dy = 1.0 / a.g.dy; a.inv_dt = 1.0 / a.g.dt;
     a.tanab = powf(tanf((float)a.g.tan_a), (float)a.g.tan_b);
     prof_begin(PK_QUERY, stream);
-    k_query<<<(unsigned)((n + 127) / 128), 128, 0, stream>>>(a);
+    const unsigned nb = (unsigned)((n + QB - 1) / QB);
+    constexpr int SM3 = QB * QStage<3>::STRIDE * 16, SM4 = QB * QStage<4>::STRIDE * 16;
+    static_assert(SM3 <= 48 * 1024 && SM4 <= 48 * 1024, "no shared-memory opt-in needed");
+    if (g.nf == 4) k_query<4><<<nb, QB, SM4, stream>>>(a);
+    else k_query<3><<<nb, QB, SM3, stream>>>(a);
     note_launch();
     prof_end(PK_QUERY, stream);
     CK(cudaGetLastError());
