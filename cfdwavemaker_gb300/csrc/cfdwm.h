@@ -150,7 +150,14 @@ struct DevSea {
     float *d_cf = nullptr;       // [NCF][npad_g]
     float *d_tab_eta = nullptr;  // grid-mask pair tiles of eta2 (A, B per pair)
     float *d_tab_grid = nullptr; // grid-mask pair tiles of uvw2
-    float *d_tab_point = nullptr;// point-API pair tiles (built on demand)
+    float *d_tab_point = nullptr;// point-API pair tiles (built on demand): velocity records, then
+    float *d_tab_pp = nullptr;   // the pressure's phase terms and
+    float *d_tab_pk = nullptr;   // its phase-free products (one allocation)
+    // their sum over the pairs as a function of the height alone (where every
+    // component has the same ramp): K, dK/dz at kin_nz heights over [-kin_h, 0]
+    double *d_kin = nullptr;
+    int kin_nz = 0;
+    double kin_h = 0;
     float *d_tab_gp = nullptr;   // grid-mask pair tiles of the s-grid pressure: Pp, Mp (phase terms)
     float *d_tab_gk = nullptr;   // grid-mask pair tiles of the phase-free pressure terms: X, Z
     int ntile_g = 0, ntile_p = 0;

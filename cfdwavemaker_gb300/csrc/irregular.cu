@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <type_traits>
 #include <vector>
 
 namespace cfdwm {
@@ -53,7 +54,13 @@ constexpr int GRIDV_NC = 8;   // uvw table: Pu, Mu, Pv, Mv, Pw, Mw, kp, km
 // and X, Z of the phase-free terms (products of the first-order profiles for
 // a pair, the linear diagonal terms on the diagonal entry)
 constexpr int GRIDP_NC = 2;
-constexpr int POINTV_NC = 12; // point table: Pu, Mu, Pv, Mv, Pw, Mw, Pp, Mp, kp, km, Xpp, Xzz
+// point tables (one allocation, in this order): the velocity records Pu, Mu,
+// Pv, Mv, Pw, Mw, kp, km; the pressure's phase terms Pp, Mp, kp, km; its
+// phase-free products Xpp, Xzz.  A velocity call and a pressure call each read
+// their own.  Two neighbouring entries of a row are interleaved (point_at), so
+// that a 16-byte word is two packed FP32x2 operands.
+constexpr int POINTV_NC = 8, POINTP_NC = 4, POINTK_NC = 2;
+__host__ __device__ inline long point_at(long entry, int nc, int q) { return ((entry / 2) * nc + q) * 2 + (entry & 1); }
 constexpr float LOG2E_F = 1.4426950408889634f;
 constexpr long SPLIT_TARGET_BLOCKS = 4 * 152;   // blocks a column-pair launch aims for
 // batches of at most this many points take the few-point kernels (a block
@@ -106,8 +113,8 @@ __device__ __forceinline__ double pair_k2(double ki, double km, double gam) {
 }
 
 // One record per (tile, entry).  mode 0: grid mask (eta + uvw tables, and
-// the pressure tables tab_gp / tab_gk), mode 1: point-API mask
-// (u2/v2/w2/dp2 table).
+// the pressure tables tab_gp / tab_gk), mode 1: point-API mask (the u2/v2/w2
+// table tab_v and the dp2 tables tab_gp, tab_gk).
 __global__ void k_build_tables(CompIn c, int TT, int nt, int mode, float *tab_eta,
                                float *tab_v, float *tab_gp, float *tab_gk) {
     long t = blockIdx.x;
@@ -245,7 +252,10 @@ __global__ void k_build_tables(CompIn c, int TT, int nt, int mode, float *tab_et
             tab_gk[base * GRIDP_NC + 0] = (float)pr[2];
             tab_gk[base * GRIDP_NC + 1] = (float)pr[3];
         } else {
-            for (int q = 0; q < POINTV_NC; q++) tab_v[base * POINTV_NC + q] = (float)out[q];
+            const int vq[POINTV_NC] = {0, 1, 2, 3, 4, 5, 8, 9}, pq[POINTP_NC] = {6, 7, 8, 9};
+            for (int q = 0; q < POINTV_NC; q++) tab_v[point_at(base, POINTV_NC, q)] = (float)out[vq[q]];
+            for (int q = 0; q < POINTP_NC; q++) tab_gp[point_at(base, POINTP_NC, q)] = (float)out[pq[q]];
+            for (int q = 0; q < POINTK_NC; q++) tab_gk[point_at(base, POINTK_NC, q)] = (float)out[10 + q];
         }
     }
 }
@@ -304,28 +314,34 @@ __global__ void k_component_coefs(CompIn c, int npad, double fx, double fy, doub
     for (int q = 0; q < NCF; q++) cf[q * npad + i] = (float)v[q];
 }
 
-constexpr int PH_REC = 13;       // floats of a phasor record
+// floats of a phasor record: kx, ky, -omega, phase0 as float pairs, then A, GX,
+// GY, GZ, GP.  Two neighbouring components' records are interleaved, float by
+// float, into packed operands (the pair is 28 floats, 7 words of 16 bytes)
+constexpr int PH_REC = 14;
 constexpr int PH_CHUNK = 128;    // records per shared-memory chunk
+__host__ __device__ inline long rec_at(long comp, int q) { return (comp / 2) * (2 * PH_REC) + 2 * q + (comp & 1); }
 
 // The phasor records of all components (time-independent, built once with the sea).
 __global__ void k_phasor_records(int n, int npad, const double *phase, const float *cf, int cs, float *rec) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npad) return;
-    float *o = rec + (long)i * PH_REC;
-    if (i >= n) {
-        for (int q = 0; q < PH_REC; q++) o[q] = 0.f;
-        return;
+    float v[PH_REC];
+    for (int q = 0; q < PH_REC; q++) v[q] = 0.f;
+    if (i < n) {
+        ff_split(phase[i], v[0], v[1]);
+        ff_split(phase[cs + i], v[2], v[3]);
+        ff_split(-phase[2 * cs + i], v[4], v[5]);
+        ff_split(phase[3 * cs + i], v[6], v[7]);
+        v[8] = cf[CF_A * cs + i];
+        v[9] = cf[CF_GX * cs + i];
+        v[10] = cf[CF_GY * cs + i];
+        v[11] = cf[CF_GZ * cs + i];
+        v[12] = cf[CF_GP * cs + i];
     }
-    ff_split(phase[i], o[0], o[1]);
-    ff_split(phase[cs + i], o[2], o[3]);
-    ff_split(-phase[2 * cs + i], o[4], o[5]);
-    ff_split(phase[3 * cs + i], o[6], o[7]);
-    o[8] = cf[CF_A * cs + i];
-    o[9] = cf[CF_GX * cs + i];
-    o[10] = cf[CF_GY * cs + i];
-    o[11] = cf[CF_GZ * cs + i];
-    o[12] = cf[CF_GP * cs + i];
+    for (int q = 0; q < PH_REC; q++) rec[rec_at(i, q)] = v[q];
 }
+
+static int point_kin_build(DevSea &sea, cudaStream_t stream);
 
 int sea_build(const Config &cfg, DevSea &sea, bool point_table, void *stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
@@ -397,11 +413,15 @@ int sea_build(const Config &cfg, DevSea &sea, bool point_table, void *stream_) {
         if (point_table) {
             long ntp = tile_index(sea.ntile_p - 1, sea.ntile_p - 1, sea.ntile_p) + 1;
             size_t entp = (size_t)ntp * POINT_TILE * POINT_TILE;
-            CK(cudaMalloc(&sea.d_tab_point, sizeof(float) * entp * POINTV_NC));
-            k_build_tables<<<(unsigned)ntp, 256, 0, stream>>>(ci, POINT_TILE, sea.ntile_p, 1,
-                                                              nullptr, sea.d_tab_point, nullptr, nullptr);
+            CK(cudaMalloc(&sea.d_tab_point, sizeof(float) * entp * (POINTV_NC + POINTP_NC + POINTK_NC)));
+            sea.d_tab_pp = sea.d_tab_point + entp * POINTV_NC;
+            sea.d_tab_pk = sea.d_tab_pp + entp * POINTP_NC;
+            k_build_tables<<<(unsigned)ntp, 256, 0, stream>>>(ci, POINT_TILE, sea.ntile_p, 1, nullptr,
+                                                              sea.d_tab_point, sea.d_tab_pp, sea.d_tab_pk);
             note_launch();
             CK(cudaGetLastError());
+            int rc = point_kin_build(sea, stream);
+            if (rc) return rc;
         }
         if (cfg.vertical_theory == 1) {
             SmitIn si;
@@ -438,13 +458,15 @@ void sea_free(DevSea &sea) {
     if (sea.d_tab_gk) cudaFree(sea.d_tab_gk);
     if (sea.d_tab_smit) cudaFree(sea.d_tab_smit);
     if (sea.d_dfcomp) cudaFree(sea.d_dfcomp);
+    if (sea.d_kin) cudaFree(sea.d_kin);
+    sea.d_kin = nullptr;
     if (sea.d_phrec) cudaFree(sea.d_phrec);
     sea.d_tab_smit = nullptr;
     sea.d_dfcomp = nullptr;
     sea.d_phrec = nullptr;
     sea.smit = false;
     sea.d_phase = nullptr; sea.d_cf = nullptr; sea.d_tab_eta = nullptr;
-    sea.d_tab_grid = nullptr; sea.d_tab_point = nullptr; sea.d_tab_gp = nullptr; sea.d_tab_gk = nullptr;
+    sea.d_tab_grid = nullptr; sea.d_tab_point = nullptr; sea.d_tab_pp = sea.d_tab_pk = nullptr; sea.d_tab_gp = nullptr; sea.d_tab_gk = nullptr;
 }
 
 int workspace_reserve(Workspace &ws, size_t bytes) {
@@ -462,8 +484,49 @@ void workspace_free(Workspace &ws) {
     ws.bytes = 0;
 }
 
+// Packed FP32x2 values as 64-bit registers.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 p_pack(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 p_un(f32x2 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+__device__ __forceinline__ float p_hsum(f32x2 a) {
+    const float2 r = p_un(a);
+    return r.x + r.y;
+}
+__device__ __forceinline__ f32x2 p_fma(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 p_mul(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 p_add(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// a packed operand that a long loop keeps: a plain pack is a move that the
+// compiler repeats at every use (6 moves a pair in k_pairs_points, velocity
+// sums 16 % slower); the result of a packed multiplication (by 1, from a kernel
+// argument) is held
+__device__ __forceinline__ f32x2 p_hold(float a, float b, f32x2 one2) { return p_mul(p_pack(a, b), one2); }
+__device__ __forceinline__ f32x2 p_ex2(f32x2 a) {
+    const float2 v = p_un(a);
+    return p_pack(ex2(v.x), ex2(v.y));
+}
+
 // ---------------------------------------------------------------------------
-// Phasor pass: one thread per point/column, all components.
+// Phasor pass: every (point or column, component).
 // ---------------------------------------------------------------------------
 struct PhArgs {
     long n;
@@ -475,9 +538,10 @@ struct PhArgs {
     int cstride;            // npad_g
     double fx, fy;
     int trivial_ramp;
-    const float *rec;       // [npad_g][PH_REC] phasor records
+    const float *rec;       // phasor records (rec_at)
+    int sums;               // which first-order sums: bit q = first[q]
     float2 *ph;             // [npad][n]
-    float *rr;              // [npad][n]
+    float *rr;              // [npad][n]; with a trivial ramp row 0 only
     double *first;          // [5][n]: eta1, gx, gy, gz, gp
 };
 
@@ -488,8 +552,42 @@ __device__ __forceinline__ void ph_kahan(float &s, float &c, float v) {
     s = t;
 }
 
-// One thread per point: the phasors (cos, sin) and ramps of every component
-// and the first-order sums eta1 and the Taylor gradients.  The phase
+// sin and cos of two phases hi + lo, FMA-only: one Cody-Waite reduction to
+// |r| <= pi/4 by multiples of pi/2 = A + B + C (A short: n A cancels hi's
+// leading bits exactly for |n| < 2^18), then the Taylor polynomials of
+// ff_sincos_poly.
+__device__ __forceinline__ void ph_sincos(f32x2 hi, f32x2 lo, f32x2 &s, f32x2 &c) {
+    auto dup = [](float v) { return p_pack(v, v); };
+    const float2 q = p_un(p_mul(hi, dup(0.636619772f)));
+    const float n0 = rintf(q.x), n1 = rintf(q.y);
+    const f32x2 nn = p_pack(-n0, -n1);
+    f32x2 r = p_fma(nn, dup(1.5703125f), hi);
+    r = p_fma(nn, dup(4.837512969970703125e-4f), r);
+    r = p_fma(nn, dup(7.549789948768648e-8f), r);
+    r = p_add(r, lo);
+    const f32x2 r2 = p_mul(r, r);
+    f32x2 ps = p_fma(r2, dup(2.7557319e-6f), dup(-1.98412698e-4f));
+    ps = p_fma(r2, p_fma(r2, ps, dup(8.33333333e-3f)), dup(-0.166666667f));
+    f32x2 pc = p_fma(r2, dup(-2.75573192e-7f), dup(2.48015873e-5f));
+    pc = p_fma(r2, p_fma(r2, p_fma(r2, pc, dup(-1.38888889e-3f)), dup(4.16666667e-2f)), dup(-0.5f));
+    const float2 sr = p_un(p_fma(p_mul(r, r2), ps, r)), cr = p_un(p_fma(r2, pc, dup(1.0f)));
+    // quarter n: sine and cosine swap when n is odd; sin is negative for n = 2,
+    // 3 and cos for n = 1, 2 (mod 4)
+    auto pick = [](float n, float sv, float cv, float &so, float &co) {
+        const unsigned k = (unsigned)(int)n;
+        const unsigned us = __float_as_uint((k & 1) ? cv : sv), uc = __float_as_uint((k & 1) ? sv : cv);
+        so = __uint_as_float(us ^ ((k & 2) << 30));
+        co = __uint_as_float(uc ^ (((k + 1) & 2) << 30));
+    };
+    float s0, c0, s1, c1;
+    pick(n0, sr.x, cr.x, s0, c0);
+    pick(n1, sr.y, cr.y, s1, c1);
+    s = p_pack(s0, s1);
+    c = p_pack(c0, c1);
+}
+
+// The phasors (cos, sin) and ramps of every component and the first-order
+// sums eta1 and the Taylor gradients.  The phase
 // kx (x - fx) + ky (y - fy) - omega t + phase0 is formed in float-float from
 // the records (the point's coordinates split by integer operations) and
 // reduced, then sine and cosine by polynomial (within 1e-7; the SFU's few
@@ -497,55 +595,134 @@ __device__ __forceinline__ void ph_kahan(float &s, float &c, float v) {
 // with Kahan compensation.  FP64 per (point, component) -- phase, reduction and FP64
 // sums -- kept the FP64 pipe the bound on this GPU.  Only non-trivial
 // component ramps are evaluated in FP64 (Irregular.cpp:200-204).
-__global__ void __launch_bounds__(128) k_phasors(PhArgs a) {
-    __shared__ float s_rec[PH_CHUNK * PH_REC];
+//
+// A block takes 32 points, a warp every PH_WARPS-th pair of components of a
+// chunk, the lanes the points (so the rows are written 256 bytes at a time);
+// the warps' shares of the sums are added in warp order, compensated, and only
+// the sums that the call's rows need are formed.  Instruction issue is the
+// bound, so two components are worked on at once in packed FP32x2 (89
+// instructions a phasor instead of 180).  A ramp that all components share is
+// evaluated once per point and written once (row 0).  With a thread per point
+// and all components in turn a batch of 5003 points was 40 blocks of one long
+// chain: 73 us at 256 components, 20 us now; 65536 points, 128 components: 60
+// us then, 38 now (4 warps a block; 2: 39, 8: 44).
+constexpr int PH_WARPS = 4;
+__global__ void __launch_bounds__(32 * PH_WARPS) k_phasors(PhArgs a) {
+    __shared__ __align__(16) float s_rec[PH_CHUNK * PH_REC];
     __shared__ float2 s_off[2];
-    const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    __shared__ float2 s_sum[PH_WARPS][5][32];
+    __shared__ float s_ramp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long p = blockIdx.x * 32L + lane;
     const bool valid = p < a.n;
     const long pc = valid ? p : 0;
     if (threadIdx.x == 0) {
         ff_split(-a.fx, s_off[0].x, s_off[0].y);
         ff_split(-a.fy, s_off[1].x, s_off[1].y);
     }
-    __syncthreads();
     const double tp = a.t[pc * a.st];
+    const double *P = a.phase;
+    const int cs = a.cstride;
+    if (warp == 1 && a.trivial_ramp) {
+        const float r0 = (float)d_freq_ramp(tp, P[4 * cs], P[5 * cs], P[6 * cs]);
+        s_ramp[lane] = r0;
+        if (valid) a.rr[p] = r0;
+    }
+    __syncthreads();
     const float2 dx = ff_add(ff_from_double(a.x[pc * a.sx]), s_off[0]);
     const float2 dy = ff_add(ff_from_double(a.y[pc * a.sy]), s_off[1]);
     const float2 tt = ff_from_double(tp);
-    const double *P = a.phase;
-    const int cs = a.cstride;
-    const float rconst = a.trivial_ramp ? (float)d_freq_ramp(tp, P[4 * cs], P[5 * cs], P[6 * cs]) : 0.f;
-    float sm[5] = {0, 0, 0, 0, 0}, cm[5] = {0, 0, 0, 0, 0};
+    const float rconst = a.trivial_ramp ? s_ramp[lane] : 0.f;
+    // everything below is on two components at once (packed FP32x2), as
+    // instruction issue is the bound
+    const f32x2 neg1 = p_pack(-1.f, -1.f);
+    auto dup = [](float v) { return p_pack(v, v); };
+    const f32x2 xh = dup(dx.x), xl = dup(dx.y), nxh = dup(-dx.x), yh = dup(dy.x), yl = dup(dy.y), nyh = dup(-dy.x);
+    const f32x2 th = dup(tt.x), tl = dup(tt.y), nth = dup(-tt.x);
+    f32x2 S[5] = {0, 0, 0, 0, 0}, C[5] = {0, 0, 0, 0, 0};
     for (int i0 = 0; i0 < a.npad; i0 += PH_CHUNK) {
         const int nrec = min(PH_CHUNK, a.npad - i0);
         __syncthreads();
-        for (int e = threadIdx.x; e < nrec * PH_REC; e += blockDim.x) s_rec[e] = a.rec[(long)i0 * PH_REC + e];
+        for (int e = threadIdx.x; e < nrec * PH_REC / 4; e += blockDim.x)
+            reinterpret_cast<float4 *>(s_rec)[e] = reinterpret_cast<const float4 *>(a.rec + (long)i0 * PH_REC)[e];
         __syncthreads();
-        if (!valid) continue;
-        for (int ii = 0; ii < nrec; ii++) {
+        for (int ii = 2 * warp; ii < nrec; ii += 2 * PH_WARPS) {
             const int i = i0 + ii;
-            const float *R = s_rec + ii * PH_REC;
-            float c = 0.f, s = 0.f, r = 0.f;
-            if (i < a.ncomp) {
-                float2 ph = ff_add(ff_mul(R[0], R[1], dx.x, dx.y), ff_mul(R[2], R[3], dy.x, dy.y));
-                ph = ff_add(ph, ff_mul(R[4], R[5], tt.x, tt.y));
-                ph = ff_add(ph, make_float2(R[6], R[7]));
-                ff_sincos_poly(ff_reduce_2pi(ph), s, c);
-                r = a.trivial_ramp ? rconst
-                                   : (float)d_freq_ramp(tp, P[4 * cs + i], P[5 * cs + i], P[6 * cs + i]);
-                const float rc = r * c, rs = r * s;
-                ph_kahan(sm[0], cm[0], rc * R[8]);
-                ph_kahan(sm[1], cm[1], rc * R[9]);
-                ph_kahan(sm[2], cm[2], rc * R[10]);
-                ph_kahan(sm[3], cm[3], rs * R[11]);
-                ph_kahan(sm[4], cm[4], rc * R[12]);
+            const ulonglong2 *R = reinterpret_cast<const ulonglong2 *>(s_rec + ii * PH_REC);
+            const ulonglong2 kx = R[0], ky = R[1], w = R[2], p0 = R[3];
+            // phase = kx x + ky y - omega t + phase0 as a pair (hi, lo): each
+            // product exact, the sums error-free in the hi parts
+            f32x2 hi = p_mul(kx.x, xh);
+            f32x2 lo = p_fma(kx.x, xl, p_fma(kx.y, xh, p_fma(kx.x, xh, p_mul(kx.x, nxh))));
+            auto add = [&](f32x2 h, f32x2 l) {
+                const f32x2 s = p_add(hi, h), bb = p_fma(hi, neg1, s);
+                const f32x2 d = p_fma(bb, neg1, s);
+                const f32x2 e = p_add(p_fma(d, neg1, hi), p_fma(bb, neg1, h));
+                hi = s;
+                lo = p_add(p_add(lo, l), e);
+            };
+            add(p_mul(ky.x, yh), p_fma(ky.x, yl, p_fma(ky.y, yh, p_fma(ky.x, yh, p_mul(ky.x, nyh)))));
+            add(p_mul(w.x, th), p_fma(w.x, tl, p_fma(w.y, th, p_fma(w.x, th, p_mul(w.x, nth)))));
+            add(p0.x, p0.y);
+            f32x2 c2, s2;
+            ph_sincos(hi, lo, s2, c2);
+            const float2 c = p_un(c2), s = p_un(s2);
+            f32x2 rc = c2, rs = s2;
+            if (a.trivial_ramp) {
+                const f32x2 r2 = dup(rconst);
+                rc = p_mul(r2, c2);
+                rs = p_mul(r2, s2);
+            } else {
+                float r[2];
+                for (int q = 0; q < 2; q++)
+                    r[q] = i + q < a.ncomp ? (float)d_freq_ramp(tp, P[4 * cs + i + q], P[5 * cs + i + q],
+                                                                P[6 * cs + i + q])
+                                           : 0.f;
+                const f32x2 r2 = p_pack(r[0], r[1]);
+                rc = p_mul(r2, c2);
+                rs = p_mul(r2, s2);
+                if (valid) {
+                    a.rr[(long)i * a.n + p] = r[0];
+                    a.rr[(long)(i + 1) * a.n + p] = r[1];
+                }
             }
-            a.ph[(long)i * a.n + p] = make_float2(c, s);
-            a.rr[(long)i * a.n + p] = r;
+            // (records past the last component are zero: phase 0, coefficients 0)
+            const ulonglong2 a0 = R[4], a1 = R[5], a2 = R[6];
+            const f32x2 cf[5] = {a0.x, a0.y, a1.x, a1.y, a2.x};
+#pragma unroll
+            for (int q = 0; q < 5; q++) {
+                if (!(a.sums & (1 << q))) continue;
+                // Kahan: y = v - C, t = S + y, C = (t - S) - y
+                const f32x2 y = p_fma(C[q], neg1, p_mul(q == 3 ? rs : rc, cf[q]));
+                const f32x2 t = p_add(S[q], y);
+                C[q] = p_fma(y, neg1, p_fma(S[q], neg1, t));
+                S[q] = t;
+            }
+            if (valid) {
+                a.ph[(long)i * a.n + p] = make_float2(c.x, s.x);
+                a.ph[(long)(i + 1) * a.n + p] = make_float2(c.y, s.y);
+            }
         }
     }
-    if (!valid) return;
-    for (int q = 0; q < 5; q++) a.first[q * a.n + p] = (double)sm[q] - (double)cm[q];
+    float sm[5], cm[5];
+    for (int q = 0; q < 5; q++) {        // the two lanes
+        const float2 t = p_un(S[q]), u = p_un(C[q]);
+        sm[q] = t.x;
+        cm[q] = u.x + u.y;
+        ph_kahan(sm[q], cm[q], t.y);
+    }
+    for (int q = 0; q < 5; q++) s_sum[warp][q][lane] = make_float2(sm[q], cm[q]);
+    __syncthreads();
+    for (int q = warp; q < 5; q += PH_WARPS) {
+        if (!valid || !(a.sums & (1 << q))) continue;
+        float v = 0.f, c = 0.f;
+        for (int w = 0; w < PH_WARPS; w++) {
+            const float2 t = s_sum[w][q][lane];
+            ph_kahan(v, c, t.x);
+            c += t.y;                    // the share is t.x - t.y
+        }
+        a.first[q * a.n + p] = (double)v - (double)c;
+    }
 }
 
 // Few points (a scalar call, a short batch): one block per point, the
@@ -569,7 +746,9 @@ __global__ void __launch_bounds__(128) k_phasors_few(PhArgs a) {
     const float rconst = a.trivial_ramp ? (float)d_freq_ramp(tp, P[4 * cs], P[5 * cs], P[6 * cs]) : 0.f;
     float sm[5] = {0, 0, 0, 0, 0}, cm[5] = {0, 0, 0, 0, 0};
     for (int i = threadIdx.x; i < a.npad; i += blockDim.x) {
-        const float *R = a.rec + (long)i * PH_REC;
+        float R[PH_REC];
+#pragma unroll
+        for (int q = 0; q < PH_REC; q++) R[q] = a.rec[rec_at(i, q)];
         float c = 0.f, sn = 0.f, r = 0.f;
         if (i < a.ncomp) {
             float2 ph = ff_add(ff_mul(R[0], R[1], dx.x, dx.y), ff_mul(R[2], R[3], dy.x, dy.y));
@@ -585,7 +764,7 @@ __global__ void __launch_bounds__(128) k_phasors_few(PhArgs a) {
             ph_kahan(sm[4], cm[4], rc * R[12]);
         }
         a.ph[(long)i * a.n + p] = make_float2(c, sn);
-        a.rr[(long)i * a.n + p] = r;
+        if (!a.trivial_ramp || i == 0) a.rr[(long)i * a.n + p] = a.trivial_ramp ? rconst : r;
     }
     double v[5];
 #pragma unroll
@@ -612,8 +791,13 @@ struct PairArgs {
     int ntile;           // component tiles of the table
     const float *tab;    // pair tiles
     const float2 *tabp;  // pressure pair tiles (Pp, Mp), column kernel with pressure
+    const float4 *tpp;   // point kernel: pressure tiles (Pp, Mp, kp, km)
+    const float4 *tpk;   // and the phase-free products (X, Z)
+    float one;           // 1 (p_hold)
+    int kin;             // few-point kernel: sum them (else the height table holds their sum)
     const float2 *ph;    // [npad][ncol]
-    const float *rr;     // [npad][ncol]
+    const float *rr;     // ramps: row stride rs (0 where every component has the same ramp)
+    long rs;
     const float *cf;     // [NCF][cstride]
     int cstride;
     const float *z0;     // [ncol*nl] evaluation heights (z0 <= 0 below the surface)
@@ -700,7 +884,7 @@ __global__ void __launch_bounds__(128) k_pairs_columns(PairArgs a) {
                 for (int ii = 0; ii < TT; ii++) {
                     const int i = I * TT + ii;
                     const float2 pi = a.ph[(long)i * a.ncol + col];
-                    const float ri = a.rr[(long)i * a.ncol + col];
+                    const float ri = a.rr[(long)i * a.rs + col];
                     // packed FP32x2 over level pairs: per pair and level,
                     // E = exp(k z), Y = exp(-k(z + 2h)) = E exp(-2k(z+h)),
                     // F = E + Y, G = E - Y (the normaliser is in the record)
@@ -767,7 +951,7 @@ __global__ void __launch_bounds__(128) k_pairs_columns(PairArgs a) {
                 for (int mm = 0; mm < TT; mm++) {
                     const int m = M * TT + mm;
                     const float2 pm = s_ph[mm * cols + cl];
-                    const float rm = a.rr[(long)m * a.ncol + col];
+                    const float rm = a.rr[(long)m * a.rs + col];
                     const float k = a.cf[CF_K * a.cstride + m], q = a.cf[CF_Q * a.cstride + m];
                     const float au_ = a.cf[CF_AU * a.cstride + m] * q * rm;
                     const float cu_ = au_ * a.cf[CF_CT * a.cstride + m] * pm.x;
@@ -812,130 +996,245 @@ __global__ void k_sum_slices(long n, int nslice, const float *part, float *out) 
     out[e] = s;
 }
 
+// Tile pair tp of a walk with the column tile M outermost: I = 0..M, so that a
+// thread's phasors of tile M stay in registers for M + 1 tile pairs.
+__device__ __forceinline__ void walk_at(int tp, int &I, int &M) {
+    M = 0;
+    while (tp > M) tp -= ++M;
+    I = tp;
+}
+
+__device__ __forceinline__ void pr_cp16(void *smem, const void *gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void pr_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void pr_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
 // Point mode: u, v, w, dp at one height per thread, point-API mask
 // (u2/v2/w2/dp2 of the reference, with rho folded into the p records).
 // VEL: the velocity sums, PR: the pressure sums (a call that asks for one of
 // them does not pay for the other; rows not computed are 0).
-template <int TT, bool VEL, bool PR>
-__global__ void __launch_bounds__(128) k_pairs_points(PairArgs a) {
+//
+// Per (pair, point) the velocity sums take 24 FMA-pipe instructions and 4
+// exponentials, the pressure's 15 and 4.  A thread keeps its phasors (and for
+// the pressure its profiles) of the 16 components of tile M in registers over
+// the walk's tiles (I, M), two components to a packed FP32x2 operand, and the
+// records, which all points share, come as broadcast reads of such operands
+// from a double-buffered stage.  Packing halves the instructions issued (the
+// FMA pipe's work is the same): unpacked, with phasors and profiles in shared
+// memory, 42 instructions a pair were issued (issue 79 % busy), now 22 (FMA pipe
+// 70 % busy, pressure: XU 66 %).  65536 points, 128 components: velocity and
+// pressure sums 1331 us together then, 894 now; 5003 points, 256 components 491
+// and 264 (tiles of 32 instead of 16 components: 1043 and 383; five blocks an
+// SM instead of six: 882 and 307).  In a tile of the diagonal the records below
+// it are zero; whole groups of four are skipped.
+// KIN: the phase-free products of the first-order profiles in the pressure,
+// summed here (otherwise the caller adds them from the height table).
+template <bool VEL, bool PR, bool KIN>
+struct PointStage {
+    static constexpr int TT = POINT_TILE;
+    static constexpr int V4 = VEL ? TT * TT * POINTV_NC / 4 : 0;      // float4 of a stage: velocity records,
+    static constexpr int P4 = PR ? TT * TT * POINTP_NC / 4 : 0;       // pressure phase terms,
+    static constexpr int K4 = KIN ? TT * TT * POINTK_NC / 4 : 0;      // phase-free products
+    static constexpr int N4 = V4 + P4 + K4;
+    static constexpr int SMEM = 2 * N4 * 16;
+    static constexpr int ROWS = VEL ? 3 : 1;                          // u, v, w or p
+};
+
+template <bool VEL, bool PR, bool KIN>
+__global__ void __launch_bounds__(128, KIN ? 2 : 6) k_pairs_points(PairArgs a) {
+    static_assert(VEL != PR && (PR || !KIN), "one group of rows a launch");
+    using ST = PointStage<VEL, PR, KIN>;
+    constexpr int TT = POINT_TILE;
     extern __shared__ float4 smem4[];
-    float *s_tab = reinterpret_cast<float *>(smem4);                        // TT*TT*12
-    float2 *s_ph = reinterpret_cast<float2 *>(s_tab + TT * TT * POINTV_NC); // TT*128
-    float2 *s_pz = s_ph + TT * 128;                                         // TT*128
-    const long p = (long)blockIdx.x * 128 + threadIdx.x;
+    const int tid = threadIdx.x;
+    const long p = (long)blockIdx.x * 128 + tid;
     const bool valid = p < a.ncol;
-    const long pc = valid ? p : 0;
-    const float z = valid ? a.z0[pc] : 0.f;
+    const long pc = valid ? p : a.ncol - 1;
+    const float z = a.z0[pc];
     const float zk = z * LOG2E_F, zetak = -2.f * (z + a.depth) * LOG2E_F;
+    const float yk = -(z + 2.f * a.depth) * LOG2E_F;
+    const f32x2 zk2 = p_pack(zk, zk), yk2 = p_pack(yk, yk), neg1 = p_pack(-1.f, -1.f);
     float su = 0, cu = 0, sv = 0, cv = 0, sw = 0, cw = 0, sq = 0, cq = 0;
-    // slice of the tile-pair loop owned by this blockIdx.y (block-uniform)
-    const int tp_lo = blockIdx.y * a.tp_per, tp_hi = tp_lo + a.tp_per;
-    int tp = -1;
-    for (int I = 0; I < a.ntile; I++) {
-        for (int M = I; M < a.ntile; M++) {
-            if (!a.pairs && M != I) continue;
-            tp++;
-            if (tp < tp_lo || tp >= tp_hi) continue;
-            __syncthreads();
-            if (a.pairs) {
-                const float4 *src = reinterpret_cast<const float4 *>(
-                    a.tab + tile_index(I, M, a.ntile) * (long)TT * TT * POINTV_NC);
-                float4 *dst = reinterpret_cast<float4 *>(s_tab);
-                for (int e = threadIdx.x; e < TT * TT * POINTV_NC / 4; e += blockDim.x) dst[e] = src[e];
+    // slice of the tile-pair loop owned by this blockIdx.y (block-uniform);
+    // without pairs the "walk" is the diagonal tiles
+    const int ntp = a.pairs ? a.ntile * (a.ntile + 1) / 2 : a.ntile;
+    const int lo = blockIdx.y * a.tp_per, hi = min(lo + a.tp_per, ntp);
+    int I = lo, M = lo;
+    if (a.pairs) walk_at(lo, I, M);
+    int lI = I, lM = M, lt = lo;         // the next tile pair to load
+    auto issue = [&]() {
+        if (a.pairs && lt < hi) {
+            const long e0 = tile_index(lI, lM, a.ntile) * (long)TT * TT;
+            float4 *dst = smem4 + ((lt - lo) & 1) * ST::N4;
+            if (VEL) {
+                const float4 *src = reinterpret_cast<const float4 *>(a.tab) + e0 * (POINTV_NC / 4);
+#pragma unroll
+                for (int e = 0; e < ST::V4; e += 128) pr_cp16(dst + e + tid, src + e + tid);
             }
-            for (int mm = 0; mm < TT; mm++) {
+            if (PR) {
+                const float4 *sp = a.tpp + e0;
+#pragma unroll
+                for (int e = 0; e < ST::P4; e += 128) pr_cp16(dst + ST::V4 + e + tid, sp + e + tid);
+            }
+            if (KIN) {
+                const float4 *sk = a.tpk + e0 / 2;
+#pragma unroll
+                for (int e = 0; e < ST::K4; e += 128) pr_cp16(dst + ST::V4 + ST::P4 + e + tid, sk + e + tid);
+            }
+            if (++lI > lM) { lI = 0; lM++; }
+        }
+        lt++;
+        pr_commit();
+    };
+    issue();
+    const f32x2 one2 = p_pack(a.one, a.one);
+    for (int t = lo; t < hi; M++) {
+        // cosines and sines of tile M's components two by two, and (KIN) px, pz
+        f32x2 pmc[TT / 2], pms[TT / 2], xmx[KIN ? TT / 2 : 1], xmz[KIN ? TT / 2 : 1];
+        {
+#pragma unroll
+            for (int mm = 0; mm < TT; mm += 2) {
                 const int m = M * TT + mm;
-                float2 pm = a.ph[(long)m * a.ncol + pc];
-                float F, G;
-                depth_fg(a.cf[CF_K * a.cstride + m], zk, zetak, F, G);
-                const float q = a.cf[CF_Q * a.cstride + m];
-                s_ph[mm * 128 + threadIdx.x] = pm;
-                s_pz[mm * 128 + threadIdx.x] = make_float2(q * F, q * G);   // px_m, pz_m
-            }
-            __syncthreads();
-            if (!valid) continue;
-            if (a.pairs) {
-                for (int ii = 0; ii < TT; ii++) {
-                    const int i = I * TT + ii;
-                    const float2 pi = a.ph[(long)i * a.ncol + p];
-                    const float ri = a.rr[(long)i * a.ncol + p];
-                    const float2 pxi = (M == I) ? s_pz[ii * 128 + threadIdx.x] : make_float2(0.f, 0.f);
-                    float2 pxz_i = pxi;
-                    if (M != I) {
-                        float F, G;
-                        depth_fg(a.cf[CF_K * a.cstride + i], zk, zetak, F, G);
-                        const float q = a.cf[CF_Q * a.cstride + i];
-                        pxz_i = make_float2(q * F, q * G);
-                    }
-                    float au = 0, av = 0, aw = 0, ap = 0, ax = 0, az = 0;
-                    const int m0 = (M == I) ? ii : 0;
-                    for (int mm = m0; mm < TT; mm++) {
-                        const float *e = s_tab + (ii * TT + mm) * POINTV_NC;
-                        const float4 c0 = *reinterpret_cast<const float4 *>(e);
-                        const float4 c1 = *reinterpret_cast<const float4 *>(e + 4);
-                        const float4 c2 = *reinterpret_cast<const float4 *>(e + 8);
-                        const float2 pm = s_ph[mm * 128 + threadIdx.x];
-                        const float2 xm = s_pz[mm * 128 + threadIdx.x];
-                        const float cc = pi.x * pm.x, ss = pi.y * pm.y;
-                        const float sc = pi.y * pm.x, cs = pi.x * pm.y;
-                        const float cp = cc - ss, cmn = cc + ss, sp = sc + cs, smn = sc - cs;
-                        float Fp, Gp, Fm, Gm;
-                        depth_fg(c2.x, zk, zetak, Fp, Gp);
-                        depth_fg(c2.y, zk, zetak, Fm, Gm);
-                        // the phase-and-depth products once, then one FMA per coefficient
-                        const float A = cp * Fp, B = cmn * Fm;
-                        if (VEL) {
-                            const float Cq = sp * Gp, D = smn * Gm;
-                            au = fmaf(c0.x, A, fmaf(c0.y, B, au));
-                            av = fmaf(c0.z, A, fmaf(c0.w, B, av));
-                            aw = fmaf(c1.x, Cq, fmaf(c1.y, D, aw));
-                        }
-                        if (PR) {
-                            ap = fmaf(c1.z, A, fmaf(c1.w, B, ap));
-                            ax = fmaf(c2.z, xm.x, ax);
-                            az = fmaf(c2.w, xm.y, az);
-                        }
-                    }
-                    if (VEL) {
-                        kahan(su, cu, ri * au);
-                        kahan(sv, cv, ri * av);
-                        kahan(sw, cw, ri * aw);
-                    }
-                    if (PR) {
-                        ap = fmaf(pxz_i.x, ax, fmaf(pxz_i.y, az, ap));
-                        kahan(sq, cq, ri * ap);
-                    }
-                }
-            }
-            if (a.first && M == I) {
-                // first-order u1, v1, w1, dp1 and the linear dp2 diagonal terms
-                for (int mm = 0; mm < TT; mm++) {
-                    const int m = M * TT + mm;
-                    const float2 pm = s_ph[mm * 128 + threadIdx.x];
-                    const float2 xm = s_pz[mm * 128 + threadIdx.x];
-                    const float rm = a.rr[(long)m * a.ncol + p];
-                    if (VEL) {
-                        const float au_ = a.cf[CF_AU * a.cstride + m] * rm;
-                        kahan(su, cu, au_ * xm.x * a.cf[CF_CT * a.cstride + m] * pm.x);
-                        kahan(sv, cv, au_ * xm.x * a.cf[CF_ST * a.cstride + m] * pm.x);
-                        kahan(sw, cw, au_ * xm.y * pm.y);
-                    }
-                    if (PR) {
-                        float pp = a.cf[CF_AP * a.cstride + m] * xm.x * pm.x;
-                        if (a.pairs)
-                            pp += a.cf[CF_X1 * a.cstride + m] * xm.x + a.cf[CF_Z1 * a.cstride + m] * xm.y;
-                        kahan(sq, cq, rm * pp);
-                    }
+                const float2 p0 = a.ph[(long)m * a.ncol + pc], p1 = a.ph[(long)(m + 1) * a.ncol + pc];
+                pmc[mm / 2] = p_hold(p0.x, p1.x, one2);
+                pms[mm / 2] = p_hold(p0.y, p1.y, one2);
+                if (KIN) {
+                    float F0, G0, F1, G1;
+                    depth_fg(a.cf[CF_K * a.cstride + m], zk, zetak, F0, G0);
+                    depth_fg(a.cf[CF_K * a.cstride + m + 1], zk, zetak, F1, G1);
+                    const float q0 = a.cf[CF_Q * a.cstride + m], q1 = a.cf[CF_Q * a.cstride + m + 1];
+                    xmx[mm / 2] = p_hold(q0 * F0, q1 * F1, one2);
+                    xmz[mm / 2] = p_hold(q0 * G0, q1 * G1, one2);
                 }
             }
         }
+        if (!a.pairs) I = M;
+        for (; I <= M && t < hi; I++, t++) {
+        issue();
+        pr_wait1();
+        __syncthreads();
+        const ulonglong2 *tv = reinterpret_cast<const ulonglong2 *>(smem4) + ((t - lo) & 1) * ST::N4, *tq = tv + ST::V4,
+                         *tx = tq + ST::P4;
+        if (a.pairs) {
+            const float2 *prow = a.ph + (long)(I * TT) * a.ncol + pc;
+            const float *rrow = a.rr + (long)(I * TT) * a.rs + pc;
+            float2 pn = *prow;
+            float rn = *rrow;
+            // off the diagonal a row is one branch-free block (its reads and
+            // exponentials scheduled across the whole row)
+            auto rows = [&](auto diag) {
+                constexpr bool DIAG = decltype(diag)::value;
+                for (int ii = 0; ii < TT; ii++) {
+                    const int i = I * TT + ii;
+                    const float2 pi = pn;
+                    const float ri = rn;
+                    if (ii + 1 < TT) {       // the next row's, under this row's sums
+                        prow += a.ncol;
+                        rrow += a.rs;
+                        pn = *prow;
+                        rn = *rrow;
+                    }
+                    const f32x2 px2 = p_pack(pi.x, pi.x), py2 = p_pack(pi.y, pi.y);
+                    const f32x2 nx2 = p_pack(-pi.x, -pi.x), ny2 = p_pack(-pi.y, -pi.y);
+                    f32x2 au = 0, av = 0, aw = 0, ap = 0, ax = 0, az = 0;
+                    // the row's records; within it every read has a constant offset
+                    const ulonglong2 *rv = tv + ii * (2 * TT), *rq = tq + ii * TT, *rx = tx + ii * (TT / 2);
+#pragma unroll
+                    for (int m4 = 0; m4 < TT; m4 += 4) {
+                        if (DIAG && m4 + 3 < ii) continue;
+#pragma unroll
+                        for (int mm = m4; mm < m4 + 4; mm += 2) {
+                            const f32x2 mc = pmc[mm / 2], ms = pms[mm / 2];
+                            ulonglong2 r0, r1, r2, rk, rp;
+                            if (VEL) {
+                                r0 = rv[2 * mm]; r1 = rv[2 * mm + 1]; r2 = rv[2 * mm + 2]; rk = rv[2 * mm + 3];
+                            }
+                            if (PR) {
+                                rp = rq[mm]; rk = rq[mm + 1];
+                            }
+                            // cos(phi_i +- phi_m), and sin below
+                            const f32x2 cc = p_mul(px2, mc);
+                            const f32x2 cp = p_fma(ny2, ms, cc), cm = p_fma(py2, ms, cc);
+                            // E = exp(kz), Y = exp(-k(z + 2h)): F = E + Y, G = E - Y (the
+                            // normaliser is in the record)
+                            const f32x2 Ep = p_ex2(p_mul(rk.x, zk2)), Yp = p_ex2(p_mul(rk.x, yk2));
+                            const f32x2 Em = p_ex2(p_mul(rk.y, zk2)), Ym = p_ex2(p_mul(rk.y, yk2));
+                            // the phase-and-depth products once, then one FMA per coefficient
+                            const f32x2 A = p_mul(cp, p_add(Ep, Yp)), B = p_mul(cm, p_add(Em, Ym));
+                            if (VEL) {
+                                const f32x2 sc = p_mul(py2, mc);
+                                const f32x2 sp = p_fma(px2, ms, sc), sm = p_fma(nx2, ms, sc);
+                                const f32x2 C = p_mul(sp, p_fma(Yp, neg1, Ep)), D = p_mul(sm, p_fma(Ym, neg1, Em));
+                                au = p_fma(r0.x, A, p_fma(r0.y, B, au));
+                                av = p_fma(r1.x, A, p_fma(r1.y, B, av));
+                                aw = p_fma(r2.x, C, p_fma(r2.y, D, aw));
+                            }
+                            if (PR) ap = p_fma(rp.x, A, p_fma(rp.y, B, ap));
+                            if (KIN) {
+                                const ulonglong2 x2 = rx[mm / 2];
+                                ax = p_fma(x2.x, xmx[mm / 2], ax);
+                                az = p_fma(x2.y, xmz[mm / 2], az);
+                            }
+                        }
+                    }
+                    if (VEL) {
+                        kahan(su, cu, ri * p_hsum(au));
+                        kahan(sv, cv, ri * p_hsum(av));
+                        kahan(sw, cw, ri * p_hsum(aw));
+                    }
+                    if (PR) {
+                        float row = p_hsum(ap);
+                        if (KIN) {
+                            float F, G;
+                            depth_fg(a.cf[CF_K * a.cstride + i], zk, zetak, F, G);
+                            const float q = a.cf[CF_Q * a.cstride + i];
+                            row = fmaf(q * F, p_hsum(ax), fmaf(q * G, p_hsum(az), row));
+                        }
+                        kahan(sq, cq, ri * row);
+                    }
+                }
+            };
+            if (M == I) rows(std::true_type{});
+            else rows(std::false_type{});
+        }
+        if (a.first && M == I) {
+            // first-order u1, v1, w1, dp1 and the linear dp2 diagonal terms
+            for (int mm = 0; mm < TT; mm++) {
+                const int m = M * TT + mm;
+                const float2 pv = a.ph[(long)m * a.ncol + pc];
+                const float rm = a.rr[(long)m * a.rs + pc];
+                float F, G;
+                depth_fg(a.cf[CF_K * a.cstride + m], zk, zetak, F, G);
+                const float q = a.cf[CF_Q * a.cstride + m];
+                const float px = q * F, pz = q * G;
+                if (VEL) {
+                    const float au_ = a.cf[CF_AU * a.cstride + m] * rm;
+                    kahan(su, cu, au_ * px * a.cf[CF_CT * a.cstride + m] * pv.x);
+                    kahan(sv, cv, au_ * px * a.cf[CF_ST * a.cstride + m] * pv.x);
+                    kahan(sw, cw, au_ * pz * pv.y);
+                }
+                if (PR) {
+                    float pp = a.cf[CF_AP * a.cstride + m] * px * pv.x;
+                    if (KIN && a.pairs) pp += a.cf[CF_X1 * a.cstride + m] * px + a.cf[CF_Z1 * a.cstride + m] * pz;
+                    kahan(sq, cq, rm * pp);
+                }
+            }
+        }
+        __syncthreads();                 // the stage is refilled by the next issue
+        }
+        I = 0;
     }
     if (!valid) return;
-    float *out = a.out + (long)blockIdx.y * 4 * a.ncol;
-    out[0 * a.ncol + p] = su;
-    out[1 * a.ncol + p] = sv;
-    out[2 * a.ncol + p] = sw;
-    out[3 * a.ncol + p] = sq;
+    float *out = a.out + (long)blockIdx.y * ST::ROWS * a.ncol;
+    if (VEL) {
+        out[p] = su;
+        out[a.ncol + p] = sv;
+        out[2 * a.ncol + p] = sw;
+    } else {
+        out[p] = sq;
+    }
 }
 
 // Few points, point mode: block (point p, slice y); thread t takes row
@@ -967,20 +1266,26 @@ __global__ void __launch_bounds__(128) k_pairs_points_few(PairArgs a, int ntp, i
         }
         const int i = I * TT + ii;
         const float2 pi = a.ph[(long)i * a.ncol + p];
-        const float ri = a.rr[(long)i * a.ncol + p];
+        const float ri = a.rr[(long)i * a.rs + p];
         float Fi, Gi;
         depth_fg(a.cf[CF_K * a.cstride + i], zk, zetak, Fi, Gi);
         const float qi = a.cf[CF_Q * a.cstride + i];
         const float2 pxz_i = make_float2(qi * Fi, qi * Gi);
         if (a.pairs) {
-            const float *T = a.tab + tile_index(I, M, a.ntile) * (long)TT * TT * POINTV_NC;
+            const long e0 = tile_index(I, M, a.ntile) * (long)TT * TT;
+            const float *TV = a.tab, *TP = reinterpret_cast<const float *>(a.tpp), *TK = reinterpret_cast<const float *>(a.tpk);
             float au = 0, av = 0, aw = 0, ap = 0, ax = 0, az = 0;
             for (int mm = (M == I) ? ii : 0; mm < TT; mm++) {
                 const int m = M * TT + mm;
-                const float *e = T + (ii * TT + mm) * POINTV_NC;
-                const float4 c0 = *reinterpret_cast<const float4 *>(e);
-                const float4 c1 = *reinterpret_cast<const float4 *>(e + 4);
-                const float4 c2 = *reinterpret_cast<const float4 *>(e + 8);
+                const long e = e0 + ii * TT + mm;
+                float c[POINTV_NC], cq_[POINTP_NC], x2[POINTK_NC];
+#pragma unroll
+                for (int q = 0; q < POINTV_NC; q++) c[q] = TV[point_at(e, POINTV_NC, q)];
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    cq_[q] = TP[point_at(e, POINTP_NC, q)];
+                    x2[q] = TK[point_at(e, POINTK_NC, q)];
+                }
                 const float2 pm = a.ph[(long)m * a.ncol + p];
                 float Fm_, Gm_;
                 depth_fg(a.cf[CF_K * a.cstride + m], zk, zetak, Fm_, Gm_);
@@ -990,15 +1295,17 @@ __global__ void __launch_bounds__(128) k_pairs_points_few(PairArgs a, int ntp, i
                 const float sc = pi.y * pm.x, cs = pi.x * pm.y;
                 const float cp = cc - ss, cmn = cc + ss, sp = sc + cs, smn = sc - cs;
                 float Fp, Gp, Fm, Gm;
-                depth_fg(c2.x, zk, zetak, Fp, Gp);
-                depth_fg(c2.y, zk, zetak, Fm, Gm);
+                depth_fg(c[6], zk, zetak, Fp, Gp);
+                depth_fg(c[7], zk, zetak, Fm, Gm);
                 const float A = cp * Fp, B = cmn * Fm, Cq = sp * Gp, D = smn * Gm;
-                au = fmaf(c0.x, A, fmaf(c0.y, B, au));
-                av = fmaf(c0.z, A, fmaf(c0.w, B, av));
-                aw = fmaf(c1.x, Cq, fmaf(c1.y, D, aw));
-                ap = fmaf(c1.z, A, fmaf(c1.w, B, ap));
-                ax = fmaf(c2.z, xm.x, ax);
-                az = fmaf(c2.w, xm.y, az);
+                au = fmaf(c[0], A, fmaf(c[1], B, au));
+                av = fmaf(c[2], A, fmaf(c[3], B, av));
+                aw = fmaf(c[4], Cq, fmaf(c[5], D, aw));
+                ap = fmaf(cq_[0], A, fmaf(cq_[1], B, ap));
+                if (a.kin) {
+                    ax = fmaf(x2[0], xm.x, ax);
+                    az = fmaf(x2[1], xm.y, az);
+                }
             }
             ap = fmaf(pxz_i.x, ax, fmaf(pxz_i.y, az, ap));
             kahan(su, cu, ri * au);
@@ -1013,7 +1320,7 @@ __global__ void __launch_bounds__(128) k_pairs_points_few(PairArgs a, int ntp, i
             kahan(sv, cv, au_ * pxz_i.x * a.cf[CF_ST * a.cstride + i] * pi.x);
             kahan(sw, cw, au_ * pxz_i.y * pi.y);
             float pp = a.cf[CF_AP * a.cstride + i] * pxz_i.x * pi.x;
-            if (a.pairs)
+            if (a.pairs && a.kin)
                 pp += a.cf[CF_X1 * a.cstride + i] * pxz_i.x + a.cf[CF_Z1 * a.cstride + i] * pxz_i.y;
             kahan(sq, cq, ri * pp);
         }
@@ -1035,47 +1342,148 @@ __global__ void __launch_bounds__(128) k_pairs_points_few(PairArgs a, int ntp, i
 // Elevation mode: eta2 from the pair cache (Irregular.cpp:223-293).  The
 // record holds A = P+M and B = M-P so that a pair contributes
 // c_i (A c_m) + s_i (B s_m); a row is c_i sum(A c_m) + s_i sum(B s_m).
-template <int TT>
+// (A, B) times (c_m, s_m) is one packed FMA, so a broadcast read of two records
+// (two of the shared memory's cycles) has to feed several points or it is the
+// bound: a thread takes two points, with their phasors of half a column tile
+// (16 components) in registers, two rows a step; the column half is outermost in the
+// walk.  65536 points, 128 components 139 us with the records and phasors read
+// per point, 90 now; 5003 points, 256 components 49 and 37 (latency of the
+// shared-memory reads and row loads; two points, one row a step: 88 and 37; four
+// points 117 and 51; a whole tile's columns 93 and 35).
+constexpr int ETA_P = 2, ETA_C = 16;                       // points a thread, columns of a walk step
+constexpr int ETA_R = 2;                                   // rows of a step
+constexpr int ETA_H = GRID_TILE / ETA_C;                   // walk steps of a tile pair
+constexpr int ETA_N4 = GRID_TILE * ETA_C * EATA_NC / 4;    // float4 of a stage
+constexpr int ETA_SMEM = 2 * ETA_N4 * 16;
 __global__ void __launch_bounds__(128) k_pairs_eta(PairArgs a) {
     extern __shared__ float4 smem4[];
-    float2 *s_tab = reinterpret_cast<float2 *>(smem4);        // TT*TT
-    float2 *s_ph = s_tab + TT * TT;                            // TT*128
-    const long p = (long)blockIdx.x * 128 + threadIdx.x;
-    const bool valid = p < a.ncol;
-    const long pc = valid ? p : 0;
-    float se = 0, ce = 0;
-    const int tp_lo = blockIdx.y * a.tp_per, tp_hi = tp_lo + a.tp_per;
-    int tp = -1;
-    for (int I = 0; I < a.ntile; I++) {
-        for (int M = I; M < a.ntile; M++) {
-            tp++;
-            if (tp < tp_lo || tp >= tp_hi) continue;   // block-uniform
-            __syncthreads();
-            const float4 *src = reinterpret_cast<const float4 *>(
-                a.tab + tile_index(I, M, a.ntile) * (long)TT * TT * 2);
-            float4 *dst = reinterpret_cast<float4 *>(s_tab);
-            for (int e = threadIdx.x; e < TT * TT / 2; e += blockDim.x) dst[e] = src[e];
-            for (int mm = 0; mm < TT; mm++)
-                s_ph[mm * 128 + threadIdx.x] = a.ph[(long)(M * TT + mm) * a.ncol + pc];
-            __syncthreads();
-            if (!valid) continue;
-            for (int ii = 0; ii < TT; ii++) {
-                const int i = I * TT + ii;
-                const float2 pi = a.ph[(long)i * a.ncol + p];
-                const float ri = a.rr[(long)i * a.ncol + p];
-                float ac = 0.f, as = 0.f;
-                const int m0 = (M == I) ? ii : 0;
-                for (int mm = m0; mm < TT; mm++) {
-                    const float2 cab = s_tab[ii * TT + mm];
-                    const float2 pm = s_ph[mm * 128 + threadIdx.x];
-                    ac = fmaf(cab.x, pm.x, ac);
-                    as = fmaf(cab.y, pm.y, as);
+    constexpr int TT = GRID_TILE;
+    const int tid = threadIdx.x;
+    long p[ETA_P];
+#pragma unroll
+    for (int k = 0; k < ETA_P; k++) p[k] = min((long)blockIdx.x * 128 * ETA_P + 128 * k + tid, a.ncol - 1);
+    float se[ETA_P], ce[ETA_P];
+#pragma unroll
+    for (int k = 0; k < ETA_P; k++) se[k] = ce[k] = 0.f;
+    // step t: tile pair t mod (M + 1) of column tile M's part H
+    const int nst = a.ntile * (a.ntile + 1) / 2 * ETA_H;
+    const int lo = blockIdx.y * a.tp_per, hi = min(lo + a.tp_per, nst);
+    int I, M, H;
+    {
+        int t = lo;
+        M = 0;
+        while (t >= ETA_H * (M + 1)) { t -= ETA_H * (M + 1); M++; }
+        H = t / (M + 1);
+        I = t % (M + 1);
+    }
+    auto next = [](int &i, int &m, int &h) {
+        if (++i > m) {
+            i = 0;
+            if (++h >= ETA_H) { h = 0; m++; }
+        }
+    };
+    int lI = I, lM = M, lH = H, lt = lo;
+    auto issue = [&]() {
+        if (lt < hi) {
+            const float4 *src = reinterpret_cast<const float4 *>(a.tab) +
+                                tile_index(lI, lM, a.ntile) * (long)(TT * TT * EATA_NC / 4) + lH * (ETA_C * EATA_NC / 4);
+            float4 *dst = smem4 + ((lt - lo) & 1) * ETA_N4;
+            constexpr int R4 = ETA_C * EATA_NC / 4;        // float4 of a row's half
+#pragma unroll
+            for (int e = 0; e < ETA_N4; e += 128)
+                pr_cp16(dst + e + tid, src + (e + tid) / R4 * (TT * EATA_NC / 4) + (e + tid) % R4);
+            next(lI, lM, lH);
+        }
+        lt++;
+        pr_commit();
+    };
+    issue();
+    const f32x2 one2 = p_pack(a.one, a.one);
+    for (int t = lo; t < hi;) {
+        f32x2 pm[ETA_P][ETA_C];
+        const int m0 = M * TT + H * ETA_C;
+        {
+#pragma unroll
+            for (int mm = 0; mm < ETA_C; mm++)
+#pragma unroll
+                for (int k = 0; k < ETA_P; k++) {
+                    const float2 v = a.ph[(long)(m0 + mm) * a.ncol + p[k]];
+                    pm[k][mm] = p_hold(v.x, v.y, one2);
                 }
-                kahan(se, ce, ri * fmaf(pi.x, ac, pi.y * as));
+        }
+        for (; I <= M && t < hi; I++, t++) {
+        issue();
+        pr_wait1();
+        __syncthreads();
+        const ulonglong2 *rec = reinterpret_cast<const ulonglong2 *>(smem4) + ((t - lo) & 1) * ETA_N4;
+        // rows past the columns of a diagonal tile are zeros
+        const int rows = M == I ? min(TT, (H + 1) * ETA_C) : TT;
+        const float2 *prow[ETA_P];
+        const float *rrow[ETA_P];
+        float2 pn[ETA_R][ETA_P];
+        float rn[ETA_R][ETA_P];
+#pragma unroll
+        for (int k = 0; k < ETA_P; k++) {
+            prow[k] = a.ph + (long)(I * TT) * a.ncol + p[k];
+            rrow[k] = a.rr + (long)(I * TT) * a.rs + p[k];
+#pragma unroll
+            for (int r = 0; r < ETA_R; r++) {
+                pn[r][k] = prow[k][(long)r * a.ncol];
+                rn[r][k] = rrow[k][(long)r * a.rs];
             }
         }
+        for (int ii = 0; ii < rows; ii += ETA_R, rec += ETA_R * (ETA_C / 2)) {
+            float2 pi[ETA_R][ETA_P];
+            float ri[ETA_R][ETA_P];
+#pragma unroll
+            for (int k = 0; k < ETA_P; k++) {
+#pragma unroll
+                for (int r = 0; r < ETA_R; r++) {
+                    pi[r][k] = pn[r][k];
+                    ri[r][k] = rn[r][k];
+                }
+                if (ii + ETA_R < rows) {                   // the next rows', under these rows' sums
+                    prow[k] += ETA_R * a.ncol;
+                    rrow[k] += ETA_R * a.rs;
+#pragma unroll
+                    for (int r = 0; r < ETA_R; r++) {
+                        pn[r][k] = prow[k][(long)r * a.ncol];
+                        rn[r][k] = rrow[k][(long)r * a.rs];
+                    }
+                }
+            }
+            f32x2 acc[ETA_R][ETA_P];                       // sums of A c_m and B s_m
+#pragma unroll
+            for (int r = 0; r < ETA_R; r++)
+#pragma unroll
+                for (int k = 0; k < ETA_P; k++) acc[r][k] = 0;
+#pragma unroll
+            for (int mm = 0; mm < ETA_C; mm += 2)
+#pragma unroll
+                for (int r = 0; r < ETA_R; r++) {
+                    const ulonglong2 c = rec[(r * ETA_C + mm) / 2];
+#pragma unroll
+                    for (int k = 0; k < ETA_P; k++)
+                        acc[r][k] = p_fma(c.y, pm[k][mm + 1], p_fma(c.x, pm[k][mm], acc[r][k]));
+                }
+#pragma unroll
+            for (int r = 0; r < ETA_R; r++)
+#pragma unroll
+                for (int k = 0; k < ETA_P; k++) {
+                    const float2 s2 = p_un(acc[r][k]);
+                    kahan(se[k], ce[k], ri[r][k] * fmaf(pi[r][k].x, s2.x, pi[r][k].y * s2.y));
+                }
+        }
+        __syncthreads();
+        }
+        I = 0;
+        if (++H >= ETA_H) { H = 0; M++; }
     }
-    if (valid) a.out[(long)blockIdx.y * a.ncol + p] = se;
+#pragma unroll
+    for (int k = 0; k < ETA_P; k++) {
+        const long q = (long)blockIdx.x * 128 * ETA_P + 128 * k + tid;
+        if (q < a.ncol) a.out[(long)blockIdx.y * a.ncol + q] = se[k];
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1094,23 +1502,26 @@ struct WsLayout {
     size_t bytes;
 };
 
-// Slices of the tile-pair loop for a launch of nblk blocks (per slice) on a
-// GPU with `slots` resident blocks: the fewest slices (at most maxs, and at
-// most one per tile pair) whose blocks fill the waves they start to 85 %, or
-// else the best filling.  A launch of 512 point blocks on 760 slots fills
-// 67 % of its one wave; 4 slices fill 90 % of three.
-static int wave_slices(long nblk, int ntp, long slots, long maxs) {
-    const long top = std::max<long>(1, std::min<long>(ntp, maxs));
-    int best = 1;
-    double beste = -1.0;
-    for (long ns = 1; ns <= top; ns++) {
-        const double w = (double)(nblk * ns) / (double)slots;
-        const double eff = w / std::ceil(w);
-        if (eff > beste + 1e-9) {
-            beste = eff;
-            best = (int)ns;
+// Tile pairs per slice of a walk of ntp tile pairs, for a launch of nblk
+// blocks per slice on a GPU with `slots` resident blocks and at most maxs
+// slices: the count whose estimated time, waves x (tile pairs + a slice's
+// fixed cost of SLICE_COST tile pairs), is the least.  Slices are whole tile
+// pairs: 4 slices of 10 tile pairs are 3 + 3 + 3 + 1.
+constexpr double SLICE_COST = 0.15;
+static int slice_plan(long nblk, int ntp, long slots, long maxs) {
+    int best = ntp;
+    double bestt = 1e300;
+    int prev = 0;
+    for (int ns = 1; ns <= ntp && ns <= maxs; ns++) {
+        const int per = (ntp + ns - 1) / ns;
+        if (per == prev) continue;              // the same slices as with fewer
+        prev = per;
+        const long n = (ntp + per - 1) / per;
+        const double t = (double)((nblk * n + slots - 1) / slots) * (per + SLICE_COST);
+        if (t < bestt) {
+            bestt = t;
+            best = per;
         }
-        if (eff >= 0.85) break;
     }
     return best;
 }
@@ -1160,6 +1571,17 @@ WsLayout layout(long n, int npad, void *base) {
     return L;
 }
 
+// K(z) of a height table [nz][2] (K, dK/dz) over [-h, 0], by cubic Hermite
+__device__ __forceinline__ double kin_at(const double *kin, int nz, double h, double z) {
+    const double dz = h / (nz - 1);
+    const double t = fmin(fmax((z + h) / dz, 0.0), (double)(nz - 1));
+    const int i = min((int)t, nz - 2);
+    const double r = t - i;
+    const double f0 = kin[2 * i], f1 = kin[2 * i + 2], d0 = kin[2 * i + 1], d1 = kin[2 * i + 3];
+    const double a = dz * d0 - (f1 - f0), b = -dz * d1 + (f1 - f0);
+    return f0 * (1.0 - r) + f1 * r + r * (1.0 - r) * (a * (1.0 - r) + b * r);
+}
+
 // z0 = min(0, z - swl) (order 2/1) or z - swl (order 0), as float
 // clamp: the seabed clamp of the wave_* calls (z below -depth evaluated at
 // -depth), or 0 for the unclamped sums of cfdwm_irregular_fields
@@ -1174,9 +1596,17 @@ __global__ void k_prep_z(long n, const double *z, double swl, int order, int cla
 // out has row stride ldo (the full batch length).
 // With any row or record of api set, the API rows and records are written
 // here (the finishing pass folded in) instead of out.
+// kt.kin: the pressure's phase-free part is added here from the height table
+// (cubic Hermite in FP64), times the point's ramp.
+struct KinTab {
+    const double *kin;      // [nz][2] over [-h, 0], or null
+    int nz;
+    double h, depth;
+    const float *rr;
+};
 __global__ void k_combine(long n, long ldo, int order, double swl, const double *z,
                           const double *first, const float *sec, const float *eta2, int mask,
-                          double *out, ApiRows api) {
+                          double *out, ApiRows api, KinTab kt) {
     long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (p >= n) return;
     double za = (order == 2) ? fmax(0.0, z[p] - swl) : 0.0;
@@ -1186,6 +1616,10 @@ __global__ void k_combine(long n, long ldo, int order, double swl, const double 
     if (mask & 4) v[2] = (double)sec[1 * n + p] + first[2 * n + p] * za;
     if (mask & 8) v[3] = (double)sec[2 * n + p] + first[3 * n + p] * za;
     if (mask & 16) v[4] = (double)sec[3 * n + p] + first[4 * n + p] * za;
+    if ((mask & 16) && kt.kin) {
+        const double z0 = fmin(0.0, fmax(-kt.depth, z[p]) - swl);
+        v[4] += (double)kt.rr[p] * kin_at(kt.kin, kt.nz, kt.h, z0);
+    }
     if (!api.any()) {
         for (int q = 0; q < 5; q++)
             if (mask & (1 << q)) out[q * ldo + p] = v[q];
@@ -1199,8 +1633,9 @@ __global__ void k_combine(long n, long ldo, int order, double swl, const double 
 
 static int launch_phasors(const DevSea &sea, long n, const double *x, const double *y,
                           const double *t, long sx, long sy, long st, int npad, float2 *ph,
-                          float *rr, double *first, cudaStream_t stream) {
+                          float *rr, double *first, cudaStream_t stream, int sums = 31) {
     PhArgs a;
+    a.sums = sums;
     a.n = n; a.x = x; a.y = y; a.t = t; a.sx = sx; a.sy = sy; a.st = st;
     a.ncomp = sea.n; a.npad = npad; a.phase = sea.d_phase; a.cf = sea.d_cf;
     a.cstride = sea.npad_g; a.fx = sea.fx; a.fy = sea.fy;
@@ -1211,7 +1646,7 @@ static int launch_phasors(const DevSea &sea, long n, const double *x, const doub
     if (n <= PH_FEW_POINTS)
         k_phasors_few<<<(unsigned)n, 128, 0, stream>>>(a);
     else
-        k_phasors<<<(unsigned)((n + 127) / 128), 128, 0, stream>>>(a);
+        k_phasors<<<(unsigned)((n + 31) / 32), 32 * PH_WARPS, 0, stream>>>(a);
     note_launch();
     prof_end(PK_PHASORS, stream);
     CK(cudaGetLastError());
@@ -1228,27 +1663,23 @@ int launch_eta_pairs(const DevSea &sea, long n, const float2 *ph, const float *r
                      cudaStream_t stream, float *split_buf = nullptr, long split_cap = 0) {
     PairArgs a{};
     a.ncol = n; a.nl = 1; a.nlg = 1; a.ntile = sea.ntile_g; a.tab = sea.d_tab_eta;
-    a.ph = ph; a.rr = rr; a.cf = sea.d_cf; a.cstride = sea.npad_g; a.out = out;
-    a.pairs = 1; a.first = 0;
-    const long nblk = (n + 127) / 128;
-    const int ntp = sea.ntile_g * (sea.ntile_g + 1) / 2;
-    const size_t smem = sizeof(float2) * (GRID_TILE * GRID_TILE + GRID_TILE * 128);
-    // set once per process (thread-safe static initialisation)
-    static const cudaError_t attr = cudaFuncSetAttribute(k_pairs_eta<GRID_TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem);
-    CK(attr);
+    a.ph = ph; a.rr = rr; a.rs = sea.trivial_ramp ? 0 : n; a.cf = sea.d_cf; a.cstride = sea.npad_g; a.out = out;
+    a.pairs = 1; a.first = 0; a.one = 1.f;
+    const long nblk = (n + 128 * ETA_P - 1) / (128 * ETA_P);
+    const int ntp = sea.ntile_g * (sea.ntile_g + 1) / 2 * ETA_H;   // steps of the walk
+    constexpr size_t smem = ETA_SMEM;
+    static_assert(smem <= 48 * 1024, "no shared-memory opt-in needed");
     static const long slots = [&] {
-        const long v = resident_slots(k_pairs_eta<GRID_TILE>, 128, smem);
+        const long v = resident_slots(k_pairs_eta, 128, smem);
         return v > 0 ? v : SPLIT_TARGET_BLOCKS;
     }();
     // the tile-pair loop split over blockIdx.y where the columns alone do
     // not fill whole waves of the resident blocks (slices summed in order)
-    int nslice = wave_slices(nblk, ntp, slots, split_buf ? split_cap / std::max<long>(1, n) : 1);
-    a.tp_per = (ntp + nslice - 1) / nslice;
-    nslice = (ntp + a.tp_per - 1) / a.tp_per;
+    a.tp_per = slice_plan(nblk, ntp, slots, split_buf ? split_cap / std::max<long>(1, n) : 1);
+    const int nslice = (ntp + a.tp_per - 1) / a.tp_per;
     if (nslice > 1) a.out = split_buf;
     prof_begin(PK_ETA_PAIRS, stream);
-    k_pairs_eta<GRID_TILE><<<dim3((unsigned)nblk, (unsigned)nslice), 128, smem, stream>>>(a);
+    k_pairs_eta<<<dim3((unsigned)nblk, (unsigned)nslice), 128, smem, stream>>>(a);
     note_launch();
     prof_end(PK_ETA_PAIRS, stream);
     CK(cudaGetLastError());
@@ -1300,7 +1731,7 @@ int launch_column_pairs(const DevSea &sea, long ncol, int nl, const float2 *ph, 
     PairArgs a{};
     a.ncol = ncol; a.nl = nl; a.nlg = nlg; a.ntile = sea.ntile_g; a.tab = sea.d_tab_grid;
     a.tabp = reinterpret_cast<const float2 *>(sea.d_tab_gp);
-    a.ph = ph; a.rr = rr; a.cf = sea.d_cf; a.cstride = sea.npad_g; a.z0 = z0;
+    a.ph = ph; a.rr = rr; a.rs = sea.trivial_ramp ? 0 : ncol; a.cf = sea.d_cf; a.cstride = sea.npad_g; a.z0 = z0;
     a.depth = (float)sea.depth; a.out = out; a.pairs = pairs; a.first = 1;
     int cols = 128 / nlg;
     // Few columns (a small grid, a column sample): split the tile-pair loop
@@ -1344,12 +1775,15 @@ int launch_column_pairs(const DevSea &sea, long ncol, int nl, const float2 *ph, 
 // ---------------------------------------------------------------------------
 struct KinArgs {
     const float2 *tabk;        // grid-mask pair tiles (X, Z)
-    int ntile, ncomp, npad, trivial_ramp, zb;
+    int tt, ntile;             // the table's tiles
+    int ncomp, npad, trivial_ramp, zb;
     const double *phase;       // [7][npad]: ramp parameters in rows 4..6
     const float *cf;           // [NCF][npad]
-    double t, depth, dz;
+    double t, depth, h, dz;    // heights -h + dz j
     int nz;
     double *kin;               // [nz][2]: K, dK/dz
+    const float *tpk;          // point-API products (point_at layout; the diagonal terms are CF_X1, CF_Z1), all
+                               // ramps 1, instead of tabk
 };
 
 constexpr int KIN_ZB = 4;      // heights per block (upper bound)
@@ -1364,12 +1798,12 @@ __global__ void __launch_bounds__(256) k_pressure_kin(KinArgs a) {
         if (i < a.ncomp) {
             k = a.cf[CF_K * np + i];
             const int ir = a.trivial_ramp ? 0 : i;
-            r = d_freq_ramp(a.t, a.phase[4 * np + ir], a.phase[5 * np + ir], a.phase[6 * np + ir]);
+            r = a.tpk ? 1.0 : d_freq_ramp(a.t, a.phase[4 * np + ir], a.phase[5 * np + ir], a.phase[6 * np + ir]);
         }
         s_k[i] = (float)k;
         s_r[i] = (float)r;
         for (int q = 0; q < zb; q++) {
-            const double z = fmin(0.0, -a.depth + a.dz * min(j0 + q, a.nz - 1));
+            const double z = fmin(0.0, -a.h + a.dz * min(j0 + q, a.nz - 1));
             // cosh(k(z+h))/cosh(kh) and sinh(k(z+h))/cosh(kh), both bounded by 1
             const double qn = 1.0 / (1.0 + exp(-2.0 * k * a.depth));
             const double E = exp(k * z), Y = exp(-k * (z + 2.0 * a.depth));
@@ -1381,15 +1815,18 @@ __global__ void __launch_bounds__(256) k_pressure_kin(KinArgs a) {
     float sK[KIN_ZB], cK[KIN_ZB], sD[KIN_ZB], cD[KIN_ZB];
 #pragma unroll
     for (int q = 0; q < KIN_ZB; q++) sK[q] = cK[q] = sD[q] = cD[q] = 0.f;
-    constexpr int TT = GRID_TILE;
+    const int TT = a.tt;
     int I = 0, M = 0;
     const long ntiles = tile_index(a.ntile - 1, a.ntile - 1, a.ntile) + 1;
     for (long t = 0; t < ntiles; t++) {
-        const float2 *tk = a.tabk + t * (long)TT * TT;
         for (int e = threadIdx.x; e < TT * TT; e += blockDim.x) {
-            const float2 c = tk[e];
-            if (c.x == 0.f && c.y == 0.f) continue;     // filtered pair or padding
+            const long g = t * (long)TT * TT + e;
             const int i = I * TT + e / TT, m = M * TT + e % TT;
+            float2 c;
+            if (!a.tpk) c = a.tabk[g];
+            else if (i == m) c = make_float2(a.cf[CF_X1 * np + i], a.cf[CF_Z1 * np + i]);
+            else c = make_float2(a.tpk[point_at(g, POINTK_NC, 0)], a.tpk[point_at(g, POINTK_NC, 1)]);
+            if (c.x == 0.f && c.y == 0.f) continue;     // filtered pair or padding
             const float ri = s_r[i], ki = s_k[i], km = s_k[m];
 #pragma unroll
             for (int q = 0; q < KIN_ZB; q++) {
@@ -1431,8 +1868,7 @@ __global__ void __launch_bounds__(256) k_pressure_kin(KinArgs a) {
     }
 }
 
-int launch_pressure_kin(const DevSea &sea, double t, int nz, double *kin, cudaStream_t stream) {
-    if (!sea.d_tab_gk || nz < 2) return E_NOT_INITIALIZED;
+static int pressure_kin(const DevSea &sea, double t, bool point, double h, int nz, double *kin, cudaStream_t stream) {
     const int np = sea.npad_g;
     // shared memory: k, ramp and zb rows of px, pz per component
     const size_t cap = 200 * 1024;
@@ -1445,26 +1881,93 @@ int launch_pressure_kin(const DevSea &sea, double t, int nz, double *kin, cudaSt
     CK(attr);
     KinArgs a;
     a.tabk = reinterpret_cast<const float2 *>(sea.d_tab_gk);
-    a.ntile = sea.ntile_g; a.ncomp = sea.n; a.npad = np; a.trivial_ramp = sea.trivial_ramp ? 1 : 0; a.zb = zb;
+    a.tt = point ? POINT_TILE : GRID_TILE; a.ntile = point ? sea.ntile_p : sea.ntile_g;
+    a.ncomp = sea.n; a.npad = np; a.trivial_ramp = sea.trivial_ramp ? 1 : 0; a.zb = zb;
     a.phase = sea.d_phase; a.cf = sea.d_cf;
-    a.t = t; a.depth = sea.depth; a.dz = sea.depth / (nz - 1); a.nz = nz; a.kin = kin;
+    a.t = t; a.depth = sea.depth; a.h = h; a.dz = h / (nz - 1); a.nz = nz; a.kin = kin;
+    a.tpk = point ? sea.d_tab_pk : nullptr;
     k_pressure_kin<<<(unsigned)((nz + zb - 1) / zb), 256, smem, stream>>>(a);
     note_launch();
     CK(cudaGetLastError());
     return OK;
 }
 
+int launch_pressure_kin(const DevSea &sea, double t, int nz, double *kin, cudaStream_t stream) {
+    if (!sea.d_tab_gk || nz < 2) return E_NOT_INITIALIZED;
+    return pressure_kin(sea, t, false, sea.depth, nz, kin, stream);
+}
+
+// The height table of the point API's phase-free pressure terms, built with
+// the sea where every component has the same ramp (which then multiplies the
+// whole sum): over [-h - max(0, swl), 0], the heights that the seabed clamp
+// leaves.  The finest wavenumber is 2 kmax; at 2 kmax dz = 0.014 the Hermite
+// interpolation's error is (2 kmax dz)^4 / 384 = 1e-10 of a term.  A sea too
+// deep for 16385 heights or with too many components for the kernel has no
+// table; its products are summed per point.
+static int point_kin_build(DevSea &sea, cudaStream_t stream) {
+    const double h = sea.depth + std::max(0.0, sea.swl);
+    const double want = 2.0 * sea.kmax * h / 0.014 + 1.0;
+    if (!sea.trivial_ramp || sea.n < 1 || !(h > 0.0) || !(want <= 16385.0)) return OK;
+    const int nz = std::max(2049, (int)std::ceil(want));
+    CK(cudaMalloc(&sea.d_kin, sizeof(double) * 2 * nz));
+    const int rc = pressure_kin(sea, 0.0, true, h, nz, sea.d_kin, stream);
+    if (rc) {
+        cudaFree(sea.d_kin);
+        sea.d_kin = nullptr;
+        return rc == E_TOO_LARGE ? OK : rc;
+    }
+    sea.kin_nz = nz;
+    sea.kin_h = h;
+    return OK;
+}
+
+// One group of rows (velocity or pressure): the tile-pair walk split into
+// slices where the points alone do not fill whole waves of the resident
+// blocks, the slices summed in order into out.
+template <bool VEL, bool PR, bool KIN>
+static int point_pairs_t(PairArgs a, long n, int ntp, float *out, float *split_buf, long split_cap,
+                         cudaStream_t stream) {
+    using ST = PointStage<VEL, PR, KIN>;
+    // set and queried once per process (thread-safe static initialisation)
+    static const cudaError_t attr = cudaFuncSetAttribute(k_pairs_points<VEL, PR, KIN>,
+                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, ST::SMEM);
+    CK(attr);
+    static const long slots = [] {
+        const long v = resident_slots(k_pairs_points<VEL, PR, KIN>, 128, ST::SMEM);
+        return v > 0 ? v : SPLIT_TARGET_BLOCKS;
+    }();
+    const long nblk = (n + 127) / 128;
+    a.tp_per = slice_plan(nblk, ntp, slots, split_buf ? split_cap / (ST::ROWS * n) : 1);
+    const int nslice = (ntp + a.tp_per - 1) / a.tp_per;
+    a.out = nslice > 1 ? split_buf : out;
+    prof_begin(PK_POINT_PAIRS, stream);
+    k_pairs_points<VEL, PR, KIN><<<dim3((unsigned)nblk, (unsigned)nslice), 128, ST::SMEM, stream>>>(a);
+    note_launch();
+    prof_end(PK_POINT_PAIRS, stream);
+    CK(cudaGetLastError());
+    if (nslice > 1) {
+        const long m = ST::ROWS * n;
+        k_sum_slices<<<(unsigned)((m + 255) / 256), 256, 0, stream>>>(m, nslice, split_buf, out);
+        note_launch();
+        CK(cudaGetLastError());
+    }
+    return OK;
+}
+
+// Rows u, v, w (mask bits 2, 4, 8) and p (16) of out [4][n]; rows not asked
+// for are not written.  kin: the pressure's phase-free products summed here.
 static int launch_point_pairs(const DevSea &sea, long n, const float2 *ph, const float *rr,
-                              const float *z0, float *out, int pairs, int mask, cudaStream_t stream,
+                              const float *z0, float *out, int pairs, int mask, bool kin, cudaStream_t stream,
                               float *split_buf, long split_cap) {
     PairArgs a{};
     a.ncol = n; a.nl = 1; a.nlg = 1; a.ntile = sea.ntile_p; a.tab = sea.d_tab_point;
-    a.ph = ph; a.rr = rr; a.cf = sea.d_cf; a.cstride = sea.npad_g; a.z0 = z0;
-    a.depth = (float)sea.depth; a.out = out; a.pairs = pairs; a.first = 1;
-    // few points: the tile-pair loop split over blockIdx.y, slices summed in order
+    a.tpp = reinterpret_cast<const float4 *>(sea.d_tab_pp);
+    a.tpk = reinterpret_cast<const float4 *>(sea.d_tab_pk);
+    a.ph = ph; a.rr = rr; a.rs = sea.trivial_ramp ? 0 : n; a.cf = sea.d_cf; a.cstride = sea.npad_g; a.z0 = z0;
+    a.depth = (float)sea.depth; a.pairs = pairs; a.first = 1; a.kin = kin ? 1 : 0; a.one = 1.f;
     const int ntp = pairs ? sea.ntile_p * (sea.ntile_p + 1) / 2 : sea.ntile_p;
     if (n <= FEW_POINTS && split_buf) {
-        // a block per (point, slice), the rows of 8 tile pairs over its threads
+        // a block per (point, slice), the rows of PER tile pairs over its threads
         constexpr int PER = 128 / POINT_TILE;
         const int npass = (ntp + PER - 1) / PER;
         int nslice = (int)std::min<long>(npass, std::max<long>(1, split_cap / (4L * n)));
@@ -1480,52 +1983,12 @@ static int launch_point_pairs(const DevSea &sea, long n, const float2 *ph, const
         CK(cudaGetLastError());
         return OK;
     }
-    const size_t smem = sizeof(float) * POINT_TILE * POINT_TILE * POINTV_NC + 2 * sizeof(float2) * POINT_TILE * 128;
-    // the same shared memory in every variant: resident blocks once per process
-    static const long slots = [&] {
-        cudaFuncSetAttribute(k_pairs_points<POINT_TILE, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-        const long v = resident_slots(k_pairs_points<POINT_TILE, true, true>, 128, smem);
-        return v > 0 ? v : SPLIT_TARGET_BLOCKS;
-    }();
-    const long nblk = (n + 127) / 128;
-    int nslice = wave_slices(nblk, ntp, slots, split_buf ? split_cap / (4L * n) : 1);
-    a.tp_per = (ntp + nslice - 1) / nslice;
-    nslice = (ntp + a.tp_per - 1) / a.tp_per;
-    if (nslice > 1) a.out = split_buf;
-    // set once per process (thread-safe static initialisation)
-    static const cudaError_t attr = [&] {
-        cudaError_t e = cudaFuncSetAttribute(k_pairs_points<POINT_TILE, true, true>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_pairs_points<POINT_TILE, true, false>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_pairs_points<POINT_TILE, false, true>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        return e;
-    }();
-    CK(attr);
-    // the velocity sums only where u, v or w is asked for, the pressure sums
-    // only where dp is
-    const bool vel = (mask & 14) != 0, pr = (mask & 16) != 0;
-    const dim3 grid((unsigned)((n + 127) / 128), (unsigned)nslice);
-    prof_begin(PK_POINT_PAIRS, stream);
-    if (vel && pr)
-        k_pairs_points<POINT_TILE, true, true><<<grid, 128, smem, stream>>>(a);
-    else if (vel)
-        k_pairs_points<POINT_TILE, true, false><<<grid, 128, smem, stream>>>(a);
-    else
-        k_pairs_points<POINT_TILE, false, true><<<grid, 128, smem, stream>>>(a);
-    note_launch();
-    prof_end(PK_POINT_PAIRS, stream);
-    CK(cudaGetLastError());
-    if (nslice > 1) {
-        k_sum_slices<<<(unsigned)((4 * n + 255) / 256), 256, 0, stream>>>(4 * n, nslice, split_buf, out);
-        note_launch();
-        CK(cudaGetLastError());
-    }
-    return OK;
+    int rc = OK;
+    if (mask & 14) rc = point_pairs_t<true, false, false>(a, n, ntp, out, split_buf, split_cap, stream);
+    if (rc == OK && (mask & 16))
+        rc = kin && pairs ? point_pairs_t<false, true, true>(a, n, ntp, out + 3 * n, split_buf, split_cap, stream)
+                          : point_pairs_t<false, true, false>(a, n, ntp, out + 3 * n, split_buf, split_cap, stream);
+    return rc;
 }
 
 // Phasor layout used by the pair kernels: the point kernel reads tiles of
@@ -1537,16 +2000,22 @@ int irregular_eval(const DevSea &sea, long n, const double *x, const double *y, 
     if (n <= 0) return OK;
     const long chunk = 1L << 18;
     const int npad = sea.npad_g;
+    // the phase-free part of the pressure from the height table: the wave_*
+    // calls clamp z to the range it covers
+    const bool table = api && sea.d_kin && sea.order == 2;
     WsLayout L0 = layout(std::min(n, chunk), npad, nullptr);
     int rc = workspace_reserve(ws, L0.bytes);
     if (rc) return rc;
     for (long b = 0; b < n; b += chunk) {
         long m = std::min(chunk, n - b);
         WsLayout L = layout(m, npad, ws.base);
-        rc = launch_phasors(sea, m, x + b, y + b, t + b, 1, 1, 1, npad, L.ph, L.rr, L.first, stream);
-        if (rc) return rc;
         // vertical_theory smit: u, v, w, dp need eta at the point first
         const bool smit = sea.smit && (mask & 30);
+        // the first-order sums behind the rows asked for (the mask's bits are
+        // those of first)
+        rc = launch_phasors(sea, m, x + b, y + b, t + b, 1, 1, 1, npad, L.ph, L.rr, L.first, stream,
+                            smit ? 1 : mask & 31);
+        if (rc) return rc;
         float *eta2 = nullptr;
         if (((mask & 1) || smit) && sea.order == 2) {
             eta2 = L.sec + 4 * m;
@@ -1564,7 +2033,7 @@ int irregular_eval(const DevSea &sea, long n, const double *x, const double *y, 
             CK(cudaGetLastError());
             // the point table is padded to POINT_TILE; the phasor rows beyond
             // npad_p are never read by the point kernel
-            rc = launch_point_pairs(sea, m, L.ph, L.rr, L.z0, L.sec, sea.order != 0 ? 1 : 0, mask, stream,
+            rc = launch_point_pairs(sea, m, L.ph, L.rr, L.z0, L.sec, sea.order != 0 ? 1 : 0, mask, !table, stream,
                                     L.split, L.split_cap);
             if (rc) return rc;
         }
@@ -1577,7 +2046,9 @@ int irregular_eval(const DevSea &sea, long n, const double *x, const double *y, 
         }
         k_combine<<<(unsigned)((m + 255) / 256), 256, 0, stream>>>(m, n, sea.order, sea.swl, z + b,
                                                                    L.first, L.sec, eta2, smit ? (mask & 1) : mask,
-                                                                   out ? out + b : nullptr, ar);
+                                                                   out ? out + b : nullptr, ar,
+                                                                   KinTab{table && !smit ? sea.d_kin : nullptr,
+                                                                          sea.kin_nz, sea.kin_h, sea.depth, L.rr});
         note_launch();
         CK(cudaGetLastError());
     }

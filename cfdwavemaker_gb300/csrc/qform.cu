@@ -393,7 +393,8 @@ struct QPlain {
     int ntile;
     const float *tab;        // plain tiles
     const float2 *ph;        // [npad][rows] (c, s)
-    const float *rr;         // [npad][rows]
+    const float *rr;         // ramps, row stride rs (0 where every component has the same ramp)
+    long rs;
     int nseg;                // segments of the tile walk (units per row block)
     int mb[QPL_MAXSEG + 1];  // segment g walks the column tiles M in [mb[g], mb[g + 1])
     float *part;             // [nseg][rows][4]: each segment's sums
@@ -465,13 +466,15 @@ __global__ void __launch_bounds__(128, 2) k_qform_plain(QPlain a) {
         // ones past the tile re-read its last component)
         const long rbase = (long)(I * QT) * a.rows;
         float2 pa0 = a.ph[rbase + q0], pa1 = a.ph[rbase + q1];
-        float ra0 = a.rr[rbase + q0], ra1 = a.rr[rbase + q1];
+        const long rr0 = (long)(I * QT) * a.rs;
+        float ra0 = a.rr[rr0 + q0], ra1 = a.rr[rr0 + q1];
         float2 pb0 = a.ph[rbase + a.rows + q0], pb1 = a.ph[rbase + a.rows + q1];
-        float rb0 = a.rr[rbase + a.rows + q0], rb1 = a.rr[rbase + a.rows + q1];
+        float rb0 = a.rr[rr0 + a.rs + q0], rb1 = a.rr[rr0 + a.rs + q1];
         for (int ii = 0; ii < QT; ii++) {
             const long rn = rbase + (long)(ii + 2 < QT ? ii + 2 : QT - 1) * a.rows;
             const float2 n0 = a.ph[rn + q0], n1 = a.ph[rn + q1];
-            const float nr0 = a.rr[rn + q0], nr1 = a.rr[rn + q1];
+            const long rrn = rr0 + (long)(ii + 2 < QT ? ii + 2 : QT - 1) * a.rs;
+            const float nr0 = a.rr[rrn + q0], nr1 = a.rr[rrn + q1];
             // (A_cos, A_sin) of each field times (c_m, s_m): the record's
             // float pairs and the phasor are the two lanes of each FFMA2
             float2 e0 = {0, 0}, u0 = {0, 0}, v0 = {0, 0}, w0 = {0, 0};
@@ -1489,7 +1492,7 @@ int qform_eval(const DevSea &sea, long n, const double *x, const double *y, cons
             if (fill > best + 1e-9) { best = fill; nseg = g; }
         }
         QPlain q;
-        q.rows = mm; q.ntile = nt; q.tab = g_q.plain_tab; q.ph = ph; q.rr = rr; q.part = part;
+        q.rows = mm; q.ntile = nt; q.tab = g_q.plain_tab; q.ph = ph; q.rr = rr; q.rs = sea.trivial_ramp ? 0 : mm; q.part = part;
         q.nseg = nseg;
         const long total = (long)nt * (nt + 1) / 2;
         q.mb[0] = 0;

@@ -178,7 +178,8 @@ struct SmitArgs {
     int ntile, cstride;
     const float *tab;
     const float2 *ph;          // [npad][n] phasors of the point phases
-    const float *rr;           // [npad][n] ramps
+    const float *rr;           // ramps, row stride rs (0 where every component has the same ramp)
+    long rs;
     const float *cf;           // [NCF][cstride]
     const double *phase;       // [7][cstride]: omega in row 2
     const float *zs, *sp1, *chain, *above;
@@ -236,14 +237,14 @@ __global__ void __launch_bounds__(128) k_smit_points(SmitArgs a) {
                 const float q = a.cf[CF_Q * a.cstride + m];
                 s_ph[mm * 128 + threadIdx.x] = a.ph[(long)m * a.n + pc];
                 s_pf[mm * 128 + threadIdx.x] = make_float2(q * F, q * G);
-                s_r[mm * 128 + threadIdx.x] = a.rr[(long)m * a.n + pc];
+                s_r[mm * 128 + threadIdx.x] = a.rr[(long)m * a.rs + pc];
             }
             __syncthreads();
             if (!valid) continue;
             for (int ii = 0; ii < TT; ii++) {
                 const int i = I * TT + ii;
                 const float2 pi = a.ph[(long)i * a.n + p];
-                const float ri = a.rr[(long)i * a.n + p];
+                const float ri = a.rr[(long)i * a.rs + p];
                 float2 pfi;
                 if (M == I) {
                     pfi = s_pf[ii * 128 + threadIdx.x];
@@ -366,7 +367,7 @@ __global__ void __launch_bounds__(128) k_smit_points_few(SmitArgs a, int ntp, in
         const int M = I + tp;
         const int i = I * TT + ii;
         const float2 pi = a.ph[(long)i * a.n + p];
-        const float ri = a.rr[(long)i * a.n + p];
+        const float ri = a.rr[(long)i * a.rs + p];
         float F, G;
         sfg(a.cf[CF_K * a.cstride + i], zk, zetak, F, G);
         const float qi = a.cf[CF_Q * a.cstride + i];
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(128) k_smit_points_few(SmitArgs a, int ntp, in
             const float4 c2 = *reinterpret_cast<const float4 *>(rec + 8);
             const float4 c3 = *reinterpret_cast<const float4 *>(rec + 12);
             const float2 pm = a.ph[(long)m * a.n + p];
-            const float rm = a.rr[(long)m * a.n + p];
+            const float rm = a.rr[(long)m * a.rs + p];
             const float km = a.cf[CF_K * a.cstride + m], am = a.cf[CF_KW * a.cstride + m];
             float Fm_, Gm_;
             sfg(km, zk, zetak, Fm_, Gm_);
@@ -492,7 +493,7 @@ int smit_eval(const DevSea &sea, long n, const double *z, const void *ph, const 
     CK(cudaGetLastError());
     SmitArgs a;
     a.n = n; a.ntile = sea.ntile_s; a.cstride = sea.npad_g; a.tab = sea.d_tab_smit;
-    a.ph = static_cast<const float2 *>(ph); a.rr = rr; a.cf = sea.d_cf; a.phase = sea.d_phase;
+    a.ph = static_cast<const float2 *>(ph); a.rr = rr; a.rs = sea.trivial_ramp ? 0 : n; a.cf = sea.d_cf; a.phase = sea.d_phase;
     a.zs = zs; a.sp1 = sp1; a.chain = chain; a.above = above;
     a.depth = (float)sea.depth; a.ldo = ldo; a.out = out;
     const int ntp = sea.ntile_s * (sea.ntile_s + 1) / 2;
