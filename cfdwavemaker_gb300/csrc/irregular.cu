@@ -63,16 +63,26 @@ constexpr int POINTV_NC = 8, POINTP_NC = 4, POINTK_NC = 2;
 __host__ __device__ inline long point_at(long entry, int nc, int q) { return ((entry / 2) * nc + q) * 2 + (entry & 1); }
 constexpr float LOG2E_F = 1.4426950408889634f;
 constexpr long SPLIT_TARGET_BLOCKS = 4 * 152;   // blocks a column-pair launch aims for
-// batches of at most this many points take the few-point kernels (a block
-// per point, the components or pair rows over its threads).  Measured on the
-// 128-component point sea, a velocity and an elevation batch: at 256 points
-// 133 us against 191 us with the per-thread kernels, at 512 166 against 187,
-// at 1024 226 against 196.
-constexpr long FEW_POINTS = 512;
-// the phasors alone: the few-point kernel up to 1024 points (a velocity and
-// an elevation batch of 1024 points 159 us against 193 us; 2048 points 210
-// against 205)
-constexpr long PH_FEW_POINTS = 1024;
+// Batches that the one-kernel evaluation (k_point_few) takes: 20 points, where
+// the per-thread kernels' blocks of 128 are nearly empty, and as many more as
+// 4e6 (pair, point) terms are, where its terms, read per point, cost less than
+// the per-thread path's eight dependent kernels.  Measured, a wave_Kinematics
+// and a pressure batch from host arrays, this kernel against the per-thread
+// ones: 24 components, 1024 points 82 and 150 us; 128 components, 256 points 100
+// and 127, 512 points 144 and 130; 256 components, 64 points 105 and 129, 128
+// points 140 and 130; 384 components, 64 points 144 and 149; 4096 components,
+// 16 points 1.9 and 2.2 ms, 64 points 7.3 and 2.2.
+constexpr long FEW_MAX_POINTS = 4096;
+constexpr size_t CNT_BYTES = sizeof(unsigned) * FEW_MAX_POINTS;
+constexpr int FEW_MAX_NPAD = 4096;   // components whose phasors, profiles and ramps fit shared memory
+static bool few_points(long n, int npad) {
+    return npad <= FEW_MAX_NPAD && n <= FEW_MAX_POINTS &&
+           (double)n <= 20.0 + 4e6 / (0.5 * npad * (npad + 1));
+}
+// the phasors alone (the Smit theory's short batches): a block per point up to
+// 300 points (120 components, a velocity and a pressure batch of 200 points 243
+// us against 257 with the limit at 1024, of 1000 points 307 against 368)
+constexpr long PH_FEW_POINTS = 300;
 
 __device__ __forceinline__ float ex2(float x) {
     float y;
@@ -586,6 +596,34 @@ __device__ __forceinline__ void ph_sincos(f32x2 hi, f32x2 lo, f32x2 &s, f32x2 &c
     c = p_pack(c0, c1);
 }
 
+// A point's offsets and time as duplicated packed operands
+struct PhPoint {
+    f32x2 xh, xl, nxh, yh, yl, nyh, th, tl, nth;
+    __device__ __forceinline__ PhPoint(float2 dx, float2 dy, float2 t)
+        : xh(p_pack(dx.x, dx.x)), xl(p_pack(dx.y, dx.y)), nxh(p_pack(-dx.x, -dx.x)), yh(p_pack(dy.x, dy.x)),
+          yl(p_pack(dy.y, dy.y)), nyh(p_pack(-dy.x, -dy.x)), th(p_pack(t.x, t.x)), tl(p_pack(t.y, t.y)),
+          nth(p_pack(-t.x, -t.x)) {}
+};
+
+// The phases kx x + ky y - omega t + phase0 of two components (records R) as
+// pairs (hi, lo): each product exact, the sums error-free in the hi parts.
+__device__ __forceinline__ void ph_phase(const ulonglong2 *R, const PhPoint &P, f32x2 &hi, f32x2 &lo) {
+    const f32x2 neg1 = p_pack(-1.f, -1.f);
+    const ulonglong2 kx = R[0], ky = R[1], w = R[2], p0 = R[3];
+    hi = p_mul(kx.x, P.xh);
+    lo = p_fma(kx.x, P.xl, p_fma(kx.y, P.xh, p_fma(kx.x, P.xh, p_mul(kx.x, P.nxh))));
+    auto add = [&](f32x2 h, f32x2 l) {
+        const f32x2 s = p_add(hi, h), bb = p_fma(hi, neg1, s);
+        const f32x2 d = p_fma(bb, neg1, s);
+        const f32x2 e = p_add(p_fma(d, neg1, hi), p_fma(bb, neg1, h));
+        hi = s;
+        lo = p_add(p_add(lo, l), e);
+    };
+    add(p_mul(ky.x, P.yh), p_fma(ky.x, P.yl, p_fma(ky.y, P.yh, p_fma(ky.x, P.yh, p_mul(ky.x, P.nyh)))));
+    add(p_mul(w.x, P.th), p_fma(w.x, P.tl, p_fma(w.y, P.th, p_fma(w.x, P.th, p_mul(w.x, P.nth)))));
+    add(p0.x, p0.y);
+}
+
 // The phasors (cos, sin) and ramps of every component and the first-order
 // sums eta1 and the Taylor gradients.  The phase
 // kx (x - fx) + ky (y - fy) - omega t + phase0 is formed in float-float from
@@ -637,8 +675,7 @@ __global__ void __launch_bounds__(32 * PH_WARPS) k_phasors(PhArgs a) {
     // instruction issue is the bound
     const f32x2 neg1 = p_pack(-1.f, -1.f);
     auto dup = [](float v) { return p_pack(v, v); };
-    const f32x2 xh = dup(dx.x), xl = dup(dx.y), nxh = dup(-dx.x), yh = dup(dy.x), yl = dup(dy.y), nyh = dup(-dy.x);
-    const f32x2 th = dup(tt.x), tl = dup(tt.y), nth = dup(-tt.x);
+    const PhPoint pt(dx, dy, tt);
     f32x2 S[5] = {0, 0, 0, 0, 0}, C[5] = {0, 0, 0, 0, 0};
     for (int i0 = 0; i0 < a.npad; i0 += PH_CHUNK) {
         const int nrec = min(PH_CHUNK, a.npad - i0);
@@ -649,21 +686,8 @@ __global__ void __launch_bounds__(32 * PH_WARPS) k_phasors(PhArgs a) {
         for (int ii = 2 * warp; ii < nrec; ii += 2 * PH_WARPS) {
             const int i = i0 + ii;
             const ulonglong2 *R = reinterpret_cast<const ulonglong2 *>(s_rec + ii * PH_REC);
-            const ulonglong2 kx = R[0], ky = R[1], w = R[2], p0 = R[3];
-            // phase = kx x + ky y - omega t + phase0 as a pair (hi, lo): each
-            // product exact, the sums error-free in the hi parts
-            f32x2 hi = p_mul(kx.x, xh);
-            f32x2 lo = p_fma(kx.x, xl, p_fma(kx.y, xh, p_fma(kx.x, xh, p_mul(kx.x, nxh))));
-            auto add = [&](f32x2 h, f32x2 l) {
-                const f32x2 s = p_add(hi, h), bb = p_fma(hi, neg1, s);
-                const f32x2 d = p_fma(bb, neg1, s);
-                const f32x2 e = p_add(p_fma(d, neg1, hi), p_fma(bb, neg1, h));
-                hi = s;
-                lo = p_add(p_add(lo, l), e);
-            };
-            add(p_mul(ky.x, yh), p_fma(ky.x, yl, p_fma(ky.y, yh, p_fma(ky.x, yh, p_mul(ky.x, nyh)))));
-            add(p_mul(w.x, th), p_fma(w.x, tl, p_fma(w.y, th, p_fma(w.x, th, p_mul(w.x, nth)))));
-            add(p0.x, p0.y);
+            f32x2 hi, lo;
+            ph_phase(R, pt, hi, lo);
             f32x2 c2, s2;
             ph_sincos(hi, lo, s2, c2);
             const float2 c = p_un(c2), s = p_un(s2);
@@ -794,7 +818,6 @@ struct PairArgs {
     const float4 *tpp;   // point kernel: pressure tiles (Pp, Mp, kp, km)
     const float4 *tpk;   // and the phase-free products (X, Z)
     float one;           // 1 (p_hold)
-    int kin;             // few-point kernel: sum them (else the height table holds their sum)
     const float2 *ph;    // [npad][ncol]
     const float *rr;     // ramps: row stride rs (0 where every component has the same ramp)
     long rs;
@@ -1237,108 +1260,6 @@ __global__ void __launch_bounds__(128, KIN ? 2 : 6) k_pairs_points(PairArgs a) {
     }
 }
 
-// Few points, point mode: block (point p, slice y); thread t takes row
-// ii = t % TT of tile pair 8 g + t / TT for g = y, y + nslice, ... (TT = 16: 8
-// tile pairs a pass).  A row is summed over its mm as in k_pairs_points (the
-// depth factors of component m formed per term here, since no other point
-// shares them), diagonal tile pairs add the first-order term of component
-// I TT + ii, each thread's rows are Kahan-summed, and the block's 128 sums
-// are added in FP32 into slice y's partial sums ([nslice][4][n], summed in
-// order by k_sum_slices).
-template <int TT>
-__global__ void __launch_bounds__(128) k_pairs_points_few(PairArgs a, int ntp, int nslice) {
-    __shared__ float s_red[4][4];
-    const long p = blockIdx.x;
-    const float z = a.z0[p];
-    const float zk = z * LOG2E_F, zetak = -2.f * (z + a.depth) * LOG2E_F;
-    const int ii = threadIdx.x % TT;
-    constexpr int PER = 128 / TT;           // tile pairs a pass
-    float su = 0, cu = 0, sv = 0, cv = 0, sw = 0, cw = 0, sq = 0, cq = 0;
-    for (int g = blockIdx.y; g * PER < ntp; g += nslice) {
-        int tp = g * PER + threadIdx.x / TT;
-        if (tp >= ntp) continue;
-        int I = 0, M = 0;
-        if (a.pairs) {
-            while (tp >= a.ntile - I) { tp -= a.ntile - I; I++; }
-            M = I + tp;
-        } else {
-            I = M = tp;
-        }
-        const int i = I * TT + ii;
-        const float2 pi = a.ph[(long)i * a.ncol + p];
-        const float ri = a.rr[(long)i * a.rs + p];
-        float Fi, Gi;
-        depth_fg(a.cf[CF_K * a.cstride + i], zk, zetak, Fi, Gi);
-        const float qi = a.cf[CF_Q * a.cstride + i];
-        const float2 pxz_i = make_float2(qi * Fi, qi * Gi);
-        if (a.pairs) {
-            const long e0 = tile_index(I, M, a.ntile) * (long)TT * TT;
-            const float *TV = a.tab, *TP = reinterpret_cast<const float *>(a.tpp), *TK = reinterpret_cast<const float *>(a.tpk);
-            float au = 0, av = 0, aw = 0, ap = 0, ax = 0, az = 0;
-            for (int mm = (M == I) ? ii : 0; mm < TT; mm++) {
-                const int m = M * TT + mm;
-                const long e = e0 + ii * TT + mm;
-                float c[POINTV_NC], cq_[POINTP_NC], x2[POINTK_NC];
-#pragma unroll
-                for (int q = 0; q < POINTV_NC; q++) c[q] = TV[point_at(e, POINTV_NC, q)];
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    cq_[q] = TP[point_at(e, POINTP_NC, q)];
-                    x2[q] = TK[point_at(e, POINTK_NC, q)];
-                }
-                const float2 pm = a.ph[(long)m * a.ncol + p];
-                float Fm_, Gm_;
-                depth_fg(a.cf[CF_K * a.cstride + m], zk, zetak, Fm_, Gm_);
-                const float qm = a.cf[CF_Q * a.cstride + m];
-                const float2 xm = make_float2(qm * Fm_, qm * Gm_);
-                const float cc = pi.x * pm.x, ss = pi.y * pm.y;
-                const float sc = pi.y * pm.x, cs = pi.x * pm.y;
-                const float cp = cc - ss, cmn = cc + ss, sp = sc + cs, smn = sc - cs;
-                float Fp, Gp, Fm, Gm;
-                depth_fg(c[6], zk, zetak, Fp, Gp);
-                depth_fg(c[7], zk, zetak, Fm, Gm);
-                const float A = cp * Fp, B = cmn * Fm, Cq = sp * Gp, D = smn * Gm;
-                au = fmaf(c[0], A, fmaf(c[1], B, au));
-                av = fmaf(c[2], A, fmaf(c[3], B, av));
-                aw = fmaf(c[4], Cq, fmaf(c[5], D, aw));
-                ap = fmaf(cq_[0], A, fmaf(cq_[1], B, ap));
-                if (a.kin) {
-                    ax = fmaf(x2[0], xm.x, ax);
-                    az = fmaf(x2[1], xm.y, az);
-                }
-            }
-            ap = fmaf(pxz_i.x, ax, fmaf(pxz_i.y, az, ap));
-            kahan(su, cu, ri * au);
-            kahan(sv, cv, ri * av);
-            kahan(sw, cw, ri * aw);
-            kahan(sq, cq, ri * ap);
-        }
-        if (a.first && M == I) {
-            // first-order u1, v1, w1, dp1 and the linear dp2 diagonal terms of component i
-            const float au_ = a.cf[CF_AU * a.cstride + i] * ri;
-            kahan(su, cu, au_ * pxz_i.x * a.cf[CF_CT * a.cstride + i] * pi.x);
-            kahan(sv, cv, au_ * pxz_i.x * a.cf[CF_ST * a.cstride + i] * pi.x);
-            kahan(sw, cw, au_ * pxz_i.y * pi.y);
-            float pp = a.cf[CF_AP * a.cstride + i] * pxz_i.x * pi.x;
-            if (a.pairs && a.kin)
-                pp += a.cf[CF_X1 * a.cstride + i] * pxz_i.x + a.cf[CF_Z1 * a.cstride + i] * pxz_i.y;
-            kahan(sq, cq, ri * pp);
-        }
-    }
-    float v[4] = {su - cu, sv - cv, sw - cw, sq - cq};
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-        for (int o = 16; o > 0; o >>= 1) v[f] += __shfl_down_sync(0xffffffffu, v[f], o);
-        if (lane == 0) s_red[warp][f] = v[f];
-    }
-    __syncthreads();
-    if (threadIdx.x < 4) {
-        const int f = threadIdx.x;
-        a.out[((long)blockIdx.y * 4 + f) * a.ncol + p] = ((s_red[0][f] + s_red[1][f]) + s_red[2][f]) + s_red[3][f];
-    }
-}
-
 // Elevation mode: eta2 from the pair cache (Irregular.cpp:223-293).  The
 // record holds A = P+M and B = M-P so that a pair contributes
 // c_i (A c_m) + s_i (B s_m); a row is c_i sum(A c_m) + s_i sum(B s_m).
@@ -1497,6 +1418,7 @@ struct WsLayout {
     double *first;
     float *z0;
     float *sec;
+    unsigned *cnt;        // the few-point kernel's counters: first, so that every layout has them there
     float *split;         // partial sums of a split point-pair launch
     long split_cap;       // its floats
     size_t bytes;
@@ -1552,6 +1474,7 @@ WsLayout layout(long n, int npad, void *base) {
     WsLayout L;
     size_t off = 0;
     auto take = [&](size_t b) { size_t o = off; off += (b + 255) & ~size_t(255); return o; };
+    const size_t o_cnt = take(CNT_BYTES);
     size_t o_ph = take(sizeof(float2) * (size_t)npad * n);
     size_t o_rr = take(sizeof(float) * (size_t)npad * n);
     size_t o_first = take(sizeof(double) * 5 * (size_t)n);
@@ -1560,6 +1483,7 @@ WsLayout layout(long n, int npad, void *base) {
     const long scap = point_split_floats(n);
     size_t o_split = take(sizeof(float) * (size_t)std::max<long>(scap, 1));
     char *b = (char *)base;
+    L.cnt = (unsigned *)(b + o_cnt);
     L.ph = (float2 *)(b + o_ph);
     L.rr = (float *)(b + o_rr);
     L.first = (double *)(b + o_first);
@@ -1627,6 +1551,254 @@ __global__ void k_combine(long n, long ldo, int order, double swl, const double 
     }
     v[5] = v[4] - api.rho * api.g * v[0];
     api_store(api, p, v);
+}
+
+// ---------------------------------------------------------------------------
+// Few points (a scalar call, a short batch): the whole evaluation in one
+// kernel.  Block (point, slice): every block forms the point's phasors in
+// shared memory (two components a thread at once), then its threads take items
+// of the sums in turn -- eight terms of a row of a tile pair of the velocity,
+// pressure or elevation tables, and the first-order terms of a component --
+// and the block's sums go to its slice's partial sums.  The last block of a
+// point to finish (a counter per point that wraps to 0) adds the slices in a
+// fixed order, assembles eta, u, v, w, dp and writes the rows.  What bounds a
+// call is latency: as separate kernels (phasors, heights, elevation and point
+// pairs, slice sums, combining pass) a wave_VeloX call of the 128-component sea
+// was five dependent kernels, 26 us; 17 us now (a launch and a synchronisation are
+// 8 of these).
+// ---------------------------------------------------------------------------
+constexpr int FEW_T = 128;           // threads of a block
+constexpr int FEW_Q = 10;            // sums: eta2, u, v, w, dp, then eta1, gx, gy, gz, gp
+constexpr int FEW_E = 8;             // terms of an item
+struct FewArgs {
+    long n, ldo;
+    const double *x, *y, *z, *t;
+    double fx, fy, swl, depth;
+    int ncomp, npad, cstride, trivial_ramp, order, clamp, kin, mask;
+    const float *rec, *cf;
+    const double *phase;
+    int ntp, ntg;                    // point and grid table tiles per side
+    const float *tabv, *tpp, *tpk, *tabe;
+    long nv, np, ne;                 // items of the velocity, pressure and elevation sums
+    float *part;                     // [slices][FEW_Q][n]
+    unsigned *cnt;                   // [n], zero before and after
+    double *out;
+    ApiRows api;
+    KinTab kt;
+};
+
+// (I, M) of tile t of an upper triangle of nt x nt tiles
+__device__ __forceinline__ void tile_at(long t, int nt, int &I, int &M) {
+    const float b = 2.f * nt + 1.f;
+    I = min(nt - 1, max(0, (int)((b - sqrtf(fmaxf(0.f, b * b - 8.f * (float)t))) * 0.5f)));
+    while (I > 0 && tile_index(I, I, nt) > t) I--;
+    while (I + 1 < nt && tile_index(I + 1, I + 1, nt) <= t) I++;
+    M = I + (int)(t - tile_index(I, I, nt));
+}
+
+__global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
+    extern __shared__ float2 s_few[];
+    float2 *s_ph = s_few;                                   // phasors [npad]
+    float2 *s_px = s_ph + a.npad;                           // kin: profiles px, pz [npad]
+    float *s_r = reinterpret_cast<float *>(s_px + (a.kin ? a.npad : 0));   // ramps [npad] (individual ramps)
+    __shared__ float s_red[FEW_T / 32][FEW_Q];
+    __shared__ float s_sum[FEW_Q];
+    __shared__ float s_ramp;
+    __shared__ int s_last;
+    const int tid = threadIdx.x;
+    const long p = blockIdx.x;
+    const int ns = gridDim.y, slice = blockIdx.y;
+    const double xp = a.x[p], yp = a.y[p], zp = a.z[p], tp = a.t[p];
+    const double *P = a.phase;
+    const int cs = a.cstride;
+    const double zz = (a.clamp ? fmax(-a.depth, zp) : zp) - a.swl;
+    const float z = (float)(a.order == 0 ? zz : fmin(0.0, zz)), h = (float)a.depth;
+    const float zk = z * LOG2E_F, yk = -(z + 2.f * h) * LOG2E_F;
+    // cosh(k(z+h))/cosh(kh), sinh(k(z+h))/cosh(kh) of component i
+    auto profile = [&](int i) {
+        const float k = a.cf[CF_K * cs + i], q = a.cf[CF_Q * cs + i];
+        const float E = ex2(k * zk), Y = ex2(k * yk);
+        return make_float2(q * (E + Y), q * (E - Y));
+    };
+    if (a.trivial_ramp) {
+        if (tid == FEW_T - 1) s_ramp = (float)d_freq_ramp(tp, P[4 * cs], P[5 * cs], P[6 * cs]);
+    } else {
+        for (int i = tid; i < a.npad; i += FEW_T)
+            s_r[i] = i < a.ncomp ? (float)d_freq_ramp(tp, P[4 * cs + i], P[5 * cs + i], P[6 * cs + i]) : 0.f;
+    }
+    {
+        float2 ox, oy;
+        ff_split(-a.fx, ox.x, ox.y);
+        ff_split(-a.fy, oy.x, oy.y);
+        const PhPoint pt(ff_add(ff_from_double(xp), ox), ff_add(ff_from_double(yp), oy), ff_from_double(tp));
+        for (int i = 2 * tid; i < a.npad; i += 2 * FEW_T) {
+            f32x2 hi, lo, s2, c2;
+            ph_phase(reinterpret_cast<const ulonglong2 *>(a.rec + (long)i * PH_REC), pt, hi, lo);
+            ph_sincos(hi, lo, s2, c2);
+            const float2 c = p_un(c2), s = p_un(s2);
+            s_ph[i] = make_float2(c.x, s.x);
+            s_ph[i + 1] = make_float2(c.y, s.y);
+        }
+    }
+    if (a.kin)
+        for (int i = tid; i < a.npad; i += FEW_T) s_px[i] = profile(i);
+    __syncthreads();
+    auto ramp = [&](int i) { return a.trivial_ramp ? s_ramp : s_r[i]; };
+    float S[FEW_Q], C[FEW_Q];
+#pragma unroll
+    for (int q = 0; q < FEW_Q; q++) S[q] = C[q] = 0.f;
+    // first order (Irregular.cpp:178-198, 394-447, 1107-1192)
+    for (int i = slice * FEW_T + tid; i < a.ncomp; i += ns * FEW_T) {
+        const float2 ph = s_ph[i];
+        const float r = ramp(i), rc = r * ph.x, rs = r * ph.y;
+        kahan(S[5], C[5], rc * a.cf[CF_A * cs + i]);
+        if (a.mask & 30) {
+            const float2 px = profile(i);
+            kahan(S[6], C[6], rc * a.cf[CF_GX * cs + i]);
+            kahan(S[7], C[7], rc * a.cf[CF_GY * cs + i]);
+            kahan(S[8], C[8], rs * a.cf[CF_GZ * cs + i]);
+            kahan(S[9], C[9], rc * a.cf[CF_GP * cs + i]);
+            const float au = a.cf[CF_AU * cs + i] * r;
+            kahan(S[1], C[1], au * px.x * a.cf[CF_CT * cs + i] * ph.x);
+            kahan(S[2], C[2], au * px.x * a.cf[CF_ST * cs + i] * ph.x);
+            kahan(S[3], C[3], au * px.y * ph.y);
+            float pp = a.cf[CF_AP * cs + i] * px.x * ph.x;
+            if (a.kin) pp += a.cf[CF_X1 * cs + i] * px.x + a.cf[CF_Z1 * cs + i] * px.y;
+            kahan(S[4], C[4], r * pp);
+        }
+    }
+    // pair items, eight terms each; the records of two neighbouring terms are
+    // interleaved (velocity, pressure) or adjacent (elevation)
+    const f32x2 zk2 = p_pack(zk, zk), yk2 = p_pack(yk, yk), neg1 = p_pack(-1.f, -1.f);
+    const long total = a.nv + a.np + a.ne;
+    for (long item = (long)slice * FEW_T + tid; item < total; item += (long)ns * FEW_T) {
+        int I, M, i, m0;
+        if (item < a.nv + a.np) {
+            const bool vel = item < a.nv;
+            const long it = vel ? item : item - a.nv;
+            constexpr int TT = POINT_TILE, CH = TT / FEW_E;
+            const int ch = (int)(it % CH), ii = (int)(it / CH % TT);
+            const long t = it / (CH * TT);
+            tile_at(t, a.ntp, I, M);
+            i = I * TT + ii;
+            m0 = M * TT + ch * FEW_E;
+            if (m0 + FEW_E <= i) continue;                  // below the diagonal: zeros
+            const long e2 = (t * TT * TT + ii * TT + ch * FEW_E) / 2;
+            const float2 pi = s_ph[i];
+            const f32x2 px2 = p_pack(pi.x, pi.x), py2 = p_pack(pi.y, pi.y), nx2 = p_pack(-pi.x, -pi.x),
+                        ny2 = p_pack(-pi.y, -pi.y);
+            const ulonglong2 *RV = reinterpret_cast<const ulonglong2 *>(a.tabv) + e2 * (POINTV_NC / 2);
+            const ulonglong2 *RP = reinterpret_cast<const ulonglong2 *>(a.tpp) + e2 * (POINTP_NC / 2);
+            const ulonglong2 *RK = reinterpret_cast<const ulonglong2 *>(a.tpk) + e2 * (POINTK_NC / 2);
+            f32x2 au = 0, av = 0, aw = 0, ap = 0, ax = 0, az = 0;
+#pragma unroll
+            for (int k = 0; k < FEW_E / 2; k++) {
+                const float2 q0 = s_ph[m0 + 2 * k], q1 = s_ph[m0 + 2 * k + 1];
+                const f32x2 mc = p_pack(q0.x, q1.x), ms = p_pack(q0.y, q1.y);
+                const f32x2 cc = p_mul(px2, mc);
+                const f32x2 cp = p_fma(ny2, ms, cc), cm = p_fma(py2, ms, cc);
+                const ulonglong2 rk = vel ? RV[4 * k + 3] : RP[2 * k + 1];
+                const f32x2 Ep = p_ex2(p_mul(rk.x, zk2)), Yp = p_ex2(p_mul(rk.x, yk2));
+                const f32x2 Em = p_ex2(p_mul(rk.y, zk2)), Ym = p_ex2(p_mul(rk.y, yk2));
+                const f32x2 A = p_mul(cp, p_add(Ep, Yp)), B = p_mul(cm, p_add(Em, Ym));
+                if (vel) {
+                    const ulonglong2 r0 = RV[4 * k], r1 = RV[4 * k + 1], r2 = RV[4 * k + 2];
+                    const f32x2 sc = p_mul(py2, mc);
+                    const f32x2 sp = p_fma(px2, ms, sc), sm = p_fma(nx2, ms, sc);
+                    const f32x2 Cc = p_mul(sp, p_fma(Yp, neg1, Ep)), D = p_mul(sm, p_fma(Ym, neg1, Em));
+                    au = p_fma(r0.x, A, p_fma(r0.y, B, au));
+                    av = p_fma(r1.x, A, p_fma(r1.y, B, av));
+                    aw = p_fma(r2.x, Cc, p_fma(r2.y, D, aw));
+                } else {
+                    const ulonglong2 rp = RP[2 * k];
+                    ap = p_fma(rp.x, A, p_fma(rp.y, B, ap));
+                    if (a.kin) {
+                        const ulonglong2 x2 = RK[k];
+                        const float2 w0 = s_px[m0 + 2 * k], w1 = s_px[m0 + 2 * k + 1];
+                        ax = p_fma(x2.x, p_pack(w0.x, w1.x), ax);
+                        az = p_fma(x2.y, p_pack(w0.y, w1.y), az);
+                    }
+                }
+            }
+            const float ri = ramp(i);
+            if (vel) {
+                kahan(S[1], C[1], ri * p_hsum(au));
+                kahan(S[2], C[2], ri * p_hsum(av));
+                kahan(S[3], C[3], ri * p_hsum(aw));
+            } else {
+                float row = p_hsum(ap);
+                if (a.kin) row = fmaf(s_px[i].x, p_hsum(ax), fmaf(s_px[i].y, p_hsum(az), row));
+                kahan(S[4], C[4], ri * row);
+            }
+        } else {
+            const long it = item - a.nv - a.np;
+            constexpr int TT = GRID_TILE, CH = TT / FEW_E;
+            const int ch = (int)(it % CH), ii = (int)(it / CH % TT);
+            const long t = it / (CH * TT);
+            tile_at(t, a.ntg, I, M);
+            i = I * TT + ii;
+            m0 = M * TT + ch * FEW_E;
+            if (m0 + FEW_E <= i) continue;
+            const ulonglong2 *RE = reinterpret_cast<const ulonglong2 *>(a.tabe) +
+                                   (t * TT * TT + ii * TT + ch * FEW_E) * EATA_NC / 4;
+            f32x2 acc = 0;                                  // sums of A c_m and B s_m
+#pragma unroll
+            for (int k = 0; k < FEW_E / 2; k++) {
+                const ulonglong2 c = RE[k];
+                const float2 q0 = s_ph[m0 + 2 * k], q1 = s_ph[m0 + 2 * k + 1];
+                acc = p_fma(c.y, p_pack(q1.x, q1.y), p_fma(c.x, p_pack(q0.x, q0.y), acc));
+            }
+            const float2 s2 = p_un(acc), pi = s_ph[i];
+            kahan(S[0], C[0], ramp(i) * fmaf(pi.x, s2.x, pi.y * s2.y));
+        }
+    }
+    // the block's sums
+#pragma unroll
+    for (int q = 0; q < FEW_Q; q++) {
+        float v = S[q] - C[q];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if ((tid & 31) == 0) s_red[tid >> 5][q] = v;
+    }
+    __syncthreads();
+    if (tid < FEW_Q) {
+        float v = 0.f;
+        for (int w = 0; w < FEW_T / 32; w++) v += s_red[w][tid];
+        s_sum[tid] = v;
+        if (ns > 1) __stcg(&a.part[((long)slice * FEW_Q + tid) * a.n + p], v);
+    }
+    if (ns > 1) {
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) s_last = atomicInc(&a.cnt[p], (unsigned)ns - 1) == (unsigned)ns - 1;
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        // a warp a sum in turn, its lanes over the slices
+        for (int q = tid >> 5; q < FEW_Q; q += FEW_T / 32) {
+            float v = 0.f, c = 0.f;
+            for (int k = tid & 31; k < ns; k += 32) kahan(v, c, __ldcg(&a.part[((long)k * FEW_Q + q) * a.n + p]));
+            v -= c;
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if ((tid & 31) == 0) s_sum[q] = v;
+        }
+    }
+    __syncthreads();
+    if (tid != 0) return;
+    // Irregular::eta/u/v/w/dp from the pieces (Irregular.cpp:9-157)
+    const double za = a.order == 2 ? fmax(0.0, zp - a.swl) : 0.0;
+    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (a.mask & 1) v[0] = a.swl + (double)s_sum[5] + (double)s_sum[0];
+    for (int q = 1; q < 5; q++)
+        if (a.mask & (1 << q)) v[q] = (double)s_sum[q] + (double)s_sum[5 + q] * za;
+    if ((a.mask & 16) && a.kt.kin)
+        v[4] += (double)s_ramp * kin_at(a.kt.kin, a.kt.nz, a.kt.h, fmin(0.0, zz));
+    if (!a.api.any()) {
+        for (int q = 0; q < 5; q++)
+            if (a.mask & (1 << q)) a.out[q * a.ldo + p] = v[q];
+        return;
+    }
+    v[5] = v[4] - a.api.rho * a.api.g * v[0];
+    api_store(a.api, p, v);
 }
 
 }  // namespace
@@ -1964,31 +2136,53 @@ static int launch_point_pairs(const DevSea &sea, long n, const float2 *ph, const
     a.tpp = reinterpret_cast<const float4 *>(sea.d_tab_pp);
     a.tpk = reinterpret_cast<const float4 *>(sea.d_tab_pk);
     a.ph = ph; a.rr = rr; a.rs = sea.trivial_ramp ? 0 : n; a.cf = sea.d_cf; a.cstride = sea.npad_g; a.z0 = z0;
-    a.depth = (float)sea.depth; a.pairs = pairs; a.first = 1; a.kin = kin ? 1 : 0; a.one = 1.f;
+    a.depth = (float)sea.depth; a.pairs = pairs; a.first = 1; a.one = 1.f;
     const int ntp = pairs ? sea.ntile_p * (sea.ntile_p + 1) / 2 : sea.ntile_p;
-    if (n <= FEW_POINTS && split_buf) {
-        // a block per (point, slice), the rows of PER tile pairs over its threads
-        constexpr int PER = 128 / POINT_TILE;
-        const int npass = (ntp + PER - 1) / PER;
-        int nslice = (int)std::min<long>(npass, std::max<long>(1, split_cap / (4L * n)));
-        nslice = std::min(nslice, 65535);
-        a.out = split_buf;
-        prof_begin(PK_POINT_PAIRS, stream);
-        k_pairs_points_few<POINT_TILE><<<dim3((unsigned)n, (unsigned)nslice), 128, 0, stream>>>(a, ntp, nslice);
-        note_launch();
-        prof_end(PK_POINT_PAIRS, stream);
-        CK(cudaGetLastError());
-        k_sum_slices<<<(unsigned)((4 * n + 255) / 256), 256, 0, stream>>>(4 * n, nslice, split_buf, out);
-        note_launch();
-        CK(cudaGetLastError());
-        return OK;
-    }
     int rc = OK;
     if (mask & 14) rc = point_pairs_t<true, false, false>(a, n, ntp, out, split_buf, split_cap, stream);
     if (rc == OK && (mask & 16))
         rc = kin && pairs ? point_pairs_t<false, true, true>(a, n, ntp, out + 3 * n, split_buf, split_cap, stream)
                           : point_pairs_t<false, true, false>(a, n, ntp, out + 3 * n, split_buf, split_cap, stream);
     return rc;
+}
+
+// The whole evaluation of a few_points() batch in one kernel.
+static int launch_point_few(const DevSea &sea, long n, const double *x, const double *y, const double *z,
+                            const double *t, int mask, double *out, bool table, const WsLayout &L,
+                            cudaStream_t stream, const ApiRows *api) {
+    FewArgs a{};
+    a.n = n; a.ldo = n; a.x = x; a.y = y; a.z = z; a.t = t;
+    a.fx = sea.fx; a.fy = sea.fy; a.swl = sea.swl; a.depth = sea.depth;
+    a.ncomp = sea.n; a.npad = sea.npad_g; a.cstride = sea.npad_g; a.trivial_ramp = sea.trivial_ramp ? 1 : 0;
+    a.order = sea.order; a.clamp = api ? 1 : 0; a.mask = mask;
+    a.rec = sea.d_phrec; a.cf = sea.d_cf; a.phase = sea.d_phase;
+    a.ntp = sea.ntile_p; a.ntg = sea.ntile_g;
+    a.tabv = sea.d_tab_point; a.tpp = sea.d_tab_pp; a.tpk = sea.d_tab_pk; a.tabe = sea.d_tab_eta;
+    const bool pairs = sea.order == 2;
+    a.kin = pairs && (mask & 16) && !table ? 1 : 0;
+    const long tp = (long)sea.ntile_p * (sea.ntile_p + 1) / 2, tg = (long)sea.ntile_g * (sea.ntile_g + 1) / 2;
+    const long ip = tp * POINT_TILE * POINT_TILE / FEW_E;
+    a.nv = pairs && (mask & 14) ? ip : 0;
+    a.np = pairs && (mask & 16) ? ip : 0;
+    a.ne = pairs && (mask & 1) ? tg * GRID_TILE * GRID_TILE / FEW_E : 0;
+    a.part = L.split; a.cnt = L.cnt; a.out = out;
+    if (api) a.api = *api;
+    if (table) a.kt = KinTab{sea.d_kin, sea.kin_nz, sea.kin_h, sea.depth, nullptr};
+    // as many slices as give every thread one item, up to about eight blocks an SM in all
+    const long want = std::max<long>(1, (a.nv + a.np + a.ne + FEW_T - 1) / FEW_T);
+    const long cap = std::max<long>(1, 2 * SPLIT_TARGET_BLOCKS / n);
+    const long ns = std::min(std::min(want, cap), std::max<long>(1, L.split_cap / (FEW_Q * n)));
+    const size_t smem = sizeof(float2) * (size_t)a.npad * (a.kin ? 2 : 1) + (sea.trivial_ramp ? 0 : sizeof(float) * a.npad);
+    // set once per process (thread-safe static initialisation)
+    static const cudaError_t attr = cudaFuncSetAttribute(k_point_few, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         FEW_MAX_NPAD * 20);
+    CK(attr);
+    prof_begin(PK_POINT_PAIRS, stream);
+    k_point_few<<<dim3((unsigned)n, (unsigned)ns), FEW_T, smem, stream>>>(a);
+    note_launch();
+    prof_end(PK_POINT_PAIRS, stream);
+    CK(cudaGetLastError());
+    return OK;
 }
 
 // Phasor layout used by the pair kernels: the point kernel reads tiles of
@@ -2004,8 +2198,12 @@ int irregular_eval(const DevSea &sea, long n, const double *x, const double *y, 
     // calls clamp z to the range it covers
     const bool table = api && sea.d_kin && sea.order == 2;
     WsLayout L0 = layout(std::min(n, chunk), npad, nullptr);
+    const void *held = ws.base;
     int rc = workspace_reserve(ws, L0.bytes);
     if (rc) return rc;
+    if (ws.base != held) CK(cudaMemsetAsync(ws.base, 0, CNT_BYTES, stream));    // the few-point counters
+    if (few_points(n, npad) && !(sea.smit && (mask & 30)))
+        return launch_point_few(sea, n, x, y, z, t, mask, out, table, layout(n, npad, ws.base), stream, api);
     for (long b = 0; b < n; b += chunk) {
         long m = std::min(chunk, n - b);
         WsLayout L = layout(m, npad, ws.base);

@@ -58,3 +58,27 @@ def test_points_vs_oracle(wm, nfreq, ndir, individual):
         rf = rf if rf.shape[0] == 5 else rf.T
         for q in range(5):
             assert np.max(np.abs(f[q] - rf[q])) <= TOL * np.max(np.abs(rf[q])), (q, m, n)
+
+
+@pytest.mark.parametrize("nfreq,ndir", [(1, 1), (33, 1), (43, 3), (130, 2)])
+def test_few_points_match_a_large_batch(wm, nfreq, ndir):
+    """The one-kernel evaluation of a short batch gives the rows that the same
+    points have in a batch too large for it (each within TOL of the sums, so
+    2 TOL apart at most), call after call."""
+    comps = ss.irregular_components(3.5, 9.0, 2.0, nfreq, 0.4, 1.9, 35.0, 8, ndir=ndir, spreading_s=5.0)
+    txt = ss.write_irregular(None, comps, 35.0, extrap=2, swl=0.4, rho=1025.0, mtheta=25.0)
+    assert wm.initialize_text(txt) == 0, cw.last_error()
+    rng = np.random.default_rng(nfreq)
+    m = 4200
+    x, y = rng.uniform(-50, 300, m), rng.uniform(-80, 80, m)
+    z, t = rng.uniform(-37.0, 3.0, m), rng.uniform(0.5, 30, m)
+
+    def rows(k):
+        p = x[:k], y[:k], z[:k], t[:k]
+        return np.array([wm.surface_elevation_batch(*p[:2], p[3]), *wm.velocity_batch(*p),
+                         wm.dynamic_pressure_batch(*p), wm.nonhydrostatic_pressure_batch(*p)])
+
+    ref = rows(m)
+    top = np.max(np.abs(ref), axis=1, keepdims=True)
+    for k in (1, 2, 17, 130, 1, 20, 400):
+        assert np.all(np.abs(rows(k) - ref[:, :k]) <= 2 * TOL * top), k
