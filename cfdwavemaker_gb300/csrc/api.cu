@@ -1143,8 +1143,7 @@ int cfdwm_surrogate_forward(const float *x, int B, int H, int W, float *y) {
     if (!x || !y || !is_device(x) || !is_device(y)) return E_BAD_ARGUMENT;
     cudaStream_t s = stream_of();
     int rc = surrogate_forward(x, B, H, W, y, s);
-    if (!rc) CKR(cudaStreamSynchronize(s));
-    if (!rc) rc = surrogate_check(s);
+    if (!rc) rc = surrogate_check(s);          // synchronises
     return rc;
 }
 

@@ -1,35 +1,40 @@
 // Valid 3x3 convolutions of the learned s-grid update as implicit GEMMs on
 // the tcgen05 tensor cores (forward, data gradient and weight gradient).
 //
-// The network (surrogate.cu) keeps its activations as FP32 planes
-// [B][C][H][W] and its weights as BF16 [O][C][9].  Each convolution is a GEMM
-// whose operand tiles the CUDA cores gather from those planes straight into
-// shared memory, in the K-major 128-byte swizzle layout the tensor cores read,
-// one 64-wide K stage at a time; two stages are in flight, so the MMAs of one
-// stage run while the threads gather the next:
 //   forward      D[pixel][o]    = sum_{tap, c} x[c][pixel + tap] w[o][c][tap]
 //   data grad    D[pixel][c]    = sum_{tap, o} dy[o][pixel - tap] w[o][c][tap]
-//   weight grad  D[tap, c][o]   = sum_{pixel}  x[c][pixel + tap] dy[o][pixel]
-//                                 (per slab of pixels; the slabs are summed in
-//                                 order afterwards, so the result is
-//                                 deterministic)
-// M = 128 rows per CTA (two threads per row, each gathering half of a K
-// stage), N = the channel count padded to 32 or 64, K = 16 per MMA; D is an
-// FP32 accumulator in TMEM, read back with tcgen05.ld by the warps of its
-// lane quarter.  The weights of a forward or data-gradient launch are packed
-// once into the K-contiguous B layout, so a stage's B tile is one 16-byte
-// copy per chunk.  The FP32 activations and
-// gradients are split into BF16 hi + lo parts (16 significant bits, error
-// <= 2^-17 of the value); the weights are BF16 already, so the forward and
-// data-gradient GEMMs take two MMAs per K step (hi, lo) and the weight
-// gradient, whose two operands are both split, three (hi hi, hi lo, lo hi).
+//   weight grad  D[dy, c][o]    = sum_{pixel}  x[c][pixel + tap] dy[o][pixel], per dx
+//
+// Operand format.  Activations and gradients are kept split into BF16 hi + lo
+// parts (16 significant bits, error <= 2^-17 of the value), eight channels to
+// 16 bytes: [b][part][C / 8][H][W][8].  A tile of pixels with its halo is then
+// one TMA box, and in shared memory every group of 8 pixels x 8 channels is a
+// core matrix of the unswizzled operand layouts, whose strides the descriptors
+// give: K-major (K = channels) for the forward and data-gradient GEMMs,
+// MN-major (K = pixels) for the weight gradient.  A tap moves the operand by
+// whole pixels, 16 bytes each, so the nine taps are nine start addresses in
+// one copy of the tile: nothing is gathered, and nothing is split twice.
+// Zero padding (ragged tiles, the data gradient's border, channels past the
+// last) is the boxes' out-of-range fill.
+//
+// The weights are BF16, so the forward and data-gradient GEMMs take two MMAs
+// per K step (hi, lo) and the weight gradient, whose two operands are both
+// split, three (hi hi, lo hi, hi lo); sums in FP32 in TMEM.  The first form
+// of these kernels gathered each operand tile from FP32 planes with the CUDA
+// cores, nine times over (issue-bound).  Network of 16 levels over a 264 x 264
+// grid: 357 us then, CT_FWD_US us now; loss and gradient of 8 patches of 72 x 72: 981
+// and CT_GRAD_US us.
+//
 // Every mbarrier wait is bounded and sets the error word when it gives up.
 #include "cfdwm.h"
+#include "convtc.h"
 #include "tc05.cuh"
 
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <mutex>
 
@@ -47,417 +52,636 @@ namespace cfdwm {
 
 namespace {
 
-constexpr int CT_M = 128;                 // GEMM rows per CTA, one per thread
-constexpr int CT_K = 64;                  // K per stage: one 128-byte swizzled row of BF16
-constexpr int CT_ATILE = CT_M * CT_K * 2; // 16 KiB, one split part of A
+constexpr int HID = CONV_HID;             // hidden channels: N of the forward and data-gradient GEMMs
+constexpr int TX = 8, TY = 16;            // pixel tile: 128 rows of D, a core matrix per tile row
+constexpr int PX = TX + 2, PY = TY + 2;   // the tile with its halo
+constexpr int KC = 4;                     // channel chunks (of 8) per stage: two K steps of 16
+constexpr int CHUNK = PX * PY * 16;       // bytes of a chunk's patch
+constexpr int APART = KC * CHUNK;         // of one split part of a stage
+constexpr int CT_THREADS = 128;           // a thread per TMEM lane
+constexpr int CT_HEAD = 64 + 4 * HID * 4; // barriers and flags, bias partial sums
 
-enum { CT_FWD = 0, CT_DATA = 1, CT_WGT = 2 };
+__device__ __forceinline__ float ct_sigmoid(float a) { return 1.f / (1.f + expf(-a)); }
 
-struct TcConv {
-    const float *x;              // FWD, WGT: input planes [*][C][H][W]
-    long xbs;                    // batch stride of x
-    const int *idx;              // sample index of batch entry b (null: b)
-    const float *dy;             // DATA, WGT: output gradient [B][O][H-2][W-2]
-    const __nv_bfloat16 *w;      // FWD, DATA: the packed B operand [NP][Kp] (k_ct_pack)
-    const float *bias;           // FWD
-    float *pre;                  // FWD: pre-activation copy (written, may be null);
-                                 // DATA: pre-activation of the input (read, may be null)
-    float *out;                  // FWD: y [B][O][H-2][W-2]; DATA: dx [B][C][H][W];
-                                 // WGT: per-slab partial sums [slab][O C 9 + O]
-    int B, C, O, H, W;
-    int act;                     // FWD: SiLU
-    int kslab;                   // WGT: output pixels per slab
-    int slabs_per_img;           // WGT
+// operand descriptor without swizzle: core matrices (8 rows of 16 bytes,
+// contiguous) lbo bytes apart along K and sbo bytes apart along M or N
+__device__ __forceinline__ uint64_t cdesc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+    return (uint64_t)((saddr & 0x3FFFF) >> 4) | (uint64_t)(lbo >> 4) << 16 | (uint64_t)(sbo >> 4) << 32 |
+           (uint64_t)1 << 46;
+}
+
+__device__ __forceinline__ void tma_4d(void *dst, const CUtensorMap *m, uint64_t *bar, int x, int y, int z, int w) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0],"
+                 " [%1, {%3, %4, %5, %6}], [%2];"
+                 ::"r"(su32(dst)), "l"(m), "r"(su32(bar)), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(su32(dst)), "l"(src), "r"(bytes), "r"(su32(bar)) : "memory");
+}
+
+__device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(slot)), "r"(cols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+}
+__device__ __forceinline__ void tmem_free(uint32_t tmem, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols));
+}
+
+// FP32 planes [idx b][C][plane] to the split format; a thread per (pixel, chunk).
+__global__ void __launch_bounds__(256) k_ct_split(const float *x, long xbs, const int *idx, int C, long plane,
+                                                  uint4 *out) {
+    const long p = blockIdx.x * 256L + threadIdx.x;
+    if (p >= plane) return;
+    const int ch = blockIdx.y, nch = gridDim.y, b = blockIdx.z;
+    const float *src = x + (long)(idx ? idx[b] : b) * xbs + (long)ch * 8 * plane + p;
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) v[e] = ch * 8 + e < C ? src[e * plane] : 0.f;
+    uint4 hi, lo;
+    conv_split8(v, hi, lo);
+    out[((long)(b * 2) * nch + ch) * plane + p] = hi;
+    out[((long)(b * 2 + 1) * nch + ch) * plane + p] = lo;
+}
+
+// ---------------------------------------------------------------------------
+// Weights: the B operands of the forward and data-gradient GEMMs,
+// [stage][tap][KC][NP][8] BF16, a stage one bulk copy; zero past the channels.
+// ---------------------------------------------------------------------------
+struct PackJobs {
+    struct Job {
+        long w, out, end;        // first weight and output element; end of the job's elements
+        int K, N, NP, sk, sn;    // channels along K and N, padded N, their weight strides
+        int flip;                // data gradient: the taps run backwards
+    } j[CONV_MAX_PACK];
+    int n;
+};
+
+__global__ void __launch_bounds__(256) k_ct_pack(PackJobs jobs, const float *w, __nv_bfloat16 *out) {
+    const long e = blockIdx.x * 256L + threadIdx.x;
+    int q = 0;
+    while (q < jobs.n && e >= jobs.j[q].end) q++;
+    if (q == jobs.n) return;
+    const PackJobs::Job &j = jobs.j[q];
+    const long i = e - j.out;
+    const int c8 = (int)(i & 7), n = (int)(i / 8 % j.NP), kc = (int)(i / (8L * j.NP) % KC);
+    const int tap = (int)(i / (8L * j.NP * KC) % 9), st = (int)(i / (8L * j.NP * KC * 9));
+    const int k = (st * KC + kc) * 8 + c8;
+    float v = 0.f;
+    if (k < j.K && n < j.N) v = w[j.w + (long)k * j.sk + (long)n * j.sn + (j.flip ? 8 - tap : tap)];
+    out[e] = __float2bfloat16_rn(v);
+}
+
+// ---------------------------------------------------------------------------
+// Forward and data gradient
+// ---------------------------------------------------------------------------
+enum { CT_HIDDEN = 0, CT_OUTPUT = 1, CT_DATA = 2 };
+
+struct ConvArgs {
+    const uint8_t *w;            // packed weights
+    const float *bias;           // HIDDEN, OUTPUT
+    const float4 *ds;            // DATA: silu' of the layer's pre-activation [b][HID / 4][Ho][Wo]
+    float4 *ds_out;              // HIDDEN: the same, or null
+    uint4 *ys;                   // HIDDEN: activations, DATA: gradient, split format
+    float *y;                    // OUTPUT: planes [b][O][Ho][Wo]
+    float *bpart;                // DATA: sums of the tile's gradient [tile][HID]
+    int nst, nch;                // stages; input chunks
+    int origin;                  // of the patch relative to the tile: 0, data gradient -2
+    int O, Ho, Wo, tiles_x;
     int *err;
 };
 
-__device__ __forceinline__ float ct_silu(float a) { return a / (1.f + expf(-a)); }
-__device__ __forceinline__ float ct_silu_d(float a) {
-    float s = 1.f / (1.f + expf(-a));
-    return s * (1.f + a * (1.f - s));
-}
-
-// byte offset of the 16-byte chunk j (elements 8j..8j+7) of row r in a K-major
-// tile of 128-byte rows with the 128-byte swizzle (8-row atoms of 1024 B)
-__device__ __forceinline__ uint32_t swz(int r, int j) {
-    return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((j ^ (r & 7)) << 4));
-}
-
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t *>(&h);
-}
-
-// eight values into the hi and lo tiles of row r, chunk j
-__device__ __forceinline__ void put8_split(uint8_t *hi, uint8_t *lo, int r, int j, const float *v) {
-    float h[8], l[8];
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-        h[e] = __bfloat162float(__float2bfloat16_rn(v[e]));
-        l[e] = v[e] - h[e];
-    }
-    const uint32_t o = swz(r, j);
-    *reinterpret_cast<uint4 *>(hi + o) =
-        make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
-    *reinterpret_cast<uint4 *>(lo + o) =
-        make_uint4(pack_bf16(l[0], l[1]), pack_bf16(l[2], l[3]), pack_bf16(l[4], l[5]), pack_bf16(l[6], l[7]));
-}
-
-constexpr int CT_THREADS = 256;           // two threads per A row, each half of its K stage
-
-template <int OP, int NP>
-struct CtCfg {
-    static constexpr int BTILE = NP * CT_K * 2;                  // B: NP rows of 128 B
-    static constexpr int NBP = OP == CT_WGT ? 2 : 1;             // split parts of B
-    static constexpr int STAGE = 2 * CT_ATILE + NBP * BTILE;     // a multiple of 1024
-    static constexpr int SMEM = 2 * STAGE + 1024 + 64 + 8 * 64 * 4;
+template <int NP> struct CtCfg {
+    static constexpr int BTILE = 9 * KC * NP * 16;
+    static constexpr int STAGE = 2 * APART + BTILE;
 };
 
-// B operand of the forward (op 0) and data-gradient (op 1) GEMMs, [NP][Kp]
-// BF16, K contiguous: forward B[o][tap C + c] = w[o][c][tap]; data gradient
-// B[c][tap O + o] = w[o][c][tap]; zero past O (C) and past 9 C (9 O).
-__global__ void k_ct_pack(const __nv_bfloat16 *w, int C, int O, int op, int NP, int Kp, __nv_bfloat16 *out) {
-    const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (e >= (long)NP * Kp) return;
-    const int n = (int)(e / Kp), k = (int)(e % Kp);
-    __nv_bfloat16 v = __float2bfloat16_rn(0.f);
-    if (op == CT_FWD) {
-        const int tap = k / C, c = k % C;
-        if (n < O && tap < 9) v = w[((long)n * C + c) * 9 + tap];
-    } else {
-        const int tap = k / O, o = k % O;
-        if (n < C && tap < 9) v = w[((long)o * C + n) * 9 + tap];
-    }
-    out[e] = v;
-}
-
-template <int OP, int NP>
-__global__ void __launch_bounds__(CT_THREADS, 2) k_conv_tc(TcConv a) {
-    using CF = CtCfg<OP, NP>;
-    constexpr int BTILE = CF::BTILE, STAGE = CF::STAGE;
-    extern __shared__ __align__(1024) uint8_t ct_raw[];
-    uint8_t *smem = (uint8_t *)(((uintptr_t)ct_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t *bar = (uint64_t *)(smem + 2 * STAGE);      // [0, 1] stage released, [2] all MMAs done
-    uint32_t *tslot = (uint32_t *)(bar + 4);
-    float *red = (float *)(bar + 8);                     // WGT: bias partial sums [8][64]
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int r = tid & (CT_M - 1), half = tid >> 7;     // A row, and which half of its K stage
-    const int Ho = a.H - 2, Wo = a.W - 2;
-    const long plane = (long)a.H * a.W, oplane = (long)Ho * Wo;
-
-    // this CTA's rows and K extent
-    int b, slab = 0;
-    long row = 0, q0 = 0, q1 = 0, K;
-    bool live;
-    if (OP == CT_WGT) {
-        slab = blockIdx.x;
-        b = slab / a.slabs_per_img;
-        q0 = (long)(slab % a.slabs_per_img) * a.kslab;
-        q1 = q0 + a.kslab < oplane ? q0 + a.kslab : oplane;
-        row = (long)blockIdx.y * CT_M + r;               // (tap, c) = (row / C, row % C)
-        live = row < 9L * a.C;
-        K = q1 - q0;
-    } else {
-        b = blockIdx.y;
-        row = (long)blockIdx.x * CT_M + r;               // pixel of the output (FWD) or input (DATA) plane
-        live = row < (OP == CT_FWD ? oplane : plane);
-        K = 9L * (OP == CT_FWD ? a.C : a.O);
-    }
-    const int nst = (int)((K + CT_K - 1) / CT_K);
-    const long Kp = (long)nst * CT_K;
-    const float *X = (OP != CT_DATA) ? a.x + (long)(a.idx ? a.idx[b] : b) * a.xbs : nullptr;
-
+// A CTA makes one tile of 16 x 8 output pixels: M = 128, N = NP (the hidden
+// channels, or the output's padded), K = 32 channels x 9 taps per stage.
+// Thread 0 copies (two stages in flight), thread 32 issues the MMAs, the four
+// warps read their TMEM lanes.  The operand's 4 KB per MMA from shared memory
+// bound the tensor cores at these N (32 cycles an MMA); up to five CTAs an SM
+// overlap copies, MMAs and epilogues of different tiles.
+template <int NP, int EPI>
+__global__ void __launch_bounds__(CT_THREADS) k_conv(const __grid_constant__ CUtensorMap xm, ConvArgs a) {
+    using CF = CtCfg<NP>;
+    extern __shared__ __align__(128) uint8_t ct_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)ct_raw + 127) & ~(uintptr_t)127);
+    const int nbuf = a.nst < 2 ? a.nst : 2;
+    uint64_t *full = (uint64_t *)(smem + nbuf * CF::STAGE), *empty = full + 2, *done = full + 4;
+    uint32_t *tslot = (uint32_t *)(full + 5);
+    volatile int *fail = (volatile int *)(full + 6);
+    float *red = (float *)(full + 8);                 // DATA: [4][HID]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int b = blockIdx.y;
+    const int x0 = (blockIdx.x % a.tiles_x) * TX, y0 = (blockIdx.x / a.tiles_x) * TY;
     if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        mbar_init(&bar[2], 1);
+        for (int q = 0; q < 5; q++) mbar_init(full + q, 1);
+        *fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    constexpr uint32_t TCOLS = NP < 32 ? 32 : NP;
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tslot)),
-                     "r"(TCOLS));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
+    if (warp == 0) tmem_alloc(tslot, NP);
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot;
 
-    // per-thread constants of the A row
-    int ay = 0, ax = 0, wc = 0, wtap = 0;
-    if (OP == CT_WGT) {
-        wtap = live ? (int)(row / a.C) : 0;
-        wc = live ? (int)(row % a.C) : 0;
-    } else if (live) {
-        const int pw = OP == CT_FWD ? Wo : a.W;
-        ay = (int)(row / pw);
-        ax = (int)(row % pw);
+    if (tid == 0) {
+        for (int s = 0; s < a.nst; s++) {
+            const int buf = s & 1;
+            if (s >= 2 && !mbar_wait(empty + buf, (uint32_t)(((s >> 1) - 1) & 1), a.err, 11)) { *fail = 1; break; }
+            uint8_t *st = smem + buf * CF::STAGE;
+            mbar_expect_tx(full + buf, CF::STAGE);
+            tma_4d(st, &xm, full + buf, (x0 + a.origin) * 8, y0 + a.origin, s * KC, b * 2);
+            bulk_load(st + 2 * APART, a.w + (long)s * CF::BTILE, CF::BTILE, full + buf);
+        }
+    } else if (tid == 32) {
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NP >> 3) << 17) |
+                               ((uint32_t)((TX * TY) >> 4) << 24);
+        for (int s = 0; s < a.nst; s++) {
+            const int buf = s & 1;
+            const uint32_t par = (uint32_t)((s >> 1) & 1);
+            if (!mbar_wait(full + buf, par, a.err, 12)) {
+                *fail = 1;
+                mbar_wait(full + buf, par, a.err, 12);
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t A = su32(smem + buf * CF::STAGE), B = A + 2 * APART;
+            const uint64_t da = cdesc(A, CHUNK, PX * 16), db = cdesc(B, NP * 16, 128);
+            const int nk = (min(KC, a.nch - s * KC) + 1) / 2;
+            for (int tap = 0; tap < 9; tap++)
+                for (int k = 0; k < nk; k++) {
+                    const uint64_t oa = (uint64_t)((2 * k * CHUNK + ((tap / 3) * PX + tap % 3) * 16) >> 4);
+                    const uint64_t ob = (uint64_t)(((tap * KC + 2 * k) * NP * 16) >> 4);
+                    umma(tmem, da + oa, db + ob, idesc, (s | tap | k) ? 1u : 0u);
+                    umma(tmem, da + oa + (APART >> 4), db + ob, idesc, 1u);
+                }
+            umma_commit(empty + buf);
+        }
+        umma_commit(done);
     }
-    // B chunks of a stage: NP rows x 8 chunks of 16 B; chunk id = tid + 256 q
-    constexpr int BCH = NP * 8 / CT_THREADS;             // 1 (NP = 32) or 2 (NP = 64)
-    float bsum[BCH];
+    __syncwarp();
+    bool ok = mbar_wait(done, 0u, a.err, 13);
+    ok = !__syncthreads_or(!ok) && !*fail;
+    if (ok) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16);
+        const int oy = y0 + (tid >> 3), ox = x0 + (tid & 7);
+        const long plane = (long)a.Ho * a.Wo, pix = (long)oy * a.Wo + ox;
+        const bool live = oy < a.Ho && ox < a.Wo;
+        if (EPI == CT_OUTPUT) {
 #pragma unroll
-    for (int q = 0; q < BCH; q++) bsum[q] = 0.f;
-
-    bool failed = false;
-    for (int s = 0; s < nst; s++) {
-        const int buf = s & 1;
-        uint8_t *st = smem + buf * STAGE;
-        uint8_t *Ahi = st, *Alo = st + CT_ATILE, *Bhi = st + 2 * CT_ATILE, *Blo = Bhi + BTILE;
-        bool ok = true;
-        if (s >= 2) ok = mbar_wait(&bar[buf], (uint32_t)(((s >> 1) - 1) & 1), a.err, 11);
-        if (__syncthreads_or(!ok)) { failed = true; break; }
-        const long k0 = (long)s * CT_K + half * (CT_K / 2);
-        // ---- half of the A row of this thread: 32 K values, gathered with all
-        // loads in flight, the K index walked incrementally
-        float v[32];
-        if (OP == CT_WGT) {
-            long q = q0 + k0;
-            int oy = (int)(q / Wo), ox = (int)(q - (long)oy * Wo);
-            const float *xr = X + (long)wc * plane + (long)(wtap / 3) * a.W + wtap % 3;
+            for (int h = 0; h < NP / 32; h++) {
+                float d[32];
+                tmem_ld32(ta + h * 32, d);
+                if (live)
 #pragma unroll
-            for (int e = 0; e < 32; e++) {
-                v[e] = (live && k0 + e < K) ? xr[(long)oy * a.W + ox] : 0.f;
-                if (++ox == Wo) { ox = 0; oy++; }
+                    for (int n = 0; n < 32; n++) {
+                        const int o = h * 32 + n;
+                        if (o >= a.O) break;
+                        a.y[((long)b * a.O + o) * plane + pix] = d[n] + a.bias[o];
+                    }
             }
         } else {
-            const int cdim = OP == CT_FWD ? a.C : a.O;
-            int tap = (int)(k0 / cdim), c = (int)(k0 - (long)tap * cdim);
+            float d[32];
+            tmem_ld32(ta, d);
 #pragma unroll
-            for (int e = 0; e < 32; e++) {
-                float val = 0.f;
-                if (live && k0 + e < K) {
-                    if (OP == CT_FWD) {
-                        val = X[(long)c * plane + (long)(ay + tap / 3) * a.W + ax + tap % 3];
-                    } else {
-                        const int yy = ay - tap / 3, xx = ax - tap % 3;
-                        if (yy >= 0 && yy < Ho && xx >= 0 && xx < Wo)
-                            val = a.dy[((long)b * a.O + c) * oplane + (long)yy * Wo + xx];
+            for (int c = 0; c < HID / 8; c++) {
+                float v[8], g[8];
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    if (EPI == CT_DATA) {
+                        float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (live) f = a.ds[((long)b * (HID / 4) + c * 2 + q) * plane + pix];
+                        g[q * 4] = f.x; g[q * 4 + 1] = f.y; g[q * 4 + 2] = f.z; g[q * 4 + 3] = f.w;
                     }
                 }
-                v[e] = val;
-                if (++c == cdim) { c = 0; tap++; }
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) put8_split(Ahi, Alo, r, half * 4 + j, v + 8 * j);
-        // ---- B chunks
-#pragma unroll
-        for (int q = 0; q < BCH; q++) {
-            const int id = tid + CT_THREADS * q, n = id >> 3, j = id & 7;
-            const long kc = (long)s * CT_K + j * 8;
-            if (OP == CT_WGT) {
-                float bv[8];
-                const float *dr = a.dy + ((long)b * a.O + n) * oplane + q0;
 #pragma unroll
                 for (int e = 0; e < 8; e++) {
-                    const float val = (n < a.O && kc + e < K) ? dr[kc + e] : 0.f;
-                    bsum[q] += val;
-                    bv[e] = val;
+                    if (EPI == CT_DATA) {
+                        v[e] = live ? d[c * 8 + e] * g[e] : 0.f;
+                        d[c * 8 + e] = v[e];
+                    } else {
+                        const float p = d[c * 8 + e] + a.bias[c * 8 + e], sg = ct_sigmoid(p);
+                        v[e] = p / (1.f + expf(-p));
+                        g[e] = sg * (1.f + p * (1.f - sg));
+                    }
                 }
-                put8_split(Bhi, Blo, n, j, bv);
-            } else {
-                // the packed weights: one 16-byte chunk
-                const uint4 c4 = *reinterpret_cast<const uint4 *>(a.w + (long)n * Kp + kc);
-                *reinterpret_cast<uint4 *>(Bhi + swz(n, j)) = c4;
-            }
-        }
-        // the generic-proxy writes become visible to the tensor cores' reads
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NP >> 3) << 17) |
-                                   ((uint32_t)(CT_M >> 4) << 24);
-            const uint64_t dAh = sdesc(su32(Ahi)), dAl = sdesc(su32(Alo)), dBh = sdesc(su32(Bhi));
-            const uint64_t dBl = sdesc(su32(Blo));
+                if (!live) continue;
+                uint4 hi, lo;
+                conv_split8(v, hi, lo);
+                a.ys[((long)(b * 2) * (HID / 8) + c) * plane + pix] = hi;
+                a.ys[((long)(b * 2 + 1) * (HID / 8) + c) * plane + pix] = lo;
+                if (EPI == CT_HIDDEN && a.ds_out)
 #pragma unroll
-            for (int k = 0; k < CT_K / 16; k++) {
-                const uint64_t o = (uint64_t)(k * 32) >> 4;        // 16 BF16 = 32 bytes per step
-                const uint32_t first = (s == 0 && k == 0) ? 0u : 1u;
-                umma(tmem, dAh + o, dBh + o, idesc, first);
-                umma(tmem, dAl + o, dBh + o, idesc, 1u);
-                if (OP == CT_WGT) umma(tmem, dAh + o, dBl + o, idesc, 1u);
+                    for (int q = 0; q < 2; q++)
+                        a.ds_out[((long)b * (HID / 4) + c * 2 + q) * plane + pix] =
+                            make_float4(g[q * 4], g[q * 4 + 1], g[q * 4 + 2], g[q * 4 + 3]);
             }
-            umma_commit(&bar[buf]);
-        }
-    }
-    if (tid == 0 && !failed) umma_commit(&bar[2]);
-    bool ok = !failed && nst > 0 && mbar_wait(&bar[2], 0u, a.err, 12);
-    ok = !__syncthreads_or(!ok);
-    if (ok) {
-        // warp w reads TMEM lane quarter w % 4, column half w / 4
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        constexpr int HC = NP / 2;
-        const int c0 = half * HC;
-        const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
-        float d[HC];
-        if constexpr (HC == 32) tmem_ld32(ta, d);
-        else tmem_ld16(ta, d);
-        if (live) {
+            if (EPI == CT_DATA) {
+                // the bias gradient's share of this tile: lane c ends with channel c of its warp's pixels
 #pragma unroll
-            for (int n = 0; n < HC; n++) {
-                const int ch = c0 + n;
-                if (OP == CT_FWD) {
-                    if (ch >= a.O) break;
-                    const long off = ((long)b * a.O + ch) * oplane + row;
-                    const float val = d[n] + a.bias[ch];
-                    if (a.pre) a.pre[off] = val;
-                    a.out[off] = a.act ? ct_silu(val) : val;
-                } else if (OP == CT_DATA) {
-                    if (ch >= a.C) break;
-                    const long off = ((long)b * a.C + ch) * plane + row;
-                    a.out[off] = a.pre ? d[n] * ct_silu_d(a.pre[off]) : d[n];
-                } else {
-                    if (ch >= a.O) break;
-                    const long per = (long)a.O * a.C * 9 + a.O;
-                    a.out[(long)slab * per + ((long)ch * a.C + wc) * 9 + wtap] = d[n];
+                for (int o = 16; o >= 1; o >>= 1) {
+                    const bool up = lane & o;
+#pragma unroll
+                    for (int i = 0; i < o; i++) {
+                        const float send = up ? d[i] : d[i + o], keep = up ? d[i + o] : d[i];
+                        d[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                    }
                 }
+                red[warp * HID + lane] = d[0];
             }
-        }
-    }
-    if (OP == CT_WGT && blockIdx.y == 0) {
-        // bias gradient of the slab: the sum of dy over its pixels, the eight
-        // chunks of a row added in a fixed order
-#pragma unroll
-        for (int q = 0; q < BCH; q++) {
-            const int id = tid + CT_THREADS * q;
-            red[(id & 7) * 64 + (id >> 3)] = bsum[q];
-        }
-        __syncthreads();
-        if (tid < NP && tid < a.O) {
-            float t = 0.f;
-            for (int j = 0; j < 8; j++) t += red[j * 64 + tid];
-            const long per = (long)a.O * a.C * 9 + a.O;
-            a.out[(long)slab * per + (long)a.O * a.C * 9 + tid] = t;
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS));
+    if (EPI == CT_DATA && ok && warp == 1)
+        a.bpart[((long)b * gridDim.x + blockIdx.x) * HID + lane] =
+            (red[lane] + red[HID + lane]) + (red[2 * HID + lane] + red[3 * HID + lane]);
+    if (warp == 0) tmem_free(tmem, NP);
 }
 
-template <int OP, int NP>
-int launch_ct(const TcConv &a, dim3 grid, cudaStream_t st) {
-    using CF = CtCfg<OP, NP>;
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_conv_tc<OP, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, CF::SMEM);
-    CK(attr);
-    k_conv_tc<OP, NP><<<grid, CT_THREADS, CF::SMEM, st>>>(a);
-    note_launch();
-    CK(cudaGetLastError());
-    return OK;
+// ---------------------------------------------------------------------------
+// Weight gradient
+// ---------------------------------------------------------------------------
+struct WgtArgs {
+    float *part;                 // [slab][3 dx][O][3 dy C]
+    int nch, rows;               // input chunks; patch rows copied
+    int ntiles, tiles_x, tiles_img;
+    int nbuf;
+    int O;
+    int *err;
+};
+
+// D's rows are (dy, c) pairs: with the patch copied as [row][chunk][pixel],
+// the row groups of 8 channels over dy and the chunks are one arithmetic
+// progression of addresses, so M = 128 holds 16 of them whatever C is (four
+// taps' worth of 32 channels; blockIdx.y counts the M tiles).  dx is a start
+// address, with an accumulator of its own.  K is the tile's pixels, two tile
+// rows per MMA.  A CTA sums its slab (every gridDim.x-th tile) in TMEM; the
+// slabs are summed in order afterwards, so the result is deterministic.
+template <int NP>
+__global__ void __launch_bounds__(CT_THREADS)
+k_conv_wgt(const __grid_constant__ CUtensorMap xm, const __grid_constant__ CUtensorMap dm, WgtArgs a) {
+    constexpr int BPART = (NP / 8) * TY * TX * 16;
+    constexpr uint32_t TCOLS = NP == 32 ? 128 : 256;
+    extern __shared__ __align__(128) uint8_t ct_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)ct_raw + 127) & ~(uintptr_t)127);
+    const int apart = a.rows * a.nch * PX * 16, abytes = (2 * apart + 127) & ~127, stage = abytes + 2 * BPART;
+    uint64_t *full = (uint64_t *)(smem + a.nbuf * stage), *empty = full + 2, *done = full + 4;
+    uint32_t *tslot = (uint32_t *)(full + 5);
+    volatile int *fail = (volatile int *)(full + 6);
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int g0 = blockIdx.y * 16, r0 = g0 / a.nch;          // first row group of this M tile, its dy
+    if (tid == 0) {
+        for (int q = 0; q < 5; q++) mbar_init(full + q, 1);
+        *fail = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) tmem_alloc(tslot, TCOLS);
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tslot;
+
+    if (tid == 0) {
+        int s = 0;
+        for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x, s++) {
+            const int buf = s % a.nbuf, use = s / a.nbuf;
+            if (use > 0 && !mbar_wait(empty + buf, (uint32_t)((use - 1) & 1), a.err, 14)) { *fail = 1; break; }
+            const int b = t / a.tiles_img, r = t % a.tiles_img;
+            const int x0 = (r % a.tiles_x) * TX, y0 = (r / a.tiles_x) * TY;
+            uint8_t *st = smem + buf * stage;
+            mbar_expect_tx(full + buf, 2 * apart + 2 * BPART);
+            tma_4d(st, &xm, full + buf, x0 * 8, 0, y0 + r0, b * 2);
+            tma_4d(st + abytes, &dm, full + buf, x0 * 8, y0, 0, b * 2);
+        }
+    } else if (tid == 32) {
+        // both operands MN-major (bits 15 and 16)
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                               ((uint32_t)(NP >> 3) << 17) | (8u << 24);
+        int s = 0;
+        for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x, s++) {
+            const int buf = s % a.nbuf;
+            const uint32_t par = (uint32_t)((s / a.nbuf) & 1);
+            if (!mbar_wait(full + buf, par, a.err, 15)) {
+                *fail = 1;
+                mbar_wait(full + buf, par, a.err, 15);
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t A = su32(smem + buf * stage), B = A + abytes;
+            const uint32_t rowb = (uint32_t)a.nch * PX * 16;
+            const uint64_t da = cdesc(A + (uint32_t)(g0 - r0 * a.nch) * PX * 16, rowb, PX * 16);
+            const uint64_t db = cdesc(B, TX * 16, TY * TX * 16);
+            const uint64_t pa = (uint64_t)(apart >> 4), pb = (uint64_t)(BPART >> 4);
+            for (int k = 0; k < TY / 2; k++)
+                for (int dx = 0; dx < 3; dx++) {
+                    const uint64_t oa = (uint64_t)((2 * k * rowb + dx * 16) >> 4);
+                    const uint64_t ob = (uint64_t)((2 * k * TX * 16) >> 4);
+                    const uint32_t d = tmem + dx * NP;
+                    umma(d, da + oa, db + ob, idesc, (s | k) ? 1u : 0u);
+                    umma(d, da + oa + pa, db + ob, idesc, 1u);
+                    umma(d, da + oa, db + ob + pb, idesc, 1u);
+                }
+            umma_commit(empty + buf);
+        }
+        umma_commit(done);
+    }
+    __syncwarp();
+    bool ok = mbar_wait(done, 0u, a.err, 16);
+    ok = !__syncthreads_or(!ok) && !*fail;
+    if (ok) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int row = g0 * 8 + tid, nrow = 3 * a.nch * 8;
+        for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+            for (int h = 0; h < NP / 32; h++) {
+                float d[32];
+                tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + dx * NP + h * 32, d);
+                if (row < nrow)
+#pragma unroll
+                    for (int n = 0; n < 32; n++) {
+                        const int o = h * 32 + n;
+                        if (o >= a.O) break;
+                        a.part[(((long)blockIdx.x * 3 + dx) * a.O + o) * nrow + row] = d[n];
+                    }
+            }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) tmem_free(tmem, TCOLS);
 }
 
-int *g_ct_err = nullptr;      // error word of the bounded waits (device)
-std::mutex g_ct_mtx;          // serialises the lazy allocations of this file
+// Sums of the slabs' partial results in slab order: 32 elements per block,
+// eight interleaved shares of the slabs each, all layers in one launch.
+struct SumJobs {
+    struct Job {
+        const float *part;
+        float *out;
+        long n, stride;          // elements, and the distance of two slabs
+        int nslab, O, C;         // C > 0: [dx][O][dy C] to [O][C][dy dx]
+        unsigned end;            // end of the job's blocks
+    } j[CONV_MAX_SUMS];
+    int n;
+};
+
+__global__ void __launch_bounds__(256) k_ct_sum(SumJobs jobs) {
+    __shared__ float red[8][32];
+    int q = 0;
+    while (blockIdx.x >= jobs.j[q].end) q++;
+    const SumJobs::Job &j = jobs.j[q];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long e = (long)(blockIdx.x - (q ? jobs.j[q - 1].end : 0)) * 32 + lane;
+    float s = 0.f;
+    if (e < j.n) {
+#pragma unroll 8
+        for (int k = w; k < j.nslab; k += 8) s += j.part[k * j.stride + e];
+    }
+    red[w][lane] = s;
+    __syncthreads();
+    if (w || e >= j.n) return;
+    for (int k = 1; k < 8; k++) s += red[k][lane];
+    long o = e;
+    if (j.C > 0) {
+        const int nrow = 3 * j.C, row = (int)(e % nrow), oc = (int)(e / nrow % j.O), dx = (int)(e / ((long)nrow * j.O));
+        o = ((long)oc * j.C + row % j.C) * 9 + (row / j.C) * 3 + dx;
+    }
+    j.out[o] = s;
+}
+
+// ---------------------------------------------------------------------------
+// Host side
+// ---------------------------------------------------------------------------
+typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiled ct_encode() {
+    static const EncodeTiled fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) !=
+                cudaSuccess || q != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return (EncodeTiled)p;
+    }();
+    return fn;
+}
+
+// The split activations [2 B][nch][H][W][8] as a 4-D map whose boxes are bx
+// pixels wide.  chunk_inner: dimensions (pixel, chunk, row, part) instead of
+// (pixel, row, chunk, part).
+int ct_map(CUtensorMap *m, const void *base, int B, int nch, int H, int W, bool chunk_inner, int bx, int brows,
+           int bch) {
+    EncodeTiled enc = ct_encode();
+    if (!enc) return E_CUDA;
+    const cuuint64_t row = (cuuint64_t)W * 16, chunk = row * H;
+    cuuint64_t dims[4] = {(cuuint64_t)W * 8, (cuuint64_t)H, (cuuint64_t)nch, (cuuint64_t)B * 2};
+    cuuint64_t strides[3] = {row, chunk, chunk * nch};
+    cuuint32_t box[4] = {(cuuint32_t)bx * 8, (cuuint32_t)brows, (cuuint32_t)bch, 2};
+    cuuint32_t es[4] = {1, 1, 1, 1};
+    if (chunk_inner) {
+        std::swap(dims[1], dims[2]);
+        std::swap(strides[0], strides[1]);
+        std::swap(box[1], box[2]);
+    }
+    const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(base), dims, strides, box, es,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? OK : E_CUDA;
+}
+
+std::mutex g_ct_mtx;          // serialises the lazy allocation of the error word
+int *g_ct_err = nullptr;      // error word of the bounded waits: mapped host memory, read after a
+                              // synchronisation without a copy
 
 int ct_err_word(int **p) {
     std::lock_guard<std::mutex> lk(g_ct_mtx);
     if (!g_ct_err) {
-        CK(cudaMalloc(&g_ct_err, sizeof(int)));
-        CK(cudaMemset(g_ct_err, 0, sizeof(int)));
+        CK(cudaHostAlloc(&g_ct_err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+        *g_ct_err = 0;
     }
-    *p = g_ct_err;
+    CK(cudaHostGetDevicePointer(p, g_ct_err, 0));
     return OK;
 }
 
-// The B operand of a forward or data-gradient launch, packed by k_ct_pack into
-// one device buffer that the launches reuse in turn.  The network is a
-// process-wide singleton driven from one stream (surrogate.cu); the buffer
-// follows the same rule, and its (re)allocation is serialised.
-__nv_bfloat16 *g_ct_w = nullptr;
-long g_ct_w_cap = 0;
+int ct_tiles_x(int Wo) { return (Wo + TX - 1) / TX; }
+int ct_tiles(int Ho, int Wo) { return ct_tiles_x(Wo) * ((Ho + TY - 1) / TY); }
 
-int ct_pack(const __nv_bfloat16 *w, int C, int O, int op, int NP, long Kp, cudaStream_t st,
-            const __nv_bfloat16 **out) {
-    std::lock_guard<std::mutex> lk(g_ct_mtx);
-    const long n = (long)NP * Kp;
-    if (n > g_ct_w_cap) {
-        if (g_ct_w) cudaFree(g_ct_w);
-        g_ct_w = nullptr;
-        g_ct_w_cap = 0;
-        CK(cudaMalloc(&g_ct_w, sizeof(__nv_bfloat16) * n));
-        g_ct_w_cap = n;
-    }
-    k_ct_pack<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(w, C, O, op, NP, (int)Kp, g_ct_w);
+template <int NP, int EPI>
+int launch_conv(const CUtensorMap &m, ConvArgs &a, int B, cudaStream_t st) {
+    const int smem = std::min(a.nst, 2) * CtCfg<NP>::STAGE + CT_HEAD + 128;
+    static const cudaError_t attr = cudaFuncSetAttribute(
+        k_conv<NP, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * CtCfg<NP>::STAGE + CT_HEAD + 128);
+    CK(attr);
+    const dim3 grid((unsigned)ct_tiles(a.Ho, a.Wo), (unsigned)B);
+    k_conv<NP, EPI><<<grid, CT_THREADS, smem, st>>>(m, a);
     note_launch();
     CK(cudaGetLastError());
-    *out = g_ct_w;
     return OK;
 }
+
+int ct_rows(int nch) {
+    int span = 0;
+    for (int g = 0; g < 3 * nch; g += 16) span = std::max(span, (g + 15) / nch - g / nch);
+    return TY + span;
+}
+
+int ct_slabs(int ntiles, int nch) { return std::min(ntiles, std::max(1, 152 / ((3 * nch + 15) / 16))); }
 
 }  // namespace
 
-// y[b][o] = act(conv3x3(x[b]) + bias), with the pre-activation copied to pre.
-int conv_tc_forward(const float *x, long xbs, const int *idx, const __nv_bfloat16 *w, const float *bias, int B,
-                    int C, int O, int H, int W, float *y, float *pre, int act, void *stream) {
-    if (O < 1 || O > 64 || C < 1 || H < 3 || W < 3 || B < 1) return E_BAD_ARGUMENT;
-    TcConv a = {};
-    a.x = x; a.xbs = xbs; a.idx = idx; a.bias = bias; a.pre = pre; a.out = y;
-    a.B = B; a.C = C; a.O = O; a.H = H; a.W = W; a.act = act;
+size_t conv_split_bytes(int B, int C, int H, int W) { return (size_t)B * 2 * ((C + 7) / 8) * H * W * 16; }
+
+int conv_split(const float *x, long xbs, const int *idx, int B, int C, int H, int W, void *xs, void *stream) {
+    const long plane = (long)H * W;
+    const dim3 grid((unsigned)((plane + 255) / 256), (unsigned)((C + 7) / 8), (unsigned)B);
+    k_ct_split<<<grid, 256, 0, (cudaStream_t)stream>>>(x, xbs, idx, C, plane, (uint4 *)xs);
+    note_launch();
+    CK(cudaGetLastError());
+    return OK;
+}
+
+long conv_pack_elems(int K, int N) { return (long)((K + 31) / 32) * 9 * KC * (N <= 32 ? 32 : 64) * 8; }
+
+int conv_pack(const ConvPack *jobs, int n, const float *w, void *out, void *stream) {
+    PackJobs p = {};
+    p.n = n;
+    long end = 0;
+    for (int q = 0; q < n; q++) {
+        PackJobs::Job &j = p.j[q];
+        const ConvPack &c = jobs[q];
+        const int C = c.C, O = c.O;
+        j.w = c.w;
+        j.out = end;
+        j.flip = c.data ? 1 : 0;
+        j.K = c.data ? O : C;
+        j.N = c.data ? C : O;
+        j.NP = j.N <= 32 ? 32 : 64;
+        j.sk = (c.data ? C : 1) * 9;
+        j.sn = (c.data ? 1 : C) * 9;
+        j.end = end += conv_pack_elems(j.K, j.N);
+    }
+    k_ct_pack<<<(unsigned)((end + 255) / 256), 256, 0, (cudaStream_t)stream>>>(p, w, (__nv_bfloat16 *)out);
+    note_launch();
+    CK(cudaGetLastError());
+    return OK;
+}
+
+static int conv_args(ConvArgs &a, CUtensorMap &m, const void *xs, const void *wp, int B, int K, int H, int W,
+                     int origin, int Ho, int Wo) {
+    a = {};
+    a.w = (const uint8_t *)wp;
+    a.nch = (K + 7) / 8;
+    a.nst = (a.nch + KC - 1) / KC;
+    a.origin = origin;
+    a.Ho = Ho; a.Wo = Wo;
+    a.tiles_x = ct_tiles_x(Wo);
     int rc = ct_err_word(&a.err);
     if (rc) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
+    return ct_map(&m, xs, B, a.nch, H, W, false, PX, PY, KC);
+}
+
+int conv_hidden(const void *xs, const void *wp, const float *bias, int B, int C, int H, int W, void *ys, void *ds,
+                void *stream) {
+    if (C < 1 || H < 3 || W < 3 || B < 1) return E_BAD_ARGUMENT;
+    ConvArgs a;
+    CUtensorMap m;
+    int rc = conv_args(a, m, xs, wp, B, C, H, W, 0, H - 2, W - 2);
+    if (rc) return rc;
+    a.bias = bias; a.ys = (uint4 *)ys; a.ds_out = (float4 *)ds;
+    return launch_conv<32, CT_HIDDEN>(m, a, B, (cudaStream_t)stream);
+}
+
+int conv_output(const void *xs, const void *wp, const float *bias, int B, int C, int O, int H, int W, float *y,
+                void *stream) {
+    if (O < 1 || O > 64 || C < 1 || H < 3 || W < 3 || B < 1) return E_BAD_ARGUMENT;
+    ConvArgs a;
+    CUtensorMap m;
+    int rc = conv_args(a, m, xs, wp, B, C, H, W, 0, H - 2, W - 2);
+    if (rc) return rc;
+    a.bias = bias; a.y = y; a.O = O;
+    return O <= 32 ? launch_conv<32, CT_OUTPUT>(m, a, B, (cudaStream_t)stream)
+                   : launch_conv<64, CT_OUTPUT>(m, a, B, (cudaStream_t)stream);
+}
+
+long conv_bias_parts(int B, int H, int W) { return (long)B * ct_tiles(H, W); }
+
+int conv_data_grad(const void *dys, const void *wp, const void *ds, int B, int O, int H, int W, void *dxs,
+                   float *bpart, void *stream) {
+    if (O < 1 || H < 3 || W < 3 || B < 1) return E_BAD_ARGUMENT;
+    ConvArgs a;
+    CUtensorMap m;
+    int rc = conv_args(a, m, dys, wp, B, O, H - 2, W - 2, -2, H, W);
+    if (rc) return rc;
+    a.ds = (const float4 *)ds; a.ys = (uint4 *)dxs; a.bpart = bpart;
+    return launch_conv<32, CT_DATA>(m, a, B, (cudaStream_t)stream);
+}
+
+long conv_wgt_part(int B, int C, int O, int H, int W, int *nslab) {
+    *nslab = ct_slabs(B * ct_tiles(H - 2, W - 2), (C + 7) / 8);
+    return (long)*nslab * 9 * O * C;
+}
+
+int conv_weight_grad(const void *xs, const void *dys, int B, int C, int O, int H, int W, float *part, void *stream) {
+    if (O < 1 || O > 64 || C < 8 || C % 8 || H < 3 || W < 3 || B < 1) return E_BAD_ARGUMENT;
     const int NP = O <= 32 ? 32 : 64;
-    const long Kp = (9L * C + CT_K - 1) / CT_K * CT_K;
-    if ((rc = ct_pack(w, C, O, CT_FWD, NP, Kp, st, &a.w))) return rc;
-    const long opl = (long)(H - 2) * (W - 2);
-    dim3 grid((unsigned)((opl + CT_M - 1) / CT_M), (unsigned)B);
-    return NP == 32 ? launch_ct<CT_FWD, 32>(a, grid, st) : launch_ct<CT_FWD, 64>(a, grid, st);
-}
-
-// dx[b][c] = conv3x3^T(dy[b]) times silu'(pre) when pre is given.
-int conv_tc_data_grad(const float *dy, const __nv_bfloat16 *w, const float *pre, int B, int C, int O, int H, int W,
-                      float *dx, void *stream) {
-    if (C < 1 || C > 64 || O < 1 || H < 3 || W < 3 || B < 1) return E_BAD_ARGUMENT;
-    TcConv a = {};
-    a.dy = dy; a.pre = const_cast<float *>(pre); a.out = dx;
-    a.B = B; a.C = C; a.O = O; a.H = H; a.W = W;
+    WgtArgs a = {};
+    a.part = part; a.O = O;
+    a.nch = C / 8;
+    a.rows = ct_rows(a.nch);
+    a.tiles_x = ct_tiles_x(W - 2);
+    a.tiles_img = ct_tiles(H - 2, W - 2);
+    a.ntiles = B * a.tiles_img;
     int rc = ct_err_word(&a.err);
     if (rc) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
-    const int NP = C <= 32 ? 32 : 64;
-    const long Kp = (9L * O + CT_K - 1) / CT_K * CT_K;
-    if ((rc = ct_pack(w, C, O, CT_DATA, NP, Kp, st, &a.w))) return rc;
-    dim3 grid((unsigned)(((long)H * W + CT_M - 1) / CT_M), (unsigned)B);
-    return NP == 32 ? launch_ct<CT_DATA, 32>(a, grid, st) : launch_ct<CT_DATA, 64>(a, grid, st);
+    CUtensorMap xm, dm;
+    if ((rc = ct_map(&xm, xs, B, a.nch, H, W, true, PX, a.rows, a.nch))) return rc;
+    if ((rc = ct_map(&dm, dys, B, (O + 7) / 8, H - 2, W - 2, false, TX, TY, NP / 8))) return rc;
+    // two stages where they fit (C <= 128 with O <= 32)
+    constexpr int LIMIT = 227 * 1024;
+    const int stage = ((2 * a.rows * a.nch * PX * 16 + 127) & ~127) + NP * TY * TX * 4;
+    a.nbuf = 2 * stage + CT_HEAD + 128 <= LIMIT ? 2 : 1;
+    const int smem = a.nbuf * stage + CT_HEAD + 128;
+    if (smem > LIMIT) return E_UNSUPPORTED;
+    const dim3 grid((unsigned)ct_slabs(a.ntiles, a.nch), (unsigned)((3 * a.nch + 15) / 16));
+    auto kern = NP == 32 ? k_conv_wgt<32> : k_conv_wgt<64>;
+    static const cudaError_t a32 =
+        cudaFuncSetAttribute(k_conv_wgt<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, LIMIT);
+    static const cudaError_t a64 =
+        cudaFuncSetAttribute(k_conv_wgt<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, LIMIT);
+    CK(a32);
+    CK(a64);
+    kern<<<grid, CT_THREADS, smem, (cudaStream_t)stream>>>(xm, dm, a);
+    note_launch();
+    CK(cudaGetLastError());
+    return OK;
 }
 
-// Slabs of the weight gradient for a batch of B (H x W) inputs.
-long conv_tc_wgt_slabs(int B, int H, int W, int *kslab, int *per_img) {
-    const long opl = (long)(H - 2) * (W - 2);
-    const int ks = 1024;
-    const int spi = (int)((opl + ks - 1) / ks);
-    if (kslab) *kslab = ks;
-    if (per_img) *per_img = spi;
-    return (long)B * spi;
+int conv_sums(const ConvSum *jobs, int n, void *stream) {
+    SumJobs p = {};
+    p.n = n;
+    unsigned end = 0;
+    for (int q = 0; q < n; q++) {
+        const ConvSum &c = jobs[q];
+        SumJobs::Job &j = p.j[q];
+        j.part = c.part; j.out = c.out; j.n = c.n; j.stride = c.stride; j.nslab = c.nslab; j.O = c.O; j.C = c.C;
+        j.end = end += (unsigned)((c.n + 31) / 32);
+    }
+    k_ct_sum<<<end, 256, 0, (cudaStream_t)stream>>>(p);
+    note_launch();
+    CK(cudaGetLastError());
+    return OK;
 }
 
-// part[slab][O C 9 + O]: the weight and bias gradients of each slab.
-int conv_tc_weight_grad(const float *x, long xbs, const int *idx, const float *dy, int B, int C, int O, int H, int W,
-                        float *part, void *stream) {
-    if (O < 1 || O > 64 || C < 1 || H < 3 || W < 3 || B < 1) return E_BAD_ARGUMENT;
-    TcConv a = {};
-    a.x = x; a.xbs = xbs; a.idx = idx; a.dy = dy; a.out = part;
-    a.B = B; a.C = C; a.O = O; a.H = H; a.W = W;
-    int rc = ct_err_word(&a.err);
-    if (rc) return rc;
-    const long nslab = conv_tc_wgt_slabs(B, H, W, &a.kslab, &a.slabs_per_img);
-    dim3 grid((unsigned)nslab, (unsigned)((9L * C + CT_M - 1) / CT_M));
-    cudaStream_t st = (cudaStream_t)stream;
-    return O <= 32 ? launch_ct<CT_WGT, 32>(a, grid, st) : launch_ct<CT_WGT, 64>(a, grid, st);
-}
-
-// The error word of the bounded waits (0: none expired); reading clears it.
-int conv_tc_error(void *stream) {
+// The error word of the bounded waits after the stream's work (0: none
+// expired); reading clears it.
+int conv_error(void *stream) {
+    if (cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) return -1;
+    std::lock_guard<std::mutex> lk(g_ct_mtx);
     if (!g_ct_err) return 0;
-    int h = 0;
-    cudaStream_t st = (cudaStream_t)stream;
-    if (cudaMemcpyAsync(&h, g_ct_err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return -1;
-    if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
-    if (h) cudaMemsetAsync(g_ct_err, 0, sizeof(int), st);
+    const int h = *(volatile int *)g_ct_err;
+    *g_ct_err = 0;
     return h;
 }
 

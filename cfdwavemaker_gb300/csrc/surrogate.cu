@@ -33,6 +33,7 @@
 // The features form their phases in float-float arithmetic in the kernel (no
 // FP64 phasor table of the halo grid).
 #include "cfdwm.h"
+#include "convtc.h"
 #include "ffmath.cuh"
 #include "sgrid_geom.cuh"
 
@@ -59,21 +60,11 @@ namespace cfdwm {
 
 GridGeom grid_geom(const DevGrid &g);
 
-// convtc.cu: valid 3x3 convolutions on the tcgen05 tensor cores
-int conv_tc_forward(const float *x, long xbs, const int *idx, const __nv_bfloat16 *w, const float *bias, int B,
-                    int C, int O, int H, int W, float *y, float *pre, int act, void *stream);
-int conv_tc_data_grad(const float *dy, const __nv_bfloat16 *w, const float *pre, int B, int C, int O, int H, int W,
-                      float *dx, void *stream);
-long conv_tc_wgt_slabs(int B, int H, int W, int *kslab, int *per_img);
-int conv_tc_weight_grad(const float *x, long xbs, const int *idx, const float *dy, int B, int C, int O, int H, int W,
-                        float *part, void *stream);
-int conv_tc_error(void *stream);
-
 namespace {
 
 constexpr int SH = 4;        // halo columns per side: 4 valid 3x3 convolutions
 constexpr int NQ = 8;        // first-order channels per level
-constexpr int HID = 32;      // hidden channels
+constexpr int HID = CONV_HID;   // hidden channels
 constexpr float LOG2E = 1.4426950408889634f;
 
 
@@ -239,46 +230,54 @@ __global__ void k_halo_coords(GridGeom g, int nxh, int nyh, double *xy) {
     xy[n + p] = g.d2 + g.dy * (jh - SH);
 }
 
-// grad[e] = sum over slabs of part[slab][e], in slab order
-__global__ void k_sum_slabs(long per, int nslab, const float *part, float *gw, float *gb, long nw) {
-    long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (e >= per) return;
-    float s = 0.f;
-    for (int k = 0; k < nslab; k++) s += part[(long)k * per + e];
-    if (e < nw) gw[e] = s;
-    else gb[e - nw] = s;
-}
-
 // Weighted mean-square loss and its gradient:
 //   L = sum_{b,o,p} w_o (y - t)^2 / (B P sum_o w_o),  dy = 2 w_o (y - t) / (B P sum w)
-__global__ void __launch_bounds__(256) k_surr_loss(const float *y, const float *tg, long tbs, const int *idx,
-                                                   int B, int O, long P, float w0, float inv_norm, float *dy,
-                                                   float *lpart) {
-    __shared__ float red[256];
-    long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    long n = (long)B * O * P;
-    float l = 0.f;
-    if (e < n) {
-        int b = (int)(e / ((long)O * P));
-        long r = e % ((long)O * P);
-        int o = (int)(r / P);
-        float wo = (o == 0) ? w0 : 1.f;
-        float t = tg[(long)(idx ? idx[b] : b) * tbs + r];
-        float d = y[e] - t;
-        l = wo * d * d * inv_norm;
-        if (dy) dy[e] = 2.f * wo * d * inv_norm;
+// A thread makes eight channels of a pixel, so that the gradient leaves in the
+// convolutions' split format; a block's sums of dy are its share of the output
+// bias gradient.
+__global__ void __launch_bounds__(256) k_surr_loss(const float *y, const float *tg, long tbs, const int *idx, int O,
+                                                   long P, float w0, float inv_norm, uint4 *dys, float *lpart,
+                                                   float *bpart) {
+    __shared__ float red[8][9];
+    const long p = blockIdx.x * 256L + threadIdx.x;
+    const int ch = blockIdx.y, nch = gridDim.y, b = blockIdx.z;
+    float v[9];                                   // dy of the eight channels, then the loss
+    v[8] = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+        const int o = ch * 8 + e;
+        v[e] = 0.f;
+        if (p < P && o < O) {
+            const float wo = (o == 0) ? w0 : 1.f;
+            const float d = y[((long)b * O + o) * P + p] - tg[(long)(idx ? idx[b] : b) * tbs + (long)o * P + p];
+            v[8] += wo * d * d * inv_norm;
+            v[e] = 2.f * wo * d * inv_norm;
+        }
     }
-    red[threadIdx.x] = l;
+    if (p < P) {
+        uint4 hi, lo;
+        conv_split8(v, hi, lo);
+        dys[((long)(b * 2) * nch + ch) * P + p] = hi;
+        dys[((long)(b * 2 + 1) * nch + ch) * P + p] = lo;
+    }
+#pragma unroll
+    for (int q = 0; q < 9; q++)
+        for (int s = 16; s > 0; s >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], s);
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int q = 0; q < 9; q++) red[threadIdx.x >> 5][q] = v[q];
     __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
+    if (threadIdx.x < 9) {
+        float t = 0.f;
+        for (int k = 0; k < 8; k++) t += red[k][threadIdx.x];
+        const long blk = (long)b * gridDim.x + blockIdx.x;
+        if (threadIdx.x < 8) bpart[(blk * nch + ch) * 8 + threadIdx.x] = t;
+        else lpart[blk * nch + ch] = t;
     }
-    if (threadIdx.x == 0) lpart[blockIdx.x] = red[0];
 }
 
 __global__ void k_adam(long n, float lr, float b1, float b2, float eps, float c1, float c2, const float *g,
-                       float *w, float *m, float *v, __nv_bfloat16 *wbf, long nweights_bf) {
+                       float *w, float *m, float *v) {
     long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (e >= n) return;
     float gg = g[e];
@@ -286,14 +285,7 @@ __global__ void k_adam(long n, float lr, float b1, float b2, float eps, float c1
     float vv = b2 * v[e] + (1.f - b2) * gg * gg;
     m[e] = mm;
     v[e] = vv;
-    float ww = w[e] - lr * (mm * c1) / (sqrtf(vv * c2) + eps);
-    w[e] = ww;
-    if (e < nweights_bf) wbf[e] = __float2bfloat16_rn(ww);
-}
-
-__global__ void k_to_bf16(long n, const float *w, __nv_bfloat16 *wbf) {
-    long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (e < n) wbf[e] = __float2bfloat16_rn(w[e]);
+    w[e] -= lr * (mm * c1) / (sqrtf(vv * c2) + eps);
 }
 
 // ---------------------------------------------------------------------------
@@ -408,13 +400,19 @@ struct Surrogate {
     int ch[5] = {0, 0, 0, 0, 0};
     long off_w[4] = {0, 0, 0, 0}, off_b[4] = {0, 0, 0, 0}, nparams = 0;
     float *w32 = nullptr, *m1 = nullptr, *m2 = nullptr, *grad = nullptr;
-    __nv_bfloat16 *wbf = nullptr;
+    // BF16 weights as the convolutions read them, laid out anew when w32
+    // changes: forward [0, 4) and data gradient [1, 4) of each layer
+    __nv_bfloat16 *wp = nullptr;
+    long off_f[4] = {0, 0, 0, 0}, off_d[4] = {0, 0, 0, 0};
+    ConvPack pack[7];
     long adam_step = 0;
     // training / gradient scratch
     void *tr = nullptr;
     size_t tr_bytes = 0;
     int *d_idx = nullptr;
     int idx_cap = 0;
+    float *h_loss = nullptr;   // pinned: the loss's block sums
+    long loss_cap = 0;
     // grid-side buffers
     int gnx = 0, gny = 0, gnl = 0;
     const float *g_eta = nullptr;      // identity of the attached grid
@@ -452,8 +450,9 @@ static void free_grid_side(Surrogate &s) {
 
 static void free_all(Surrogate &s) {
     free_grid_side(s);
-    void *q[] = {s.w32, s.m1, s.m2, s.grad, s.wbf, s.tr, s.d_idx};
+    void *q[] = {s.w32, s.m1, s.m2, s.grad, s.wp, s.tr, s.d_idx};
     for (void *p : q) if (p) cudaFree(p);
+    if (s.h_loss) cudaFreeHost(s.h_loss);
     s = Surrogate();
 }
 
@@ -467,6 +466,8 @@ static double rnd_unit(unsigned long long &st) {
     return ((z >> 11) + 0.5) * (1.0 / 9007199254740992.0);
 }
 
+static int pack_weights(const Surrogate &s, cudaStream_t st) { return conv_pack(s.pack, 7, s.w32, s.wp, st); }
+
 int surrogate_create(int nl, unsigned long long seed, void *stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
     if (nl < 1 || nl > 32) return E_BAD_ARGUMENT;
@@ -478,10 +479,18 @@ int surrogate_create(int nl, unsigned long long seed, void *stream_) {
     int ch[5] = {s.cin, HID, HID, HID, s.cout};
     std::memcpy(s.ch, ch, sizeof(ch));
     long off = 0;
-    // all weight blocks first (they have BF16 copies), then the biases
+    // all weight blocks first, then the biases
     for (int l = 0; l < 4; l++) { s.off_w[l] = off; off += (long)ch[l + 1] * ch[l] * 9; }
     for (int l = 0; l < 4; l++) { s.off_b[l] = off; off += ch[l + 1]; }
     s.nparams = off;
+    long op = 0;
+    for (int q = 0; q < 7; q++) {
+        const bool data = q >= 4;
+        const int l = data ? q - 3 : q;
+        s.pack[q] = {s.off_w[l], ch[l], ch[l + 1], data};
+        (data ? s.off_d : s.off_f)[l] = op;
+        op += data ? conv_pack_elems(ch[l + 1], ch[l]) : conv_pack_elems(ch[l], ch[l + 1]);
+    }
     std::vector<float> w(off, 0.f);
     unsigned long long st = seed;
     for (int l = 0; l < 4; l++) {
@@ -495,13 +504,12 @@ int surrogate_create(int nl, unsigned long long seed, void *stream_) {
     CK(cudaMalloc(&s.m1, sizeof(float) * off));
     CK(cudaMalloc(&s.m2, sizeof(float) * off));
     CK(cudaMalloc(&s.grad, sizeof(float) * off));
-    CK(cudaMalloc(&s.wbf, sizeof(__nv_bfloat16) * s.off_b[0]));
+    CK(cudaMalloc(&s.wp, sizeof(__nv_bfloat16) * op));
     CK(cudaMemcpyAsync(s.w32, w.data(), sizeof(float) * off, cudaMemcpyHostToDevice, stream));
     CK(cudaMemsetAsync(s.m1, 0, sizeof(float) * off, stream));
     CK(cudaMemsetAsync(s.m2, 0, sizeof(float) * off, stream));
-    k_to_bf16<<<(unsigned)((s.off_b[0] + 255) / 256), 256, 0, stream>>>(s.off_b[0], s.w32, s.wbf);
-    note_launch();
-    CK(cudaGetLastError());
+    int rc = pack_weights(s, stream);
+    if (rc) return rc;
     CK(cudaStreamSynchronize(stream));
     s.ready = true;
     return OK;
@@ -528,46 +536,18 @@ int surrogate_set_params(const float *src, long n, void *stream_) {
     CK(cudaMemsetAsync(g_s.m1, 0, sizeof(float) * n, stream));
     CK(cudaMemsetAsync(g_s.m2, 0, sizeof(float) * n, stream));
     g_s.adam_step = 0;
-    k_to_bf16<<<(unsigned)((g_s.off_b[0] + 255) / 256), 256, 0, stream>>>(g_s.off_b[0], g_s.w32, g_s.wbf);
-    note_launch();
-    CK(cudaGetLastError());
+    int rc = pack_weights(g_s, stream);
+    if (rc) return rc;
     CK(cudaStreamSynchronize(stream));
     return OK;
 }
 
-// ---- layer launchers ------------------------------------------------------
+// ---- layers ---------------------------------------------------------------
 // The convolutions run as implicit GEMMs on the tcgen05 tensor cores
 // (convtc.cu); the error word of their bounded waits is read where a call
 // synchronises anyway.
-static int conv_fwd(const Surrogate &s, int l, const float *x, long xbs, const int *idx, int B, int H, int W,
-                    float *y, float *pre, int act, cudaStream_t st) {
-    return conv_tc_forward(x, xbs, idx, s.wbf + s.off_w[l], s.w32 + s.off_b[l], B, s.ch[l], s.ch[l + 1], H, W, y,
-                           pre, act, st);
-}
-
-static int conv_bwd_data(const Surrogate &s, int l, const float *dy, const float *pre, int B, int H, int W,
-                         float *dx, cudaStream_t st) {
-    return conv_tc_data_grad(dy, s.wbf + s.off_w[l], pre, B, s.ch[l], s.ch[l + 1], H, W, dx, st);
-}
-
-static long wgt_slabs(int B, int H, int W) { return conv_tc_wgt_slabs(B, H, W, nullptr, nullptr); }
-
-static int conv_bwd_wgt(Surrogate &s, int l, const float *x, long xbs, const int *idx, const float *dy, int B,
-                        int H, int W, float *part, cudaStream_t st) {
-    const int C = s.ch[l], O = s.ch[l + 1];
-    int rc = conv_tc_weight_grad(x, xbs, idx, dy, B, C, O, H, W, part, st);
-    if (rc) return rc;
-    const long nslab = wgt_slabs(B, H, W);
-    long nw = (long)O * C * 9, per = nw + O;
-    k_sum_slabs<<<(unsigned)((per + 255) / 256), 256, 0, st>>>(per, (int)nslab, part, s.grad + s.off_w[l],
-                                                                s.grad + s.off_b[l], nw);
-    note_launch();
-    CK(cudaGetLastError());
-    return OK;
-}
-
 static int conv_check(cudaStream_t st) {
-    int e = conv_tc_error(st);
+    int e = conv_error(st);
     if (e == 0) return OK;
     std::fprintf(stderr, "cfdwm: a bounded wait of the tensor-core convolutions expired (code %d)\n", e);
     return E_CUDA;
@@ -583,66 +563,104 @@ static int reserve_tr(Surrogate &s, size_t bytes) {
     return OK;
 }
 
+static size_t up256(size_t b) { return (b + 255) / 256 * 256; }
+
+// The network over split inputs xs: hidden activations h[1..3] (split) and,
+// for the backward pass, silu' of their pre-activations ds[1..3] (null: not
+// kept); output planes y.
+static int net_forward(const Surrogate &s, const void *xs, int B, int H, int W, void *const *h, void *const *ds,
+                       float *y, cudaStream_t st) {
+    const void *in = xs;
+    for (int l = 0; l < 3; l++) {
+        int rc = conv_hidden(in, s.wp + s.off_f[l], s.w32 + s.off_b[l], B, s.ch[l], H - 2 * l, W - 2 * l, h[l + 1],
+                             ds ? ds[l + 1] : nullptr, st);
+        if (rc) return rc;
+        in = h[l + 1];
+    }
+    return conv_output(in, s.wp + s.off_f[3], s.w32 + s.off_b[3], B, HID, s.cout, H - 6, W - 6, y, st);
+}
+
 // Forward + loss + backward into s.grad.  x: [*][cin][H][W], tg: [*][cout][H-8][W-8],
-// batch entries idx[0..B) (device) or 0..B-1.
+// batch entries idx[0..B) (device) or 0..B-1.  The loss's nloss block sums
+// come to s.h_loss when want_loss is set (finish_loss).
 static int loss_grad(Surrogate &s, const float *x, const float *tg, const int *idx, int B, int H, int W,
-                     double *loss, cudaStream_t st) {
-    if (H < 9 || W < 9 || B < 1) return E_BAD_ARGUMENT;
-    const long P1 = (long)(H - 2) * (W - 2), P2 = (long)(H - 4) * (W - 4), P3 = (long)(H - 6) * (W - 6),
-               P4 = (long)(H - 8) * (W - 8);
-    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-    size_t n1 = up(sizeof(float) * B * HID * P1), n2 = up(sizeof(float) * B * HID * P2),
-           n3 = up(sizeof(float) * B * HID * P3), n4 = up(sizeof(float) * B * s.cout * P4);
-    long maxpart = 0;
-    int HH[4] = {H, H - 2, H - 4, H - 6}, WW[4] = {W, W - 2, W - 4, W - 6};
-    for (int l = 0; l < 4; l++)
-        maxpart = std::max(maxpart, wgt_slabs(B, HH[l], WW[l]) * ((long)s.ch[l + 1] * s.ch[l] * 9 + s.ch[l + 1]));
-    long nl4 = ((long)B * s.cout * P4 + 255) / 256;
-    size_t npart = up(sizeof(float) * maxpart), nloss = up(sizeof(float) * nl4);
-    // a1 h1 a2 h2 a3 h3 y dy da3 da2 da1 part lpart
-    size_t bytes = 2 * n1 + 2 * n2 + 2 * n3 + 2 * n4 + n3 + n2 + n1 + npart + nloss;
+                     bool want_loss, long *nloss, cudaStream_t st) {
+    if (H < 9 || W < 9 || B < 1 || s.cout > 64) return E_BAD_ARGUMENT;
+    const long P4 = (long)(H - 8) * (W - 8);
+    const int nco = (s.cout + 7) / 8;
+    const long lblk = (P4 + 255) / 256, nl4 = lblk * nco * B;
+    // split input, h ds da of the hidden layers, y, dys, partial sums
+    size_t bytes = 0;
+    auto take = [&](size_t n) { size_t o = bytes; bytes += up256(n); return o; };
+    const size_t o_x = take(conv_split_bytes(B, s.cin, H, W));
+    size_t o_h[4] = {}, o_s[4] = {}, o_a[4] = {}, o_p[4] = {}, o_b[4] = {};
+    int slabs[4];
+    for (int l = 0; l < 4; l++) {
+        const int h = H - 2 * l, w = W - 2 * l;
+        o_p[l] = take(sizeof(float) * conv_wgt_part(B, s.ch[l], s.ch[l + 1], h, w, &slabs[l]));
+        if (l == 0) continue;
+        const size_t n = conv_split_bytes(B, HID, h, w);
+        o_h[l] = take(n);
+        o_s[l] = take(n);
+        o_a[l] = take(n);
+        o_b[l] = take(sizeof(float) * HID * conv_bias_parts(B, h, w));
+    }
+    const size_t o_y = take(sizeof(float) * B * s.cout * P4), o_dy = take(conv_split_bytes(B, s.cout, H - 8, W - 8));
+    const size_t o_l = take(sizeof(float) * nl4), o_bo = take(sizeof(float) * nl4 * 8);
     int rc = reserve_tr(s, bytes);
     if (rc) return rc;
-    char *p = (char *)s.tr;
-    float *a1 = (float *)p; p += n1;
-    float *h1 = (float *)p; p += n1;
-    float *a2 = (float *)p; p += n2;
-    float *h2 = (float *)p; p += n2;
-    float *a3 = (float *)p; p += n3;
-    float *h3 = (float *)p; p += n3;
-    float *y = (float *)p; p += n4;
-    float *dy = (float *)p; p += n4;
-    float *da3 = (float *)p; p += n3;
-    float *da2 = (float *)p; p += n2;
-    float *da1 = (float *)p; p += n1;
-    float *part = (float *)p; p += npart;
-    float *lpart = (float *)p;
-    const long xbs = (long)s.cin * H * W, tbs = (long)s.cout * P4;
-    if ((rc = conv_fwd(s, 0, x, xbs, idx, B, H, W, h1, a1, 1, st))) return rc;
-    if ((rc = conv_fwd(s, 1, h1, (long)HID * P1, nullptr, B, H - 2, W - 2, h2, a2, 1, st))) return rc;
-    if ((rc = conv_fwd(s, 2, h2, (long)HID * P2, nullptr, B, H - 4, W - 4, h3, a3, 1, st))) return rc;
-    if ((rc = conv_fwd(s, 3, h3, (long)HID * P3, nullptr, B, H - 6, W - 6, y, nullptr, 0, st))) return rc;
+    char *base = (char *)s.tr;
+    void *h[4], *ds[4], *da[5];
+    for (int l = 1; l < 4; l++) { h[l] = base + o_h[l]; ds[l] = base + o_s[l]; da[l] = base + o_a[l]; }
+    h[0] = base + o_x;
+    da[4] = base + o_dy;
+    float *y = (float *)(base + o_y), *lpart = (float *)(base + o_l), *bout = (float *)(base + o_bo);
+    const long tbs = (long)s.cout * P4;
+    if ((rc = conv_split(x, (long)s.cin * H * W, idx, B, s.cin, H, W, h[0], st))) return rc;
+    if ((rc = net_forward(s, h[0], B, H, W, h, ds, y, st))) return rc;
     const float w0 = (float)s.nl;
     const float inv_norm = (float)(1.0 / ((double)B * P4 * (w0 + (s.cout - 1))));
-    k_surr_loss<<<(unsigned)nl4, 256, 0, st>>>(y, tg, tbs, idx, B, s.cout, P4, w0, inv_norm, dy, lpart);
+    k_surr_loss<<<dim3((unsigned)lblk, (unsigned)nco, (unsigned)B), 256, 0, st>>>(
+        y, tg, tbs, idx, s.cout, P4, w0, inv_norm, (uint4 *)da[4], lpart, bout);
     note_launch();
     CK(cudaGetLastError());
-    if ((rc = conv_bwd_wgt(s, 3, h3, (long)HID * P3, nullptr, dy, B, H - 6, W - 6, part, st))) return rc;
-    if ((rc = conv_bwd_data(s, 3, dy, a3, B, H - 6, W - 6, da3, st))) return rc;
-    if ((rc = conv_bwd_wgt(s, 2, h2, (long)HID * P2, nullptr, da3, B, H - 4, W - 4, part, st))) return rc;
-    if ((rc = conv_bwd_data(s, 2, da3, a2, B, H - 4, W - 4, da2, st))) return rc;
-    if ((rc = conv_bwd_wgt(s, 1, h1, (long)HID * P1, nullptr, da2, B, H - 2, W - 2, part, st))) return rc;
-    if ((rc = conv_bwd_data(s, 1, da2, a1, B, H - 2, W - 2, da1, st))) return rc;
-    if ((rc = conv_bwd_wgt(s, 0, x, xbs, idx, da1, B, H, W, part, st))) return rc;
-    if (loss) {
-        std::vector<float> lp(nl4);
-        CK(cudaMemcpyAsync(lp.data(), lpart, sizeof(float) * nl4, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        double L = 0.0;
-        for (float v : lp) L += v;
-        *loss = L;
-        return conv_check(st);
+    ConvSum sums[8];
+    for (int l = 3; l >= 0; l--) {
+        const int hh = H - 2 * l, ww = W - 2 * l, C = s.ch[l], O = s.ch[l + 1];
+        float *part = (float *)(base + o_p[l]);
+        if ((rc = conv_weight_grad(h[l], da[l + 1], B, C, O, hh, ww, part, st))) return rc;
+        if (l && (rc = conv_data_grad(da[l + 1], s.wp + s.off_d[l], ds[l], B, O, hh, ww, da[l],
+                                      (float *)(base + o_b[l]), st)))
+            return rc;
+        sums[l] = {part, s.grad + s.off_w[l], 9L * O * C, 9L * O * C, slabs[l], O, C};
+        if (l == 3)
+            sums[4 + l] = {bout, s.grad + s.off_b[l], s.cout, 8L * nco, (int)(lblk * B), 0, 0};
+        else
+            sums[4 + l] = {(float *)(base + o_b[l + 1]), s.grad + s.off_b[l], HID, HID,
+                           (int)conv_bias_parts(B, hh - 2, ww - 2), 0, 0};
     }
+    if ((rc = conv_sums(sums, 8, st))) return rc;
+    *nloss = nl4;
+    if (want_loss) {
+        if (s.loss_cap < nl4) {
+            if (s.h_loss) cudaFreeHost(s.h_loss);
+            s.h_loss = nullptr;
+            s.loss_cap = 0;
+            CK(cudaMallocHost(&s.h_loss, sizeof(float) * nl4));
+            s.loss_cap = nl4;
+        }
+        CK(cudaMemcpyAsync(s.h_loss, lpart, sizeof(float) * nl4, cudaMemcpyDeviceToHost, st));
+    }
+    return OK;
+}
+
+// Synchronises; the loss from its block sums.
+static int finish_loss(const Surrogate &s, long nloss, double *loss, cudaStream_t st) {
+    int rc = conv_check(st);
+    if (rc) return rc;
+    double L = 0.0;
+    for (long k = 0; k < nloss; k++) L += s.h_loss[k];
+    *loss = L;
     return OK;
 }
 
@@ -661,9 +679,11 @@ int surrogate_loss_grad(const float *x, const float *tg, int B, int H, int W, do
                         void *stream_) {
     cudaStream_t st = (cudaStream_t)stream_;
     if (!g_s.ready) return E_NOT_INITIALIZED;
-    int rc = loss_grad(g_s, x, tg, nullptr, B, H, W, loss, st);
+    long nloss;
+    int rc = loss_grad(g_s, x, tg, nullptr, B, H, W, loss != nullptr, &nloss, st);
     if (rc) return rc;
     if (grad) CK(cudaMemcpyAsync(grad, g_s.grad, sizeof(float) * g_s.nparams, cudaMemcpyDefault, st));
+    if (loss) return finish_loss(g_s, nloss, loss, st);
     CK(cudaStreamSynchronize(st));
     return OK;
 }
@@ -678,17 +698,19 @@ int surrogate_train_step(const float *xs, const float *ts, long nsamples, const 
         if (idx_host[b] < 0 || idx_host[b] >= nsamples) return E_BAD_ARGUMENT;
     int rc = put_idx(s, idx_host, B, st);
     if (rc) return rc;
-    rc = loss_grad(s, xs, ts, s.d_idx, B, H, W, loss, st);
+    long nloss;
+    rc = loss_grad(s, xs, ts, s.d_idx, B, H, W, loss != nullptr, &nloss, st);
+    if (!rc && loss) rc = finish_loss(s, nloss, loss, st);
     if (rc) return rc;
     s.adam_step++;
     const double b1 = 0.9, b2 = 0.999;
     float c1 = (float)(1.0 / (1.0 - std::pow(b1, (double)s.adam_step)));
     float c2 = (float)(1.0 / (1.0 - std::pow(b2, (double)s.adam_step)));
     k_adam<<<(unsigned)((s.nparams + 255) / 256), 256, 0, st>>>(s.nparams, lr, (float)b1, (float)b2, 1e-8f, c1, c2,
-                                                                s.grad, s.w32, s.m1, s.m2, s.wbf, s.off_b[0]);
+                                                                s.grad, s.w32, s.m1, s.m2);
     note_launch();
     CK(cudaGetLastError());
-    return OK;
+    return pack_weights(s, st);
 }
 
 int surrogate_check(void *stream) { return conv_check((cudaStream_t)stream); }
@@ -697,19 +719,16 @@ int surrogate_forward(const float *x, int B, int H, int W, float *y, void *strea
     cudaStream_t st = (cudaStream_t)stream_;
     Surrogate &s = g_s;
     if (!s.ready) return E_NOT_INITIALIZED;
-    if (H < 9 || W < 9 || B < 1) return E_BAD_ARGUMENT;
-    const long P1 = (long)(H - 2) * (W - 2), P2 = (long)(H - 4) * (W - 4), P3 = (long)(H - 6) * (W - 6);
-    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-    size_t n1 = up(sizeof(float) * B * HID * P1), n2 = up(sizeof(float) * B * HID * P2),
-           n3 = up(sizeof(float) * B * HID * P3);
-    int rc = reserve_tr(s, n1 + n2 + n3);
+    if (H < 9 || W < 9 || B < 1 || s.cout > 64) return E_BAD_ARGUMENT;
+    size_t off[5] = {};
+    for (int l = 0; l < 4; l++) off[l + 1] = off[l] + up256(conv_split_bytes(B, s.ch[l], H - 2 * l, W - 2 * l));
+    int rc = reserve_tr(s, off[4]);
     if (rc) return rc;
-    float *h1 = (float *)s.tr, *h2 = (float *)((char *)s.tr + n1), *h3 = (float *)((char *)s.tr + n1 + n2);
+    void *h[4];
+    for (int l = 0; l < 4; l++) h[l] = (char *)s.tr + off[l];
     prof_begin(PK_SURR_NET, st);
-    if ((rc = conv_fwd(s, 0, x, (long)s.cin * H * W, nullptr, B, H, W, h1, nullptr, 1, st))) return rc;
-    if ((rc = conv_fwd(s, 1, h1, (long)HID * P1, nullptr, B, H - 2, W - 2, h2, nullptr, 1, st))) return rc;
-    if ((rc = conv_fwd(s, 2, h2, (long)HID * P2, nullptr, B, H - 4, W - 4, h3, nullptr, 1, st))) return rc;
-    rc = conv_fwd(s, 3, h3, (long)HID * P3, nullptr, B, H - 6, W - 6, y, nullptr, 0, st);
+    rc = conv_split(x, (long)s.cin * H * W, nullptr, B, s.cin, H, W, h[0], st);
+    if (!rc) rc = net_forward(s, h[0], B, H, W, h, nullptr, y, st);
     prof_end(PK_SURR_NET, st);
     return rc;
 }
