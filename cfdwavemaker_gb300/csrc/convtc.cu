@@ -37,6 +37,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <mutex>
+#include <utility>
 
 namespace cfdwm {
 
@@ -53,13 +54,8 @@ namespace cfdwm {
 namespace {
 
 constexpr int HID = CONV_HID;             // hidden channels: N of the forward and data-gradient GEMMs
-constexpr int TX = 8, TY = 16;            // pixel tile: 128 rows of D, a core matrix per tile row
-constexpr int PX = TX + 2, PY = TY + 2;   // the tile with its halo
-constexpr int KC = 4;                     // channel chunks (of 8) per stage: two K steps of 16
-constexpr int CHUNK = PX * PY * 16;       // bytes of a chunk's patch
-constexpr int APART = KC * CHUNK;         // of one split part of a stage
-constexpr int CT_THREADS = 128;           // a thread per TMEM lane
-constexpr int CT_HEAD = 64 + 4 * HID * 4; // barriers and flags, bias partial sums
+constexpr int SMS = 152;
+constexpr int SMEM_SM = 227 * 1024, SMEM_HALF = 112 * 1024;   // a CTA's shared memory, one or two on an SM
 
 __device__ __forceinline__ float ct_sigmoid(float a) { return 1.f / (1.f + expf(-a)); }
 
@@ -88,9 +84,17 @@ __device__ __forceinline__ void tmem_free(uint32_t tmem, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols));
 }
 
+// A launch may start while the one before it in the stream drains: what
+// precedes pdl_wait touches nothing that the earlier kernels write, and every
+// kernel of the chain waits, so that all earlier ones are complete after it.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // FP32 planes [idx b][C][plane] to the split format; a thread per (pixel, chunk).
 __global__ void __launch_bounds__(256) k_ct_split(const float *x, long xbs, const int *idx, int C, long plane,
                                                   uint4 *out) {
+    pdl_next();
+    pdl_wait();
     const long p = blockIdx.x * 256L + threadIdx.x;
     if (p >= plane) return;
     const int ch = blockIdx.y, nch = gridDim.y, b = blockIdx.z;
@@ -106,7 +110,7 @@ __global__ void __launch_bounds__(256) k_ct_split(const float *x, long xbs, cons
 
 // ---------------------------------------------------------------------------
 // Weights: the B operands of the forward and data-gradient GEMMs,
-// [stage][tap][KC][NP][8] BF16, a stage one bulk copy; zero past the channels.
+// [16 input channels][dy][2 chunks][dx][NP][8] BF16; zero past the channels.
 // ---------------------------------------------------------------------------
 struct PackJobs {
     struct Job {
@@ -124,9 +128,9 @@ __global__ void __launch_bounds__(256) k_ct_pack(PackJobs jobs, const float *w, 
     if (q == jobs.n) return;
     const PackJobs::Job &j = jobs.j[q];
     const long i = e - j.out;
-    const int c8 = (int)(i & 7), n = (int)(i / 8 % j.NP), kc = (int)(i / (8L * j.NP) % KC);
-    const int tap = (int)(i / (8L * j.NP * KC) % 9), st = (int)(i / (8L * j.NP * KC * 9));
-    const int k = (st * KC + kc) * 8 + c8;
+    const int c8 = (int)(i & 7), n = (int)(i / 8 % j.NP), dx = (int)(i / (8L * j.NP) % 3);
+    const int kc = (int)(i / (24L * j.NP) % 2), dy = (int)(i / (48L * j.NP) % 3), st = (int)(i / (144L * j.NP));
+    const int k = (st * 2 + kc) * 8 + c8, tap = dy * 3 + dx;
     float v = 0.f;
     if (k < j.K && n < j.N) v = w[j.w + (long)k * j.sk + (long)n * j.sn + (j.flip ? 8 - tap : tap)];
     out[e] = __float2bfloat16_rn(v);
@@ -137,6 +141,20 @@ __global__ void __launch_bounds__(256) k_ct_pack(PackJobs jobs, const float *w, 
 // ---------------------------------------------------------------------------
 enum { CT_HIDDEN = 0, CT_OUTPUT = 1, CT_DATA = 2 };
 
+// M = 128: 8 rows of 16 pixels.  An MMA costs about 33 + N / 2 cycles here (its
+// 4 KB of A from shared memory, measured with N = 32 and 64), so the three dx
+// of a kernel row share one MMA with N = 3 NP on the unshifted pixels, and the
+// epilogue adds the neighbouring pixels' columns: 81 cycles for what takes
+// 3 x 49 with a shifted operand per tap, less the two of 16 columns that give
+// no output.  16 pixels wide rather than 32: training patches are small (70
+// pixels are 5 tiles of 14, 3 of 30).
+constexpr int FW = 16, FX = FW - 2, FY = 8;          // patch width, output tile
+constexpr int FCHUNK = (FY + 2) * FW * 16;           // bytes of 8 channels' patch
+constexpr int FPART = 2 * FCHUNK, FSTAGE = 2 * FPART;   // 16 channels, hi and lo
+constexpr int FRING = 6;                             // stages in flight at most
+constexpr int F_THREADS = 320;
+constexpr int FHEAD = 256 + 4 * HID * 4;             // barriers and flags, bias sums
+
 struct ConvArgs {
     const uint8_t *w;            // packed weights
     const float *bias;           // HIDDEN, OUTPUT
@@ -144,272 +162,324 @@ struct ConvArgs {
     float4 *ds_out;              // HIDDEN: the same, or null
     uint4 *ys;                   // HIDDEN: activations, DATA: gradient, split format
     float *y;                    // OUTPUT: planes [b][O][Ho][Wo]
-    float *bpart;                // DATA: sums of the tile's gradient [tile][HID]
-    int nst, nch;                // stages; input chunks
+    float *bpart;                // DATA: sums of the CTA's gradients [CTA][HID]
+    int nst, ring;               // K stages of 16 channels; stage buffers
     int origin;                  // of the patch relative to the tile: 0, data gradient -2
-    int O, Ho, Wo, tiles_x;
+    int O, Ho, Wo, tiles_x, tiles_img, ntiles;
     int *err;
 };
 
 template <int NP> struct CtCfg {
-    static constexpr int BTILE = 9 * KC * NP * 16;
-    static constexpr int STAGE = 2 * APART + BTILE;
+    static constexpr int N = 3 * NP;
+    static constexpr int WSTAGE = 3 * 2 * N * 16;    // weights of a K stage
+    static constexpr int NACC = NP == 32 ? 2 : 1;    // accumulators, so that two CTAs fit an SM's TMEM
+    static constexpr uint32_t ACOLS = NP == 32 ? 128 : 256, TCOLS = NACC * ACOLS;
 };
 
-// A CTA makes one tile of 16 x 8 output pixels: M = 128, N = NP (the hidden
-// channels, or the output's padded), K = 32 channels x 9 taps per stage.
-// Thread 0 copies (two stages in flight), thread 32 issues the MMAs, the four
-// warps read their TMEM lanes.  The operand's 4 KB per MMA from shared memory
-// bound the tensor cores at these N (32 cycles an MMA); up to five CTAs an SM
-// overlap copies, MMAs and epilogues of different tiles.
+// A persistent CTA, two on an SM: the weights stay in shared memory, warp 0
+// copies patches through a ring of stages, warp 1 issues the MMAs, warps 2 to 9
+// (two to a lane quarter, half of the channels each) make the epilogue of one
+// tile while the next one accumulates.
 template <int NP, int EPI>
-__global__ void __launch_bounds__(CT_THREADS) k_conv(const __grid_constant__ CUtensorMap xm, ConvArgs a) {
+__global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ CUtensorMap xm, ConvArgs a) {
     using CF = CtCfg<NP>;
     extern __shared__ __align__(128) uint8_t ct_raw[];
-    uint8_t *smem = (uint8_t *)(((uintptr_t)ct_raw + 127) & ~(uintptr_t)127);
-    const int nbuf = a.nst < 2 ? a.nst : 2;
-    uint64_t *full = (uint64_t *)(smem + nbuf * CF::STAGE), *empty = full + 2, *done = full + 4;
-    uint32_t *tslot = (uint32_t *)(full + 5);
-    volatile int *fail = (volatile int *)(full + 6);
-    float *red = (float *)(full + 8);                 // DATA: [4][HID]
+    uint8_t *wsm = (uint8_t *)(((uintptr_t)ct_raw + 127) & ~(uintptr_t)127);
+    uint8_t *asm_ = wsm + a.nst * CF::WSTAGE;
+    uint64_t *full = (uint64_t *)(asm_ + a.ring * FSTAGE), *empty = full + FRING, *wfull = empty + FRING;
+    uint64_t *afull = wfull + 1, *aempty = afull + 2;
+    uint32_t *tslot = (uint32_t *)(aempty + 2);
+    volatile int *fail = (volatile int *)(tslot + 1);
+    float *red = (float *)(full + 32);                // DATA: [4][HID]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int b = blockIdx.y;
-    const int x0 = (blockIdx.x % a.tiles_x) * TX, y0 = (blockIdx.x / a.tiles_x) * TY;
     if (tid == 0) {
-        for (int q = 0; q < 5; q++) mbar_init(full + q, 1);
+        for (int q = 0; q < 2 * FRING + 3; q++) mbar_init(full + q, 1);
+        for (int q = 0; q < 2; q++) mbar_init(aempty + q, 8);
         *fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) tmem_alloc(tslot, NP);
+    if (warp == 0) tmem_alloc(tslot, CF::TCOLS);
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot;
+    pdl_next();
+    float bs = 0.f;
 
-    if (tid == 0) {
-        for (int s = 0; s < a.nst; s++) {
-            const int buf = s & 1;
-            if (s >= 2 && !mbar_wait(empty + buf, (uint32_t)(((s >> 1) - 1) & 1), a.err, 11)) { *fail = 1; break; }
-            uint8_t *st = smem + buf * CF::STAGE;
-            mbar_expect_tx(full + buf, CF::STAGE);
-            tma_4d(st, &xm, full + buf, (x0 + a.origin) * 8, y0 + a.origin, s * KC, b * 2);
-            bulk_load(st + 2 * APART, a.w + (long)s * CF::BTILE, CF::BTILE, full + buf);
-        }
-    } else if (tid == 32) {
-        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NP >> 3) << 17) |
-                               ((uint32_t)((TX * TY) >> 4) << 24);
-        for (int s = 0; s < a.nst; s++) {
-            const int buf = s & 1;
-            const uint32_t par = (uint32_t)((s >> 1) & 1);
-            if (!mbar_wait(full + buf, par, a.err, 12)) {
-                *fail = 1;
-                mbar_wait(full + buf, par, a.err, 12);
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t A = su32(smem + buf * CF::STAGE), B = A + 2 * APART;
-            const uint64_t da = cdesc(A, CHUNK, PX * 16), db = cdesc(B, NP * 16, 128);
-            const int nk = (min(KC, a.nch - s * KC) + 1) / 2;
-            for (int tap = 0; tap < 9; tap++)
-                for (int k = 0; k < nk; k++) {
-                    const uint64_t oa = (uint64_t)((2 * k * CHUNK + ((tap / 3) * PX + tap % 3) * 16) >> 4);
-                    const uint64_t ob = (uint64_t)(((tap * KC + 2 * k) * NP * 16) >> 4);
-                    umma(tmem, da + oa, db + ob, idesc, (s | tap | k) ? 1u : 0u);
-                    umma(tmem, da + oa + (APART >> 4), db + ob, idesc, 1u);
+    if (warp == 0) {
+        if (lane == 0) {
+            mbar_expect_tx(wfull, a.nst * CF::WSTAGE);
+            for (int s = 0; s < a.nst; s++)
+                bulk_load(wsm + s * CF::WSTAGE, a.w + (long)s * CF::WSTAGE, CF::WSTAGE, wfull);
+            pdl_wait();
+            int k = 0;                                // stages copied
+            bool ok = true;
+            for (int t = blockIdx.x; ok && t < a.ntiles; t += gridDim.x) {
+                const int b = t / a.tiles_img, r = t % a.tiles_img;
+                const int x0 = (r % a.tiles_x) * FX + a.origin, y0 = (r / a.tiles_x) * FY + a.origin;
+                for (int s = 0; s < a.nst; s++, k++) {
+                    const int buf = k % a.ring, use = k / a.ring;
+                    if (use && !mbar_wait(empty + buf, (uint32_t)((use - 1) & 1), a.err, 11)) { ok = false; break; }
+                    mbar_expect_tx(full + buf, FSTAGE);
+                    tma_4d(asm_ + buf * FSTAGE, &xm, full + buf, x0 * 8, y0, s * 2, b * 2);
                 }
-            umma_commit(empty + buf);
+            }
+            if (!ok) {
+                *fail = 1;                            // let the copies in flight land
+                for (int q = max(0, k - a.ring); q < k; q++)
+                    mbar_wait(full + q % a.ring, (uint32_t)((q / a.ring) & 1), a.err, 11);
+            }
         }
-        umma_commit(done);
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(CF::N >> 3) << 17) | (8u << 24);
+            const uint32_t W = su32(wsm);
+            bool ok = mbar_wait(wfull, 0u, a.err, 12);
+            int k = 0, i = 0;                         // stages, tiles
+            for (int t = blockIdx.x; ok && t < a.ntiles; t += gridDim.x, i++) {
+                const int acc = i % CF::NACC, use = i / CF::NACC;
+                if (use && !mbar_wait(aempty + acc, (uint32_t)((use - 1) & 1), a.err, 13)) { ok = false; break; }
+                const uint32_t d = tmem + acc * CF::ACOLS;
+                for (int s = 0; s < a.nst; s++, k++) {
+                    const int buf = k % a.ring;
+                    if (!mbar_wait(full + buf, (uint32_t)((k / a.ring) & 1), a.err, 14)) { ok = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t da = cdesc(su32(asm_ + buf * FSTAGE), FCHUNK, 128);
+                    const uint64_t db = cdesc(W + s * CF::WSTAGE, CF::N * 16, 128);
+                    for (int dy = 0; dy < 3; dy++) {
+                        const uint64_t oa = (uint64_t)((dy * FW * 16) >> 4), ob = (uint64_t)((dy * 2 * CF::N * 16) >> 4);
+                        umma(d, da + oa, db + ob, idesc, (s | dy) ? 1u : 0u);
+                        umma(d, da + oa + (FPART >> 4), db + ob, idesc, 1u);
+                    }
+                    umma_commit(empty + buf);
+                }
+                if (ok) umma_commit(afull + acc);
+            }
+            if (!ok) *fail = 1;
+        }
+    } else {
+        pdl_wait();
+        const int q = warp & 3, hf = (warp - 2) >> 2; // TMEM lane quarter, half of the channels
+        const int m = q * 32 + lane;                  // row of D
+        const int col = m & (FW - 1);
+        const long plane = (long)a.Ho * a.Wo;
+        int i = 0;
+        for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x, i++) {
+            const int acc = i % CF::NACC;
+            bool ok = mbar_wait(afull + acc, (uint32_t)((i / CF::NACC) & 1), a.err, 15);
+            if (!__all_sync(0xffffffffu, ok)) { *fail = 1; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + acc * CF::ACOLS;
+            const int b = t / a.tiles_img, r = t % a.tiles_img;
+            const int oy = (r / a.tiles_x) * FY + (m / FW), ox = (r % a.tiles_x) * FX + col;
+            const long pix = (long)oy * a.Wo + ox;
+            const bool live = col < FX && oy < a.Ho && ox < a.Wo;
+#pragma unroll
+            for (int k = 0; k < NP / 32; k++) {
+                const int h = hf * (NP / 32) + k;
+                float d[16], e1[16], e2[16];
+                tmem_ld16x3(ta + h * 16, NP, d, e1, e2);
+                if (k == NP / 32 - 1) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(aempty + acc);
+                }
+#pragma unroll
+                for (int n = 0; n < 16; n++)
+                    d[n] += __shfl_down_sync(0xffffffffu, e1[n], 1) + __shfl_down_sync(0xffffffffu, e2[n], 2);
+                if (EPI == CT_OUTPUT) {
+                    if (live)
+#pragma unroll
+                        for (int n = 0; n < 16; n++)
+                            if (h * 16 + n < a.O)
+                                a.y[((long)b * a.O + h * 16 + n) * plane + pix] = d[n] + a.bias[h * 16 + n];
+                }
+#pragma unroll
+                for (int c = 0; c < (EPI == CT_OUTPUT ? 0 : 2); c++) {
+                    float *v = d + c * 8, g[8];
+                    const int ch = h * 2 + c;                     // channel chunk
+                    if (EPI == CT_DATA) {
+#pragma unroll
+                        for (int f = 0; f < 2; f++) {
+                            float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (live) w = a.ds[((long)b * (HID / 4) + ch * 2 + f) * plane + pix];
+                            g[f * 4] = w.x; g[f * 4 + 1] = w.y; g[f * 4 + 2] = w.z; g[f * 4 + 3] = w.w;
+                        }
+#pragma unroll
+                        for (int e = 0; e < 8; e++) v[e] = live ? v[e] * g[e] : 0.f;
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; e++) {
+                            const float p = v[e] + a.bias[ch * 8 + e], sg = ct_sigmoid(p);
+                            v[e] = p * sg;
+                            g[e] = sg * (1.f + p * (1.f - sg));
+                        }
+                    }
+                    if (!live) continue;
+                    uint4 hi, lo;
+                    conv_split8(v, hi, lo);
+                    a.ys[((long)(b * 2) * (HID / 8) + ch) * plane + pix] = hi;
+                    a.ys[((long)(b * 2 + 1) * (HID / 8) + ch) * plane + pix] = lo;
+                    if (EPI == CT_HIDDEN && a.ds_out)
+#pragma unroll
+                        for (int f = 0; f < 2; f++)
+                            a.ds_out[((long)b * (HID / 4) + ch * 2 + f) * plane + pix] =
+                                make_float4(g[f * 4], g[f * 4 + 1], g[f * 4 + 2], g[f * 4 + 3]);
+                }
+                if (EPI == CT_DATA) {
+                    // the bias gradient's share: lane n ends with channel n of the warp's pixels
+#pragma unroll
+                    for (int o = 8; o >= 1; o >>= 1) {
+                        const bool up = lane & o;
+#pragma unroll
+                        for (int n = 0; n < o; n++) {
+                            const float send = up ? d[n] : d[n + o], keep = up ? d[n + o] : d[n];
+                            d[n] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                        }
+                    }
+                    bs += d[0] + __shfl_xor_sync(0xffffffffu, d[0], 16);
+                }
+            }
+        }
+        if (EPI == CT_DATA && lane < 16) red[q * HID + hf * 16 + lane] = bs;
     }
     __syncwarp();
-    bool ok = mbar_wait(done, 0u, a.err, 13);
-    ok = !__syncthreads_or(!ok) && !*fail;
-    if (ok) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16);
-        const int oy = y0 + (tid >> 3), ox = x0 + (tid & 7);
-        const long plane = (long)a.Ho * a.Wo, pix = (long)oy * a.Wo + ox;
-        const bool live = oy < a.Ho && ox < a.Wo;
-        if (EPI == CT_OUTPUT) {
-#pragma unroll
-            for (int h = 0; h < NP / 32; h++) {
-                float d[32];
-                tmem_ld32(ta + h * 32, d);
-                if (live)
-#pragma unroll
-                    for (int n = 0; n < 32; n++) {
-                        const int o = h * 32 + n;
-                        if (o >= a.O) break;
-                        a.y[((long)b * a.O + o) * plane + pix] = d[n] + a.bias[o];
-                    }
-            }
-        } else {
-            float d[32];
-            tmem_ld32(ta, d);
-#pragma unroll
-            for (int c = 0; c < HID / 8; c++) {
-                float v[8], g[8];
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    if (EPI == CT_DATA) {
-                        float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (live) f = a.ds[((long)b * (HID / 4) + c * 2 + q) * plane + pix];
-                        g[q * 4] = f.x; g[q * 4 + 1] = f.y; g[q * 4 + 2] = f.z; g[q * 4 + 3] = f.w;
-                    }
-                }
-#pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    if (EPI == CT_DATA) {
-                        v[e] = live ? d[c * 8 + e] * g[e] : 0.f;
-                        d[c * 8 + e] = v[e];
-                    } else {
-                        const float p = d[c * 8 + e] + a.bias[c * 8 + e], sg = ct_sigmoid(p);
-                        v[e] = p / (1.f + expf(-p));
-                        g[e] = sg * (1.f + p * (1.f - sg));
-                    }
-                }
-                if (!live) continue;
-                uint4 hi, lo;
-                conv_split8(v, hi, lo);
-                a.ys[((long)(b * 2) * (HID / 8) + c) * plane + pix] = hi;
-                a.ys[((long)(b * 2 + 1) * (HID / 8) + c) * plane + pix] = lo;
-                if (EPI == CT_HIDDEN && a.ds_out)
-#pragma unroll
-                    for (int q = 0; q < 2; q++)
-                        a.ds_out[((long)b * (HID / 4) + c * 2 + q) * plane + pix] =
-                            make_float4(g[q * 4], g[q * 4 + 1], g[q * 4 + 2], g[q * 4 + 3]);
-            }
-            if (EPI == CT_DATA) {
-                // the bias gradient's share of this tile: lane c ends with channel c of its warp's pixels
-#pragma unroll
-                for (int o = 16; o >= 1; o >>= 1) {
-                    const bool up = lane & o;
-#pragma unroll
-                    for (int i = 0; i < o; i++) {
-                        const float send = up ? d[i] : d[i + o], keep = up ? d[i + o] : d[i];
-                        d[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-                    }
-                }
-                red[warp * HID + lane] = d[0];
-            }
-        }
-    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (EPI == CT_DATA && ok && warp == 1)
-        a.bpart[((long)b * gridDim.x + blockIdx.x) * HID + lane] =
+    if (EPI == CT_DATA && warp == 2 && !*fail)
+        a.bpart[(long)blockIdx.x * HID + lane] =
             (red[lane] + red[HID + lane]) + (red[2 * HID + lane] + red[3 * HID + lane]);
-    if (warp == 0) tmem_free(tmem, NP);
+    if (warp == 0) tmem_free(tmem, CF::TCOLS);
 }
 
 // ---------------------------------------------------------------------------
 // Weight gradient
 // ---------------------------------------------------------------------------
-struct WgtArgs {
-    float *part;                 // [slab][3 dx][O][3 dy C]
-    int nch, rows;               // input chunks; patch rows copied
+constexpr int TX = 8, TY = 16;            // pixel tile: K = 128, a core matrix per tile row
+constexpr int PX = TX + 2;                // width of the patch
+constexpr int QCHUNK = TX * TY * 16;      // bytes of 8 channels of the plain tile
+constexpr int W_THREADS = 128;
+constexpr int W_UNITS = 12;               // (layer, M tile, N block) triples of a launch at most
+constexpr int WHEAD = 128;
+
+struct WgtUnit {
+    float *part;                 // [slab][dx][q][3 P]: the slabs' sums
+    int layer;                   // tensor maps
+    int nch, rows;               // P's chunks, patch rows copied
+    int g0, q0, N, Q;            // first row group, first q chunk, N of the MMAs, q channels in all
+    int origin;                  // of the patch relative to the tile: 0, or -2 (P is dy)
     int ntiles, tiles_x, tiles_img;
-    int nbuf;
-    int O;
+    int nslab, end;              // CTAs; end of the unit's blocks
+};
+
+struct WgtArgs {
+    CUtensorMap p[4], q[4];
+    WgtUnit u[W_UNITS];
     int *err;
 };
 
-// D's rows are (dy, c) pairs: with the patch copied as [row][chunk][pixel],
-// the row groups of 8 channels over dy and the chunks are one arithmetic
-// progression of addresses, so M = 128 holds 16 of them whatever C is (four
-// taps' worth of 32 channels; blockIdx.y counts the M tiles).  dx is a start
-// address, with an accumulator of its own.  K is the tile's pixels, two tile
-// rows per MMA.  A CTA sums its slab (every gridDim.x-th tile) in TMEM; the
-// slabs are summed in order afterwards, so the result is deterministic.
-template <int NP>
-__global__ void __launch_bounds__(CT_THREADS)
-k_conv_wgt(const __grid_constant__ CUtensorMap xm, const __grid_constant__ CUtensorMap dm, WgtArgs a) {
-    constexpr int BPART = (NP / 8) * TY * TX * 16;
-    constexpr uint32_t TCOLS = NP == 32 ? 128 : 256;
+// All layers in one launch, a CTA per SM.  D's rows are (t, p): with the patch
+// of P copied as [row][chunk][pixel], the row groups of 8 channels over the
+// three kernel rows t and the chunks are one arithmetic progression of
+// addresses, so M = 128 holds 16 of them (the kernel rows of 32 channels, and
+// a fourth that is not kept).  dx is a start address, with an accumulator of
+// its own; N are Q's channels, K the tile's pixels, two tile rows per MMA.
+// P is x and Q dy, or, where x has more channels, the other way round (taps
+// then run backwards): the layer with 128 inputs needs one M tile instead of
+// three, 97 cycles an MMA (33 + N / 2) instead of 3 x 49.
+// A CTA sums its slab (every nslab-th tile) in TMEM; the slabs are summed in
+// order afterwards, so the result is deterministic.  The CTAs are divided
+// between the units by their MMA cycles.
+__global__ void __launch_bounds__(W_THREADS) k_conv_wgt(const __grid_constant__ WgtArgs a) {
     extern __shared__ __align__(128) uint8_t ct_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)ct_raw + 127) & ~(uintptr_t)127);
-    const int apart = a.rows * a.nch * PX * 16, abytes = (2 * apart + 127) & ~127, stage = abytes + 2 * BPART;
-    uint64_t *full = (uint64_t *)(smem + a.nbuf * stage), *empty = full + 2, *done = full + 4;
+    uint64_t *full = (uint64_t *)smem, *empty = full + 2, *done = full + 4;
     uint32_t *tslot = (uint32_t *)(full + 5);
     volatile int *fail = (volatile int *)(full + 6);
+    smem += WHEAD;
     const int tid = threadIdx.x, warp = tid >> 5;
-    const int g0 = blockIdx.y * 16, r0 = g0 / a.nch;          // first row group of this M tile, its dy
+    int ui = 0;
+    while ((int)blockIdx.x >= a.u[ui].end) ui++;
+    const WgtUnit &u = a.u[ui];
+    const int slab = (int)blockIdx.x - (u.end - u.nslab);
+    const int r0 = u.g0 / u.nch, ppart = u.rows * u.nch * PX * 16, pbytes = (2 * ppart + 127) & ~127;
+    const int qpart = (u.N / 8) * QCHUNK, stage = pbytes + 2 * qpart;
     if (tid == 0) {
-        for (int q = 0; q < 5; q++) mbar_init(full + q, 1);
+        for (int k = 0; k < 5; k++) mbar_init(full + k, 1);
         *fail = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) tmem_alloc(tslot, TCOLS);
+    if (warp == 0) tmem_alloc(tslot, 512);
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot;
+    pdl_next();
+    pdl_wait();
 
     if (tid == 0) {
-        int s = 0;
-        for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x, s++) {
-            const int buf = s % a.nbuf, use = s / a.nbuf;
-            if (use > 0 && !mbar_wait(empty + buf, (uint32_t)((use - 1) & 1), a.err, 14)) { *fail = 1; break; }
-            const int b = t / a.tiles_img, r = t % a.tiles_img;
-            const int x0 = (r % a.tiles_x) * TX, y0 = (r / a.tiles_x) * TY;
+        const CUtensorMap *pm = &a.p[u.layer], *qm = &a.q[u.layer];
+        int k = 0;
+        bool ok = true;
+        for (int t = slab; t < u.ntiles; t += u.nslab, k++) {
+            const int buf = k & 1;
+            if (k > 1 && !mbar_wait(empty + buf, (uint32_t)(((k >> 1) - 1) & 1), a.err, 21)) { ok = false; break; }
+            const int b = t / u.tiles_img, r = t % u.tiles_img;
+            const int x0 = (r % u.tiles_x) * TX, y0 = (r / u.tiles_x) * TY;
             uint8_t *st = smem + buf * stage;
-            mbar_expect_tx(full + buf, 2 * apart + 2 * BPART);
-            tma_4d(st, &xm, full + buf, x0 * 8, 0, y0 + r0, b * 2);
-            tma_4d(st + abytes, &dm, full + buf, x0 * 8, y0, 0, b * 2);
+            mbar_expect_tx(full + buf, 2 * ppart + 2 * qpart);
+            tma_4d(st, pm, full + buf, (x0 + u.origin) * 8, 0, y0 + u.origin + r0, b * 2);
+            tma_4d(st + pbytes, qm, full + buf, x0 * 8, y0, u.q0, b * 2);
+        }
+        if (!ok) {
+            *fail = 1;                                // let the copies in flight land
+            for (int j = max(0, k - 2); j < k; j++) mbar_wait(full + (j & 1), (uint32_t)((j >> 1) & 1), a.err, 21);
         }
     } else if (tid == 32) {
         // both operands MN-major (bits 15 and 16)
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
-                               ((uint32_t)(NP >> 3) << 17) | (8u << 24);
-        int s = 0;
-        for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x, s++) {
-            const int buf = s % a.nbuf;
-            const uint32_t par = (uint32_t)((s / a.nbuf) & 1);
-            if (!mbar_wait(full + buf, par, a.err, 15)) {
-                *fail = 1;
-                mbar_wait(full + buf, par, a.err, 15);
-                break;
-            }
+                               ((uint32_t)(u.N >> 3) << 17) | (8u << 24);
+        int k = 0;
+        bool ok = true;
+        for (int t = slab; t < u.ntiles; t += u.nslab, k++) {
+            const int buf = k & 1;
+            if (!mbar_wait(full + buf, (uint32_t)((k >> 1) & 1), a.err, 22)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t A = su32(smem + buf * stage), B = A + abytes;
-            const uint32_t rowb = (uint32_t)a.nch * PX * 16;
-            const uint64_t da = cdesc(A + (uint32_t)(g0 - r0 * a.nch) * PX * 16, rowb, PX * 16);
-            const uint64_t db = cdesc(B, TX * 16, TY * TX * 16);
-            const uint64_t pa = (uint64_t)(apart >> 4), pb = (uint64_t)(BPART >> 4);
-            for (int k = 0; k < TY / 2; k++)
+            const uint32_t P = su32(smem + buf * stage), Q = P + pbytes, rowb = (uint32_t)u.nch * PX * 16;
+            const uint64_t dp = cdesc(P + (uint32_t)(u.g0 - r0 * u.nch) * PX * 16, rowb, PX * 16);
+            const uint64_t dq = cdesc(Q, TX * 16, QCHUNK);
+            const uint64_t lp = (uint64_t)(ppart >> 4), lq = (uint64_t)(qpart >> 4);
+            for (int y = 0; y < TY; y += 2)
                 for (int dx = 0; dx < 3; dx++) {
-                    const uint64_t oa = (uint64_t)((2 * k * rowb + dx * 16) >> 4);
-                    const uint64_t ob = (uint64_t)((2 * k * TX * 16) >> 4);
-                    const uint32_t d = tmem + dx * NP;
-                    umma(d, da + oa, db + ob, idesc, (s | k) ? 1u : 0u);
-                    umma(d, da + oa + pa, db + ob, idesc, 1u);
-                    umma(d, da + oa, db + ob + pb, idesc, 1u);
+                    const uint64_t op = (uint64_t)((y * rowb + dx * 16) >> 4), oq = (uint64_t)((y * TX * 16) >> 4);
+                    const uint32_t d = tmem + dx * u.N;
+                    umma(d, dp + op, dq + oq, idesc, (k | y) ? 1u : 0u);
+                    umma(d, dp + op + lp, dq + oq, idesc, 1u);
+                    umma(d, dp + op, dq + oq + lq, idesc, 1u);
                 }
             umma_commit(empty + buf);
         }
+        if (!ok) *fail = 1;
         umma_commit(done);
     }
     __syncwarp();
-    bool ok = mbar_wait(done, 0u, a.err, 16);
+    bool ok = mbar_wait(done, 0u, a.err, 23);
     ok = !__syncthreads_or(!ok) && !*fail;
     if (ok) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int row = g0 * 8 + tid, nrow = 3 * a.nch * 8;
+        const int row = u.g0 * 8 + tid, nrow = 3 * u.nch * 8, nq = min(u.N, u.Q - u.q0 * 8);
         for (int dx = 0; dx < 3; dx++)
-#pragma unroll
-            for (int h = 0; h < NP / 32; h++) {
-                float d[32];
-                tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + dx * NP + h * 32, d);
+            for (int h = 0; h < u.N; h += 16) {
+                float d[16];
+                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + dx * u.N + h, d);
                 if (row < nrow)
 #pragma unroll
-                    for (int n = 0; n < 32; n++) {
-                        const int o = h * 32 + n;
-                        if (o >= a.O) break;
-                        a.part[(((long)blockIdx.x * 3 + dx) * a.O + o) * nrow + row] = d[n];
-                    }
+                    for (int n = 0; n < 16; n++)
+                        if (h + n < nq)
+                            u.part[(((long)slab * 3 + dx) * u.Q + u.q0 * 8 + h + n) * nrow + row] = d[n];
             }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) tmem_free(tmem, TCOLS);
+    if (warp == 0) tmem_free(tmem, 512);
 }
 
 // Sums of the slabs' partial results in slab order: 32 elements per block,
@@ -419,7 +489,7 @@ struct SumJobs {
         const float *part;
         float *out;
         long n, stride;          // elements, and the distance of two slabs
-        int nslab, O, C;         // C > 0: [dx][O][dy C] to [O][C][dy dx]
+        int nslab, P, Q, swap;   // P > 0: [dx][q][t p] to [o][c][dy dx]
         unsigned end;            // end of the job's blocks
     } j[CONV_MAX_SUMS];
     int n;
@@ -427,6 +497,8 @@ struct SumJobs {
 
 __global__ void __launch_bounds__(256) k_ct_sum(SumJobs jobs) {
     __shared__ float red[8][32];
+    pdl_next();
+    pdl_wait();
     int q = 0;
     while (blockIdx.x >= jobs.j[q].end) q++;
     const SumJobs::Job &j = jobs.j[q];
@@ -442,9 +514,10 @@ __global__ void __launch_bounds__(256) k_ct_sum(SumJobs jobs) {
     if (w || e >= j.n) return;
     for (int k = 1; k < 8; k++) s += red[k][lane];
     long o = e;
-    if (j.C > 0) {
-        const int nrow = 3 * j.C, row = (int)(e % nrow), oc = (int)(e / nrow % j.O), dx = (int)(e / ((long)nrow * j.O));
-        o = ((long)oc * j.C + row % j.C) * 9 + (row / j.C) * 3 + dx;
+    if (j.P > 0) {
+        const int p = (int)(e % j.P), t = (int)(e / j.P % 3), c = (int)(e / (3L * j.P) % j.Q);
+        const int dx = (int)(e / (3L * j.P * j.Q));
+        o = j.swap ? ((long)p * j.Q + c) * 9 + (2 - t) * 3 + 2 - dx : ((long)c * j.P + p) * 9 + t * 3 + dx;
     }
     j.out[o] = s;
 }
@@ -505,29 +578,43 @@ int ct_err_word(int **p) {
     return OK;
 }
 
-int ct_tiles_x(int Wo) { return (Wo + TX - 1) / TX; }
-int ct_tiles(int Ho, int Wo) { return ct_tiles_x(Wo) * ((Ho + TY - 1) / TY); }
+int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
-template <int NP, int EPI>
-int launch_conv(const CUtensorMap &m, ConvArgs &a, int B, cudaStream_t st) {
-    const int smem = std::min(a.nst, 2) * CtCfg<NP>::STAGE + CT_HEAD + 128;
-    static const cudaError_t attr = cudaFuncSetAttribute(
-        k_conv<NP, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * CtCfg<NP>::STAGE + CT_HEAD + 128);
-    CK(attr);
-    const dim3 grid((unsigned)ct_tiles(a.Ho, a.Wo), (unsigned)B);
-    k_conv<NP, EPI><<<grid, CT_THREADS, smem, st>>>(m, a);
+// a launch that may start while the kernel before it drains (pdl_wait)
+template <class... P, class... A>
+int launch_pdl(void (*kern)(P...), dim3 grid, int threads, int smem, cudaStream_t st, A &&...args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = dim3((unsigned)threads);
+    c.dynamicSmemBytes = (size_t)smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    CK(cudaLaunchKernelEx(&c, kern, std::forward<A>(args)...));
     note_launch();
-    CK(cudaGetLastError());
     return OK;
 }
 
-int ct_rows(int nch) {
-    int span = 0;
-    for (int g = 0; g < 3 * nch; g += 16) span = std::max(span, (g + 15) / nch - g / nch);
-    return TY + span;
-}
+int conv_ctas(int ntiles) { return std::min(ntiles, 2 * SMS); }
 
-int ct_slabs(int ntiles, int nch) { return std::min(ntiles, std::max(1, 152 / ((3 * nch + 15) / 16))); }
+template <int NP, int EPI>
+int launch_conv(const CUtensorMap &m, ConvArgs &a, int B, cudaStream_t st) {
+    const int wbytes = a.nst * CtCfg<NP>::WSTAGE, head = wbytes + FHEAD + 128;
+    // two CTAs on an SM where the weights leave room for three stages each
+    const int room = head + 3 * FSTAGE <= SMEM_HALF ? SMEM_HALF : SMEM_SM;
+    a.ring = std::min(FRING, (room - head) / FSTAGE);
+    if (a.ring < 1) return E_UNSUPPORTED;
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(k_conv<NP, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_SM);
+    CK(attr);
+    a.tiles_x = ceil_div(a.Wo, FX);
+    a.tiles_img = a.tiles_x * ceil_div(a.Ho, FY);
+    a.ntiles = B * a.tiles_img;
+    return launch_pdl(k_conv<NP, EPI>, dim3((unsigned)conv_ctas(a.ntiles)), F_THREADS, head + a.ring * FSTAGE, st, m, a);
+}
 
 }  // namespace
 
@@ -536,13 +623,15 @@ size_t conv_split_bytes(int B, int C, int H, int W) { return (size_t)B * 2 * ((C
 int conv_split(const float *x, long xbs, const int *idx, int B, int C, int H, int W, void *xs, void *stream) {
     const long plane = (long)H * W;
     const dim3 grid((unsigned)((plane + 255) / 256), (unsigned)((C + 7) / 8), (unsigned)B);
+    // an ordinary launch: the kernels that may overlap it read the weights
+    // before their pdl_wait, so everything earlier has to be complete
     k_ct_split<<<grid, 256, 0, (cudaStream_t)stream>>>(x, xbs, idx, C, plane, (uint4 *)xs);
     note_launch();
     CK(cudaGetLastError());
     return OK;
 }
 
-long conv_pack_elems(int K, int N) { return (long)((K + 31) / 32) * 9 * KC * (N <= 32 ? 32 : 64) * 8; }
+long conv_pack_elems(int K, int N) { return (long)ceil_div(K, 16) * 144 * (N <= 32 ? 32 : 64); }
 
 int conv_pack(const ConvPack *jobs, int n, const float *w, void *out, void *stream) {
     PackJobs p = {};
@@ -572,14 +661,12 @@ static int conv_args(ConvArgs &a, CUtensorMap &m, const void *xs, const void *wp
                      int origin, int Ho, int Wo) {
     a = {};
     a.w = (const uint8_t *)wp;
-    a.nch = (K + 7) / 8;
-    a.nst = (a.nch + KC - 1) / KC;
+    a.nst = ceil_div(K, 16);
     a.origin = origin;
     a.Ho = Ho; a.Wo = Wo;
-    a.tiles_x = ct_tiles_x(Wo);
     int rc = ct_err_word(&a.err);
     if (rc) return rc;
-    return ct_map(&m, xs, B, a.nch, H, W, false, PX, PY, KC);
+    return ct_map(&m, xs, B, ceil_div(K, 8), H, W, false, FW, FY + 2, 2);
 }
 
 int conv_hidden(const void *xs, const void *wp, const float *bias, int B, int C, int H, int W, void *ys, void *ds,
@@ -605,7 +692,7 @@ int conv_output(const void *xs, const void *wp, const float *bias, int B, int C,
                    : launch_conv<64, CT_OUTPUT>(m, a, B, (cudaStream_t)stream);
 }
 
-long conv_bias_parts(int B, int H, int W) { return (long)B * ct_tiles(H, W); }
+int conv_bias_parts(int B, int H, int W) { return conv_ctas(B * ceil_div(W, FX) * ceil_div(H, FY)); }
 
 int conv_data_grad(const void *dys, const void *wp, const void *ds, int B, int O, int H, int W, void *dxs,
                    float *bpart, void *stream) {
@@ -618,44 +705,84 @@ int conv_data_grad(const void *dys, const void *wp, const void *ds, int B, int O
     return launch_conv<32, CT_DATA>(m, a, B, (cudaStream_t)stream);
 }
 
-long conv_wgt_part(int B, int C, int O, int H, int W, int *nslab) {
-    *nslab = ct_slabs(B * ct_tiles(H - 2, W - 2), (C + 7) / 8);
-    return (long)*nslab * 9 * O * C;
+// The units of the layers' weight gradients and their CTAs.
+static int wgt_units(ConvWgt *l, int n, int B, WgtUnit *u, int *smem) {
+    int nu = 0;
+    double cost[W_UNITS], total = 0.0;
+    *smem = 0;
+    for (int i = 0; i < n; i++) {
+        if (l[i].O < 1 || l[i].O > 64 || l[i].C < 8 || l[i].C % 8) return E_BAD_ARGUMENT;
+        l[i].swap = 3 * l[i].C > 128 && l[i].O == HID;      // more than one M tile otherwise
+        const int P = l[i].swap ? l[i].O : l[i].C, Q = l[i].swap ? l[i].C : l[i].O, nch = P / 8;
+        const int H = l[i].swap ? l[i].H : l[i].H - 2, W = l[i].swap ? l[i].W : l[i].W - 2;   // Q's planes
+        int span = 0;
+        for (int g = 0; g < 3 * nch; g += 16) span = std::max(span, (g + 15) / nch - g / nch);
+        for (int g = 0; g < 3 * nch; g += 16)
+            for (int q0 = 0; q0 < ceil_div(Q, 8); q0 += 16, nu++) {
+                if (nu == W_UNITS) return E_UNSUPPORTED;
+                WgtUnit &v = u[nu];
+                v = {};
+                v.layer = i;
+                v.nch = nch;
+                v.rows = TY + span;
+                v.g0 = g;
+                v.q0 = q0;
+                v.N = std::min(128, ceil_div(Q, 16) * 16);
+                v.Q = Q;
+                v.origin = l[i].swap ? -2 : 0;
+                v.tiles_x = ceil_div(W, TX);
+                v.tiles_img = v.tiles_x * ceil_div(H, TY);
+                v.ntiles = B * v.tiles_img;
+                *smem = std::max(*smem, 2 * (((2 * v.rows * nch * PX * 16 + 127) & ~127) + 2 * (v.N / 8) * QCHUNK));
+                total += cost[nu] = (33.0 + 0.5 * v.N) * v.ntiles;
+            }
+    }
+    *smem += WHEAD + 128;
+    int end = 0;
+    for (int k = 0; k < nu; k++) {
+        // the units of a layer have the same slabs
+        u[k].nslab = k && u[k].layer == u[k - 1].layer
+                         ? u[k - 1].nslab
+                         : std::min(u[k].ntiles, std::max(1, (int)(SMS * cost[k] / total)));
+        u[k].end = end += u[k].nslab;
+        l[u[k].layer].nslab = u[k].nslab;
+    }
+    return *smem <= SMEM_SM ? nu : E_UNSUPPORTED;
 }
 
-int conv_weight_grad(const void *xs, const void *dys, int B, int C, int O, int H, int W, float *part, void *stream) {
-    if (O < 1 || O > 64 || C < 8 || C % 8 || H < 3 || W < 3 || B < 1) return E_BAD_ARGUMENT;
-    const int NP = O <= 32 ? 32 : 64;
+int conv_wgt_plan(ConvWgt *l, int n, int B) {
+    WgtUnit u[W_UNITS];
+    int smem;
+    const int nu = wgt_units(l, n, B, u, &smem);
+    return nu < 0 ? nu : OK;
+}
+
+int conv_weight_grads(ConvWgt *l, int n, int B, void *stream) {
+    if (n < 1 || n > 4) return E_BAD_ARGUMENT;
     WgtArgs a = {};
-    a.part = part; a.O = O;
-    a.nch = C / 8;
-    a.rows = ct_rows(a.nch);
-    a.tiles_x = ct_tiles_x(W - 2);
-    a.tiles_img = ct_tiles(H - 2, W - 2);
-    a.ntiles = B * a.tiles_img;
+    int smem;
+    const int nu = wgt_units(l, n, B, a.u, &smem);
+    if (nu < 0) return nu;
     int rc = ct_err_word(&a.err);
     if (rc) return rc;
-    CUtensorMap xm, dm;
-    if ((rc = ct_map(&xm, xs, B, a.nch, H, W, true, PX, a.rows, a.nch))) return rc;
-    if ((rc = ct_map(&dm, dys, B, (O + 7) / 8, H - 2, W - 2, false, TX, TY, NP / 8))) return rc;
-    // two stages where they fit (C <= 128 with O <= 32)
-    constexpr int LIMIT = 227 * 1024;
-    const int stage = ((2 * a.rows * a.nch * PX * 16 + 127) & ~127) + NP * TY * TX * 4;
-    a.nbuf = 2 * stage + CT_HEAD + 128 <= LIMIT ? 2 : 1;
-    const int smem = a.nbuf * stage + CT_HEAD + 128;
-    if (smem > LIMIT) return E_UNSUPPORTED;
-    const dim3 grid((unsigned)ct_slabs(a.ntiles, a.nch), (unsigned)((3 * a.nch + 15) / 16));
-    auto kern = NP == 32 ? k_conv_wgt<32> : k_conv_wgt<64>;
-    static const cudaError_t a32 =
-        cudaFuncSetAttribute(k_conv_wgt<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, LIMIT);
-    static const cudaError_t a64 =
-        cudaFuncSetAttribute(k_conv_wgt<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, LIMIT);
-    CK(a32);
-    CK(a64);
-    kern<<<grid, CT_THREADS, smem, (cudaStream_t)stream>>>(xm, dm, a);
-    note_launch();
-    CK(cudaGetLastError());
-    return OK;
+    for (int k = 0; k < nu; k++) a.u[k].part = l[a.u[k].layer].part;
+    for (int i = 0; i < n; i++) {
+        const ConvWgt &c = l[i];
+        int k = 0;
+        while (a.u[k].layer != i) k++;
+        const WgtUnit &v = a.u[k];
+        const int cc = c.C / 8, co = ceil_div(c.O, 8), H = c.H, W = c.W;
+        rc = c.swap ? ct_map(&a.p[i], c.dys, B, co, H - 2, W - 2, true, PX, v.rows, co)
+                    : ct_map(&a.p[i], c.xs, B, cc, H, W, true, PX, v.rows, cc);
+        if (rc) return rc;
+        rc = c.swap ? ct_map(&a.q[i], c.xs, B, cc, H, W, false, TX, TY, v.N / 8)
+                    : ct_map(&a.q[i], c.dys, B, co, H - 2, W - 2, false, TX, TY, v.N / 8);
+        if (rc) return rc;
+    }
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(k_conv_wgt, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_SM);
+    CK(attr);
+    return launch_pdl(k_conv_wgt, dim3((unsigned)a.u[nu - 1].end), W_THREADS, smem, (cudaStream_t)stream, a);
 }
 
 int conv_sums(const ConvSum *jobs, int n, void *stream) {
@@ -665,13 +792,15 @@ int conv_sums(const ConvSum *jobs, int n, void *stream) {
     for (int q = 0; q < n; q++) {
         const ConvSum &c = jobs[q];
         SumJobs::Job &j = p.j[q];
-        j.part = c.part; j.out = c.out; j.n = c.n; j.stride = c.stride; j.nslab = c.nslab; j.O = c.O; j.C = c.C;
+        j.part = c.part; j.out = c.out; j.n = c.n; j.stride = c.stride; j.nslab = c.nslab;
+        if (c.wgt) {
+            j.swap = c.wgt->swap;
+            j.P = j.swap ? c.wgt->O : c.wgt->C;
+            j.Q = j.swap ? c.wgt->C : c.wgt->O;
+        }
         j.end = end += (unsigned)((c.n + 31) / 32);
     }
-    k_ct_sum<<<end, 256, 0, (cudaStream_t)stream>>>(p);
-    note_launch();
-    CK(cudaGetLastError());
-    return OK;
+    return launch_pdl(k_ct_sum, dim3(end), 256, 0, (cudaStream_t)stream, p);
 }
 
 // The error word of the bounded waits after the stream's work (0: none

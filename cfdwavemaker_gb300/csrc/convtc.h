@@ -50,15 +50,23 @@ int conv_hidden(const void *xs, const void *wp, const float *bias, int B, int C,
 // y[b][O][H-2][W-2] = conv(xs) + bias, O <= 64
 int conv_output(const void *xs, const void *wp, const float *bias, int B, int C, int O, int H, int W, float *y,
                 void *stream);
-// dxs[b][HID channels][H][W] = conv^T(dys) ds; bpart[conv_bias_parts(B, H, W)][HID]: its sums over pixel tiles
-long conv_bias_parts(int B, int H, int W);
+// dxs[b][HID channels][H][W] = conv^T(dys) ds; bpart[conv_bias_parts(B, H, W)][HID]: sums of shares of it
+int conv_bias_parts(int B, int H, int W);
 int conv_data_grad(const void *dys, const void *wp, const void *ds, int B, int O, int H, int W, void *dxs,
                    float *bpart, void *stream);
-// part: nslab partial weight gradients of 9 O C elements each (C a multiple of 8, O <= 64)
-long conv_wgt_part(int B, int C, int O, int H, int W, int *nslab);
-int conv_weight_grad(const void *xs, const void *dys, int B, int C, int O, int H, int W, float *part, void *stream);
-// sums over nslab of part[slab * stride + e], e < n; C > 0: a weight gradient's elements put in [O][C][9] order
-struct ConvSum { const float *part; float *out; long n, stride; int nslab, O, C; };
+// the weight gradients of up to four layers (C a multiple of 8, O <= 64), each
+// as nslab partial sums of 9 O C elements; the plan sets nslab and swap
+struct ConvWgt {
+    const void *xs, *dys;
+    int C, O, H, W;
+    float *part;
+    int nslab;
+    bool swap;
+};
+int conv_wgt_plan(ConvWgt *l, int n, int B);
+int conv_weight_grads(ConvWgt *l, int n, int B, void *stream);
+// sums over nslab of part[slab * stride + e], e < n; wgt: a weight gradient's elements, put in [O][C][9] order
+struct ConvSum { const float *part; float *out; long n, stride; int nslab; const ConvWgt *wgt; };
 int conv_sums(const ConvSum *jobs, int n, void *stream);
 
 int conv_error(void *stream);         // synchronises; error word of the bounded waits

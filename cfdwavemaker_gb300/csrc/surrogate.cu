@@ -594,10 +594,15 @@ static int loss_grad(Surrogate &s, const float *x, const float *tg, const int *i
     auto take = [&](size_t n) { size_t o = bytes; bytes += up256(n); return o; };
     const size_t o_x = take(conv_split_bytes(B, s.cin, H, W));
     size_t o_h[4] = {}, o_s[4] = {}, o_a[4] = {}, o_p[4] = {}, o_b[4] = {};
-    int slabs[4];
+    ConvWgt wg[4] = {};
+    for (int l = 0; l < 4; l++) {
+        wg[l].C = s.ch[l]; wg[l].O = s.ch[l + 1]; wg[l].H = H - 2 * l; wg[l].W = W - 2 * l;
+    }
+    int rc = conv_wgt_plan(wg, 4, B);
+    if (rc) return rc;
     for (int l = 0; l < 4; l++) {
         const int h = H - 2 * l, w = W - 2 * l;
-        o_p[l] = take(sizeof(float) * conv_wgt_part(B, s.ch[l], s.ch[l + 1], h, w, &slabs[l]));
+        o_p[l] = take(sizeof(float) * 9 * s.ch[l] * s.ch[l + 1] * wg[l].nslab);
         if (l == 0) continue;
         const size_t n = conv_split_bytes(B, HID, h, w);
         o_h[l] = take(n);
@@ -607,7 +612,7 @@ static int loss_grad(Surrogate &s, const float *x, const float *tg, const int *i
     }
     const size_t o_y = take(sizeof(float) * B * s.cout * P4), o_dy = take(conv_split_bytes(B, s.cout, H - 8, W - 8));
     const size_t o_l = take(sizeof(float) * nl4), o_bo = take(sizeof(float) * nl4 * 8);
-    int rc = reserve_tr(s, bytes);
+    rc = reserve_tr(s, bytes);
     if (rc) return rc;
     char *base = (char *)s.tr;
     void *h[4], *ds[4], *da[5];
@@ -625,20 +630,21 @@ static int loss_grad(Surrogate &s, const float *x, const float *tg, const int *i
     note_launch();
     CK(cudaGetLastError());
     ConvSum sums[8];
-    for (int l = 3; l >= 0; l--) {
-        const int hh = H - 2 * l, ww = W - 2 * l, C = s.ch[l], O = s.ch[l + 1];
-        float *part = (float *)(base + o_p[l]);
-        if ((rc = conv_weight_grad(h[l], da[l + 1], B, C, O, hh, ww, part, st))) return rc;
-        if (l && (rc = conv_data_grad(da[l + 1], s.wp + s.off_d[l], ds[l], B, O, hh, ww, da[l],
-                                      (float *)(base + o_b[l]), st)))
-            return rc;
-        sums[l] = {part, s.grad + s.off_w[l], 9L * O * C, 9L * O * C, slabs[l], O, C};
-        if (l == 3)
-            sums[4 + l] = {bout, s.grad + s.off_b[l], s.cout, 8L * nco, (int)(lblk * B), 0, 0};
-        else
-            sums[4 + l] = {(float *)(base + o_b[l + 1]), s.grad + s.off_b[l], HID, HID,
-                           (int)conv_bias_parts(B, hh - 2, ww - 2), 0, 0};
+    for (int l = 3; l >= 1; l--) {
+        const int hh = H - 2 * l, ww = W - 2 * l;
+        float *bp = (float *)(base + o_b[l]);
+        if ((rc = conv_data_grad(da[l + 1], s.wp + s.off_d[l], ds[l], B, s.ch[l + 1], hh, ww, da[l], bp, st))) return rc;
+        sums[4 + l] = {bp, s.grad + s.off_b[l - 1], HID, HID, conv_bias_parts(B, hh, ww), nullptr};
     }
+    sums[4] = {bout, s.grad + s.off_b[3], s.cout, 8L * nco, (int)(lblk * B), nullptr};
+    for (int l = 0; l < 4; l++) {
+        const long n = 9L * s.ch[l] * s.ch[l + 1];
+        wg[l].xs = h[l];
+        wg[l].dys = da[l + 1];
+        wg[l].part = (float *)(base + o_p[l]);
+        sums[l] = {wg[l].part, s.grad + s.off_w[l], n, n, wg[l].nslab, &wg[l]};
+    }
+    if ((rc = conv_weight_grads(wg, 4, B, st))) return rc;
     if ((rc = conv_sums(sums, 8, st))) return rc;
     *nloss = nl4;
     if (want_loss) {

@@ -24,6 +24,9 @@ __device__ __forceinline__ bool mbar_try(uint64_t *b, uint32_t parity) {
                  : "=r"(ok) : "r"(su32(b)), "r"(parity) : "memory");
     return ok != 0;
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t *b) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(b)) : "memory");
+}
 // bounded wait: false (and the error word set) after WAIT_LIMIT cycles
 __device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity, int *err, int code) {
     long long t0 = clock64();
@@ -70,6 +73,26 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
           "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
         : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// columns taddr, taddr + step and taddr + 2 step, 16 each
+__device__ __forceinline__ void tmem_ld16x3(uint32_t taddr, uint32_t step, float *u, float *v, float *w) {
+    float *o[3] = {u, v, w};
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        float *r = o[k];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+            : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]),
+              "=f"(r[8]), "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
+            : "r"(taddr + k * step));
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    // the registers are not read before the wait
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+        for (int n = 0; n < 16; n++) asm volatile("" : "+f"(o[k][n]));
 }
 
 }  // namespace cfdwm
