@@ -12,9 +12,8 @@
 // core matrix of the unswizzled operand layouts, whose strides the descriptors
 // give: K-major (K = channels) for the forward and data-gradient GEMMs,
 // MN-major (K = pixels) for the weight gradient.  A tap moves the operand by
-// whole pixels, 16 bytes each, so the nine taps are nine start addresses in
-// one copy of the tile: nothing is gathered, and nothing is split twice.
-// Zero padding (ragged tiles, the data gradient's border, channels past the
+// whole pixels, 16 bytes each, so the taps are start addresses in one copy of
+// the tile: nothing is gathered, and nothing is split twice.  Zero padding (ragged tiles, the data gradient's border, channels past the
 // last) is the boxes' out-of-range fill.
 //
 // The weights are BF16, so the forward and data-gradient GEMMs take two MMAs
@@ -22,8 +21,9 @@
 // split, three (hi hi, lo hi, hi lo); sums in FP32 in TMEM.  The first form
 // of these kernels gathered each operand tile from FP32 planes with the CUDA
 // cores, nine times over (issue-bound).  Network of 16 levels over a 264 x 264
-// grid: 357 us then, CT_FWD_US us now; loss and gradient of 8 patches of 72 x 72: 981
-// and CT_GRAD_US us.
+// grid, the whole call: 356 us then, 67 now (11 of them the split of the input
+// planes, at the memory's rate; 10 of them launch overlap).  Loss and gradient
+// of eight 72 x 72 patches: 975 and 133 us.
 //
 // Every mbarrier wait is bounded and sets the error word when it gives up.
 #include "cfdwm.h"
@@ -70,6 +70,9 @@ __device__ __forceinline__ void tma_4d(void *dst, const CUtensorMap *m, uint64_t
     asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0],"
                  " [%1, {%3, %4, %5, %6}], [%2];"
                  ::"r"(su32(dst)), "l"(m), "r"(su32(bar)), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void tma_prefetch(const CUtensorMap *m) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
 }
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -139,7 +142,7 @@ __global__ void __launch_bounds__(256) k_ct_pack(PackJobs jobs, const float *w, 
 // ---------------------------------------------------------------------------
 // Forward and data gradient
 // ---------------------------------------------------------------------------
-enum { CT_HIDDEN = 0, CT_OUTPUT = 1, CT_DATA = 2 };
+enum { CT_HIDDEN = 0, CT_OUTPUT = 1, CT_DATA = 2, CT_LOSS = 3 };
 
 // M = 128: 8 rows of 16 pixels.  An MMA costs about 33 + N / 2 cycles here (its
 // 4 KB of A from shared memory, measured with N = 32 and 64), so the three dx
@@ -153,16 +156,21 @@ constexpr int FCHUNK = (FY + 2) * FW * 16;           // bytes of 8 channels' pat
 constexpr int FPART = 2 * FCHUNK, FSTAGE = 2 * FPART;   // 16 channels, hi and lo
 constexpr int FRING = 6;                             // stages in flight at most
 constexpr int F_THREADS = 320;
-constexpr int FHEAD = 256 + 4 * HID * 4;             // barriers and flags, bias sums
+constexpr int FHEAD = 256 + 4 * 64 * 4 + 32;         // barriers and flags, bias and loss sums
 
 struct ConvArgs {
     const uint8_t *w;            // packed weights
-    const float *bias;           // HIDDEN, OUTPUT
+    const float *bias;           // HIDDEN, OUTPUT, LOSS
     const float4 *ds;            // DATA: silu' of the layer's pre-activation [b][HID / 4][Ho][Wo]
     float4 *ds_out;              // HIDDEN: the same, or null
-    uint4 *ys;                   // HIDDEN: activations, DATA: gradient, split format
+    uint4 *ys;                   // HIDDEN: activations, DATA, LOSS: gradient, split format
     float *y;                    // OUTPUT: planes [b][O][Ho][Wo]
-    float *bpart;                // DATA: sums of the CTA's gradients [CTA][HID]
+    float *bpart;                // DATA, LOSS: sums of the CTA's gradients [CTA][NP]
+    const float *tg;             // LOSS: targets, their batch stride and samples (ConvLoss)
+    long tbs;
+    const int *idx;
+    float w0, inv_norm;
+    float *lpart;                // LOSS: the CTA's share
     int nst, ring;               // K stages of 16 channels; stage buffers
     int origin;                  // of the patch relative to the tile: 0, data gradient -2
     int O, Ho, Wo, tiles_x, tiles_img, ntiles;
@@ -190,12 +198,13 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ C
     uint64_t *afull = wfull + 1, *aempty = afull + 2;
     uint32_t *tslot = (uint32_t *)(aempty + 2);
     volatile int *fail = (volatile int *)(tslot + 1);
-    float *red = (float *)(full + 32);                // DATA: [4][HID]
+    float *red = (float *)(full + 32);                // DATA, LOSS: [4][NP], then [8]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         for (int q = 0; q < 2 * FRING + 3; q++) mbar_init(full + q, 1);
         for (int q = 0; q < 2; q++) mbar_init(aempty + q, 8);
         *fail = 0;
+        tma_prefetch(&xm);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) tmem_alloc(tslot, CF::TCOLS);
@@ -203,7 +212,7 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ C
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tslot;
     pdl_next();
-    float bs = 0.f;
+    float bs[NP / 32] = {}, ls = 0.f;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -211,16 +220,17 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ C
             for (int s = 0; s < a.nst; s++)
                 bulk_load(wsm + s * CF::WSTAGE, a.w + (long)s * CF::WSTAGE, CF::WSTAGE, wfull);
             pdl_wait();
-            int k = 0;                                // stages copied
+            int k = 0, buf = 0;                       // stages copied
+            uint32_t par = 1;                         // of the stage buffer's last release
             bool ok = true;
             for (int t = blockIdx.x; ok && t < a.ntiles; t += gridDim.x) {
-                const int b = t / a.tiles_img, r = t % a.tiles_img;
-                const int x0 = (r % a.tiles_x) * FX + a.origin, y0 = (r / a.tiles_x) * FY + a.origin;
+                const int b = t / a.tiles_img, r = t - b * a.tiles_img, ty = r / a.tiles_x;
+                const int x0 = (r - ty * a.tiles_x) * FX + a.origin, y0 = ty * FY + a.origin;
                 for (int s = 0; s < a.nst; s++, k++) {
-                    const int buf = k % a.ring, use = k / a.ring;
-                    if (use && !mbar_wait(empty + buf, (uint32_t)((use - 1) & 1), a.err, 11)) { ok = false; break; }
+                    if (k >= a.ring && !mbar_wait(empty + buf, par, a.err, 11)) { ok = false; break; }
                     mbar_expect_tx(full + buf, FSTAGE);
                     tma_4d(asm_ + buf * FSTAGE, &xm, full + buf, x0 * 8, y0, s * 2, b * 2);
+                    if (++buf == a.ring) { buf = 0; par ^= 1; }
                 }
             }
             if (!ok) {
@@ -234,25 +244,27 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ C
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(CF::N >> 3) << 17) | (8u << 24);
             const uint32_t W = su32(wsm);
             bool ok = mbar_wait(wfull, 0u, a.err, 12);
-            int k = 0, i = 0;                         // stages, tiles
+            int buf = 0, acc = 0, i = 0;              // stage buffer, accumulator, tiles
+            uint32_t par = 0, apar = 1;
             for (int t = blockIdx.x; ok && t < a.ntiles; t += gridDim.x, i++) {
-                const int acc = i % CF::NACC, use = i / CF::NACC;
-                if (use && !mbar_wait(aempty + acc, (uint32_t)((use - 1) & 1), a.err, 13)) { ok = false; break; }
+                if (i >= CF::NACC && !mbar_wait(aempty + acc, apar, a.err, 13)) { ok = false; break; }
                 const uint32_t d = tmem + acc * CF::ACOLS;
-                for (int s = 0; s < a.nst; s++, k++) {
-                    const int buf = k % a.ring;
-                    if (!mbar_wait(full + buf, (uint32_t)((k / a.ring) & 1), a.err, 14)) { ok = false; break; }
+                for (int s = 0; s < a.nst; s++) {
+                    if (!mbar_wait(full + buf, par, a.err, 14)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t da = cdesc(su32(asm_ + buf * FSTAGE), FCHUNK, 128);
                     const uint64_t db = cdesc(W + s * CF::WSTAGE, CF::N * 16, 128);
+#pragma unroll
                     for (int dy = 0; dy < 3; dy++) {
                         const uint64_t oa = (uint64_t)((dy * FW * 16) >> 4), ob = (uint64_t)((dy * 2 * CF::N * 16) >> 4);
                         umma(d, da + oa, db + ob, idesc, (s | dy) ? 1u : 0u);
                         umma(d, da + oa + (FPART >> 4), db + ob, idesc, 1u);
                     }
                     umma_commit(empty + buf);
+                    if (++buf == a.ring) { buf = 0; par ^= 1; }
                 }
                 if (ok) umma_commit(afull + acc);
+                if (++acc == CF::NACC) { acc = 0; apar ^= 1; }
             }
             if (!ok) *fail = 1;
         }
@@ -262,10 +274,10 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ C
         const int m = q * 32 + lane;                  // row of D
         const int col = m & (FW - 1);
         const long plane = (long)a.Ho * a.Wo;
-        int i = 0;
-        for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x, i++) {
-            const int acc = i % CF::NACC;
-            bool ok = mbar_wait(afull + acc, (uint32_t)((i / CF::NACC) & 1), a.err, 15);
+        int acc = 0;
+        uint32_t par = 0;
+        for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
+            bool ok = mbar_wait(afull + acc, par, a.err, 15);
             if (!__all_sync(0xffffffffu, ok)) { *fail = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + acc * CF::ACOLS;
@@ -276,16 +288,51 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ C
 #pragma unroll
             for (int k = 0; k < NP / 32; k++) {
                 const int h = hf * (NP / 32) + k;
+                // the epilogue's inputs first, all in flight
+                float in[16];
+                if (EPI == CT_DATA) {
+#pragma unroll
+                    for (int f = 0; f < 4; f++) {
+                        float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (live) w = a.ds[((long)b * (HID / 4) + h * 4 + f) * plane + pix];
+                        in[f * 4] = w.x; in[f * 4 + 1] = w.y; in[f * 4 + 2] = w.z; in[f * 4 + 3] = w.w;
+                    }
+                } else if (EPI == CT_LOSS) {
+                    const float *tg = a.tg + (long)(live && a.idx ? a.idx[b] : b) * a.tbs + pix;
+#pragma unroll
+                    for (int n = 0; n < 16; n++) in[n] = live && h * 16 + n < a.O ? tg[(h * 16 + n) * plane] : 0.f;
+                }
                 float d[16], e1[16], e2[16];
                 tmem_ld16x3(ta + h * 16, NP, d, e1, e2);
                 if (k == NP / 32 - 1) {
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
                     if (lane == 0) mbar_arrive(aempty + acc);
+                    if (++acc == CF::NACC) { acc = 0; par ^= 1; }
                 }
 #pragma unroll
                 for (int n = 0; n < 16; n++)
                     d[n] += __shfl_down_sync(0xffffffffu, e1[n], 1) + __shfl_down_sync(0xffffffffu, e2[n], 2);
+                if (EPI == CT_LOSS) {
+                    // L = sum w_o (y - t)^2 inv_norm, dy = 2 w_o (y - t) inv_norm
+#pragma unroll
+                    for (int n = 0; n < 16; n++) {
+                        const int o = h * 16 + n;
+                        const float wo = o == 0 ? a.w0 : 1.f;
+                        const float df = live && o < a.O ? d[n] + a.bias[o] - in[n] : 0.f;
+                        ls += wo * df * df * a.inv_norm;
+                        d[n] = 2.f * wo * df * a.inv_norm;
+                    }
+                    const int nco = (a.O + 7) / 8;
+#pragma unroll
+                    for (int c = 0; c < 2; c++) {
+                        if (!live || h * 2 + c >= nco) break;
+                        uint4 hi, lo;
+                        conv_split8(d + c * 8, hi, lo);
+                        a.ys[((long)(b * 2) * nco + h * 2 + c) * plane + pix] = hi;
+                        a.ys[((long)(b * 2 + 1) * nco + h * 2 + c) * plane + pix] = lo;
+                    }
+                }
                 if (EPI == CT_OUTPUT) {
                     if (live)
 #pragma unroll
@@ -294,18 +341,12 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ C
                                 a.y[((long)b * a.O + h * 16 + n) * plane + pix] = d[n] + a.bias[h * 16 + n];
                 }
 #pragma unroll
-                for (int c = 0; c < (EPI == CT_OUTPUT ? 0 : 2); c++) {
+                for (int c = 0; c < (EPI == CT_OUTPUT || EPI == CT_LOSS ? 0 : 2); c++) {
                     float *v = d + c * 8, g[8];
                     const int ch = h * 2 + c;                     // channel chunk
                     if (EPI == CT_DATA) {
 #pragma unroll
-                        for (int f = 0; f < 2; f++) {
-                            float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
-                            if (live) w = a.ds[((long)b * (HID / 4) + ch * 2 + f) * plane + pix];
-                            g[f * 4] = w.x; g[f * 4 + 1] = w.y; g[f * 4 + 2] = w.z; g[f * 4 + 3] = w.w;
-                        }
-#pragma unroll
-                        for (int e = 0; e < 8; e++) v[e] = live ? v[e] * g[e] : 0.f;
+                        for (int e = 0; e < 8; e++) v[e] = live ? v[e] * in[c * 8 + e] : 0.f;
                     } else {
 #pragma unroll
                         for (int e = 0; e < 8; e++) {
@@ -325,7 +366,7 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ C
                             a.ds_out[((long)b * (HID / 4) + ch * 2 + f) * plane + pix] =
                                 make_float4(g[f * 4], g[f * 4 + 1], g[f * 4 + 2], g[f * 4 + 3]);
                 }
-                if (EPI == CT_DATA) {
+                if (EPI == CT_DATA || EPI == CT_LOSS) {
                     // the bias gradient's share: lane n ends with channel n of the warp's pixels
 #pragma unroll
                     for (int o = 8; o >= 1; o >>= 1) {
@@ -336,18 +377,29 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ C
                             d[n] = keep + __shfl_xor_sync(0xffffffffu, send, o);
                         }
                     }
-                    bs += d[0] + __shfl_xor_sync(0xffffffffu, d[0], 16);
+                    bs[k] += d[0] + __shfl_xor_sync(0xffffffffu, d[0], 16);
                 }
             }
         }
-        if (EPI == CT_DATA && lane < 16) red[q * HID + hf * 16 + lane] = bs;
+        if ((EPI == CT_DATA || EPI == CT_LOSS) && lane < 16)
+#pragma unroll
+            for (int k = 0; k < NP / 32; k++) red[q * NP + (hf * (NP / 32) + k) * 16 + lane] = bs[k];
+        if (EPI == CT_LOSS) {
+            for (int o = 16; o >= 1; o >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, o);
+            if (lane == 0) red[4 * NP + warp - 2] = ls;
+        }
     }
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (EPI == CT_DATA && warp == 2 && !*fail)
-        a.bpart[(long)blockIdx.x * HID + lane] =
-            (red[lane] + red[HID + lane]) + (red[2 * HID + lane] + red[3 * HID + lane]);
+    if ((EPI == CT_DATA || EPI == CT_LOSS) && tid < NP && !*fail) {
+        a.bpart[(long)blockIdx.x * NP + tid] = (red[tid] + red[NP + tid]) + (red[2 * NP + tid] + red[3 * NP + tid]);
+        if (EPI == CT_LOSS && tid == 0) {
+            float l = 0.f;
+            for (int k = 0; k < 8; k++) l += red[4 * NP + k];
+            a.lpart[blockIdx.x] = l;
+        }
+    }
     if (warp == 0) tmem_free(tmem, CF::TCOLS);
 }
 
@@ -357,7 +409,7 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ C
 constexpr int TX = 8, TY = 16;            // pixel tile: K = 128, a core matrix per tile row
 constexpr int PX = TX + 2;                // width of the patch
 constexpr int QCHUNK = TX * TY * 16;      // bytes of 8 channels of the plain tile
-constexpr int W_THREADS = 128;
+constexpr int W_THREADS = 256;
 constexpr int W_UNITS = 12;               // (layer, M tile, N block) triples of a launch at most
 constexpr int WHEAD = 128;
 
@@ -406,6 +458,8 @@ __global__ void __launch_bounds__(W_THREADS) k_conv_wgt(const __grid_constant__ 
     if (tid == 0) {
         for (int k = 0; k < 5; k++) mbar_init(full + k, 1);
         *fail = 0;
+        tma_prefetch(&a.p[u.layer]);
+        tma_prefetch(&a.q[u.layer]);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) tmem_alloc(tslot, 512);
@@ -465,25 +519,28 @@ __global__ void __launch_bounds__(W_THREADS) k_conv_wgt(const __grid_constant__ 
     ok = !__syncthreads_or(!ok) && !*fail;
     if (ok) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int row = u.g0 * 8 + tid, nrow = 3 * u.nch * 8, nq = min(u.N, u.Q - u.q0 * 8);
-        for (int dx = 0; dx < 3; dx++)
-            for (int h = 0; h < u.N; h += 16) {
+        // warp w reads lane quarter w % 4, every other 16 columns
+        const int row = u.g0 * 8 + (tid & 127), nrow = 3 * u.nch * 8, nq = min(u.N, u.Q - u.q0 * 8);
+        const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        for (int dx = 0; dx < 3; dx++) {
+            float *out = u.part + (((long)slab * 3 + dx) * u.Q + u.q0 * 8) * nrow + row;
+            for (int h = (warp >> 2) * 16; h < u.N; h += 32) {
                 float d[16];
-                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + dx * u.N + h, d);
+                tmem_ld16(ta + dx * u.N + h, d);
                 if (row < nrow)
 #pragma unroll
                     for (int n = 0; n < 16; n++)
-                        if (h + n < nq)
-                            u.part[(((long)slab * 3 + dx) * u.Q + u.q0 * 8 + h + n) * nrow + row] = d[n];
+                        if (h + n < nq) out[(h + n) * nrow] = d[n];
             }
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) tmem_free(tmem, 512);
 }
 
-// Sums of the slabs' partial results in slab order: 32 elements per block,
-// eight interleaved shares of the slabs each, all layers in one launch.
+// Sums of the slabs' partial results, all layers in one launch: 32 elements
+// per block, 32 interleaved shares of the slabs, added in a fixed order.
 struct SumJobs {
     struct Job {
         const float *part;
@@ -496,27 +553,38 @@ struct SumJobs {
 };
 
 __global__ void __launch_bounds__(256) k_ct_sum(SumJobs jobs) {
+    __shared__ float4 part[32][8];
     __shared__ float red[8][32];
     pdl_next();
     pdl_wait();
     int q = 0;
     while (blockIdx.x >= jobs.j[q].end) q++;
     const SumJobs::Job &j = jobs.j[q];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const long e = (long)(blockIdx.x - (q ? jobs.j[q - 1].end : 0)) * 32 + lane;
-    float s = 0.f;
-    if (e < j.n) {
-#pragma unroll 8
-        for (int k = w; k < j.nslab; k += 8) s += j.part[k * j.stride + e];
+    const long e0 = (long)(blockIdx.x - (q ? jobs.j[q - 1].end : 0)) * 32;
+    {
+        const int v = threadIdx.x & 7, w = threadIdx.x >> 3;     // four elements, share
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (e0 + v * 4 < j.n) {
+#pragma unroll 4
+            for (int k = w; k < j.nslab; k += 32) {
+                const float4 f = *reinterpret_cast<const float4 *>(j.part + k * j.stride + e0 + v * 4);
+                s.x += f.x; s.y += f.y; s.z += f.z; s.w += f.w;
+            }
+        }
+        part[w][v] = s;
     }
-    red[w][lane] = s;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long e = e0 + lane;
+    const float *ps = reinterpret_cast<const float *>(&part[w * 4][0]) + lane;
+    red[w][lane] = (ps[0] + ps[32]) + (ps[64] + ps[96]);
     __syncthreads();
     if (w || e >= j.n) return;
+    float s = red[0][lane];
     for (int k = 1; k < 8; k++) s += red[k][lane];
     long o = e;
     if (j.P > 0) {
-        const int p = (int)(e % j.P), t = (int)(e / j.P % 3), c = (int)(e / (3L * j.P) % j.Q);
-        const int dx = (int)(e / (3L * j.P * j.Q));
+        const int i = (int)e, p = i % j.P, tc = i / j.P, t = tc % 3, cd = tc / 3, c = cd % j.Q, dx = cd / j.Q;
         o = j.swap ? ((long)p * j.Q + c) * 9 + (2 - t) * 3 + 2 - dx : ((long)c * j.P + p) * 9 + t * 3 + dx;
     }
     j.out[o] = s;
@@ -690,6 +758,19 @@ int conv_output(const void *xs, const void *wp, const float *bias, int B, int C,
     a.bias = bias; a.y = y; a.O = O;
     return O <= 32 ? launch_conv<32, CT_OUTPUT>(m, a, B, (cudaStream_t)stream)
                    : launch_conv<64, CT_OUTPUT>(m, a, B, (cudaStream_t)stream);
+}
+
+int conv_loss(const void *xs, const void *wp, const float *bias, int B, int C, int O, int H, int W,
+              const ConvLoss &l, void *dys, float *bpart, float *lpart, void *stream) {
+    if (O < 1 || O > 64 || C < 1 || H < 3 || W < 3 || B < 1) return E_BAD_ARGUMENT;
+    ConvArgs a;
+    CUtensorMap m;
+    int rc = conv_args(a, m, xs, wp, B, C, H, W, 0, H - 2, W - 2);
+    if (rc) return rc;
+    a.bias = bias; a.O = O; a.ys = (uint4 *)dys; a.bpart = bpart; a.lpart = lpart;
+    a.tg = l.tg; a.tbs = l.tbs; a.idx = l.idx; a.w0 = l.w0; a.inv_norm = l.inv_norm;
+    return O <= 32 ? launch_conv<32, CT_LOSS>(m, a, B, (cudaStream_t)stream)
+                   : launch_conv<64, CT_LOSS>(m, a, B, (cudaStream_t)stream);
 }
 
 int conv_bias_parts(int B, int H, int W) { return conv_ctas(B * ceil_div(W, FX) * ceil_div(H, FY)); }

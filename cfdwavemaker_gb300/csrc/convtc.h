@@ -50,6 +50,17 @@ int conv_hidden(const void *xs, const void *wp, const float *bias, int B, int C,
 // y[b][O][H-2][W-2] = conv(xs) + bias, O <= 64
 int conv_output(const void *xs, const void *wp, const float *bias, int B, int C, int O, int H, int W, float *y,
                 void *stream);
+// that output against targets tg[idx[b] or b][O] (batch stride tbs), channel 0 weighted by w0:
+// loss = sum w (y - t)^2 inv_norm as conv_bias_parts shares lpart, dys its gradient in the split
+// format, bpart[share][32 or 64] its sums per channel
+struct ConvLoss {
+    const float *tg;
+    long tbs;
+    const int *idx;
+    float w0, inv_norm;
+};
+int conv_loss(const void *xs, const void *wp, const float *bias, int B, int C, int O, int H, int W,
+              const ConvLoss &l, void *dys, float *bpart, float *lpart, void *stream);
 // dxs[b][HID channels][H][W] = conv^T(dys) ds; bpart[conv_bias_parts(B, H, W)][HID]: sums of shares of it
 int conv_bias_parts(int B, int H, int W);
 int conv_data_grad(const void *dys, const void *wp, const void *ds, int B, int O, int H, int W, void *dxs,
@@ -65,7 +76,7 @@ struct ConvWgt {
 };
 int conv_wgt_plan(ConvWgt *l, int n, int B);
 int conv_weight_grads(ConvWgt *l, int n, int B, void *stream);
-// sums over nslab of part[slab * stride + e], e < n; wgt: a weight gradient's elements, put in [O][C][9] order
+// sums over nslab of part[slab * stride + e], e < n (16-byte aligned, stride a multiple of 4 >= n); wgt: a weight gradient's elements, put in [O][C][9] order
 struct ConvSum { const float *part; float *out; long n, stride; int nslab; const ConvWgt *wgt; };
 int conv_sums(const ConvSum *jobs, int n, void *stream);
 

@@ -230,52 +230,6 @@ __global__ void k_halo_coords(GridGeom g, int nxh, int nyh, double *xy) {
     xy[n + p] = g.d2 + g.dy * (jh - SH);
 }
 
-// Weighted mean-square loss and its gradient:
-//   L = sum_{b,o,p} w_o (y - t)^2 / (B P sum_o w_o),  dy = 2 w_o (y - t) / (B P sum w)
-// A thread makes eight channels of a pixel, so that the gradient leaves in the
-// convolutions' split format; a block's sums of dy are its share of the output
-// bias gradient.
-__global__ void __launch_bounds__(256) k_surr_loss(const float *y, const float *tg, long tbs, const int *idx, int O,
-                                                   long P, float w0, float inv_norm, uint4 *dys, float *lpart,
-                                                   float *bpart) {
-    __shared__ float red[8][9];
-    const long p = blockIdx.x * 256L + threadIdx.x;
-    const int ch = blockIdx.y, nch = gridDim.y, b = blockIdx.z;
-    float v[9];                                   // dy of the eight channels, then the loss
-    v[8] = 0.f;
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-        const int o = ch * 8 + e;
-        v[e] = 0.f;
-        if (p < P && o < O) {
-            const float wo = (o == 0) ? w0 : 1.f;
-            const float d = y[((long)b * O + o) * P + p] - tg[(long)(idx ? idx[b] : b) * tbs + (long)o * P + p];
-            v[8] += wo * d * d * inv_norm;
-            v[e] = 2.f * wo * d * inv_norm;
-        }
-    }
-    if (p < P) {
-        uint4 hi, lo;
-        conv_split8(v, hi, lo);
-        dys[((long)(b * 2) * nch + ch) * P + p] = hi;
-        dys[((long)(b * 2 + 1) * nch + ch) * P + p] = lo;
-    }
-#pragma unroll
-    for (int q = 0; q < 9; q++)
-        for (int s = 16; s > 0; s >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], s);
-    if ((threadIdx.x & 31) == 0)
-#pragma unroll
-        for (int q = 0; q < 9; q++) red[threadIdx.x >> 5][q] = v[q];
-    __syncthreads();
-    if (threadIdx.x < 9) {
-        float t = 0.f;
-        for (int k = 0; k < 8; k++) t += red[k][threadIdx.x];
-        const long blk = (long)b * gridDim.x + blockIdx.x;
-        if (threadIdx.x < 8) bpart[(blk * nch + ch) * 8 + threadIdx.x] = t;
-        else lpart[blk * nch + ch] = t;
-    }
-}
-
 __global__ void k_adam(long n, float lr, float b1, float b2, float eps, float c1, float c2, const float *g,
                        float *w, float *m, float *v) {
     long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -565,19 +519,16 @@ static int reserve_tr(Surrogate &s, size_t bytes) {
 
 static size_t up256(size_t b) { return (b + 255) / 256 * 256; }
 
-// The network over split inputs xs: hidden activations h[1..3] (split) and,
+// The hidden layers over split inputs h[0]: activations h[1..3] (split) and,
 // for the backward pass, silu' of their pre-activations ds[1..3] (null: not
-// kept); output planes y.
-static int net_forward(const Surrogate &s, const void *xs, int B, int H, int W, void *const *h, void *const *ds,
-                       float *y, cudaStream_t st) {
-    const void *in = xs;
+// kept).
+static int net_hidden(const Surrogate &s, int B, int H, int W, void *const *h, void *const *ds, cudaStream_t st) {
     for (int l = 0; l < 3; l++) {
-        int rc = conv_hidden(in, s.wp + s.off_f[l], s.w32 + s.off_b[l], B, s.ch[l], H - 2 * l, W - 2 * l, h[l + 1],
+        int rc = conv_hidden(h[l], s.wp + s.off_f[l], s.w32 + s.off_b[l], B, s.ch[l], H - 2 * l, W - 2 * l, h[l + 1],
                              ds ? ds[l + 1] : nullptr, st);
         if (rc) return rc;
-        in = h[l + 1];
     }
-    return conv_output(in, s.wp + s.off_f[3], s.w32 + s.off_b[3], B, HID, s.cout, H - 6, W - 6, y, st);
+    return OK;
 }
 
 // Forward + loss + backward into s.grad.  x: [*][cin][H][W], tg: [*][cout][H-8][W-8],
@@ -587,9 +538,8 @@ static int loss_grad(Surrogate &s, const float *x, const float *tg, const int *i
                      bool want_loss, long *nloss, cudaStream_t st) {
     if (H < 9 || W < 9 || B < 1 || s.cout > 64) return E_BAD_ARGUMENT;
     const long P4 = (long)(H - 8) * (W - 8);
-    const int nco = (s.cout + 7) / 8;
-    const long lblk = (P4 + 255) / 256, nl4 = lblk * nco * B;
-    // split input, h ds da of the hidden layers, y, dys, partial sums
+    const int nl4 = conv_bias_parts(B, H - 8, W - 8), npo = s.cout <= 32 ? 32 : 64;
+    // split input, h ds da of the hidden layers, dys, partial sums
     size_t bytes = 0;
     auto take = [&](size_t n) { size_t o = bytes; bytes += up256(n); return o; };
     const size_t o_x = take(conv_split_bytes(B, s.cin, H, W));
@@ -610,8 +560,8 @@ static int loss_grad(Surrogate &s, const float *x, const float *tg, const int *i
         o_a[l] = take(n);
         o_b[l] = take(sizeof(float) * HID * conv_bias_parts(B, h, w));
     }
-    const size_t o_y = take(sizeof(float) * B * s.cout * P4), o_dy = take(conv_split_bytes(B, s.cout, H - 8, W - 8));
-    const size_t o_l = take(sizeof(float) * nl4), o_bo = take(sizeof(float) * nl4 * 8);
+    const size_t o_dy = take(conv_split_bytes(B, s.cout, H - 8, W - 8));
+    const size_t o_l = take(sizeof(float) * nl4), o_bo = take(sizeof(float) * nl4 * npo);
     rc = reserve_tr(s, bytes);
     if (rc) return rc;
     char *base = (char *)s.tr;
@@ -619,16 +569,16 @@ static int loss_grad(Surrogate &s, const float *x, const float *tg, const int *i
     for (int l = 1; l < 4; l++) { h[l] = base + o_h[l]; ds[l] = base + o_s[l]; da[l] = base + o_a[l]; }
     h[0] = base + o_x;
     da[4] = base + o_dy;
-    float *y = (float *)(base + o_y), *lpart = (float *)(base + o_l), *bout = (float *)(base + o_bo);
+    float *lpart = (float *)(base + o_l), *bout = (float *)(base + o_bo);
     const long tbs = (long)s.cout * P4;
     if ((rc = conv_split(x, (long)s.cin * H * W, idx, B, s.cin, H, W, h[0], st))) return rc;
-    if ((rc = net_forward(s, h[0], B, H, W, h, ds, y, st))) return rc;
-    const float w0 = (float)s.nl;
-    const float inv_norm = (float)(1.0 / ((double)B * P4 * (w0 + (s.cout - 1))));
-    k_surr_loss<<<dim3((unsigned)lblk, (unsigned)nco, (unsigned)B), 256, 0, st>>>(
-        y, tg, tbs, idx, s.cout, P4, w0, inv_norm, (uint4 *)da[4], lpart, bout);
-    note_launch();
-    CK(cudaGetLastError());
+    if ((rc = net_hidden(s, B, H, W, h, ds, st))) return rc;
+    // L = sum_{b,o,p} w_o (y - t)^2 / (B P sum_o w_o), w_0 = nl (the elevation), 1 else
+    ConvLoss cl = {tg, tbs, idx, (float)s.nl, 0.f};
+    cl.inv_norm = (float)(1.0 / ((double)B * P4 * (cl.w0 + (s.cout - 1))));
+    if ((rc = conv_loss(h[3], s.wp + s.off_f[3], s.w32 + s.off_b[3], B, HID, s.cout, H - 6, W - 6, cl, da[4], bout,
+                        lpart, st)))
+        return rc;
     ConvSum sums[8];
     for (int l = 3; l >= 1; l--) {
         const int hh = H - 2 * l, ww = W - 2 * l;
@@ -636,7 +586,7 @@ static int loss_grad(Surrogate &s, const float *x, const float *tg, const int *i
         if ((rc = conv_data_grad(da[l + 1], s.wp + s.off_d[l], ds[l], B, s.ch[l + 1], hh, ww, da[l], bp, st))) return rc;
         sums[4 + l] = {bp, s.grad + s.off_b[l - 1], HID, HID, conv_bias_parts(B, hh, ww), nullptr};
     }
-    sums[4] = {bout, s.grad + s.off_b[3], s.cout, 8L * nco, (int)(lblk * B), nullptr};
+    sums[4] = {bout, s.grad + s.off_b[3], s.cout, npo, nl4, nullptr};
     for (int l = 0; l < 4; l++) {
         const long n = 9L * s.ch[l] * s.ch[l + 1];
         wg[l].xs = h[l];
@@ -734,7 +684,8 @@ int surrogate_forward(const float *x, int B, int H, int W, float *y, void *strea
     for (int l = 0; l < 4; l++) h[l] = (char *)s.tr + off[l];
     prof_begin(PK_SURR_NET, st);
     rc = conv_split(x, (long)s.cin * H * W, nullptr, B, s.cin, H, W, h[0], st);
-    if (!rc) rc = net_forward(s, h[0], B, H, W, h, nullptr, y, st);
+    if (!rc) rc = net_hidden(s, B, H, W, h, nullptr, st);
+    if (!rc) rc = conv_output(h[3], s.wp + s.off_f[3], s.w32 + s.off_b[3], B, HID, s.cout, H - 6, W - 6, y, st);
     prof_end(PK_SURR_NET, st);
     return rc;
 }

@@ -29,6 +29,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *b) {
 }
 // bounded wait: false (and the error word set) after WAIT_LIMIT cycles
 __device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity, int *err, int code) {
+    if (mbar_try(b, parity)) return true;
     long long t0 = clock64();
     while (!mbar_try(b, parity)) {
         if (clock64() - t0 > WAIT_LIMIT) {
