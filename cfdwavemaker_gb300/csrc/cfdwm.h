@@ -4,6 +4,7 @@
 // C ABI lives in include/cfdwavemaker_gb300.h.
 #pragma once
 
+#include <vector_types.h>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -134,7 +135,6 @@ enum CompCoef {
 constexpr int GRID_TILE = 32;
 constexpr int POINT_TILE = 16;
 constexpr int SMIT_TILE = 16;
-constexpr int DF_COMP_FLOATS = 14;   // floats of one depthform.cu component record
 
 struct DevSea {
     int n = 0;              // components
@@ -165,13 +165,13 @@ struct DevSea {
     bool smit = false;
     float *d_tab_smit = nullptr;
     int npad_s = 0, ntile_s = 0;
-    // per-launch component records of the first-order kernels: float-pair
-    // phase coefficients, ramp, 5 coefficients; three regions of npad_g
-    // records (depthform.cu surface and levels, surrogate.cu features)
-    float *d_dfcomp = nullptr;
     // per-component records of the point phasor kernel (irregular.cu):
     // kx, ky, -omega, phase0 as float pairs, then A, GX, GY, GZ, GP
     float *d_phrec = nullptr;
+    // the components by wave number: their indices, and where each group of
+    // one (FP32) wave number begins (ngrp + 1 entries)
+    int *d_kperm = nullptr, *d_kgrp = nullptr;
+    int ngrp = 0;
 };
 
 // Seeded JONSWAP / cos-2s component columns [5][nfreq ndir] (omega, A, k,
@@ -375,10 +375,41 @@ struct TcForm {
 };
 int tcform_split(TcForm &f, const double *coef64, const int *bmap_host, int nblk, int nout, int npad, bool fp16,
                  void *stream, bool one_acc = false);
+// at points (x, y, t), or (cols given) at the columns of a grid at the time of its tables
+struct GridCols;
+struct GridTab;
 int tcform_eval(TcForm &f, const DevSea &sea, long n, const double *x, const double *y, const double *t, long st,
-                float *out, void *stream, int *tc_error);
+                float *out, void *stream, int *tc_error, const GridTab *tab = nullptr, const GridCols *cols = nullptr);
 void tcform_free(TcForm &f);
 constexpr int TC_NPAD = 256;    // the component count of a TcForm is a multiple of this
+
+// First-order sums over the columns of a regular grid (firstorder.cu).
+// Columns: index act[q] (null: q) = i ny + j, at (d0 + dx (i - off), d2 + dy (j - off)).
+struct GridCols {
+    double d0, d2, dx, dy;
+    int nx, ny, off;
+    const int *act;
+    long n;
+};
+// The components' phasors at the grid's x and y indices at one time, and their
+// coefficient records: a column's phasor is the product X[q][i] Y[q][j], q in
+// the order of DevSea::d_kperm (groups grp of one wave number; zero up to ncp).
+// Xt, Yt by [index][component] (ncp a row) and ramp: in the sea's order.
+struct GridTab {
+    const float2 *X, *Y, *Xt, *Yt;
+    const float *rec, *ramp;
+    const int *grp;
+    int ngrp, ncp, sx, sy;       // sx, sy: row strides of X and Y (zero past nx, ny)
+};
+int first_order_load();
+size_t grid_tab_bytes(const DevSea &sea, int nx, int ny);
+// transposed: with Xt and Yt
+int grid_tab(const DevSea &sea, const GridCols &c, double t, void *mem, bool transposed, GridTab *T, void *stream);
+// first [5][n]: eta1 and the Taylor gradients phi1_dxdz, phi1_dydz, phi1_dzdz, dp1_dz
+int first_surface(const GridTab &T, const GridCols &c, double *first, void *stream);
+// sec [nf][n nl]: u1, v1, w1 (nf = 4: and dp1) at the heights z0 [n nl]
+int first_levels(const GridTab &T, const GridCols &c, int nl, int nf, double depth, const float *z0, float *sec,
+                 void *stream);
 
 // Depth-separable tensor-core form of the s-grid column sums (depthform.cu).
 struct DepthForm {
@@ -394,14 +425,9 @@ struct DepthForm {
 // nf = 3: u, v, w; nf = 4: and the phase terms of the pressure
 int depthform_build(const Config &cfg, const DevSea &sea, DepthForm &df, int nf, void *stream);
 void depthform_free(DepthForm &df);
-int depthform_columns(DepthForm &df, const DevSea &sea, long nact, const double *x, const double *y,
-                      const double *tdev, float *eta2, void *stream);
+int depthform_columns(DepthForm &df, const DevSea &sea, const GridTab &T, const GridCols &c, float *eta2,
+                      void *stream);
 int depthform_combine(DepthForm &df, long nact, int nl, const float *z0, float *sec, void *stream);
-// First-order sums of the tensor-core path (float-float phases): first [5][n]
-// (eta1 and the Taylor gradients) and/or sec [nf][n nl] (u1, v1, w1, and dp1
-// when nf = 4, at z0).
-int depthform_first(const DevSea &sea, long nact, int nl, const double *xy, double t, const float *z0,
-                    double *first, float *sec, int nf, void *stream);
 int depthform_error(DepthForm &df, void *stream);
 int depthform_basis_info(double K, double h, int *R, double *err);
 

@@ -13,8 +13,9 @@
 // give: K-major (K = channels) for the forward and data-gradient GEMMs,
 // MN-major (K = pixels) for the weight gradient.  A tap moves the operand by
 // whole pixels, 16 bytes each, so the taps are start addresses in one copy of
-// the tile: nothing is gathered, and nothing is split twice.  Zero padding (ragged tiles, the data gradient's border, channels past the
-// last) is the boxes' out-of-range fill.
+// the tile: nothing is gathered, and nothing is split twice.  Zero padding
+// (ragged tiles, the data gradient's border, channels past the last) is the
+// boxes' out-of-range fill.
 //
 // The weights are BF16, so the forward and data-gradient GEMMs take two MMAs
 // per K step (hi, lo) and the weight gradient, whose two operands are both
@@ -882,6 +883,25 @@ int conv_sums(const ConvSum *jobs, int n, void *stream) {
         j.end = end += (unsigned)((c.n + 31) / 32);
     }
     return launch_pdl(k_ct_sum, dim3(end), 256, 0, (cudaStream_t)stream, p);
+}
+
+// Loads the kernels (the first launch of each would otherwise).
+int conv_load() {
+    static const cudaError_t rc = [] {
+        const void *k[] = {(const void *)k_ct_split, (const void *)k_ct_pack, (const void *)k_ct_sum,
+                           (const void *)k_conv_wgt, (const void *)k_conv<32, CT_HIDDEN>,
+                           (const void *)k_conv<32, CT_OUTPUT>, (const void *)k_conv<64, CT_OUTPUT>,
+                           (const void *)k_conv<32, CT_LOSS>, (const void *)k_conv<64, CT_LOSS>,
+                           (const void *)k_conv<32, CT_DATA>};
+        cudaFuncAttributes at;
+        for (const void *f : k) {
+            const cudaError_t e = cudaFuncGetAttributes(&at, f);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }();
+    CK(rc);
+    return OK;
 }
 
 // The error word of the bounded waits after the stream's work (0: none

@@ -35,6 +35,7 @@ __device__ __forceinline__ void conv_split8(const float *v, uint4 &hi, uint4 &lo
 }
 #endif
 
+int conv_load();
 size_t conv_split_bytes(int B, int C, int H, int W);
 // planes x[idx[b] or b][C][H][W] (batch stride xbs) to the split format
 int conv_split(const float *x, long xbs, const int *idx, int B, int C, int H, int W, void *xs, void *stream);

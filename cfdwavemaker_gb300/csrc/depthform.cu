@@ -18,7 +18,7 @@
 // same shape as the precision form at z = 0 -- so the 3R forms and eta2 run
 // as one tcgen05 GEMM over all columns (qform.cu), and the levels only
 // combine R numbers per field.  The first-order sums stay exact
-// (k_pairs_columns with pairs = 0).
+// (firstorder.cu).
 //
 // Set-up (host, FP64): Gauss-Legendre nodes on [-h, 0], the weighted kernel
 // matrix, its eigenvectors by cyclic Jacobi rotations, b_r on a fine z table
@@ -29,8 +29,6 @@
 // (about 5e-6 of their maximum), and the whole field (first order included)
 // differs from the plain form by a few 1e-7.
 #include "cfdwm.h"
-#include "ffmath.cuh"
-#include "sgrid_geom.cuh"
 
 #include <cuda_runtime.h>
 
@@ -330,201 +328,6 @@ __global__ void k_depth_coef(DfCoefArgs a) {
     }
 }
 
-// ---------------------------------------------------------------------------
-// First-order sums of the columns for the tensor-core path, with float-float
-// phases (the plain path's FP64 phasor pass and its per-(component, column)
-// phasor table are not needed here):
-//   mode 0: eta1 and the Taylor gradients phi1_dxdz, phi1_dydz, phi1_dzdz,
-//           dp1_dz per column (Irregular.cpp:178-198, 1107-1192) into first[5][n];
-//   mode 1: u1, v1, w1 (nf = 4: and dp1) at the level heights z0
-//           (Irregular.cpp:394-447, 1107-1120) into sec[nf][n nl].
-// Sums are FP32 with Kahan compensation.
-// ---------------------------------------------------------------------------
-struct DfFirstArgs {
-    long n;
-    const double *xy;          // [2][n]
-    double t, fx, fy;
-    const double *phase;       // [7][cstride]: kx, ky, omega, phase0, ramp parameters
-    const float *cf;           // [NCF][cstride]
-    int cstride, ncomp, trivial_ramp;
-    int nl, nf;
-    const float *z0;           // [n nl] (mode 1)
-    float depth;
-    double *first;             // [5][n] (mode 0)
-    float *sec;                // [nf][n nl] (mode 1)
-    const void *comps;         // this launch's component records (DfComp, ncomp of them)
-};
-
-constexpr int DFC = 128;       // components per shared-memory chunk
-constexpr float LOG2E_DF = 1.4426950408889634f;
-
-__device__ __forceinline__ float df_ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ void df_kahan(float &s, float &c, float v) {
-    float y = v - c;
-    float t = s + y;
-    c = (t - s) - y;
-    s = t;
-}
-
-// shared record of a component: phase coefficients as float pairs, ramp, 5 coefficients
-struct DfComp {
-    FfComp f;
-    float c[5];
-};
-
-static_assert(sizeof(DfComp) == DF_COMP_FLOATS * sizeof(float), "component record size");
-
-// The records of all components at this launch's time, one thread each:
-// converting the FP64 phase rows and evaluating the FP64 ramp once here, not
-// in every block (FP64 runs at a small fraction of the FP32 rate on this GPU;
-// done per block it kept the FP64 pipe 71% busy in the level kernel).
-template <int MODE>
-__global__ void k_df_comps(DfFirstArgs a, DfComp *out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.ncomp) return;
-    const int cs = a.cstride;
-    DfComp d;
-    d.f = ff_component(a.phase, cs, i, a.trivial_ramp, a.t);
-    if (MODE == 0) {
-        d.c[0] = a.cf[CF_A * cs + i];
-        d.c[1] = a.cf[CF_GX * cs + i];
-        d.c[2] = a.cf[CF_GY * cs + i];
-        d.c[3] = a.cf[CF_GZ * cs + i];
-        d.c[4] = a.cf[CF_GP * cs + i];
-    } else {
-        const float au = a.cf[CF_AU * cs + i] * a.cf[CF_Q * cs + i];
-        d.c[0] = a.cf[CF_K * cs + i];
-        d.c[1] = au * a.cf[CF_CT * cs + i];
-        d.c[2] = au * a.cf[CF_ST * cs + i];
-        d.c[3] = au;
-        d.c[4] = a.cf[CF_AP * cs + i] * a.cf[CF_Q * cs + i];
-    }
-    out[i] = d;
-}
-
-// a chunk of DFC records into shared memory (zero past the last component)
-__device__ __forceinline__ void df_stage(const DfFirstArgs &a, int i0, DfComp *sc) {
-    const float *src = reinterpret_cast<const float *>(a.comps) + (long)i0 * DF_COMP_FLOATS;
-    float *dst = reinterpret_cast<float *>(sc);
-    const int nrec = min(DFC, a.ncomp - i0);
-    for (int e = threadIdx.x; e < DFC * DF_COMP_FLOATS; e += blockDim.x)
-        dst[e] = e < nrec * DF_COMP_FLOATS ? src[e] : 0.f;
-}
-
-__global__ void __launch_bounds__(128) k_df_first_surface(DfFirstArgs a) {
-    __shared__ DfComp sc[DFC];
-    const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    const bool valid = p < a.n;
-    const long pc = valid ? p : 0;
-    float dxh, dxl, dyh, dyl, th, tl;
-    ff_split(a.xy[pc] - a.fx, dxh, dxl);
-    ff_split(a.xy[a.n + pc] - a.fy, dyh, dyl);
-    ff_split(a.t, th, tl);
-    float s[5] = {0, 0, 0, 0, 0}, k[5] = {0, 0, 0, 0, 0};
-    for (int i0 = 0; i0 < a.ncomp; i0 += DFC) {
-        __syncthreads();
-        df_stage(a, i0, sc);
-        __syncthreads();
-        const int iend = min(DFC, a.ncomp - i0);
-        for (int ii = 0; ii < iend; ii++) {
-            const DfComp &d = sc[ii];
-            float c, sn;
-            ff_phasor(d.f, dxh, dxl, dyh, dyl, th, tl, c, sn);
-            const float rc = d.f.r * c, rs = d.f.r * sn;
-            df_kahan(s[0], k[0], rc * d.c[0]);
-            df_kahan(s[1], k[1], rc * d.c[1]);
-            df_kahan(s[2], k[2], rc * d.c[2]);
-            df_kahan(s[3], k[3], rs * d.c[3]);
-            df_kahan(s[4], k[4], rc * d.c[4]);
-        }
-    }
-    if (!valid) return;
-    for (int q = 0; q < 5; q++) a.first[q * a.n + p] = (double)s[q] - (double)k[q];
-}
-
-// blockDim = 32 columns x up to 8 level groups of 4 levels; blockIdx.y: further level groups.
-// The warps of a block hold the same 32 columns: each computes the phasors of
-// every nw-th component of a chunk into shared memory, and all of them read
-// the whole chunk, so a (column, component) phasor is formed once per block.
-// A chunk's terms are summed in FP32 and the chunk sum is added to a Kahan
-// (sum, carry) pair per output.
-__global__ void __launch_bounds__(256) k_df_first_levels(DfFirstArgs a) {
-    __shared__ DfComp sc[DFC];
-    __shared__ float2 s_ph[DFC][32];     // (r cos, r sin) of (component, column)
-    const int cl = threadIdx.x & 31, wg = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int lg = blockIdx.y * nw + wg;
-    const long p = (long)blockIdx.x * 32 + cl;
-    const bool valid = p < a.n;
-    const long pc = valid ? p : 0;
-    float dxh, dxl, dyh, dyl, th, tl;
-    ff_split(a.xy[pc] - a.fx, dxh, dxl);
-    ff_split(a.xy[a.n + pc] - a.fy, dyh, dyl);
-    ff_split(a.t, th, tl);
-    float zk[4], yk[4];
-#pragma unroll
-    for (int l = 0; l < 4; l++) {
-        const int m = lg * 4 + l;
-        const float z = (valid && m < a.nl) ? a.z0[pc * a.nl + m] : 0.f;
-        zk[l] = z * LOG2E_DF;
-        yk[l] = -(z + 2.f * a.depth) * LOG2E_DF;
-    }
-    float su[4] = {0, 0, 0, 0}, sv[4] = {0, 0, 0, 0}, sw[4] = {0, 0, 0, 0}, sp[4] = {0, 0, 0, 0};
-    float cu[4] = {0, 0, 0, 0}, cv[4] = {0, 0, 0, 0}, cw[4] = {0, 0, 0, 0}, cp[4] = {0, 0, 0, 0};
-    const bool pres = a.nf == 4;
-    for (int i0 = 0; i0 < a.ncomp; i0 += DFC) {
-        __syncthreads();
-        df_stage(a, i0, sc);
-        __syncthreads();
-        const int iend = min(DFC, a.ncomp - i0);
-        for (int ii = wg; ii < iend; ii += nw) {
-            float c, sn;
-            ff_phasor(sc[ii].f, dxh, dxl, dyh, dyl, th, tl, c, sn);
-            s_ph[ii][cl] = make_float2(sc[ii].f.r * c, sc[ii].f.r * sn);
-        }
-        __syncthreads();
-        float tu[4] = {0, 0, 0, 0}, tv[4] = {0, 0, 0, 0}, tw[4] = {0, 0, 0, 0}, tp[4] = {0, 0, 0, 0};
-        for (int ii = 0; ii < iend; ii++) {
-            const DfComp &d = sc[ii];
-            const float2 ph = s_ph[ii][cl];
-            const float au = d.c[1] * ph.x, av = d.c[2] * ph.x, aw = d.c[3] * ph.y, k = d.c[0];
-            const float ap = d.c[4] * ph.x;
-#pragma unroll
-            for (int l = 0; l < 4; l++) {
-                // cosh(k(z+h))/cosh(kh) = q (E + Y), sinh(k(z+h))/cosh(kh) = q (E - Y)
-                const float E = df_ex2(k * zk[l]), Y = df_ex2(k * yk[l]);
-                const float F = E + Y, G = E - Y;
-                tu[l] = fmaf(au, F, tu[l]);
-                tv[l] = fmaf(av, F, tv[l]);
-                tw[l] = fmaf(aw, G, tw[l]);
-                if (pres) tp[l] = fmaf(ap, F, tp[l]);
-            }
-        }
-#pragma unroll
-        for (int l = 0; l < 4; l++) {
-            df_kahan(su[l], cu[l], tu[l]);
-            df_kahan(sv[l], cv[l], tv[l]);
-            df_kahan(sw[l], cw[l], tw[l]);
-            if (pres) df_kahan(sp[l], cp[l], tp[l]);
-        }
-    }
-    if (!valid) return;
-    const long tot = a.n * a.nl;
-#pragma unroll
-    for (int l = 0; l < 4; l++) {
-        const int m = lg * 4 + l;
-        if (m >= a.nl) continue;
-        const long o = p * a.nl + m;
-        a.sec[o] = su[l];
-        a.sec[tot + o] = sv[l];
-        a.sec[2 * tot + o] = sw[l];
-        if (pres) a.sec[3 * tot + o] = sp[l];
-    }
-}
-
 // eta2 of the columns from output column 0
 __global__ void k_df_take(long n, int nout, const float *out, float *eta2) {
     long q = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -680,9 +483,10 @@ void depthform_free(DepthForm &df) {
 
 // second-order sums of the columns act[0..nact): eta2 [nact] and the basis
 // coefficients of the level sums in qout (combined by depthform_combine)
-int depthform_columns(DepthForm &df, const DevSea &sea, long nact, const double *x, const double *y,
-                      const double *tdev, float *eta2, void *stream_) {
+int depthform_columns(DepthForm &df, const DevSea &sea, const GridTab &T, const GridCols &c, float *eta2,
+                      void *stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
+    const long nact = c.n;
     if (!df.built) return E_NOT_INITIALIZED;
     if (df.qcap < nact) {
         if (df.qout) cudaFree(df.qout);
@@ -691,45 +495,11 @@ int depthform_columns(DepthForm &df, const DevSea &sea, long nact, const double 
         CK(cudaMalloc(&df.qout, sizeof(float) * df.nout * nact));
         df.qcap = nact;
     }
-    int rc = tcform_eval(df.tc, sea, nact, x, y, tdev, 0, df.qout, stream, nullptr);
+    int rc = tcform_eval(df.tc, sea, nact, nullptr, nullptr, nullptr, 0, df.qout, stream, nullptr, &T, &c);
     if (rc) return rc;
     k_df_take<<<(unsigned)((nact + 255) / 256), 256, 0, stream>>>(nact, df.nout, df.qout, eta2);
     note_launch();
     CK(cudaGetLastError());
-    return OK;
-}
-
-int depthform_first(const DevSea &sea, long nact, int nl, const double *xy, double t, const float *z0,
-                    double *first, float *sec, int nf, void *stream_) {
-    cudaStream_t stream = (cudaStream_t)stream_;
-    if (nact <= 0) return OK;
-    DfFirstArgs a;
-    a.n = nact; a.xy = xy; a.t = t; a.fx = sea.fx; a.fy = sea.fy;
-    a.phase = sea.d_phase; a.cf = sea.d_cf; a.cstride = sea.npad_g; a.ncomp = sea.n;
-    a.trivial_ramp = sea.trivial_ramp ? 1 : 0;
-    a.nl = nl; a.nf = nf; a.z0 = z0; a.depth = (float)sea.depth; a.first = first; a.sec = sec;
-    if (!sea.d_dfcomp) return E_NOT_INITIALIZED;
-    DfComp *recs = reinterpret_cast<DfComp *>(sea.d_dfcomp);
-    const unsigned cb = (unsigned)((sea.n + 127) / 128);
-    if (first) {
-        k_df_comps<0><<<cb, 128, 0, stream>>>(a, recs);
-        note_launch();
-        a.comps = recs;
-        k_df_first_surface<<<(unsigned)((nact + 127) / 128), 128, 0, stream>>>(a);
-        note_launch();
-        CK(cudaGetLastError());
-    }
-    if (sec) {
-        const int ngrp = (nl + 3) / 4;
-        const int gpb = std::min(ngrp, 8);
-        dim3 grid((unsigned)((nact + 31) / 32), (unsigned)((ngrp + gpb - 1) / gpb));
-        k_df_comps<1><<<cb, 128, 0, stream>>>(a, recs + sea.npad_g);
-        note_launch();
-        a.comps = recs + sea.npad_g;
-        k_df_first_levels<<<grid, 32 * gpb, 0, stream>>>(a);
-        note_launch();
-        CK(cudaGetLastError());
-    }
     return OK;
 }
 

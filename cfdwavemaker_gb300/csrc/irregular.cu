@@ -26,6 +26,7 @@
 //  * Accumulation is compensated: a tile row is summed in FP32, then added to
 //    a Kahan (sum, carry) pair per output.
 #include "cfdwm.h"
+#include "f32x2.cuh"
 #include "ffmath.cuh"
 #include "ramp.cuh"
 
@@ -33,6 +34,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <type_traits>
 #include <vector>
 
@@ -84,11 +86,6 @@ static bool few_points(long n, int npad) {
 // us against 257 with the limit at 1024, of 1000 points 307 against 368)
 constexpr long PH_FEW_POINTS = 300;
 
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 __device__ __forceinline__ void kahan(float &s, float &c, float v) {
     float y = v - c;
     float t = s + y;
@@ -393,7 +390,6 @@ int sea_build(const Config &cfg, DevSea &sea, bool point_table, void *stream_) {
 
     CK(cudaMalloc(&sea.d_phase, sizeof(double) * 7 * sea.npad_g));
     CK(cudaMalloc(&sea.d_cf, sizeof(float) * NCF * sea.npad_g));
-    CK(cudaMalloc(&sea.d_dfcomp, sizeof(float) * DF_COMP_FLOATS * 3 * sea.npad_g));
     // records for up to the next multiple of 256 components (the plain
     // precision form pads to 256), zero past the last component
     const int nrec_cap = ((sea.npad_g + 255) / 256) * 256;
@@ -407,6 +403,25 @@ int sea_build(const Config &cfg, DevSea &sea, bool point_table, void *stream_) {
                                                                  sea.npad_g, sea.d_phrec);
     note_launch();
     CK(cudaGetLastError());
+
+    {
+        std::vector<int> perm(n), grp(1, 0);
+        std::vector<unsigned> key(n);
+        for (int i = 0; i < n; i++) {
+            const float k = (float)cfg.k[i];
+            std::memcpy(&key[i], &k, sizeof(k));
+            perm[i] = i;
+        }
+        std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) { return key[a] < key[b]; });
+        for (int i = 1; i <= n; i++)
+            if (i == n || key[perm[i]] != key[perm[i - 1]]) grp.push_back(i);
+        sea.ngrp = (int)grp.size() - 1;
+        CK(cudaMalloc(&sea.d_kperm, sizeof(int) * nn));
+        CK(cudaMalloc(&sea.d_kgrp, sizeof(int) * grp.size()));
+        if (n) CK(cudaMemcpyAsync(sea.d_kperm, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice, stream));
+        CK(cudaMemcpyAsync(sea.d_kgrp, grp.data(), sizeof(int) * grp.size(), cudaMemcpyHostToDevice, stream));
+        CK(cudaStreamSynchronize(stream));      // the host arrays go out of scope
+    }
 
     if (cfg.order == 2) {
         long ntiles = tile_index(sea.ntile_g - 1, sea.ntile_g - 1, sea.ntile_g) + 1;
@@ -467,12 +482,13 @@ void sea_free(DevSea &sea) {
     if (sea.d_tab_gp) cudaFree(sea.d_tab_gp);
     if (sea.d_tab_gk) cudaFree(sea.d_tab_gk);
     if (sea.d_tab_smit) cudaFree(sea.d_tab_smit);
-    if (sea.d_dfcomp) cudaFree(sea.d_dfcomp);
     if (sea.d_kin) cudaFree(sea.d_kin);
     sea.d_kin = nullptr;
     if (sea.d_phrec) cudaFree(sea.d_phrec);
+    if (sea.d_kperm) cudaFree(sea.d_kperm);
+    if (sea.d_kgrp) cudaFree(sea.d_kgrp);
+    sea.d_kperm = sea.d_kgrp = nullptr;
     sea.d_tab_smit = nullptr;
-    sea.d_dfcomp = nullptr;
     sea.d_phrec = nullptr;
     sea.smit = false;
     sea.d_phase = nullptr; sea.d_cf = nullptr; sea.d_tab_eta = nullptr;
@@ -492,47 +508,6 @@ void workspace_free(Workspace &ws) {
     if (ws.base) cudaFree(ws.base);
     ws.base = nullptr;
     ws.bytes = 0;
-}
-
-// Packed FP32x2 values as 64-bit registers.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 p_pack(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 p_un(f32x2 a) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
-    return r;
-}
-__device__ __forceinline__ float p_hsum(f32x2 a) {
-    const float2 r = p_un(a);
-    return r.x + r.y;
-}
-__device__ __forceinline__ f32x2 p_fma(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 p_mul(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 p_add(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-// a packed operand that a long loop keeps: a plain pack is a move that the
-// compiler repeats at every use (6 moves a pair in k_pairs_points, velocity
-// sums 16 % slower); the result of a packed multiplication (by 1, from a kernel
-// argument) is held
-__device__ __forceinline__ f32x2 p_hold(float a, float b, f32x2 one2) { return p_mul(p_pack(a, b), one2); }
-__device__ __forceinline__ f32x2 p_ex2(f32x2 a) {
-    const float2 v = p_un(a);
-    return p_pack(ex2(v.x), ex2(v.y));
 }
 
 // ---------------------------------------------------------------------------

@@ -65,11 +65,8 @@ __global__ void k_column_coords(GridGeom g, long nact, const int *act, double *x
 // ETA of the slot, the level heights and the level offsets above swl.
 // blockDim 128; the stretched coordinate of each level (which depends on the
 // level only) is formed once per block
-__global__ void k_levels(GridGeom g, long nact, const int *act, const double *first,
+__global__ void k_levels(GridGeom g, long nact, const int *act, const double *sig, const double *first,
                          const float *eta2, int slot, float *ETA, float *zmin, float *zmax) {
-    __shared__ double s_sig[128];
-    for (int m = threadIdx.x; m < g.nl; m += blockDim.x) s_sig[m] = d_sigma_level(g, m);
-    __syncthreads();
     long q = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (q >= nact) return;
     int c = act[q];
@@ -79,7 +76,7 @@ __global__ void k_levels(GridGeom g, long nact, const int *act, const double *fi
     for (int m = 0; m < g.nl; m++) {
         // the reference evaluates the levels from the stored value; the FP32
         // store is the value the query sees, so use it here too
-        double z = d_s2z(g, s_sig[m], (double)ef);
+        double z = d_s2z(g, sig[m], (double)ef);
         zmin[q * g.nl + m] = (float)fmin(0.0, z);
         zmax[q * g.nl + m] = (float)fmax(0.0, z - g.swl);
     }
@@ -424,6 +421,7 @@ struct GridExtra {
     double *xy = nullptr;      // [2][ncol]
     float *zmin = nullptr, *zmax = nullptr, *sec = nullptr;
     float *eta2 = nullptr;
+    double *sig = nullptr;     // stretched coordinate of each level
     double *tdev = nullptr;    // the slot time, read with stride 0 by the phasor pass
     float *split = nullptr;    // slices of a split column-pair launch
     long split_cap = 0;
@@ -504,6 +502,10 @@ int grid_create(const Config &cfg, DevGrid &g, void *stream_) {
     CK(cudaMalloc(&x->sec, sizeof(float) * 4 * v));
     CK(cudaMalloc(&x->eta2, sizeof(float) * c));
     CK(cudaMalloc(&x->tdev, sizeof(double)));
+    CK(cudaMalloc(&x->sig, sizeof(double) * g.nl));
+    int rc = grid_sigma_table(geom(g), x->sig, stream);
+    if (!rc) rc = first_order_load();
+    if (rc) return rc;
     x->split_cap = column_pairs_split_floats(g.nl);
     CK(cudaMalloc(&x->split, sizeof(float) * x->split_cap));
     CK(cudaMalloc(&g.QIMG, sizeof(float4) * 10 * v));
@@ -531,7 +533,7 @@ void grid_free(DevGrid &g) {
     for (auto it = g_extra.begin(); it != g_extra.end(); ++it)
         if (it->first == &g) {
             GridExtra &x = it->second;
-            void *q[] = {x.act_all, x.act_live, x.xy, x.zmin, x.zmax, x.sec, x.eta2, x.tdev, x.split, x.kin};
+            void *q[] = {x.act_all, x.act_live, x.xy, x.zmin, x.zmax, x.sec, x.eta2, x.sig, x.tdev, x.split, x.kin};
             for (void *p : q) if (p) cudaFree(p);
             depthform_free(x.df);
             g_extra.erase(it);
@@ -552,30 +554,35 @@ static int fill_cols(DevGrid &g, const DevSea &sea, Workspace &ws, const int *ac
     const bool tc = g.method == 1 && x->df.built;
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
     // workspace: plain: phasors [npad][nact], ramps [npad][nact], first-order
-    // sums [5][nact]; tensor-core: the first-order sums only
-    size_t b_ph = tc ? 0 : up(sizeof(float2) * (size_t)npad * nact);
+    // sums [5][nact]; tensor-core: the first-order sums and the phasor tables
+    size_t b_ph = tc ? up(grid_tab_bytes(sea, g.nx, g.ny)) : up(sizeof(float2) * (size_t)npad * nact);
     size_t b_rr = tc ? 0 : up(sizeof(float) * (size_t)npad * nact);
     int rc = workspace_reserve(ws, b_ph + b_rr + sizeof(double) * 5 * nact);
     if (rc) return rc;
     char *b = (char *)ws.base;
-    float2 *ph = (float2 *)b;
-    float *rr = (float *)(b + b_ph);
     double *first = (double *)(b + b_ph + b_rr);
-    k_column_coords<<<(unsigned)((nact + 255) / 256), 256, 0, stream>>>(G, nact, act, x->xy);
-    note_launch();
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(x->tdev, &t, sizeof(double), cudaMemcpyHostToDevice, stream));
+    // the grid's own list of all columns (ascending) needs no look-up
+    const bool all = (act == x->act_all || act == x->act_live) && nact == x->n_all;
+    const GridCols cols = {G.d0, G.d2, G.dx, G.dy, g.nx, g.ny, 0, all ? nullptr : act, nact};
+    GridTab tab;
     if (tc) {
-        // eta1 and the Taylor gradients (float-float phases), then eta2 and the
-        // 3R depth-separated quadratic forms of every column in one GEMM
-        rc = depthform_first(sea, nact, g.nl, x->xy, t, nullptr, first, nullptr, 3, stream);
-        if (!rc) rc = depthform_columns(x->df, sea, nact, x->xy, x->xy + nact, x->tdev, x->eta2, stream);
+        // eta1 and the Taylor gradients, then eta2 and the 3R depth-separated
+        // quadratic forms of every column in one GEMM
+        rc = grid_tab(sea, cols, t, b, true, &tab, stream);
+        if (!rc) rc = first_surface(tab, cols, first, stream);
+        if (!rc) rc = depthform_columns(x->df, sea, tab, cols, x->eta2, stream);
     } else {
+        float2 *ph = (float2 *)b;
+        float *rr = (float *)(b + b_ph);
+        k_column_coords<<<(unsigned)((nact + 255) / 256), 256, 0, stream>>>(G, nact, act, x->xy);
+        note_launch();
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(x->tdev, &t, sizeof(double), cudaMemcpyHostToDevice, stream));
         rc = launch_phasors_public(sea, nact, x->xy, x->xy + nact, x->tdev, 1, 1, 0, npad, ph, rr, first, stream);
         if (!rc) rc = launch_eta_pairs(sea, nact, ph, rr, x->eta2, stream, x->split, x->split_cap);
     }
     if (rc) return rc;
-    k_levels<<<(unsigned)((nact + 127) / 128), 128, 0, stream>>>(G, nact, act, first, x->eta2, slot, ETA,
+    k_levels<<<(unsigned)((nact + 127) / 128), 128, 0, stream>>>(G, nact, act, x->sig, first, x->eta2, slot, ETA,
                                                                  x->zmin, x->zmax);
     note_launch();
     CK(cudaGetLastError());
@@ -585,11 +592,11 @@ static int fill_cols(DevGrid &g, const DevSea &sea, Workspace &ws, const int *ac
         // (the form holds the pressure blocks when the grid holds pressure;
         // a fill without P leaves them unused)
         if (pres && x->df.nf != 4) return E_NOT_INITIALIZED;
-        rc = depthform_first(sea, nact, g.nl, x->xy, t, x->zmin, nullptr, x->sec, x->df.nf, stream);
+        rc = first_levels(tab, cols, g.nl, x->df.nf, sea.depth, x->zmin, x->sec, stream);
         if (!rc) rc = depthform_combine(x->df, nact, g.nl, x->zmin, x->sec, stream);
     } else {
         // first and second order per (pair, level)
-        rc = launch_column_pairs(sea, nact, g.nl, ph, rr, x->zmin, x->sec, 1, stream, x->split, x->split_cap,
+        rc = launch_column_pairs(sea, nact, g.nl, (float2 *)b, (float *)(b + b_ph), x->zmin, x->sec, 1, stream, x->split, x->split_cap,
                                  pres);
     }
     if (rc) return rc;
@@ -645,6 +652,7 @@ void grid_live_columns(DevGrid &g, const int **act, long *n) {
 }
 
 GridGeom grid_geom(const DevGrid &g) { return geom(g); }
+const double *grid_sigma(const DevGrid &g) { return extra(g)->sig; }
 
 static int gradients(DevGrid &g, cudaStream_t stream) {
     GradArgs a;

@@ -23,8 +23,15 @@ __device__ __forceinline__ double d_sigma_level(const GridGeom &g, int m) {
 __device__ __forceinline__ double d_s2z(const GridGeom &g, double sigma, double e) {
     return (e - g.swl) + sigma * (g.depth + (e - g.swl));
 }
-__device__ __forceinline__ double d_sigmaS2cart(const GridGeom &g, int m, double e) {
-    return d_s2z(g, d_sigma_level(g, m), e);
-}
+// firstorder.cu: the stretched coordinates of all levels; the first-order
+// channels of the learned update at the levels under eta1 (first: first_surface's
+// sums), scaled, as planes feat and / or in the convolutions' split format xs,
+// and the interior columns' first order with the Taylor term (base) and eta1
+struct GridCols;
+struct GridTab;
+int grid_sigma_table(const GridGeom &g, double *sig, void *stream);
+int first_features(const GridTab &T, const GridCols &c, const GridGeom &g, int halo, const double *sig,
+                   const double *first, float inv_su, float inv_sp, float *feat, void *xs, float *base, float *eta1,
+                   void *stream);
 
 }  // namespace cfdwm

@@ -30,11 +30,9 @@
 // GB300 notes: the convolutions (forward, data and weight gradients) run as
 // implicit GEMMs on the tcgen05 tensor cores (convtc.cu), with the FP32
 // activations split into BF16 hi + lo parts and FP32 accumulation in TMEM.
-// The features form their phases in float-float arithmetic in the kernel (no
-// FP64 phasor table of the halo grid).
+// The features (firstorder.cu) leave in the convolutions' operand format.
 #include "cfdwm.h"
 #include "convtc.h"
-#include "ffmath.cuh"
 #include "sgrid_geom.cuh"
 
 #include <cuda_bf16.h>
@@ -59,177 +57,13 @@ namespace cfdwm {
     } while (0)
 
 GridGeom grid_geom(const DevGrid &g);
+const double *grid_sigma(const DevGrid &g);
 
 namespace {
 
 constexpr int SH = 4;        // halo columns per side: 4 valid 3x3 convolutions
 constexpr int NQ = 8;        // first-order channels per level
 constexpr int HID = CONV_HID;   // hidden channels
-constexpr float LOG2E = 1.4426950408889634f;
-
-
-__device__ __forceinline__ float ex2f(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-// ---------------------------------------------------------------------------
-// First-order channels
-// ---------------------------------------------------------------------------
-struct FeatArgs {
-    GridGeom g;
-    int nxh, nyh;
-    long ncolh;
-    const double *xy;      // [2][ncolh] coordinates of the halo columns
-    double t, fx, fy;
-    const double *phase;   // [7][cstride]: kx, ky, omega, phase0, ramp parameters
-    int trivial_ramp;
-    const double *first;   // [5][ncolh]: eta1, phi1_dxdz, phi1_dydz, phi1_dzdz, dp1_dz
-    const float *cf;
-    int cstride, ncomp;
-    float inv_su, inv_sp;  // 1 / (sigma omega_m), 1 / sigma
-    float *feat;           // [NQ nl][ncolh]
-    float *base;           // [3][nx ny nl] first order with the Taylor term (interior), or null
-    float *eta1;           // [nx ny] (interior), or null
-    const void *recs;      // this launch's component records (SurrRec, ncomp of them)
-};
-
-constexpr int FC = 128;      // components per shared-memory chunk
-
-// a component's record: float-pair phase coefficients and ramp at the
-// launch's time, then k, cu, cv, cw, cp
-struct SurrRec {
-    FfComp f;
-    float c[5];
-};
-static_assert(sizeof(SurrRec) == DF_COMP_FLOATS * sizeof(float), "component record size");
-
-// The records of all components, one thread each: the FP64 phase rows and
-// ramps converted once per launch instead of in every block (FP64 runs at a
-// small fraction of the FP32 rate on this GPU).
-__global__ void k_surr_recs(FeatArgs a, SurrRec *out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.ncomp) return;
-    const int cs = a.cstride;
-    SurrRec d;
-    d.f = ff_component(a.phase, cs, i, a.trivial_ramp, a.t);
-    const float q = a.cf[CF_Q * cs + i];
-    const float au = a.cf[CF_AU * cs + i] * q;
-    d.c[0] = a.cf[CF_K * cs + i];
-    d.c[1] = au * a.cf[CF_CT * cs + i];
-    d.c[2] = au * a.cf[CF_ST * cs + i];
-    d.c[3] = au;
-    d.c[4] = a.cf[CF_A * cs + i] * q;
-    out[i] = d;
-}
-
-// blockDim = 32 columns x ceil(nl / 4) level groups of 4 levels.  The warps
-// hold the same 32 columns: each forms the float-float phasors of every
-// nw-th component of a chunk into shared memory, and all of them read the
-// whole chunk, so a (column, component) phasor is formed once per block.
-__global__ void __launch_bounds__(256) k_surr_features(FeatArgs a) {
-    __shared__ FfComp s_f[FC];
-    __shared__ float s_c[5][FC];         // k, cu, cv, cw, cp of the chunk's components
-    __shared__ float2 s_ph[FC][32];      // (r cos, r sin) of (component, column)
-    const int cl = threadIdx.x & 31, lg = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const long p = (long)blockIdx.x * 32 + cl;
-    const bool valid = p < a.ncolh;
-    const long pc = valid ? p : 0;
-    const GridGeom &g = a.g;
-    float dxh, dxl, dyh, dyl, th, tl;
-    ff_split(a.xy[pc] - a.fx, dxh, dxl);
-    ff_split(a.xy[a.ncolh + pc] - a.fy, dyh, dyl);
-    ff_split(a.t, th, tl);
-    const double e1 = a.first[pc];
-    float zk[4], yk[4], za[4];
-#pragma unroll
-    for (int l = 0; l < 4; l++) {
-        int m = lg * 4 + l;
-        double z = d_sigmaS2cart(g, m < g.nl ? m : g.nl - 1, e1 + g.swl);
-        double z0 = fmin(0.0, z);
-        za[l] = (float)fmax(0.0, z - g.swl);
-        zk[l] = (float)z0 * LOG2E;
-        yk[l] = -((float)z0 + 2.f * (float)g.depth) * LOG2E;
-    }
-    float acc[4][NQ];
-#pragma unroll
-    for (int l = 0; l < 4; l++)
-#pragma unroll
-        for (int q = 0; q < NQ; q++) acc[l][q] = 0.f;
-    for (int i0 = 0; i0 < a.ncomp; i0 += FC) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < FC; e += blockDim.x) {
-            const int i = i0 + e;
-            SurrRec d = {};
-            if (i < a.ncomp) d = reinterpret_cast<const SurrRec *>(a.recs)[i];
-            s_f[e] = d.f;
-            s_c[0][e] = d.c[0]; s_c[1][e] = d.c[1]; s_c[2][e] = d.c[2]; s_c[3][e] = d.c[3]; s_c[4][e] = d.c[4];
-        }
-        __syncthreads();
-        const int iend = min(FC, a.ncomp - i0);
-        for (int ii = lg; ii < iend; ii += nw) {
-            float c, sn;
-            ff_phasor(s_f[ii], dxh, dxl, dyh, dyl, th, tl, c, sn);
-            s_ph[ii][cl] = make_float2(s_f[ii].r * c, s_f[ii].r * sn);
-        }
-        __syncthreads();
-        for (int ii = 0; ii < iend; ii++) {
-            const float2 pv = s_ph[ii][cl];
-            const float rc = pv.x, rs = pv.y;
-            const float k = s_c[0][ii];
-            const float q0 = s_c[1][ii] * rc, q1 = s_c[1][ii] * rs;
-            const float q2 = s_c[2][ii] * rc, q3 = s_c[2][ii] * rs;
-            const float q4 = s_c[3][ii] * rs, q5 = -s_c[3][ii] * rc;
-            const float q6 = s_c[4][ii] * rc, q7 = s_c[4][ii] * rs;
-#pragma unroll
-            for (int l = 0; l < 4; l++) {
-                // profile factors with the normaliser in the coefficient:
-                // cosh(k(z+h))/cosh(kh) = q (E + Y), sinh(k(z+h))/cosh(kh) = q (E - Y)
-                const float E = ex2f(k * zk[l]), Y = ex2f(k * yk[l]);
-                const float F = E + Y, G = E - Y;
-                acc[l][0] = fmaf(q0, F, acc[l][0]);
-                acc[l][1] = fmaf(q1, F, acc[l][1]);
-                acc[l][2] = fmaf(q2, F, acc[l][2]);
-                acc[l][3] = fmaf(q3, F, acc[l][3]);
-                acc[l][4] = fmaf(q4, G, acc[l][4]);
-                acc[l][5] = fmaf(q5, G, acc[l][5]);
-                acc[l][6] = fmaf(q6, F, acc[l][6]);
-                acc[l][7] = fmaf(q7, F, acc[l][7]);
-            }
-        }
-    }
-    if (!valid) return;
-    const int ih = (int)(p / a.nyh), jh = (int)(p % a.nyh);
-    const int i = ih - SH, j = jh - SH;
-    const bool inner = i >= 0 && i < g.nx && j >= 0 && j < g.ny;
-    const long c = (long)i * g.ny + j;
-    const long nxy = (long)g.nx * g.ny;
-#pragma unroll
-    for (int l = 0; l < 4; l++) {
-        int m = lg * 4 + l;
-        if (m >= g.nl) continue;
-#pragma unroll
-        for (int q = 0; q < NQ; q++)
-            a.feat[(long)(m * NQ + q) * a.ncolh + p] = acc[l][q] * (q < 6 ? a.inv_su : a.inv_sp);
-        if (inner && a.base) {
-            for (int f = 0; f < 3; f++)
-                a.base[(long)f * nxy * g.nl + c * g.nl + m] =
-                    acc[l][2 * f] + (float)a.first[(long)(1 + f) * a.ncolh + p] * za[l];
-        }
-    }
-    if (inner && a.eta1 && lg == 0) a.eta1[c] = (float)e1;
-}
-
-__global__ void k_halo_coords(GridGeom g, int nxh, int nyh, double *xy) {
-    long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    long n = (long)nxh * nyh;
-    if (p >= n) return;
-    int ih = (int)(p / nyh), jh = (int)(p % nyh);
-    xy[p] = g.d0 + g.dx * (ih - SH);
-    xy[n + p] = g.d2 + g.dy * (jh - SH);
-}
-
 __global__ void k_adam(long n, float lr, float b1, float b2, float eps, float c1, float c2, const float *g,
                        float *w, float *m, float *v) {
     long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -371,8 +205,8 @@ struct Surrogate {
     int gnx = 0, gny = 0, gnl = 0;
     const float *g_eta = nullptr;      // identity of the attached grid
     double g_dx = 0, g_dy = 0, g_dom[4] = {0, 0, 0, 0}, g_ign[4] = {0, 0, 0, 0};
-    double *xyh = nullptr;
-    float *feat = nullptr, *base = nullptr, *eta1 = nullptr, *pred = nullptr, *hbuf = nullptr;
+    void *xs = nullptr;        // first-order channels, split (convtc.h)
+    float *base = nullptr, *eta1 = nullptr, *pred = nullptr, *hbuf = nullptr;
     float *R = nullptr;        // residual (plain - network) of the last plain slot, [cout][nx ny]
     float *Rtmp = nullptr;
     bool have_res = false;
@@ -389,10 +223,10 @@ struct Surrogate {
 static Surrogate g_s;
 
 static void free_grid_side(Surrogate &s) {
-    void *q[] = {s.xyh, s.feat, s.base, s.eta1, s.pred, s.hbuf, s.rETA, s.rU[0], s.rU[1], s.rU[2],
+    void *q[] = {s.xs, s.base, s.eta1, s.pred, s.hbuf, s.rETA, s.rU[0], s.rU[1], s.rU[2],
                  s.d_sample, s.d_err, s.R, s.Rtmp};
     for (void *p : q) if (p) cudaFree(p);
-    s.xyh = nullptr; s.feat = s.base = s.eta1 = s.pred = s.hbuf = s.rETA = s.R = nullptr;
+    s.xs = nullptr; s.base = s.eta1 = s.pred = s.hbuf = s.rETA = s.R = nullptr;
     s.Rtmp = nullptr;
     s.have_res = false;
     s.rU[0] = s.rU[1] = s.rU[2] = nullptr;
@@ -462,7 +296,8 @@ int surrogate_create(int nl, unsigned long long seed, void *stream_) {
     CK(cudaMemcpyAsync(s.w32, w.data(), sizeof(float) * off, cudaMemcpyHostToDevice, stream));
     CK(cudaMemsetAsync(s.m1, 0, sizeof(float) * off, stream));
     CK(cudaMemsetAsync(s.m2, 0, sizeof(float) * off, stream));
-    int rc = pack_weights(s, stream);
+    int rc = conv_load();
+    if (!rc) rc = pack_weights(s, stream);
     if (rc) return rc;
     CK(cudaStreamSynchronize(stream));
     s.ready = true;
@@ -671,23 +506,28 @@ int surrogate_train_step(const float *xs, const float *ts, long nsamples, const 
 
 int surrogate_check(void *stream) { return conv_check((cudaStream_t)stream); }
 
-int surrogate_forward(const float *x, int B, int H, int W, float *y, void *stream_) {
-    cudaStream_t st = (cudaStream_t)stream_;
-    Surrogate &s = g_s;
-    if (!s.ready) return E_NOT_INITIALIZED;
+// The network over planes x or split inputs xs.
+static int forward(Surrogate &s, const float *x, void *xs, int B, int H, int W, float *y, cudaStream_t st) {
     if (H < 9 || W < 9 || B < 1 || s.cout > 64) return E_BAD_ARGUMENT;
     size_t off[5] = {};
-    for (int l = 0; l < 4; l++) off[l + 1] = off[l] + up256(conv_split_bytes(B, s.ch[l], H - 2 * l, W - 2 * l));
+    for (int l = 0; l < 4; l++)
+        off[l + 1] = off[l] + (l == 0 && xs ? 0 : up256(conv_split_bytes(B, s.ch[l], H - 2 * l, W - 2 * l)));
     int rc = reserve_tr(s, off[4]);
     if (rc) return rc;
     void *h[4];
     for (int l = 0; l < 4; l++) h[l] = (char *)s.tr + off[l];
+    if (xs) h[0] = xs;
     prof_begin(PK_SURR_NET, st);
-    rc = conv_split(x, (long)s.cin * H * W, nullptr, B, s.cin, H, W, h[0], st);
+    if (!xs) rc = conv_split(x, (long)s.cin * H * W, nullptr, B, s.cin, H, W, h[0], st);
     if (!rc) rc = net_hidden(s, B, H, W, h, nullptr, st);
     if (!rc) rc = conv_output(h[3], s.wp + s.off_f[3], s.w32 + s.off_b[3], B, HID, s.cout, H - 6, W - 6, y, st);
     prof_end(PK_SURR_NET, st);
     return rc;
+}
+
+int surrogate_forward(const float *x, int B, int H, int W, float *y, void *stream) {
+    if (!g_s.ready) return E_NOT_INITIALIZED;
+    return forward(g_s, x, nullptr, B, H, W, y, (cudaStream_t)stream);
 }
 
 // ---- grid side ------------------------------------------------------------
@@ -709,7 +549,7 @@ static void sea_scales(const Config &cfg, double &sigma, double &om, double &km)
 // The grid-side buffers follow the grid: their sizes its dimensions, the
 // halo coordinates and the live-column list its placement and ignore area.
 static bool same_grid(const Surrogate &s, const DevGrid &g) {
-    if (!(s.gnx == g.nx && s.gny == g.ny && s.gnl == g.nl && s.feat)) return false;
+    if (!(s.gnx == g.nx && s.gny == g.ny && s.gnl == g.nl && s.xs)) return false;
     if (s.g_eta != g.ETA || s.g_dx != g.dx || s.g_dy != g.dy) return false;
     for (int q = 0; q < 4; q++)
         if (s.g_dom[q] != g.cfg.domain[q] || s.g_ign[q] != g.cfg.domain_ignore[q]) return false;
@@ -721,9 +561,8 @@ static int attach_grid(Surrogate &s, DevGrid &g, cudaStream_t st) {
     if (same_grid(s, g)) return OK;
     free_grid_side(s);
     const int nxh = g.nx + 2 * SH, nyh = g.ny + 2 * SH;
-    const long nh = (long)nxh * nyh, nxy = (long)g.nx * g.ny, n = nxy * g.nl;
-    CK(cudaMalloc(&s.xyh, sizeof(double) * 2 * nh));
-    CK(cudaMalloc(&s.feat, sizeof(float) * s.cin * nh));
+    const long nxy = (long)g.nx * g.ny, n = nxy * g.nl;
+    CK(cudaMalloc(&s.xs, conv_split_bytes(1, s.cin, nxh, nyh)));
     CK(cudaMalloc(&s.base, sizeof(float) * 3 * n));
     CK(cudaMalloc(&s.eta1, sizeof(float) * nxy));
     CK(cudaMalloc(&s.pred, sizeof(float) * s.cout * nxy));
@@ -733,10 +572,6 @@ static int attach_grid(Surrogate &s, DevGrid &g, cudaStream_t st) {
     for (int f = 0; f < 3; f++) CK(cudaMalloc(&s.rU[f], sizeof(float) * n));
     CK(cudaMalloc(&s.d_err, sizeof(unsigned) * 8));
     CK(cudaMalloc(&s.d_sample, sizeof(int) * 4096));
-    GridGeom G = grid_geom(g);
-    k_halo_coords<<<(unsigned)((nh + 255) / 256), 256, 0, st>>>(G, nxh, nyh, s.xyh);
-    note_launch();
-    CK(cudaGetLastError());
     const int *act;
     long nlive;
     grid_live_columns(g, &act, &nlive);
@@ -751,41 +586,30 @@ static int attach_grid(Surrogate &s, DevGrid &g, cudaStream_t st) {
     return OK;
 }
 
-// First-order channels of the attached grid at time t into s.feat/s.base/s.eta1
-// (or the given outputs).
-static int features(Surrogate &s, const Config &cfg, const DevSea &sea, DevGrid &g, Workspace &ws, double t,
-                    float *feat, float *base, float *eta1, cudaStream_t st) {
+// First-order channels of the attached grid at time t into planes feat and / or
+// the split format xs (null: not wanted), base and eta1.
+static int features(const Config &cfg, const DevSea &sea, DevGrid &g, Workspace &ws, double t, float *feat, void *xs,
+                    float *base, float *eta1, cudaStream_t st) {
     const int nxh = g.nx + 2 * SH, nyh = g.ny + 2 * SH;
     const long nh = (long)nxh * nyh;
-    int rc = workspace_reserve(ws, sizeof(double) * 5 * nh);
+    const size_t tabs = up256(grid_tab_bytes(sea, nxh, nyh));
+    int rc = workspace_reserve(ws, tabs + sizeof(double) * 5 * nh);
     if (rc) return rc;
-    double *first = (double *)ws.base;
-    // eta1 and the Taylor gradients of the halo columns (float-float phases)
-    rc = depthform_first(sea, nh, g.nl, s.xyh, t, nullptr, first, nullptr, 3, st);
-    if (rc) return rc;
+    double *first = (double *)((char *)ws.base + tabs);
+    const GridGeom G = grid_geom(g);
+    const GridCols cols = {G.d0, G.d2, G.dx, G.dy, nxh, nyh, SH, nullptr, nh};
+    GridTab tab;
+    prof_begin(PK_SURR_FEATURES, st);
+    rc = grid_tab(sea, cols, t, ws.base, false, &tab, st);
+    // eta1 and the Taylor gradients of the halo columns
+    if (!rc) rc = first_surface(tab, cols, first, st);
     double sigma, om, km;
     sea_scales(cfg, sigma, om, km);
-    FeatArgs a;
-    a.g = grid_geom(g);
-    a.nxh = nxh; a.nyh = nyh; a.ncolh = nh;
-    a.xy = s.xyh; a.t = t; a.fx = sea.fx; a.fy = sea.fy; a.phase = sea.d_phase;
-    a.trivial_ramp = sea.trivial_ramp ? 1 : 0;
-    a.first = first; a.cf = sea.d_cf; a.cstride = sea.npad_g; a.ncomp = sea.n;
-    a.inv_su = (float)(1.0 / (sigma * om));
-    a.inv_sp = (float)(1.0 / sigma);
-    a.feat = feat; a.base = base; a.eta1 = eta1;
-    if (!sea.d_dfcomp) return E_NOT_INITIALIZED;
-    SurrRec *recs = reinterpret_cast<SurrRec *>(sea.d_dfcomp) + 2L * sea.npad_g;
-    k_surr_recs<<<(unsigned)((sea.n + 127) / 128), 128, 0, st>>>(a, recs);
-    note_launch();
-    a.recs = recs;
-    int ngrp = (g.nl + 3) / 4;
-    prof_begin(PK_SURR_FEATURES, st);
-    k_surr_features<<<(unsigned)((nh + 31) / 32), 32 * ngrp, 0, st>>>(a);
-    note_launch();
+    if (!rc)
+        rc = first_features(tab, cols, G, SH, grid_sigma(g), first, (float)(1.0 / (sigma * om)), (float)(1.0 / sigma),
+                            feat, xs, base, eta1, st);
     prof_end(PK_SURR_FEATURES, st);
-    CK(cudaGetLastError());
-    return OK;
+    return rc;
 }
 
 int surrogate_features(const Config &cfg, const DevSea &sea, DevGrid &g, Workspace &ws, double t, float *feat,
@@ -795,7 +619,7 @@ int surrogate_features(const Config &cfg, const DevSea &sea, DevGrid &g, Workspa
     if (!s.ready) return E_NOT_INITIALIZED;
     int rc = attach_grid(s, g, st);
     if (rc) return rc;
-    return features(s, cfg, sea, g, ws, t, feat ? feat : s.feat, base ? base : s.base, eta1 ? eta1 : s.eta1, st);
+    return features(cfg, sea, g, ws, t, feat, feat ? nullptr : s.xs, base ? base : s.base, eta1 ? eta1 : s.eta1, st);
 }
 
 int surrogate_targets(const Config &cfg, DevGrid &g, int slot, const float *base, const float *eta1, float *tg,
@@ -832,13 +656,17 @@ static int slot_max(Surrogate &s, DevGrid &g, const float *ETA, float *const U[3
     return OK;
 }
 
+// s.base, s.eta1 and the network's output s.pred at time t.
+static int predict(Surrogate &s, const Config &cfg, const DevSea &sea, DevGrid &g, Workspace &ws, double t,
+                   cudaStream_t st) {
+    int rc = features(cfg, sea, g, ws, t, nullptr, s.xs, s.base, s.eta1, st);
+    return rc ? rc : forward(s, nullptr, s.xs, 1, g.nx + 2 * SH, g.ny + 2 * SH, s.pred, st);
+}
+
 // Predicts slot `slot` at time t for the live columns.
 static int predict_slot(Surrogate &s, const Config &cfg, const DevSea &sea, DevGrid &g, Workspace &ws, int slot,
                         double t, bool carry, cudaStream_t st) {
-    int rc = features(s, cfg, sea, g, ws, t, s.feat, s.base, s.eta1, st);
-    if (rc) return rc;
-    const int nxh = g.nx + 2 * SH, nyh = g.ny + 2 * SH;
-    rc = surrogate_forward(s.feat, 1, nxh, nyh, s.pred, st);
+    int rc = predict(s, cfg, sea, g, ws, t, st);
     if (rc) return rc;
     double sigma, om, km;
     sea_scales(cfg, sigma, om, km);
@@ -887,9 +715,7 @@ static int refresh_residual(Surrogate &s, const Config &cfg, const DevSea &sea, 
                             int slot, double t, bool have_pred, cudaStream_t st) {
     int rc;
     if (!have_pred) {
-        rc = features(s, cfg, sea, g, ws, t, s.feat, s.base, s.eta1, st);
-        if (rc) return rc;
-        rc = surrogate_forward(s.feat, 1, g.nx + 2 * SH, g.ny + 2 * SH, s.pred, st);
+        rc = predict(s, cfg, sea, g, ws, t, st);
         if (rc) return rc;
     }
     rc = surrogate_targets(cfg, g, slot, s.base, s.eta1, s.R, st);
