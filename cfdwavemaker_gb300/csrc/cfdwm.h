@@ -206,6 +206,30 @@ int sea_build(const Config &cfg, DevSea &sea, bool point_table, void *stream);
 void sea_free(DevSea &sea);
 
 // Scratch workspace for one batch: phasors and first-order sums.
+// Tile pairs per slice of a walk of ntp tile pairs, for a launch of nblk
+// blocks per slice on a GPU with `slots` resident blocks and at most maxs
+// slices: the count whose estimated time, waves x (tile pairs + a slice's
+// fixed cost of SLICE_COST tile pairs), is the least.  Slices are whole tile
+// pairs: 4 slices of 10 tile pairs are 3 + 3 + 3 + 1.
+constexpr double SLICE_COST = 0.15;
+inline int slice_plan(long nblk, int ntp, long slots, long maxs) {
+    int best = ntp;
+    double bestt = 1e300;
+    int prev = 0;
+    for (int ns = 1; ns <= ntp && ns <= maxs; ns++) {
+        const int per = (ntp + ns - 1) / ns;
+        if (per == prev) continue;              // the same slices as with fewer
+        prev = per;
+        const long n = (ntp + per - 1) / per;
+        const double t = (double)((nblk * n + slots - 1) / slots) * (per + SLICE_COST);
+        if (t < bestt) {
+            bestt = t;
+            best = per;
+        }
+    }
+    return best;
+}
+
 struct Workspace {
     size_t bytes = 0;
     void *base = nullptr;

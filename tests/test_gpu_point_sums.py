@@ -82,3 +82,32 @@ def test_few_points_match_a_large_batch(wm, nfreq, ndir):
     top = np.max(np.abs(ref), axis=1, keepdims=True)
     for k in (1, 2, 17, 130, 1, 20, 400):
         assert np.all(np.abs(rows(k) - ref[:, :k]) <= 2 * TOL * top), k
+
+
+@pytest.mark.parametrize("individual", [False, True])
+@pytest.mark.parametrize("nfreq,ndir", [(1, 1), (15, 1), (17, 1), (11, 3)])
+def test_smit_tiles_and_batches(wm, nfreq, ndir, individual):
+    """The Smit theory's sums at the edges of its 16-component tiles, in batches
+    for the kernel of 128 points a block against the FP64 oracle, and in short
+    ones, a block per point, against those."""
+    depth = 35.0
+    comps = ss.irregular_components(3.0, 9.0, 2.0, nfreq, 0.4, 1.9, depth, 8, ndir=ndir, spreading_s=5.0)
+    n = nfreq * ndir
+    rng = np.random.default_rng(n)
+    ramps = [np.full(n, 4.0), rng.uniform(0, 3, n), np.full(n, 500.0)] if individual else None
+    txt = ss.write_irregular(None, comps, depth, extrap=2, swl=0.4, rho=1025.0, mtheta=25.0, ramp_columns=ramps,
+                             vertical_theory="smit")
+    assert wm.initialize_text(txt) == 0, cw.last_error()
+    model = oracle.Model(oracle.waveinput.read_text(txt))
+    for m in (513, 1100):
+        x, y = rng.uniform(-50, 300, m), rng.uniform(-80, 80, m)
+        z, t = rng.uniform(-depth - 2.0, 1.0, m), rng.uniform(5.0, 30, m)
+        ref = model.api(x, y, z, t)
+        u, v, w = wm.velocity_batch(x, y, z, t)
+        p = wm.dynamic_pressure_batch(x, y, z, t)
+        for q, a in ((1, u), (2, v), (3, w), (4, p)):
+            assert np.max(np.abs(a - ref[:, q])) <= TOL * np.max(np.abs(ref[:, q])), (q, m, n)
+        for k in (1, 9):
+            part = [*wm.velocity_batch(x[:k], y[:k], z[:k], t[:k]), wm.dynamic_pressure_batch(x[:k], y[:k], z[:k], t[:k])]
+            for a, b in zip(part, (u, v, w, p)):
+                assert np.max(np.abs(a - b[:k])) <= 2 * TOL * np.max(np.abs(b)), (m, n, k)
