@@ -305,6 +305,8 @@ int grid_write_vtu(const DevGrid &g, const std::string &path, const std::string 
 int grid_dump_vtu(const DevGrid &g, bool last, void *stream);
 // Plain fill of a column subset into ring slot `slot` of the given arrays
 // (the grid's own ETA/U or a scratch copy with the same layout).
+// It takes grid_fill_bytes of ws.
+size_t grid_fill_bytes(DevGrid &g, const DevSea &sea, long nact);
 int grid_fill_columns(DevGrid &g, const DevSea &sea, Workspace &ws, const int *act, long nact, double t,
                       float *ETA, float *const U[3], int slot, void *stream);
 // Plain fill of all live columns of slot `slot` of the grid at time t.

@@ -541,6 +541,22 @@ void grid_free(DevGrid &g) {
         }
 }
 
+// Workspace of a fill.  Plain: phasors [npad][nact], ramps [npad][nact],
+// first-order sums [5][nact]; tensor-core: phasor tables and the first-order sums.
+struct FillBytes {
+    size_t ph, rr, all;
+};
+static FillBytes fill_bytes(DevGrid &g, const DevSea &sea, long nact) {
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const bool tc = g.method == 1 && extra(g)->df.built;
+    FillBytes b;
+    b.ph = up(tc ? grid_tab_bytes(sea, g.nx, g.ny) : sizeof(float2) * (size_t)sea.npad_g * nact);
+    b.rr = tc ? 0 : up(sizeof(float) * (size_t)sea.npad_g * nact);
+    b.all = b.ph + b.rr + sizeof(double) * 5 * nact;
+    return b;
+}
+size_t grid_fill_bytes(DevGrid &g, const DevSea &sea, long nact) { return fill_bytes(g, sea, nact).all; }
+
 // Plain second-order fill of the columns act[0..nact) at time t into ring
 // slot `slot` of the arrays ETA ([slot][nx*ny]) and U[f] ([slot][nx*ny*nl]);
 // P (or null): the pressure field, when the grid holds one.
@@ -552,15 +568,11 @@ static int fill_cols(DevGrid &g, const DevSea &sea, Workspace &ws, const int *ac
     GridGeom G = geom(g);
     const int npad = sea.npad_g;
     const bool tc = g.method == 1 && x->df.built;
-    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-    // workspace: plain: phasors [npad][nact], ramps [npad][nact], first-order
-    // sums [5][nact]; tensor-core: the first-order sums and the phasor tables
-    size_t b_ph = tc ? up(grid_tab_bytes(sea, g.nx, g.ny)) : up(sizeof(float2) * (size_t)npad * nact);
-    size_t b_rr = tc ? 0 : up(sizeof(float) * (size_t)npad * nact);
-    int rc = workspace_reserve(ws, b_ph + b_rr + sizeof(double) * 5 * nact);
+    const FillBytes fb = fill_bytes(g, sea, nact);
+    int rc = workspace_reserve(ws, fb.all);
     if (rc) return rc;
     char *b = (char *)ws.base;
-    double *first = (double *)(b + b_ph + b_rr);
+    double *first = (double *)(b + fb.ph + fb.rr);
     // the grid's own list of all columns (ascending) needs no look-up
     const bool all = (act == x->act_all || act == x->act_live) && nact == x->n_all;
     const GridCols cols = {G.d0, G.d2, G.dx, G.dy, g.nx, g.ny, 0, all ? nullptr : act, nact};
@@ -573,7 +585,7 @@ static int fill_cols(DevGrid &g, const DevSea &sea, Workspace &ws, const int *ac
         if (!rc) rc = depthform_columns(x->df, sea, tab, cols, x->eta2, stream);
     } else {
         float2 *ph = (float2 *)b;
-        float *rr = (float *)(b + b_ph);
+        float *rr = (float *)(b + fb.ph);
         k_column_coords<<<(unsigned)((nact + 255) / 256), 256, 0, stream>>>(G, nact, act, x->xy);
         note_launch();
         CK(cudaGetLastError());
@@ -596,7 +608,7 @@ static int fill_cols(DevGrid &g, const DevSea &sea, Workspace &ws, const int *ac
         if (!rc) rc = depthform_combine(x->df, nact, g.nl, x->zmin, x->sec, stream);
     } else {
         // first and second order per (pair, level)
-        rc = launch_column_pairs(sea, nact, g.nl, (float2 *)b, (float *)(b + b_ph), x->zmin, x->sec, 1, stream, x->split, x->split_cap,
+        rc = launch_column_pairs(sea, nact, g.nl, (float2 *)b, (float *)(b + fb.ph), x->zmin, x->sec, 1, stream, x->split, x->split_cap,
                                  pres);
     }
     if (rc) return rc;

@@ -214,6 +214,9 @@ struct Surrogate {
     float *rETA = nullptr, *rU[3] = {nullptr, nullptr, nullptr};
     int *d_sample = nullptr;
     unsigned *d_err = nullptr;
+    // the checked columns' plain fill runs beside the prediction
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     std::vector<int> live;
     float fmax_eta = 0.f, fmax_u = 0.f;
     unsigned long long rng = 0x2545F4914F6CDD1DULL;
@@ -241,6 +244,9 @@ static void free_all(Surrogate &s) {
     void *q[] = {s.w32, s.m1, s.m2, s.grad, s.wp, s.tr, s.d_idx};
     for (void *p : q) if (p) cudaFree(p);
     if (s.h_loss) cudaFreeHost(s.h_loss);
+    if (s.fork) cudaEventDestroy(s.fork);
+    if (s.join) cudaEventDestroy(s.join);
+    if (s.side) cudaStreamDestroy(s.side);
     s = Surrogate();
 }
 
@@ -288,6 +294,9 @@ int surrogate_create(int nl, unsigned long long seed, void *stream_) {
             w[s.off_w[l] + e] = (float)(sd * std::sqrt(-2.0 * std::log(u1)) * std::cos(6.283185307179586 * u2));
         }
     }
+    CK(cudaStreamCreateWithFlags(&s.side, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming));
     CK(cudaMalloc(&s.w32, sizeof(float) * off));
     CK(cudaMalloc(&s.m1, sizeof(float) * off));
     CK(cudaMalloc(&s.m2, sizeof(float) * off));
@@ -586,16 +595,20 @@ static int attach_grid(Surrogate &s, DevGrid &g, cudaStream_t st) {
     return OK;
 }
 
+static size_t features_bytes(const DevSea &sea, const DevGrid &g) {
+    const int nxh = g.nx + 2 * SH, nyh = g.ny + 2 * SH;
+    return up256(grid_tab_bytes(sea, nxh, nyh)) + up256(sizeof(double) * 5 * nxh * nyh);
+}
+
 // First-order channels of the attached grid at time t into planes feat and / or
 // the split format xs (null: not wanted), base and eta1.
 static int features(const Config &cfg, const DevSea &sea, DevGrid &g, Workspace &ws, double t, float *feat, void *xs,
                     float *base, float *eta1, cudaStream_t st) {
     const int nxh = g.nx + 2 * SH, nyh = g.ny + 2 * SH;
     const long nh = (long)nxh * nyh;
-    const size_t tabs = up256(grid_tab_bytes(sea, nxh, nyh));
-    int rc = workspace_reserve(ws, tabs + sizeof(double) * 5 * nh);
+    int rc = workspace_reserve(ws, features_bytes(sea, g));
     if (rc) return rc;
-    double *first = (double *)((char *)ws.base + tabs);
+    double *first = (double *)((char *)ws.base + up256(grid_tab_bytes(sea, nxh, nyh)));
     const GridGeom G = grid_geom(g);
     const GridCols cols = {G.d0, G.d2, G.dx, G.dy, nxh, nyh, SH, nullptr, nh};
     GridTab tab;
@@ -812,16 +825,32 @@ int surrogate_step(const Config &cfg, const DevSea &sea, DevGrid &g, Workspace &
             if (rc) return rc;
         }
         long ns = std::min<long>(nsample, (long)s.live.size());
-        if (mode == 1 && ns > 0) {
+        // the plain fill of a few columns leaves most of the GPU idle (64
+        // columns: 190 us of latency and one read of the GEMM's weights), so it
+        // runs on a stream and a part of the workspace of its own beside the
+        // prediction, which shares no buffer with it: 706 us a step in one
+        // stream, 642 (the GEMM itself needs whole SMs)
+        const bool check = mode == 1 && ns > 0;
+        if (check) {
             std::vector<int> pick(ns);
             for (long q = 0; q < ns; q++) pick[q] = s.live[lcg(s.rng) % s.live.size()];
             CK(cudaMemcpyAsync(s.d_sample, pick.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, st));
+            CK(cudaEventRecord(s.fork, st));
+            CK(cudaStreamWaitEvent(s.side, s.fork, 0));
             float *rU[3] = {s.rU[0], s.rU[1], s.rU[2]};
-            rc = grid_fill_columns(g, sea, ws, s.d_sample, ns, t2, s.rETA, rU, 0, st);
-            if (rc) return rc;
+            const size_t own = features_bytes(sea, g), part = grid_fill_bytes(g, sea, ns);
+            rc = workspace_reserve(ws, own + part);
+            Workspace side;
+            side.bytes = part;
+            side.base = (char *)ws.base + own;
+            if (!rc) rc = grid_fill_columns(g, sea, side, s.d_sample, ns, t2, s.rETA, rU, 0, s.side);
         }
-        rc = predict_slot(s, cfg, sea, g, ws, slot, t2, carry, st);
-        if (rc) return rc;
+        const int rp = rc ? rc : predict_slot(s, cfg, sea, g, ws, slot, t2, carry, st);
+        if (check) {
+            CK(cudaEventRecord(s.join, s.side));
+            CK(cudaStreamWaitEvent(st, s.join, 0));
+        }
+        if (rc || rp) return rc ? rc : rp;
         s.steps++;
         if (mode == 1 && ns > 0) {
             rc = compare(s, g, slot, s.d_sample, ns, 1.f / std::max(s.fmax_eta, 1e-30f),
