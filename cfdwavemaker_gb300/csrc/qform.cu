@@ -636,6 +636,7 @@ constexpr int QTC_MAXCU = 256;
 struct QTC {
     long rows;               // rows of this chunk
     int npad;                // components (multiple of 256)
+    int ncomp;               // of them in use
     int ntn;                 // column tiles per block (npad / N)
     int group_m;             // row blocks per tile group
     int nblk;                // coefficient blocks of W
@@ -686,6 +687,7 @@ __device__ __forceinline__ bool mbar_wait_ec(uint64_t *b, uint32_t parity, int *
 struct TileInfo {
     long rb;
     int blk, tn, kb0, kb1;
+    int bn;                  // columns
 };
 
 // grouped tile order: a group of group_m row units sweeps all column tiles.
@@ -716,8 +718,13 @@ __device__ __forceinline__ bool tile_of(const QTC &a, long nru, long t, int cran
     } else {
         ti.tn = cu;
         ti.kb0 = 0;
-        ti.kb1 = (cu * BN + BN) / TBK;          // upper triangle: i < m0 + BN
+        ti.kb1 = min((cu * BN + BN) / TBK, (a.ncomp + TBK - 1) / TBK);    // upper triangle: i < m0 + BN
     }
+    // past the last component there are only zeros: K blocks are left out (of
+    // the segments when they are made), and the last column tile has as many
+    // columns as it needs, by 32.  320 components in 512, 1786 columns: 107 us
+    // with whole tiles, 84
+    ti.bn = min(BN, (a.ncomp - ti.tn * BN + 31) / 32 * 32);
     return true;
 }
 
@@ -821,7 +828,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
                     if (leader) mbar_expect_tx(&full[s], CS * STAGE_BYTES);
                     int kx = khalf * a.npad + kb * TBK;
                     int ky = (int)(ti.rb * TBM);
-                    int wy = ti.blk * a.npad + m0 + crank * BROWS;
+                    int wy = ti.blk * a.npad + m0 + crank * (ti.bn / CS);
                     if (PAIR) {
                         const uint32_t fb = full0 + (uint32_t)(s * 8);
                         tma_2d_pair(st, &mXh, fb, kx, ky);
@@ -847,8 +854,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
         if (lane == 0 && leader) {
             // kind::f16, D = F32, A/B = bf16 (1) or f16 (0), both K-major, N = BN, M = 128 CS
             const uint32_t fmt = a.fp16 ? 0u : 1u;
-            const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(BN >> 3) << 17) |
-                                   ((uint32_t)((CS * TBM) >> 4) << 24);
+            const uint32_t idesc0 = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)((CS * TBM) >> 4) << 24);
             long g = 0;
             int j = 0;
             bool ok = true;
@@ -864,6 +870,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc = tmem + (uint32_t)(buf * ACOLS);
                 const uint32_t acc2 = TWO ? acc + BN : acc;     // fp16: cross products
+                const uint32_t idesc = idesc0 | ((uint32_t)(ti.bn >> 3) << 17);
                 for (int kb = ti.kb0; kb < ti.kb1; kb++, g++) {
                     int s = (int)(g % TSTAGES);
                     uint32_t ph = (uint32_t)((g / TSTAGES) & 1);
@@ -910,6 +917,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
             const uint32_t use = (uint32_t)(j / NBUF);
             const int yhalf = a.bmap[3 * ti.blk + 1], outcol = a.bmap[3 * ti.blk + 2];
             const int c0 = ti.tn * BN + hc * HC;       // first column of this warp
+            const int nch = (ti.bn - hc * HC) / 32;    // its chunks of 32 columns in use (may be none)
             const long row = ti.rb * TBM + q * 32 + lane;
             const bool live = row < a.rows;
             const float *Yc = a.Y + ((long)yhalf * a.npad + c0) * a.ldy + (live ? row : 0);
@@ -928,6 +936,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
                 float tv[NCH][32];
 #pragma unroll
                 for (int c = 0; c < NCH; c++) {
+                    if (c >= nch) break;
                     tmem_ld32(acc + c * 32, tv[c]);
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
@@ -950,6 +959,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
                     for (int c = 0; c < NCH; c++)
 #pragma unroll
                         for (int jj = 0; jj < 32; jj += 4) {
+                            if (c >= nch) break;
                             const float4 s4 = __ldg(reinterpret_cast<const float4 *>(cs + c * 32 + jj));
                             const float y0 = __ldg(Yc + (long)(c * 32 + jj) * a.ldy);
                             const float y1 = __ldg(Yc + (long)(c * 32 + jj + 1) * a.ldy);
@@ -993,6 +1003,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
             float part = 0.f;
 #pragma unroll
             for (int c = 0; c < NCH; c++) {
+                if (c >= nch) break;
                 const int sl = c % NSL;
                 if (c >= NSL) {
                     // loaded while chunk c - NSL was reduced
@@ -1327,7 +1338,7 @@ int tcform_eval(TcForm &f, const DevSea &sea, long n, const double *x, const dou
             make_map(&mWl, f.Wlo, (long)f.nblk * npad, npad, BN / CSZ, f.fp16))
             return E_CUDA;
         QTC q;
-        q.rows = mm; q.npad = npad; q.ntn = npad / BN; q.group_m = tc_group_m(); q.nblk = f.nblk; q.nout = f.nout;
+        q.rows = mm; q.npad = npad; q.ncomp = sea.n; q.ntn = npad / BN; q.group_m = tc_group_m(); q.nblk = f.nblk; q.nout = f.nout;
         q.bmap = f.bmap; q.Y = Y; q.ldy = mpad; q.colscale = f.colscale;
         q.out = out + (long)f.nout * b; q.fp16 = f.fp16 ? 1 : 0; q.err = f.err;
         // column units: each column tile's upper-triangle K range, cut into
@@ -1340,7 +1351,7 @@ int tcform_eval(TcForm &f, const DevSea &sea, long n, const double *x, const dou
             q.ncu = 0;
             q.seg = 1;
             for (int tn = 0; tn < q.ntn; tn++) {
-                const int nkb = (tn * BN + BN) / TBK;
+                const int nkb = std::min((tn * BN + BN) / TBK, (sea.n + TBK - 1) / TBK);
                 int nseg = (nkb + f.kseg - 1) / f.kseg;
                 if (q.ntn * nseg > QTC_MAXCU) nseg = 1;
                 for (int sg = 0; sg < nseg; sg++) {
