@@ -392,13 +392,18 @@ struct TcForm {
     int kseg = 0;
     void *Whi = nullptr, *Wlo = nullptr;
     float *colscale = nullptr;
-    int *bmap = nullptr;        // per block: X half, Y half, output column
+    int *bmap = nullptr;        // per block: X half, Y half, output column, kind (TC_*)
+    float *wt = nullptr;        // [3][npad] column weights of the TC_WEIGHTED blocks
     int *err = nullptr;
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
     void *aux = nullptr;        // stream of the operand preparation (several chunks)
     void *ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
 };
+// Kinds of blocks.  Triangular: coefficients of i <= m, one output.  Full: of all
+// (i, m), one output, or TC_WEIGHTED: nw outputs, each with its own column
+// weights, at the output column, the next one and (the third) two further on.
+enum { TC_TRI = 0, TC_FULL = 1, TC_WEIGHTED2 = 2, TC_WEIGHTED3 = 3 };
 int tcform_split(TcForm &f, const double *coef64, const int *bmap_host, int nblk, int nout, int npad, bool fp16,
                  void *stream, bool one_acc = false);
 // at points (x, y, t), or (cols given) at the columns of a grid at the time of its tables

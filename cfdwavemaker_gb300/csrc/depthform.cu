@@ -15,10 +15,19 @@
 // to 1e-8 with R of about 16 terms (a Karhunen-Loeve expansion).  Then
 //   u2(z) = sum_r b_r(z) Q^u_r,   Q^u_r = sum_pairs r_i [Pu f_r(k+) cos(.+.) + Mu f_r(k-) cos(.-.)],
 // and every Q_r is a quadratic form in the column's phasor vector -- the
-// same shape as the precision form at z = 0 -- so the 3R forms and eta2 run
+// same shape as the precision form at z = 0 -- so the forms and eta2 run
 // as one tcgen05 GEMM over all columns (qform.cu), and the levels only
 // combine R numbers per field.  The first-order sums stay exact
 // (firstorder.cu).
+//
+// With individual ramps (r_i weights the first component of a pair) a basis
+// function takes six triangular blocks (eight with the pressure); with one ramp
+// for all components three full ones (k_depth_coef_pot).  Full blocks have no
+// zero half, whose MMAs cost time but little power: 1024 components, 65536
+// columns 10.0 ms triangular, 8.5 to 8.9 as potentials (at the rate the power
+// allows); 320 components, 1786 columns with pressure 84 and 48 us.  Largest
+// errors of the fields against FP64 over 24 to 640 components: 1.8e-7 to 6.6e-7
+// triangular, 1.8e-7 to 8.1e-7.
 //
 // Set-up (host, FP64): Gauss-Legendre nodes on [-h, 0], the weighted kernel
 // matrix, its eigenvectors by cyclic Jacobi rotations, b_r on a fine z table
@@ -274,7 +283,10 @@ __device__ __forceinline__ void cubic_w(double t, int n, int &i0, double wt[4]) 
 }
 
 struct DfCoefArgs {
-    int n, npad, ntile, R, nf;
+    int n, npad, ntile, R, nf, cstride;
+    const double *phase;      // [7][cstride]: kx, ky, omega in rows 0 to 2
+    double rho;
+    float *wt;                // [3][npad]
     const float *tab_grid, *tab_eta, *tab_gp;
     const double *fk, *gk;    // [R][DF_NK]
     double inv_dk;
@@ -325,6 +337,64 @@ __global__ void k_depth_coef(DfCoefArgs a) {
             c[6 * nn] = Pp * fp + Mp * fm; // p, c c
             c[7 * nn] = Mp * fm - Pp * fp; // p, s s
         }
+    }
+}
+
+// The potential form's blocks.  With one ramp for all components the pair sums are
+// the derivatives of sum_{i < m} [P sin(phi_i + phi_m) F(k+) + M sin(phi_i - phi_m) F(k-)]:
+// Pu = P (kx_i + kx_m), Mu = M (kx_i - kx_m), v and the pressure alike with ky and rho
+// omega.  P is symmetric and M antisymmetric in (i, m), so over all ordered pairs
+//   u = sum_m kx_m [c_m sum_i (P - M) c_i - s_m sum_i (P + M) s_i],
+// the same two forms for u, v (and p) with other column weights, and
+//   w = sum_m c_m sum_i (Pw + Mw) s_i, Pw = k+ P G(k+), Mw = k- M G(k-),
+// three full blocks per basis function instead of six triangular ones (eight
+// with the pressure).  Diagonal: twice the pair's, which the sum meets once.
+__global__ void k_depth_coef_pot(DfCoefArgs a) {
+    long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    long tot = (long)a.npad * a.npad;
+    if (e >= tot) return;
+    const int m = (int)(e / a.npad), i = (int)(e % a.npad);
+    const long nn = tot;
+    if (i == 0)
+        for (int q = 0; q < 3; q++)
+            a.wt[(long)q * a.npad + m] = m < a.n ? (float)((q == 2 ? a.rho : 1.0) * a.phase[q * a.cstride + m]) : 0.f;
+    const int nb = 2 + 3 * a.R;
+    if (i >= a.n || m >= a.n) {
+        for (int b = 0; b < nb; b++) a.coef[(long)b * nn + e] = 0.0;
+        return;
+    }
+    const int lo = min(i, m), hi = max(i, m), I = lo / DF_TT, M = hi / DF_TT, ii = lo % DF_TT, mm = hi % DF_TT;
+    const long rec = df_tile_index(I, M, a.ntile) * DF_TT * DF_TT + ii * DF_TT + mm;
+    const float *g = a.tab_grid + rec * GRIDV_NC_DF;
+    const double kp = g[6], km = g[7], two = i == m ? 2.0 : 1.0, sg = i < m ? 1.0 : -1.0;
+    double Pw = two * g[4], Mw = sg * g[5], Pf, Mf;
+    if (a.nf == 4) {
+        const double wi = a.phase[2 * a.cstride + lo], wm = a.phase[2 * a.cstride + hi];
+        Pf = two * a.tab_gp[rec * 2] / (a.rho * (wi + wm));
+        Mf = wi != wm ? sg * a.tab_gp[rec * 2 + 1] / (a.rho * (wi - wm)) : 0.0;
+    } else {
+        Pf = kp > 0.0 ? Pw / kp : 0.0;
+        Mf = km > 0.0 ? Mw / km : 0.0;
+    }
+    a.coef[e] = i <= m ? a.tab_eta[rec * EATA_NC_DF + 0] : 0.0;
+    a.coef[nn + e] = i <= m ? a.tab_eta[rec * EATA_NC_DF + 1] : 0.0;
+    int ip, im;
+    double wp[4], wq[4];
+    cubic_w(kp * a.inv_dk, DF_NK, ip, wp);
+    cubic_w(km * a.inv_dk, DF_NK, im, wq);
+    for (int r = 0; r < a.R; r++) {
+        const double *fr = a.fk + (long)r * DF_NK, *gr = a.gk + (long)r * DF_NK;
+        double fp = 0, fm = 0, gp = 0, gm = 0;
+        for (int q = 0; q < 4; q++) {
+            fp += wp[q] * fr[ip + q];
+            gp += wp[q] * gr[ip + q];
+            fm += wq[q] * fr[im + q];
+            gm += wq[q] * gr[im + q];
+        }
+        double *c = a.coef + (long)(2 + 3 * r) * nn + e;
+        c[0] = Pf * fp - Mf * fm;          // u, v (p): c c
+        c[nn] = -(Pf * fp + Mf * fm);      // u, v (p): s s
+        c[2 * nn] = Pw * gp + Mw * gm;     // w: s c
     }
 }
 
@@ -422,39 +492,56 @@ int depthform_build(const Config &cfg, const DevSea &sea, DepthForm &df, int nf,
     CK(cudaMemcpyAsync(d_fk, fk.data(), sizeof(double) * fk.size(), cudaMemcpyHostToDevice, stream));
     CK(cudaMemcpyAsync(d_gk, gk.data(), sizeof(double) * gk.size(), cudaMemcpyHostToDevice, stream));
     const int npad = ((sea.n + TC_NPAD - 1) / TC_NPAD) * TC_NPAD;
-    const int nblk = 2 + 2 * nf * R;
+    const bool pot = sea.trivial_ramp && df_one_acc();
+    const int nblk = 2 + (pot ? 3 : 2 * nf) * R;
     CK(cudaMalloc(&coef, sizeof(double) * (size_t)nblk * npad * npad));
-    DfCoefArgs a;
+    DfCoefArgs a = {};
     a.n = sea.n; a.npad = npad; a.ntile = sea.ntile_g; a.R = R; a.nf = nf;
     a.tab_grid = sea.d_tab_grid; a.tab_eta = sea.d_tab_eta; a.tab_gp = sea.d_tab_gp; a.fk = d_fk; a.gk = d_gk;
     a.inv_dk = 1.0 / dk; a.coef = coef;
+    a.cstride = sea.npad_g; a.phase = sea.d_phase; a.rho = sea.rho;
+    CK(cudaMalloc(&a.wt, sizeof(float) * 3 * npad));
     long tot = (long)npad * npad;
-    k_depth_coef<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(a);
+    if (pot) k_depth_coef_pot<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(a);
+    else k_depth_coef<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(a);
     note_launch();
     CK(cudaGetLastError());
-    // blocks: eta (c c, s s), then per r: u (c c, s s), v (c c, s s), w (c s, s c)
-    // and, nf = 4, p (c c, s s)
-    std::vector<int> bmap(3 * nblk);
-    auto setb = [&](int b, int kh, int yh, int col) { bmap[3 * b] = kh; bmap[3 * b + 1] = yh; bmap[3 * b + 2] = col; };
-    setb(0, 0, 0, 0);
-    setb(1, 1, 1, 0);
+    // blocks: eta (c c, s s), then per r the potential form's three, or u (c c,
+    // s s), v (c c, s s), w (c s, s c) and, nf = 4, p (c c, s s)
+    std::vector<int> bmap(4 * nblk);
+    auto setb = [&](int b, int kh, int yh, int col, int kind) {
+        const int v[4] = {kh, yh, col, kind};
+        std::copy(v, v + 4, bmap.begin() + 4 * b);
+    };
+    setb(0, 0, 0, 0, TC_TRI);
+    setb(1, 1, 1, 0, TC_TRI);
     for (int r = 0; r < R; r++) {
-        int b = 2 + 2 * nf * r, o = 1 + nf * r;
-        setb(b + 0, 0, 0, o);
-        setb(b + 1, 1, 1, o);
-        setb(b + 2, 0, 0, o + 1);
-        setb(b + 3, 1, 1, o + 1);
-        setb(b + 4, 0, 1, o + 2);
-        setb(b + 5, 1, 0, o + 2);
+        const int o = 1 + nf * r;
+        if (pot) {
+            const int b = 2 + 3 * r, kind = nf == 4 ? TC_WEIGHTED3 : TC_WEIGHTED2;
+            setb(b + 0, 0, 0, o, kind);
+            setb(b + 1, 1, 1, o, kind);
+            setb(b + 2, 1, 0, o + 2, TC_FULL);
+            continue;
+        }
+        const int b = 2 + 2 * nf * r;
+        setb(b + 0, 0, 0, o, TC_TRI);
+        setb(b + 1, 1, 1, o, TC_TRI);
+        setb(b + 2, 0, 0, o + 1, TC_TRI);
+        setb(b + 3, 1, 1, o + 1, TC_TRI);
+        setb(b + 4, 0, 1, o + 2, TC_TRI);
+        setb(b + 5, 1, 0, o + 2, TC_TRI);
         if (nf == 4) {
-            setb(b + 6, 0, 0, o + 3);
-            setb(b + 7, 1, 1, o + 3);
+            setb(b + 6, 0, 0, o + 3, TC_TRI);
+            setb(b + 7, 1, 1, o + 3, TC_TRI);
         }
     }
     // fp16 split with one accumulator: the K range of a tile is short here
     // (256-1024 components), so the cross products keep their bits in the hi
     // accumulator, and the two accumulator buffers hide each tile's epilogue
+    // (the potential form's weights are in that epilogue only)
     rc = tcform_split(df.tc, coef, bmap.data(), nblk, df.nout, npad, true, stream, df_one_acc());
+    df.tc.wt = a.wt;
     cudaFree(coef);
     cudaFree(d_fk);
     cudaFree(d_gk);

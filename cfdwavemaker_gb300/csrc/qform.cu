@@ -641,7 +641,8 @@ struct QTC {
     int group_m;             // row blocks per tile group
     int nblk;                // coefficient blocks of W
     int nout;                // outputs per row
-    const int *bmap;         // per block: X half, Y half, output column
+    const int *bmap;         // per block: X half, Y half, output column, kind
+    const float *wt;         // [3][npad] column weights of the weighted blocks
     const float *Y;          // [2 npad][ldy], column-major
     long ldy;
     const float *colscale;   // [nblk][npad] (1 for bf16)
@@ -718,7 +719,9 @@ __device__ __forceinline__ bool tile_of(const QTC &a, long nru, long t, int cran
     } else {
         ti.tn = cu;
         ti.kb0 = 0;
-        ti.kb1 = min((cu * BN + BN) / TBK, (a.ncomp + TBK - 1) / TBK);    // upper triangle: i < m0 + BN
+        // upper triangle: i < m0 + BN
+        ti.kb1 = (a.ncomp + TBK - 1) / TBK;
+        if (a.bmap[4 * ti.blk + 3] == TC_TRI) ti.kb1 = min(ti.kb1, (cu * BN + BN) / TBK);
     }
     // past the last component there are only zeros: K blocks are left out (of
     // the segments when they are made), and the last column tile has as many
@@ -817,7 +820,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
             for (long t = cid; t < ntiles && ok; t += ncl) {
                 TileInfo ti;
                 if (!tile_of<BN, CS>(a, nru, t, crank, ti)) continue;
-                const int khalf = a.bmap[3 * ti.blk];
+                const int khalf = a.bmap[4 * ti.blk];
                 const int m0 = ti.tn * BN;
                 for (int kb = ti.kb0; kb < ti.kb1; kb++, g++) {
                     int s = (int)(g % TSTAGES);
@@ -915,7 +918,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
             if (!tile_of<BN, CS>(a, nru, t, crank, ti)) continue;
             const int buf = j % NBUF;
             const uint32_t use = (uint32_t)(j / NBUF);
-            const int yhalf = a.bmap[3 * ti.blk + 1], outcol = a.bmap[3 * ti.blk + 2];
+            const int yhalf = a.bmap[4 * ti.blk + 1], outcol = a.bmap[4 * ti.blk + 2];
+            const int nw = TWO ? 0 : a.bmap[4 * ti.blk + 3];      // >= TC_WEIGHTED2: its outputs
             const int c0 = ti.tn * BN + hc * HC;       // first column of this warp
             const int nch = (ti.bn - hc * HC) / 32;    // its chunks of 32 columns in use (may be none)
             const long row = ti.rb * TBM + q * 32 + lane;
@@ -1000,7 +1004,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * ACOLS) + (uint32_t)(hc * HC);
-            float part = 0.f;
+            float part = 0.f, part1 = 0.f, part2 = 0.f;
 #pragma unroll
             for (int c = 0; c < NCH; c++) {
                 if (c >= nch) break;
@@ -1018,8 +1022,31 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
                 }
                 float v[32];
                 tmem_ld32(acc + c * 32, v);
+                if (nw < TC_WEIGHTED2) {
 #pragma unroll
-                for (int jj = 0; jj < 32; jj++) part = fmaf(v[jj], ys[sl][jj], part);
+                    for (int jj = 0; jj < 32; jj++) part = fmaf(v[jj], ys[sl][jj], part);
+                } else {
+                    const float *wt = a.wt + c0 + c * 32;
+#pragma unroll
+                    for (int jj = 0; jj < 32; jj++) v[jj] *= ys[sl][jj];
+#pragma unroll
+                    for (int jj = 0; jj < 32; jj += 4) {
+                        const float4 w = __ldg(reinterpret_cast<const float4 *>(wt + jj));
+                        part = fmaf(v[jj], w.x, fmaf(v[jj + 1], w.y, fmaf(v[jj + 2], w.z, fmaf(v[jj + 3], w.w, part))));
+                    }
+#pragma unroll
+                    for (int jj = 0; jj < 32; jj += 4) {
+                        const float4 w = __ldg(reinterpret_cast<const float4 *>(wt + a.npad + jj));
+                        part1 = fmaf(v[jj], w.x, fmaf(v[jj + 1], w.y, fmaf(v[jj + 2], w.z, fmaf(v[jj + 3], w.w, part1))));
+                    }
+                    if (nw == TC_WEIGHTED3)
+#pragma unroll
+                        for (int jj = 0; jj < 32; jj += 4) {
+                            const float4 w = __ldg(reinterpret_cast<const float4 *>(wt + 2 * a.npad + jj));
+                            part2 = fmaf(v[jj], w.x,
+                                         fmaf(v[jj + 1], w.y, fmaf(v[jj + 2], w.z, fmaf(v[jj + 3], w.w, part2))));
+                        }
+                }
                 if (TWO) {
                     // cross products: lo parts carry a factor 2^11
                     float w[32];
@@ -1041,7 +1068,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
                 if (PAIR) mbar_arrive_remote(acce0 + (uint32_t)(buf * 8));
                 else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(&acce[buf])) : "memory");
             }
-            if (live) atomicAdd(a.out + row * a.nout + outcol, part);
+            if (live) {
+                float *o = a.out + row * a.nout + outcol;
+                atomicAdd(o, part);
+                if (nw >= TC_WEIGHTED2) atomicAdd(o + 1, part1);
+                if (nw == TC_WEIGHTED3) atomicAdd(o + 3, part2);
+            }
             j++;
         }
     }
@@ -1109,7 +1141,7 @@ int launch_phasors_public(const DevSea &sea, long n, const double *x, const doub
                           cudaStream_t stream);
 
 void tcform_free(TcForm &f) {
-    void *q[] = {f.Whi, f.Wlo, f.colscale, f.bmap, f.err, f.scratch};
+    void *q[] = {f.Whi, f.Wlo, f.colscale, f.bmap, f.wt, f.err, f.scratch};
     for (void *p : q) if (p) cudaFree(p);
     for (void *e : f.ev) if (e) cudaEventDestroy((cudaEvent_t)e);
     if (f.aux) cudaStreamDestroy((cudaStream_t)f.aux);
@@ -1127,8 +1159,8 @@ int tcform_split(TcForm &f, const double *coef64, const int *bmap_host, int nblk
     CK(cudaMalloc(&f.Whi, 2 * wel));
     CK(cudaMalloc(&f.Wlo, 2 * wel));
     CK(cudaMalloc(&f.colscale, sizeof(float) * nblk * npad));
-    CK(cudaMalloc(&f.bmap, sizeof(int) * 3 * nblk));
-    CK(cudaMemcpyAsync(f.bmap, bmap_host, sizeof(int) * 3 * nblk, cudaMemcpyHostToDevice, stream));
+    CK(cudaMalloc(&f.bmap, sizeof(int) * 4 * nblk));
+    CK(cudaMemcpyAsync(f.bmap, bmap_host, sizeof(int) * 4 * nblk, cudaMemcpyHostToDevice, stream));
     dim3 gt((unsigned)npad, (unsigned)nblk);
     if (fp16)
         k_qform_split<__half><<<gt, 256, 0, stream>>>(npad, 1, f.one_acc ? 1.0 : 2048.0, coef64, (__half *)f.Whi,
@@ -1339,7 +1371,7 @@ int tcform_eval(TcForm &f, const DevSea &sea, long n, const double *x, const dou
             return E_CUDA;
         QTC q;
         q.rows = mm; q.npad = npad; q.ncomp = sea.n; q.ntn = npad / BN; q.group_m = tc_group_m(); q.nblk = f.nblk; q.nout = f.nout;
-        q.bmap = f.bmap; q.Y = Y; q.ldy = mpad; q.colscale = f.colscale;
+        q.bmap = f.bmap; q.wt = f.wt; q.Y = Y; q.ldy = mpad; q.colscale = f.colscale;
         q.out = out + (long)f.nout * b; q.fp16 = f.fp16 ? 1 : 0; q.err = f.err;
         // column units: each column tile's upper-triangle K range, cut into
         // segments of at most f.kseg K blocks when the form asks for it
@@ -1435,12 +1467,13 @@ int qform_build(const Config &cfg, const DevSea &sea, bool fp16, void *stream_) 
     CK(cudaGetLastError());
     // block b: field (b & 3) -- eta, u, v, w -- X half (b >> 2); the w blocks
     // take the other half of Y (sin(a +- b) = s c +- c s)
-    int bmap[24];
+    int bmap[32];
     for (int b = 0; b < 8; b++) {
         int field = b & 3, kh = b >> 2;
-        bmap[3 * b] = kh;
-        bmap[3 * b + 1] = field == 3 ? 1 - kh : kh;
-        bmap[3 * b + 2] = field;
+        bmap[4 * b] = kh;
+        bmap[4 * b + 1] = field == 3 ? 1 - kh : kh;
+        bmap[4 * b + 2] = field;
+        bmap[4 * b + 3] = TC_TRI;
     }
     // fp16: the cross products in the hi accumulator over K segments of at
     // most 8 blocks (512 terms), so that the FP32 accumulation keeps their

@@ -97,3 +97,33 @@ def test_first_order_channels(wm):
         for f in range(3):
             assert np.max(np.abs(got[1][f, :i, :j] - ref[1][f, :i, :j])) <= TOL * np.max(np.abs(ref[1][f]))
         assert np.max(np.abs(got[2][:i, :j] - ref[2][:i, :j])) <= TOL * np.max(np.abs(ref[2]))
+
+
+@pytest.mark.parametrize("pressure", [False, True])
+@pytest.mark.parametrize("nfreq,ndir", [(1, 1), (31, 1), (257, 1), (43, 3)])
+def test_potential_form(wm, monkeypatch, nfreq, ndir, pressure):
+    """One ramp for all components: the potential form's three full blocks per
+    depth function against the plain pair sums and against the triangular blocks.
+    Each tensor-core form is within 1e-5 of the second-order sums, a few per cent
+    of the fields."""
+    comps = ss.irregular_components(4.0, 9.0, 2.0, nfreq, 0.4, 1.8, 45.0, 3, ndir=ndir, spreading_s=6.0)
+    nx, ny, nl = 13, 17, 10
+    got = {}
+    for form in ("plain", "potential", "triangular"):
+        if form == "triangular":
+            monkeypatch.setenv("CFDWM_DF_TWO_ACC", "1")
+        grid = {"bounds": (-40.0, -40.0 + D * (nx - 1), 10.0, 10.0 + D * (ny - 1)), "nx": nx, "ny": ny, "nl": nl,
+                "t0": 7.5, "dt": 0.5, "stretch": (0.7, 1.5)}
+        txt = ss.write_irregular(None, comps, 45.0, extrap=2, swl=0.3, mtheta=20.0, lsgrid=grid)
+        assert wm.initialize_text(txt) == 0, cw.last_error()
+        wm.sgrid_method(0 if form == "plain" else 1)
+        if pressure:
+            wm.sgrid_pressure(True)
+        got[form] = _newest(wm, nx, ny, nl)
+        if pressure:
+            p = np.zeros((nx, ny, nl), np.float32)
+            assert wm.lib.cfdwm_sgrid_block_export(4, 0, nx, cw._ptr(p)) == 0, cw.last_error()
+            got[form].append(p)
+    for form in ("potential", "triangular"):
+        for f, (a, b) in enumerate(zip(got[form], got["plain"])):
+            assert np.max(np.abs(a - b)) <= 2e-6 * np.max(np.abs(b)), (form, f, np.max(np.abs(a - b)) / np.max(np.abs(b)))
