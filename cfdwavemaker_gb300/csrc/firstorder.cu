@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(512, 1) k_first_levels(LevelArgs a, int rows) 
                 float4 sc[2], ss[2];
 #pragma unroll
                 for (int h = 0; h < 2; h++) sc[h] = ss[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll(TILE || MODE == LV_FEAT ? 4 : 8)
+#pragma unroll(MODE == LV_FEAT ? 4 : 8)
                 for (int q = qb; q < qe; q++) {
                     const float2 *X = a.T.X + (long)q * a.T.sx, *Y = a.T.Y + (long)q * a.T.sy;
                     float2 x[2], y[2];
