@@ -22,7 +22,7 @@
 // split, three (hi hi, lo hi, hi lo); sums in FP32 in TMEM.  The first form
 // of these kernels gathered each operand tile from FP32 planes with the CUDA
 // cores, nine times over (issue-bound).  Network of 16 levels over a 264 x 264
-// grid, the whole call: 356 us then, 67 now (11 of them the split of the input
+// grid, the whole call: 356 us then, 61 now (11 of them the split of the input
 // planes, at the memory's rate; 10 of them launch overlap).  Loss and gradient
 // of eight 72 x 72 patches: 975 and 133 us.
 //
@@ -145,16 +145,17 @@ __global__ void __launch_bounds__(256) k_ct_pack(PackJobs jobs, const float *w, 
 // ---------------------------------------------------------------------------
 enum { CT_HIDDEN = 0, CT_OUTPUT = 1, CT_DATA = 2, CT_LOSS = 3 };
 
-// M = 128: 8 rows of 16 pixels.  An MMA costs about 33 + N / 2 cycles here (its
-// 4 KB of A from shared memory, measured with N = 32 and 64), so the three dx
-// of a kernel row share one MMA with N = 3 NP on the unshifted pixels, and the
-// epilogue adds the neighbouring pixels' columns: 81 cycles for what takes
-// 3 x 49 with a shifted operand per tap, less the two of 16 columns that give
-// no output.  16 pixels wide rather than 32: training patches are small (70
-// pixels are 5 tiles of 14, 3 of 30).
-constexpr int FW = 16, FX = FW - 2, FY = 8;          // patch width, output tile
-constexpr int FCHUNK = (FY + 2) * FW * 16;           // bytes of 8 channels' patch
-constexpr int FPART = 2 * FCHUNK, FSTAGE = 2 * FPART;   // 16 channels, hi and lo
+// M = 128: 8 rows of 16 pixels, or 4 of 32.  An MMA costs about 33 + N / 2 cycles
+// here (its 4 KB of A from shared memory, measured with N = 32 and 64), so the
+// three dx of a kernel row share one MMA with N = 3 NP on the unshifted pixels,
+// and the epilogue adds the neighbouring pixels' columns: 81 cycles for what
+// takes 3 x 49 with a shifted operand per tap, less the two columns of a row
+// that give no output.
+template <int FW> struct Tile {
+    static constexpr int W = FW, X = FW - 2, Y = 128 / FW;           // patch width, output tile
+    static constexpr int CHUNK = (Y + 2) * W * 16;                   // bytes of 8 channels' patch
+    static constexpr int PART = 2 * CHUNK, STAGE = 2 * PART;         // 16 channels, hi and lo
+};
 constexpr int FRING = 6;                             // stages in flight at most
 constexpr int F_THREADS = 320;
 constexpr int FHEAD = 256 + 4 * 64 * 4 + 32;         // barriers and flags, bias and loss sums
@@ -189,13 +190,14 @@ template <int NP> struct CtCfg {
 // copies patches through a ring of stages, warp 1 issues the MMAs, warps 2 to 9
 // (two to a lane quarter, half of the channels each) make the epilogue of one
 // tile while the next one accumulates.
-template <int NP, int EPI>
+template <int NP, int EPI, int FW>
 __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ CUtensorMap xm, ConvArgs a) {
     using CF = CtCfg<NP>;
+    using T = Tile<FW>;
     extern __shared__ __align__(128) uint8_t ct_raw[];
     uint8_t *wsm = (uint8_t *)(((uintptr_t)ct_raw + 127) & ~(uintptr_t)127);
     uint8_t *asm_ = wsm + a.nst * CF::WSTAGE;
-    uint64_t *full = (uint64_t *)(asm_ + a.ring * FSTAGE), *empty = full + FRING, *wfull = empty + FRING;
+    uint64_t *full = (uint64_t *)(asm_ + a.ring * T::STAGE), *empty = full + FRING, *wfull = empty + FRING;
     uint64_t *afull = wfull + 1, *aempty = afull + 2;
     uint32_t *tslot = (uint32_t *)(aempty + 2);
     volatile int *fail = (volatile int *)(tslot + 1);
@@ -226,11 +228,11 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ C
             bool ok = true;
             for (int t = blockIdx.x; ok && t < a.ntiles; t += gridDim.x) {
                 const int b = t / a.tiles_img, r = t - b * a.tiles_img, ty = r / a.tiles_x;
-                const int x0 = (r - ty * a.tiles_x) * FX + a.origin, y0 = ty * FY + a.origin;
+                const int x0 = (r - ty * a.tiles_x) * T::X + a.origin, y0 = ty * T::Y + a.origin;
                 for (int s = 0; s < a.nst; s++, k++) {
                     if (k >= a.ring && !mbar_wait(empty + buf, par, a.err, 11)) { ok = false; break; }
-                    mbar_expect_tx(full + buf, FSTAGE);
-                    tma_4d(asm_ + buf * FSTAGE, &xm, full + buf, x0 * 8, y0, s * 2, b * 2);
+                    mbar_expect_tx(full + buf, T::STAGE);
+                    tma_4d(asm_ + buf * T::STAGE, &xm, full + buf, x0 * 8, y0, s * 2, b * 2);
                     if (++buf == a.ring) { buf = 0; par ^= 1; }
                 }
             }
@@ -253,13 +255,13 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ C
                 for (int s = 0; s < a.nst; s++) {
                     if (!mbar_wait(full + buf, par, a.err, 14)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t da = cdesc(su32(asm_ + buf * FSTAGE), FCHUNK, 128);
+                    const uint64_t da = cdesc(su32(asm_ + buf * T::STAGE), T::CHUNK, 128);
                     const uint64_t db = cdesc(W + s * CF::WSTAGE, CF::N * 16, 128);
 #pragma unroll
                     for (int dy = 0; dy < 3; dy++) {
                         const uint64_t oa = (uint64_t)((dy * FW * 16) >> 4), ob = (uint64_t)((dy * 2 * CF::N * 16) >> 4);
                         umma(d, da + oa, db + ob, idesc, (s | dy) ? 1u : 0u);
-                        umma(d, da + oa + (FPART >> 4), db + ob, idesc, 1u);
+                        umma(d, da + oa + (T::PART >> 4), db + ob, idesc, 1u);
                     }
                     umma_commit(empty + buf);
                     if (++buf == a.ring) { buf = 0; par ^= 1; }
@@ -283,9 +285,9 @@ __global__ void __launch_bounds__(F_THREADS, 2) k_conv(const __grid_constant__ C
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + acc * CF::ACOLS;
             const int b = t / a.tiles_img, r = t % a.tiles_img;
-            const int oy = (r / a.tiles_x) * FY + (m / FW), ox = (r % a.tiles_x) * FX + col;
+            const int oy = (r / a.tiles_x) * T::Y + (m / FW), ox = (r % a.tiles_x) * T::X + col;
             const long pix = (long)oy * a.Wo + ox;
-            const bool live = col < FX && oy < a.Ho && ox < a.Wo;
+            const bool live = col < T::X && oy < a.Ho && ox < a.Wo;
 #pragma unroll
             for (int k = 0; k < NP / 32; k++) {
                 const int h = hf * (NP / 32) + k;
@@ -669,20 +671,55 @@ int launch_pdl(void (*kern)(P...), dim3 grid, int threads, int smem, cudaStream_
 
 int conv_ctas(int ntiles) { return std::min(ntiles, 2 * SMS); }
 
-template <int NP, int EPI>
-int launch_conv(const CUtensorMap &m, ConvArgs &a, int B, cudaStream_t st) {
+// Tiles of B output planes.  32 pixels wide where that takes fewer rounds of the
+// resident CTAs: the network of 264 x 264 has 627 tiles of 14 x 8 outputs a layer, a
+// third round for 19 of them, and 594 of 30 x 4: first layer 16.2 and 14.7 us, the next two
+// 10.8 and 9.9.  Otherwise 16, whose
+// halo is smaller and which suits small planes (70 pixels are 5 tiles of 14, 3 of 30).
+struct ConvTiles {
+    int fw, tx, img, n;
+};
+ConvTiles conv_tiles(int B, int Ho, int Wo) {
+    auto make = [&](int fw) {
+        ConvTiles t;
+        t.fw = fw;
+        t.tx = ceil_div(Wo, fw - 2);
+        t.img = t.tx * ceil_div(Ho, 128 / fw);
+        t.n = B * t.img;
+        return t;
+    };
+    const ConvTiles a = make(16), b = make(32);
+    return ceil_div(b.n, 2 * SMS) < ceil_div(a.n, 2 * SMS) ? b : a;
+}
+
+template <int NP, int EPI, int FW>
+int launch_conv_t(const CUtensorMap &m, ConvArgs &a, cudaStream_t st) {
+    constexpr int STAGE = Tile<FW>::STAGE;
     const int wbytes = a.nst * CtCfg<NP>::WSTAGE, head = wbytes + FHEAD + 128;
     // two CTAs on an SM where the weights leave room for three stages each
-    const int room = head + 3 * FSTAGE <= SMEM_HALF ? SMEM_HALF : SMEM_SM;
-    a.ring = std::min(FRING, (room - head) / FSTAGE);
+    const int room = head + 3 * STAGE <= SMEM_HALF ? SMEM_HALF : SMEM_SM;
+    a.ring = std::min(FRING, (room - head) / STAGE);
     if (a.ring < 1) return E_UNSUPPORTED;
     static const cudaError_t attr =
-        cudaFuncSetAttribute(k_conv<NP, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_SM);
+        cudaFuncSetAttribute(k_conv<NP, EPI, FW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_SM);
     CK(attr);
-    a.tiles_x = ceil_div(a.Wo, FX);
-    a.tiles_img = a.tiles_x * ceil_div(a.Ho, FY);
-    a.ntiles = B * a.tiles_img;
-    return launch_pdl(k_conv<NP, EPI>, dim3((unsigned)conv_ctas(a.ntiles)), F_THREADS, head + a.ring * FSTAGE, st, m, a);
+    return launch_pdl(k_conv<NP, EPI, FW>, dim3((unsigned)conv_ctas(a.ntiles)), F_THREADS, head + a.ring * STAGE, st, m,
+                      a);
+}
+
+// The convolution of split inputs xs (K channels, H x W) to Ho x Wo outputs.
+template <int NP, int EPI>
+int launch_conv(ConvArgs &a, const void *xs, int B, int K, int H, int W, cudaStream_t st) {
+    const ConvTiles t = conv_tiles(B, a.Ho, a.Wo);
+    a.nst = ceil_div(K, 16);
+    a.tiles_x = t.tx;
+    a.tiles_img = t.img;
+    a.ntiles = t.n;
+    int rc = ct_err_word(&a.err);
+    if (rc) return rc;
+    CUtensorMap m;
+    if ((rc = ct_map(&m, xs, B, ceil_div(K, 8), H, W, false, t.fw, 128 / t.fw + 2, 2))) return rc;
+    return t.fw == 32 ? launch_conv_t<NP, EPI, 32>(m, a, st) : launch_conv_t<NP, EPI, 16>(m, a, st);
 }
 
 }  // namespace
@@ -726,65 +763,45 @@ int conv_pack(const ConvPack *jobs, int n, const float *w, void *out, void *stre
     return OK;
 }
 
-static int conv_args(ConvArgs &a, CUtensorMap &m, const void *xs, const void *wp, int B, int K, int H, int W,
-                     int origin, int Ho, int Wo) {
-    a = {};
-    a.w = (const uint8_t *)wp;
-    a.nst = ceil_div(K, 16);
-    a.origin = origin;
-    a.Ho = Ho; a.Wo = Wo;
-    int rc = ct_err_word(&a.err);
-    if (rc) return rc;
-    return ct_map(&m, xs, B, ceil_div(K, 8), H, W, false, FW, FY + 2, 2);
-}
-
 int conv_hidden(const void *xs, const void *wp, const float *bias, int B, int C, int H, int W, void *ys, void *ds,
                 void *stream) {
     if (C < 1 || H < 3 || W < 3 || B < 1) return E_BAD_ARGUMENT;
-    ConvArgs a;
-    CUtensorMap m;
-    int rc = conv_args(a, m, xs, wp, B, C, H, W, 0, H - 2, W - 2);
-    if (rc) return rc;
+    ConvArgs a = {};
+    a.w = (const uint8_t *)wp; a.Ho = H - 2; a.Wo = W - 2;
     a.bias = bias; a.ys = (uint4 *)ys; a.ds_out = (float4 *)ds;
-    return launch_conv<32, CT_HIDDEN>(m, a, B, (cudaStream_t)stream);
+    return launch_conv<32, CT_HIDDEN>(a, xs, B, C, H, W, (cudaStream_t)stream);
 }
 
 int conv_output(const void *xs, const void *wp, const float *bias, int B, int C, int O, int H, int W, float *y,
                 void *stream) {
     if (O < 1 || O > 64 || C < 1 || H < 3 || W < 3 || B < 1) return E_BAD_ARGUMENT;
-    ConvArgs a;
-    CUtensorMap m;
-    int rc = conv_args(a, m, xs, wp, B, C, H, W, 0, H - 2, W - 2);
-    if (rc) return rc;
+    ConvArgs a = {};
+    a.w = (const uint8_t *)wp; a.Ho = H - 2; a.Wo = W - 2;
     a.bias = bias; a.y = y; a.O = O;
-    return O <= 32 ? launch_conv<32, CT_OUTPUT>(m, a, B, (cudaStream_t)stream)
-                   : launch_conv<64, CT_OUTPUT>(m, a, B, (cudaStream_t)stream);
+    return O <= 32 ? launch_conv<32, CT_OUTPUT>(a, xs, B, C, H, W, (cudaStream_t)stream)
+                   : launch_conv<64, CT_OUTPUT>(a, xs, B, C, H, W, (cudaStream_t)stream);
 }
 
 int conv_loss(const void *xs, const void *wp, const float *bias, int B, int C, int O, int H, int W,
               const ConvLoss &l, void *dys, float *bpart, float *lpart, void *stream) {
     if (O < 1 || O > 64 || C < 1 || H < 3 || W < 3 || B < 1) return E_BAD_ARGUMENT;
-    ConvArgs a;
-    CUtensorMap m;
-    int rc = conv_args(a, m, xs, wp, B, C, H, W, 0, H - 2, W - 2);
-    if (rc) return rc;
+    ConvArgs a = {};
+    a.w = (const uint8_t *)wp; a.Ho = H - 2; a.Wo = W - 2;
     a.bias = bias; a.O = O; a.ys = (uint4 *)dys; a.bpart = bpart; a.lpart = lpart;
     a.tg = l.tg; a.tbs = l.tbs; a.idx = l.idx; a.w0 = l.w0; a.inv_norm = l.inv_norm;
-    return O <= 32 ? launch_conv<32, CT_LOSS>(m, a, B, (cudaStream_t)stream)
-                   : launch_conv<64, CT_LOSS>(m, a, B, (cudaStream_t)stream);
+    return O <= 32 ? launch_conv<32, CT_LOSS>(a, xs, B, C, H, W, (cudaStream_t)stream)
+                   : launch_conv<64, CT_LOSS>(a, xs, B, C, H, W, (cudaStream_t)stream);
 }
 
-int conv_bias_parts(int B, int H, int W) { return conv_ctas(B * ceil_div(W, FX) * ceil_div(H, FY)); }
+int conv_bias_parts(int B, int H, int W) { return conv_ctas(conv_tiles(B, H, W).n); }
 
 int conv_data_grad(const void *dys, const void *wp, const void *ds, int B, int O, int H, int W, void *dxs,
                    float *bpart, void *stream) {
     if (O < 1 || H < 3 || W < 3 || B < 1) return E_BAD_ARGUMENT;
-    ConvArgs a;
-    CUtensorMap m;
-    int rc = conv_args(a, m, dys, wp, B, O, H - 2, W - 2, -2, H, W);
-    if (rc) return rc;
+    ConvArgs a = {};
+    a.w = (const uint8_t *)wp; a.origin = -2; a.Ho = H; a.Wo = W;
     a.ds = (const float4 *)ds; a.ys = (uint4 *)dxs; a.bpart = bpart;
-    return launch_conv<32, CT_DATA>(m, a, B, (cudaStream_t)stream);
+    return launch_conv<32, CT_DATA>(a, dys, B, O, H - 2, W - 2, (cudaStream_t)stream);
 }
 
 // The units of the layers' weight gradients and their CTAs.
@@ -889,10 +906,13 @@ int conv_sums(const ConvSum *jobs, int n, void *stream) {
 int conv_load() {
     static const cudaError_t rc = [] {
         const void *k[] = {(const void *)k_ct_split, (const void *)k_ct_pack, (const void *)k_ct_sum,
-                           (const void *)k_conv_wgt, (const void *)k_conv<32, CT_HIDDEN>,
-                           (const void *)k_conv<32, CT_OUTPUT>, (const void *)k_conv<64, CT_OUTPUT>,
-                           (const void *)k_conv<32, CT_LOSS>, (const void *)k_conv<64, CT_LOSS>,
-                           (const void *)k_conv<32, CT_DATA>};
+                           (const void *)k_conv_wgt, (const void *)k_conv<32, CT_HIDDEN, 16>,
+                           (const void *)k_conv<32, CT_OUTPUT, 16>, (const void *)k_conv<64, CT_OUTPUT, 16>,
+                           (const void *)k_conv<32, CT_LOSS, 16>, (const void *)k_conv<64, CT_LOSS, 16>,
+                           (const void *)k_conv<32, CT_DATA, 16>, (const void *)k_conv<32, CT_HIDDEN, 32>,
+                           (const void *)k_conv<32, CT_OUTPUT, 32>, (const void *)k_conv<64, CT_OUTPUT, 32>,
+                           (const void *)k_conv<32, CT_LOSS, 32>, (const void *)k_conv<64, CT_LOSS, 32>,
+                           (const void *)k_conv<32, CT_DATA, 32>};
         cudaFuncAttributes at;
         for (const void *f : k) {
             const cudaError_t e = cudaFuncGetAttributes(&at, f);

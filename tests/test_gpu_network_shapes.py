@@ -1,7 +1,8 @@
 """The learned update's network at the edges of its kernels' tiles: planes
 smaller than a tile, one more and one less than whole tiles, several images,
 level counts whose channels are not whole groups of 16, need one or several
-blocks of the weight gradient, or fill the output's 64."""
+blocks of the weight gradient, or fill the output's 64; planes that take the
+wide tiles."""
 import ctypes
 
 import numpy as np
@@ -17,7 +18,8 @@ TOL_NET, TOL_GRAD = 1e-5, 1e-4          # the bars of test_gpu_surrogate.py
 
 
 @pytest.mark.parametrize("nl,b,h,w", [(1, 1, 9, 9), (2, 3, 10, 23), (3, 2, 16, 15), (5, 1, 17, 38), (6, 2, 25, 24),
-                                      (10, 1, 24, 64), (11, 1, 31, 22), (16, 2, 22, 37), (21, 1, 18, 30)])
+                                      (10, 1, 24, 64), (11, 1, 31, 22), (16, 2, 22, 37), (21, 1, 18, 30),
+                                      (2, 2, 250, 62), (11, 2, 247, 61)])
 def test_network_and_gradient(nl, b, h, w):
     torch = pytest.importorskip("torch")
     lib = cw.load()
