@@ -673,9 +673,9 @@ int conv_ctas(int ntiles) { return std::min(ntiles, 2 * SMS); }
 
 // Tiles of B output planes.  32 pixels wide where that takes fewer rounds of the
 // resident CTAs: the network of 264 x 264 has 627 tiles of 14 x 8 outputs a layer, a
-// third round for 19 of them, and 594 of 30 x 4: first layer 16.2 and 14.7 us, the next two
-// 10.8 and 9.9.  Otherwise 16, whose
-// halo is smaller and which suits small planes (70 pixels are 5 tiles of 14, 3 of 30).
+// third round for 19 of them, and 594 of 30 x 4: first layer 16.2 and 14.7 us, the
+// next two 10.8 and 9.9.  Otherwise 16, whose halo is smaller and which suits small
+// planes (70 pixels are 5 tiles of 14, 3 of 30).
 struct ConvTiles {
     int fw, tx, img, n;
 };
