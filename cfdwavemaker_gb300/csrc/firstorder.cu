@@ -262,6 +262,8 @@ template <int MODE, bool FEW> struct LvCfg {
     }
 };
 
+__device__ __forceinline__ void lv_prefetch(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 // A block holds `rows` sets of 32 columns (TILE: rows of the grid, which share
 // their y entries; else listed columns), a warp 8 levels of one set.  The depth
 // profiles
@@ -277,8 +279,8 @@ template <int MODE, bool FEW> struct LvCfg {
 // of the pass before.  With the profiles per component the second half was
 // bound by the FMA and SFU pipes (58 % and 30 % busy).  16 levels, 1024 components
 // in 64 groups, features of 69696 columns: one level at a time with float-float
-// phases 1263 us, packed 805, by groups 204; levels of 65536 columns: 675, 660
-// and 164.
+// phases 1263 us, packed 805, by groups 186; levels of 65536 columns: 675, 660
+// and 158.
 template <int MODE, bool TILE, bool FEW>
 __global__ void __launch_bounds__(512, 1) k_first_levels(LevelArgs a, int rows) {
     using CF = LvCfg<MODE, FEW>;
@@ -408,6 +410,16 @@ __global__ void __launch_bounds__(512, 1) k_first_levels(LevelArgs a, int rows) 
     __syncthreads();
     for (int g0 = 0, buf = 0, since = 1; g0 < a.T.ngrp; g0 += LGC, buf ^= 1, since++) {
         if (g0 + LGC < a.T.ngrp) sums(g0 + LGC, buf ^ 1);
+        // the entries of this warp's group of the pass after next, toward L1, many
+        // lines an instruction (features 201 and 186 us)
+        if (TILE && w < LGC && g0 + 2 * LGC + w < a.T.ngrp) {
+            const int qb = a.T.grp[g0 + 2 * LGC + w], qe = a.T.grp[g0 + 2 * LGC + w + 1];
+            for (int q = qb + (lane >> 1); q < qe; q += 16) {
+                lv_prefetch(a.T.Y + (long)q * a.T.sy + blockIdx.x * 32 + (lane & 1) * 16);
+                if (lane & 1) lv_prefetch(a.T.X + (long)q * a.T.sx + blockIdx.y * rows);
+                else lv_prefetch(a.T.rec + (long)q * REC + REC_L);
+            }
+        }
         const int ngc = min(LGC, a.T.ngrp - g0);
         for (int gi = 0; gi < (worker ? ngc : 0); gi++) {
             const ulonglong2 rk = *reinterpret_cast<const ulonglong2 *>(s_k + buf * LGC + gi);
