@@ -279,8 +279,9 @@ __device__ __forceinline__ void lv_prefetch(const void *p) { asm volatile("prefe
 // of the pass before.  With the profiles per component the second half was
 // bound by the FMA and SFU pipes (58 % and 30 % busy).  16 levels, 1024 components
 // in 64 groups, features of 69696 columns: one level at a time with float-float
-// phases 1263 us, packed 805, by groups 186; levels of 65536 columns: 675, 660
-// and 158.
+// phases 1263 us, packed 805, by groups 169; levels of 65536 columns: 675, 660
+// and 121 (the kernel alone on the GPU; beside the checked columns of a learned
+// update the features take 290).
 template <int MODE, bool TILE, bool FEW>
 __global__ void __launch_bounds__(512, 1) k_first_levels(LevelArgs a, int rows) {
     using CF = LvCfg<MODE, FEW>;
@@ -411,7 +412,8 @@ __global__ void __launch_bounds__(512, 1) k_first_levels(LevelArgs a, int rows) 
     for (int g0 = 0, buf = 0, since = 1; g0 < a.T.ngrp; g0 += LGC, buf ^= 1, since++) {
         if (g0 + LGC < a.T.ngrp) sums(g0 + LGC, buf ^ 1);
         // the entries of this warp's group of the pass after next, toward L1, many
-        // lines an instruction (features 201 and 186 us)
+        // lines an instruction (levels of 65536 columns 123 and 121 us; features
+        // alone 169 us with and without; a learned update 592-600 and 577-586 us)
         if (TILE && w < LGC && g0 + 2 * LGC + w < a.T.ngrp) {
             const int qb = a.T.grp[g0 + 2 * LGC + w], qe = a.T.grp[g0 + 2 * LGC + w + 1];
             for (int q = qb + (lane >> 1); q < qe; q += 16) {
