@@ -500,7 +500,7 @@ int depthform_build(const Config &cfg, const DevSea &sea, DepthForm &df, int nf,
     a.tab_grid = sea.d_tab_grid; a.tab_eta = sea.d_tab_eta; a.tab_gp = sea.d_tab_gp; a.fk = d_fk; a.gk = d_gk;
     a.inv_dk = 1.0 / dk; a.coef = coef;
     a.cstride = sea.npad_g; a.phase = sea.d_phase; a.rho = sea.rho;
-    CK(cudaMalloc(&a.wt, sizeof(float) * 3 * npad));
+    if (pot) CK(cudaMalloc(&a.wt, sizeof(float) * 3 * npad));
     long tot = (long)npad * npad;
     if (pot) k_depth_coef_pot<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(a);
     else k_depth_coef<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(a);

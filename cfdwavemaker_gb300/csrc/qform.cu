@@ -37,6 +37,7 @@
 //    visited.  Every mbarrier wait is bounded; a timeout sets an error word.
 //  * k_qform_plain: the same sums on FP32 CUDA cores (the plain form).
 #include "cfdwm.h"
+#include "f32x2.cuh"
 #include "ffmath.cuh"
 #include "tc05.cuh"
 
@@ -47,6 +48,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 namespace cfdwm {
@@ -244,49 +246,57 @@ __global__ void k_qform_split(int npad, int fp16, double lo_scale, const double 
 // lo) coordinates, then reduced by a three-part 2 pi (Cody-Waite) before the
 // FP32 sincos.  Error: a few 1e-7 rad at |phase| ~ 1e4.
 // ---------------------------------------------------------------------------
-struct QRow {     // per row: dx, dy, t as float pairs and the ramp (trivial ramps)
-    float dxh, dxl, dyh, dyl, th, tl, ramp, pad;
+// Per row: dx, dy, t as float pairs (the products' error terms are formed with
+// the negated parts) and the ramp (trivial ramps), each twice: the operands of
+// packed arithmetic on two components.
+struct alignas(16) QRow {
+    float2 dxh, ndxh, ndxl, dyh, ndyh, ndyl, th, nth, ntl, ramp;
 };
-struct QComp {    // per component: kx, ky, -omega, phase0 as float pairs
-    float kxh, kxl, kyh, kyl, wh, wl, ph, pl;
-};
+// Per component, rows of npad: kx, ky, -omega, phase0 as float pairs (hi, lo;
+// phase0's lo part negated).
+constexpr int QCOMP = 8;
 
 __global__ void k_qform_rows(long rows, const double *x, const double *y, const double *t, long st, double fx,
                              double fy, const double *phase, int cstride, QRow *out) {
     long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (p >= rows) return;
-    double dx = x[p] - fx, dy = y[p] - fy, tt = t[p * st];
+    const double v[3] = {x[p] - fx, y[p] - fy, t[p * st]};
+    float h[3], l[3];
+    for (int q = 0; q < 3; q++) { h[q] = (float)v[q]; l[q] = (float)(v[q] - (double)h[q]); }
+    auto two = [](float a) { return make_float2(a, a); };
     QRow r;
-    r.dxh = (float)dx; r.dxl = (float)(dx - (double)r.dxh);
-    r.dyh = (float)dy; r.dyl = (float)(dy - (double)r.dyh);
-    r.th = (float)tt; r.tl = (float)(tt - (double)r.th);
-    r.ramp = (float)q_freq_ramp(tt, phase[4 * cstride], phase[5 * cstride], phase[6 * cstride]);
-    r.pad = 0.f;
+    r.dxh = two(h[0]); r.ndxh = two(-h[0]); r.ndxl = two(-l[0]);
+    r.dyh = two(h[1]); r.ndyh = two(-h[1]); r.ndyl = two(-l[1]);
+    r.th = two(h[2]); r.nth = two(-h[2]); r.ntl = two(-l[2]);
+    r.ramp = two((float)q_freq_ramp(v[2], phase[4 * cstride], phase[5 * cstride], phase[6 * cstride]));
     out[p] = r;
 }
 
-__global__ void k_qform_comps(int n, int npad, const double *phase, int cstride, QComp *out) {
+__global__ void k_qform_comps(int n, int npad, const double *phase, int cstride, float *out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npad) return;
-    QComp c = {0, 0, 0, 0, 0, 0, 0, 0};
+    double v[4] = {0, 0, 0, 0};
     if (i < n) {
-        double v[4] = {phase[i], phase[cstride + i], -phase[2 * cstride + i], phase[3 * cstride + i]};
-        float h[4], l[4];
-        for (int q = 0; q < 4; q++) { h[q] = (float)v[q]; l[q] = (float)(v[q] - (double)h[q]); }
-        c = {h[0], l[0], h[1], l[1], h[2], l[2], h[3], l[3]};
+        v[0] = phase[i]; v[1] = phase[cstride + i]; v[2] = -phase[2 * cstride + i]; v[3] = phase[3 * cstride + i];
     }
-    out[i] = c;
+    for (int q = 0; q < 4; q++) {
+        const float h = (float)v[q], l = (float)(v[q] - (double)h);
+        out[(long)(2 * q) * npad + i] = h;
+        out[(long)(2 * q + 1) * npad + i] = q == 3 ? -l : l;
+    }
 }
 
 struct QPrep {
     long rows;
     const QRow *row;
-    const QComp *comp;
+    const float *comp;
     const double *phase;       // [7][cstride] (ramp parameters for non-trivial ramps)
     const double *t;
     long st;                   // element stride of t
     int cstride, ncomp, npad;
     int trivial_ramp, fp16;
+    f32x2 none;              // (-1, -1): a - b is fma(b, -1, a), rounded alike
+    f32x2 ninv, P[3];        // -1 / 2 pi, 2 pi in three parts (ff_reduce_2pi)
     float lo_scale;          // fp16: factor of the lo parts (2^11 with a cross accumulator, else 1)
     void *Xhi, *Xlo;           // [rows][2 npad]
     float *Y;                  // [2 npad][ldy], column-major: rows adjacent
@@ -298,7 +308,21 @@ struct QPrep {
     long row0;
 };
 
-constexpr int PREP_ROWS = 16;      // rows per block of the operand preparation
+constexpr int PREP_ROWS = 8;      // rows per block of the operand preparation
+
+// The arithmetic of the two components is packed (ff_mul, ff_add of
+// ffmath.cuh with the error terms carried negated).
+__device__ __forceinline__ void qp_mul(f32x2 ah, f32x2 al, f32x2 bh, f32x2 nbh, f32x2 nbl, f32x2 &p, f32x2 &ne) {
+    p = p_mul(ah, bh);
+    ne = p_fma(ah, nbl, p_fma(al, nbh, p_fma(ah, nbh, p)));
+}
+__device__ __forceinline__ void qp_add(f32x2 &a, f32x2 &na, f32x2 b, f32x2 nb, f32x2 none) {
+    const f32x2 s = p_add(a, b), bb = p_fma(a, none, s);
+    const f32x2 e = p_add(p_fma(p_fma(bb, none, s), none, a), p_fma(bb, none, b));
+    na = p_add(p_fma(e, none, na), nb);
+    a = s;
+}
+__device__ __forceinline__ f32x2 qp_ld(const float2 &v) { return *reinterpret_cast<const f32x2 *>(&v); }
 
 // blockDim 128: thread t owns components i = 256 blockIdx.x + 2t and i + 1
 // (their float-float coefficients stay in registers); blockIdx.y: a group of
@@ -314,82 +338,98 @@ template <bool GRID>
 __global__ void __launch_bounds__(128) k_qform_prep(QPrep a) {
     __shared__ float s_y[512][PREP_ROWS + 1];     // [cos 256 | sin 256][row]
     const int i = blockIdx.x * 256 + 2 * threadIdx.x;
-    QComp K[2];
-    bool on[2];
+    const bool on0 = i < a.ncomp, on1 = i + 1 < a.ncomp;
+    f32x2 K[QCOMP], gr = 0ull;
+    if (GRID) {
+        if (on0) gr = p_pack(a.T.ramp[i], on1 ? a.T.ramp[i + 1] : 0.f);
+    } else {
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
-        on[q] = i + q < a.ncomp;
-        K[q] = on[q] && !GRID ? a.comp[i + q] : QComp{0, 0, 0, 0, 0, 0, 0, 0};
+        for (int q = 0; q < QCOMP; q++) K[q] = *reinterpret_cast<const f32x2 *>(a.comp + (long)q * a.npad + i);
     }
-    float gr[2] = {0.f, 0.f};
-    if (GRID)
-#pragma unroll
-        for (int q = 0; q < 2; q++)
-            if (on[q]) gr[q] = a.T.ramp[i + q];
+    const f32x2 none = a.none;
     const long p0 = (long)blockIdx.y * PREP_ROWS;
     for (int rr = 0; rr < PREP_ROWS; rr++) {
         const long p = p0 + rr;
-        float c[2] = {0.f, 0.f}, s[2] = {0.f, 0.f}, r[2] = {0.f, 0.f};
+        f32x2 c = 0ull, s = 0ull, r = 0ull;
         if (GRID) {
-            if (p < a.rows && on[0]) {
+            if (p < a.rows && on0) {
                 const int col = a.act ? a.act[a.row0 + p] : (int)(a.row0 + p), ix = col / a.gny, iy = col - ix * a.gny;
                 // the tables are padded with zeros to a multiple of 128 components
                 const float4 X = *reinterpret_cast<const float4 *>(a.T.Xt + (long)ix * a.T.ncp + i);
                 const float4 Y = *reinterpret_cast<const float4 *>(a.T.Yt + (long)iy * a.T.ncp + i);
-                c[0] = fmaf(X.x, Y.x, -(X.y * Y.y)); s[0] = fmaf(X.y, Y.x, X.x * Y.y);
-                c[1] = fmaf(X.z, Y.z, -(X.w * Y.w)); s[1] = fmaf(X.w, Y.z, X.z * Y.w);
-                r[0] = gr[0];
-                r[1] = gr[1];
+                c = p_pack(fmaf(X.x, Y.x, -(X.y * Y.y)), fmaf(X.z, Y.z, -(X.w * Y.w)));
+                s = p_pack(fmaf(X.y, Y.x, X.x * Y.y), fmaf(X.w, Y.z, X.z * Y.w));
+                r = gr;
             }
-        } else if (p < a.rows) {
-            const QRow R = a.row[p];
+        } else if (p < a.rows && on0) {
+            const QRow &R = a.row[p];
+            f32x2 ph, nl, q, nq;
+            qp_mul(K[0], K[1], qp_ld(R.dxh), qp_ld(R.ndxh), qp_ld(R.ndxl), ph, nl);
+            qp_mul(K[2], K[3], qp_ld(R.dyh), qp_ld(R.ndyh), qp_ld(R.ndyl), q, nq);
+            qp_add(ph, nl, q, nq, none);
+            qp_mul(K[4], K[5], qp_ld(R.th), qp_ld(R.nth), qp_ld(R.ntl), q, nq);
+            qp_add(ph, nl, q, nq, none);
+            qp_add(ph, nl, K[6], K[7], none);
+            // ff_reduce_2pi
+            const float2 n = p_un(p_mul(ph, a.ninv));
+            const f32x2 nn = p_pack(rintf(n.x), rintf(n.y));
+            const float2 x = p_un(p_fma(nl, none, p_fma(nn, a.P[2], p_fma(nn, a.P[1], p_fma(nn, a.P[0], ph)))));
+            float c0, s0, c1, s1;
+            __sincosf(x.x, &s0, &c0);
+            __sincosf(x.y, &s1, &c1);
+            c = p_pack(c0, on1 ? c1 : 0.f);
+            s = p_pack(s0, on1 ? s1 : 0.f);
+            if (a.trivial_ramp) r = qp_ld(R.ramp);
+            else {
+                float f[2] = {0.f, 0.f};
 #pragma unroll
-            for (int q = 0; q < 2; q++) {
-                if (!on[q]) continue;
-                float2 ph = ff_add(ff_mul(K[q].kxh, K[q].kxl, R.dxh, R.dxl), ff_mul(K[q].kyh, K[q].kyl, R.dyh, R.dyl));
-                ph = ff_add(ph, ff_mul(K[q].wh, K[q].wl, R.th, R.tl));
-                ph = ff_add(ph, make_float2(K[q].ph, K[q].pl));
-                __sincosf(ff_reduce_2pi(ph), &s[q], &c[q]);
-                r[q] = a.trivial_ramp ? R.ramp
-                                      : (float)q_freq_ramp(a.t[p * a.st], a.phase[4 * a.cstride + i + q],
-                                                           a.phase[5 * a.cstride + i + q],
-                                                           a.phase[6 * a.cstride + i + q]);
+                for (int k = 0; k < 2; k++)
+                    if (k == 0 || on1)
+                        f[k] = (float)q_freq_ramp(a.t[p * a.st], a.phase[4 * a.cstride + i + k],
+                                                  a.phase[5 * a.cstride + i + k], a.phase[6 * a.cstride + i + k]);
+                r = p_pack(f[0], f[1]);
             }
         }
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-            s_y[2 * threadIdx.x + q][rr] = c[q];
-            s_y[256 + 2 * threadIdx.x + q][rr] = s[q];
-        }
+        const float2 cu = p_un(c), su = p_un(s);
+        s_y[2 * threadIdx.x][rr] = cu.x;
+        s_y[2 * threadIdx.x + 1][rr] = cu.y;
+        s_y[256 + 2 * threadIdx.x][rr] = su.x;
+        s_y[256 + 2 * threadIdx.x + 1][rr] = su.y;
         if (p >= a.rows) continue;
         const long o = p * 2 * a.npad + i;
-        const float xc0 = r[0] * c[0], xc1 = r[1] * c[1], xs0 = r[0] * s[0], xs1 = r[1] * s[1];
+        const f32x2 xc = p_mul(r, c), xs = p_mul(r, s);
+        const float2 fxc = p_un(xc), fxs = p_un(xs);
         if (a.fp16) {
-            const __half2 hc = __floats2half2_rn(xc0, xc1), hs = __floats2half2_rn(xs0, xs1);
+            const __half2 hc = __floats2half2_rn(fxc.x, fxc.y), hs = __floats2half2_rn(fxs.x, fxs.y);
             const float2 fc = __half22float2(hc), fs = __half22float2(hs);
+            const f32x2 ls = p_pack(a.lo_scale, a.lo_scale);
+            const float2 lc = p_un(p_mul(p_fma(p_pack(fc.x, fc.y), none, xc), ls));
+            const float2 lsn = p_un(p_mul(p_fma(p_pack(fs.x, fs.y), none, xs), ls));
             __half2 *H = reinterpret_cast<__half2 *>((__half *)a.Xhi + o);
             __half2 *L = reinterpret_cast<__half2 *>((__half *)a.Xlo + o);
             H[0] = hc;
             H[a.npad / 2] = hs;
-            L[0] = __floats2half2_rn((xc0 - fc.x) * a.lo_scale, (xc1 - fc.y) * a.lo_scale);
-            L[a.npad / 2] = __floats2half2_rn((xs0 - fs.x) * a.lo_scale, (xs1 - fs.y) * a.lo_scale);
+            L[0] = __floats2half2_rn(lc.x, lc.y);
+            L[a.npad / 2] = __floats2half2_rn(lsn.x, lsn.y);
         } else {
-            const __nv_bfloat162 hc = __floats2bfloat162_rn(xc0, xc1), hs = __floats2bfloat162_rn(xs0, xs1);
+            const __nv_bfloat162 hc = __floats2bfloat162_rn(fxc.x, fxc.y), hs = __floats2bfloat162_rn(fxs.x, fxs.y);
             const float2 fc = __bfloat1622float2(hc), fs = __bfloat1622float2(hs);
+            const float2 lc = p_un(p_fma(p_pack(fc.x, fc.y), none, xc)), lsn = p_un(p_fma(p_pack(fs.x, fs.y), none, xs));
             __nv_bfloat162 *H = reinterpret_cast<__nv_bfloat162 *>((__nv_bfloat16 *)a.Xhi + o);
             __nv_bfloat162 *L = reinterpret_cast<__nv_bfloat162 *>((__nv_bfloat16 *)a.Xlo + o);
             H[0] = hc;
             H[a.npad / 2] = hs;
-            L[0] = __floats2bfloat162_rn(xc0 - fc.x, xc1 - fc.y);
-            L[a.npad / 2] = __floats2bfloat162_rn(xs0 - fs.x, xs1 - fs.y);
+            L[0] = __floats2bfloat162_rn(lc.x, lc.y);
+            L[a.npad / 2] = __floats2bfloat162_rn(lsn.x, lsn.y);
         }
     }
     __syncthreads();
-    // Y: warp w writes columns 2 k + (lane >> 4), k = w, w + 4, ..., rows lane & 15
+    // Y: a warp writes 32 / PREP_ROWS adjacent columns at a time, each
+    // column's rows by adjacent threads
+    constexpr int CW = 32 / PREP_ROWS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rr = lane & (PREP_ROWS - 1);
-    const int i0 = blockIdx.x * 256;
-    for (int col = 2 * warp + (lane >> 4); col < 512; col += 8) {
+    const int rr = lane & (PREP_ROWS - 1), i0 = blockIdx.x * 256;
+    for (int col = CW * warp + lane / PREP_ROWS; col < 512; col += 4 * CW) {
         const long gcol = col < 256 ? (long)i0 + col : (long)a.npad + i0 + (col - 256);
         a.Y[gcol * a.ldy + p0 + rr] = s_y[col][rr];
     }
@@ -753,7 +793,7 @@ __device__ __forceinline__ bool tile_of(const QTC &a, long nru, long t, int cran
 constexpr int TC_THREADS = 320;            // producer, MMA and 8 epilogue warps
 constexpr int TC_EPI_WARPS = 8;
 
-template <int BN, bool TWO, bool PAIR>
+template <int BN, bool TWO, bool PAIR, bool WT>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constant__ CUtensorMap mXh,
                                                      const __grid_constant__ CUtensorMap mXl,
                                                      const __grid_constant__ CUtensorMap mWh,
@@ -919,7 +959,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
             const int buf = j % NBUF;
             const uint32_t use = (uint32_t)(j / NBUF);
             const int yhalf = a.bmap[4 * ti.blk + 1], outcol = a.bmap[4 * ti.blk + 2];
-            const int nw = TWO ? 0 : a.bmap[4 * ti.blk + 3];      // >= TC_WEIGHTED2: its outputs
+            const int nw = WT ? a.bmap[4 * ti.blk + 3] : 0;       // >= TC_WEIGHTED2: its outputs
             const int c0 = ti.tn * BN + hc * HC;       // first column of this warp
             const int nch = (ti.bn - hc * HC) / 32;    // its chunks of 32 columns in use (may be none)
             const long row = ti.rb * TBM + q * 32 + lane;
@@ -1022,7 +1062,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
                 }
                 float v[32];
                 tmem_ld32(acc + c * 32, v);
-                if (nw < TC_WEIGHTED2) {
+                if (!WT || nw < TC_WEIGHTED2) {
 #pragma unroll
                     for (int jj = 0; jj < 32; jj++) part = fmaf(v[jj], ys[sl][jj], part);
                 } else {
@@ -1071,8 +1111,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
             if (live) {
                 float *o = a.out + row * a.nout + outcol;
                 atomicAdd(o, part);
-                if (nw >= TC_WEIGHTED2) atomicAdd(o + 1, part1);
-                if (nw == TC_WEIGHTED3) atomicAdd(o + 3, part2);
+                if (WT && nw >= TC_WEIGHTED2) atomicAdd(o + 1, part1);
+                if (WT && nw == TC_WEIGHTED3) atomicAdd(o + 3, part2);
             }
             j++;
         }
@@ -1192,13 +1232,13 @@ static int tc_group_m() {
     return g;
 }
 
-template <int BN, bool TWO, bool PAIR>
+template <int BN, bool TWO, bool PAIR, bool WT>
 static int tc_max_units() {
     using CF = TcCfg<BN, TWO, PAIR>;
     // computed on the device current at the first call and kept for the
     // process (the library serves one device: the model's)
     static const int maxunits = [] {
-        if (cudaFuncSetAttribute(k_qform_tc<BN, TWO, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, CF::SMEM) !=
+        if (cudaFuncSetAttribute(k_qform_tc<BN, TWO, PAIR, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, CF::SMEM) !=
             cudaSuccess) {
             cudaGetLastError();     // a failure here only selects the other form
             return -1;
@@ -1222,7 +1262,7 @@ static int tc_max_units() {
         c.attrs = at;
         c.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, k_qform_tc<BN, TWO, PAIR>, &c) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveClusters(&n, k_qform_tc<BN, TWO, PAIR, WT>, &c) != cudaSuccess) {
             cudaGetLastError();
             return -1;
         }
@@ -1231,18 +1271,18 @@ static int tc_max_units() {
     return maxunits;
 }
 
-template <int BN, bool TWO, bool PAIR>
+template <int BN, bool TWO, bool PAIR, bool WT>
 static int launch_tc(const CUtensorMap &mXh, const CUtensorMap &mXl, const CUtensorMap &mWh, const CUtensorMap &mWl,
                      const QTC &q, long nunits, cudaStream_t stream) {
     using CF = TcCfg<BN, TWO, PAIR>;
-    const int maxunits = tc_max_units<BN, TWO, PAIR>();
+    const int maxunits = tc_max_units<BN, TWO, PAIR, WT>();
     if (maxunits <= 0) {
         std::fprintf(stderr, "cfdwm: the tensor-core form (pair %d) does not fit on this device\n", (int)PAIR);
         return E_CUDA;
     }
     const long nu = std::min<long>(nunits, maxunits);
     if (!PAIR) {
-        k_qform_tc<BN, TWO, false><<<(unsigned)nu, TC_THREADS, CF::SMEM, stream>>>(mXh, mXl, mWh, mWl, q);
+        k_qform_tc<BN, TWO, false, WT><<<(unsigned)nu, TC_THREADS, CF::SMEM, stream>>>(mXh, mXl, mWh, mWl, q);
     } else {
         cudaLaunchConfig_t c = {};
         cudaLaunchAttribute at[1];
@@ -1256,7 +1296,7 @@ static int launch_tc(const CUtensorMap &mXh, const CUtensorMap &mXl, const CUten
         c.stream = stream;
         c.attrs = at;
         c.numAttrs = 1;
-        CK(cudaLaunchKernelEx(&c, k_qform_tc<BN, TWO, true>, mXh, mXl, mWh, mWl, q));
+        CK(cudaLaunchKernelEx(&c, k_qform_tc<BN, TWO, true, WT>, mXh, mXl, mWh, mWl, q));
     }
     note_launch();
     CK(cudaGetLastError());
@@ -1270,6 +1310,12 @@ static bool tc_pair() {
     const char *e = std::getenv("CFDWM_TC_PAIR");
     if (e && (e[0] == '0' || e[0] == '1') && e[1] == 0) return e[0] == '1';
     return true;
+}
+
+static f32x2 f2_dup(float v) {
+    unsigned u;
+    std::memcpy(&u, &v, 4);
+    return (f32x2)u << 32 | u;
 }
 
 static int tc_reserve(TcForm &f, size_t bytes) {
@@ -1302,7 +1348,7 @@ int tcform_eval(TcForm &f, const DevSea &sea, long n, const double *x, const dou
     // overlap where the SMs have room (measured: 1277 against 1323 ms per step
     // of 4e6 points)
     const int nbuf = n > chunk ? 2 : 1;
-    const size_t bufb = ((2 * xb + yb + sizeof(QRow) * chunk + sizeof(QComp) * npad + 4095) / 4096) * 4096;
+    const size_t bufb = ((2 * xb + yb + sizeof(QRow) * chunk + sizeof(float) * QCOMP * npad + 4095) / 4096) * 4096;
     int rc = tc_reserve(f, nbuf * bufb);
     if (rc) return rc;
     cudaStream_t pst = stream;
@@ -1323,7 +1369,9 @@ int tcform_eval(TcForm &f, const DevSea &sea, long n, const double *x, const dou
     // two accumulators (hi, cross) for the fp16 split unless the form keeps
     // the cross products in the hi accumulator
     const bool two = f.fp16 && !f.one_acc;
-    const bool pair = tc_pair() && (two ? tc_max_units<256, true, true>() : tc_max_units<256, false, true>()) > 0;
+    const bool pair = tc_pair() && (two ? tc_max_units<256, true, true, false>()
+                                   : f.wt ? tc_max_units<256, false, true, true>()
+                                          : tc_max_units<256, false, true, false>()) > 0;
     const int CSZ = pair ? 2 : 1;
     int j = 0;
     for (long b = 0; b < n; b += chunk, j++) {
@@ -1335,7 +1383,7 @@ int tcform_eval(TcForm &f, const DevSea &sea, long n, const double *x, const dou
         void *Xh = base, *Xl = base + xb;
         float *Y = (float *)(base + 2 * xb);
         QRow *rowrec = (QRow *)(base + 2 * xb + yb);
-        QComp *comprec = (QComp *)(base + 2 * xb + yb + sizeof(QRow) * chunk);
+        float *comprec = (float *)(base + 2 * xb + yb + sizeof(QRow) * chunk);
         if (!tab) {
             k_qform_rows<<<(unsigned)((mm + 255) / 256), 256, 0, pst>>>(mm, x + b, y + b, t + b * st, st, sea.fx,
                                                                         sea.fy, sea.d_phase, sea.npad_g, rowrec);
@@ -1348,6 +1396,8 @@ int tcform_eval(TcForm &f, const DevSea &sea, long n, const double *x, const dou
         pp.rows = mm; pp.row = rowrec; pp.comp = comprec; pp.phase = sea.d_phase; pp.t = tab ? nullptr : t + b * st; pp.st = st;
         pp.cstride = sea.npad_g; pp.ncomp = sea.n; pp.npad = npad;
         pp.trivial_ramp = sea.trivial_ramp ? 1 : 0; pp.fp16 = f.fp16 ? 1 : 0;
+        pp.none = f2_dup(-1.f); pp.ninv = f2_dup(-0.15915494309189535f);
+        pp.P[0] = f2_dup(6.28125f); pp.P[1] = f2_dup(1.9353071693331003e-3f); pp.P[2] = f2_dup(1.0253376273028358e-11f);
         pp.lo_scale = two ? 2048.0f : 1.0f;
         pp.Xhi = Xh; pp.Xlo = Xl; pp.Y = Y; pp.ldy = mpad;
         if (tab) {
@@ -1398,11 +1448,13 @@ int tcform_eval(TcForm &f, const DevSea &sea, long n, const double *x, const dou
         long nunits = (nrb + CSZ - 1) / CSZ * (long)f.nblk * q.ncu;
         prof_begin(PK_QFORM, stream);
         if (!two)
-            rc = pair ? launch_tc<256, false, true>(mXh, mXl, mWh, mWl, q, nunits, stream)
-                      : launch_tc<256, false, false>(mXh, mXl, mWh, mWl, q, nunits, stream);
+            rc = pair ? (f.wt ? launch_tc<256, false, true, true> : launch_tc<256, false, true, false>)(
+                            mXh, mXl, mWh, mWl, q, nunits, stream)
+                      : (f.wt ? launch_tc<256, false, false, true> : launch_tc<256, false, false, false>)(
+                            mXh, mXl, mWh, mWl, q, nunits, stream);
         else
-            rc = pair ? launch_tc<256, true, true>(mXh, mXl, mWh, mWl, q, nunits, stream)
-                      : launch_tc<256, true, false>(mXh, mXl, mWh, mWl, q, nunits, stream);
+            rc = pair ? launch_tc<256, true, true, false>(mXh, mXl, mWh, mWl, q, nunits, stream)
+                      : launch_tc<256, true, false, false>(mXh, mXl, mWh, mWl, q, nunits, stream);
         prof_end(PK_QFORM, stream);
         if (rc) return rc;
         if (nbuf == 2) CK(cudaEventRecord(ev[3 + buf], stream));
