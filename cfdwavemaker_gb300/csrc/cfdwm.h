@@ -390,6 +390,9 @@ struct TcForm {
     // K blocks (of 64) per accumulation segment of a column tile, 0: the whole
     // upper-triangle K range in one accumulation
     int kseg = 0;
+    // consecutive blocks with the same X half that a column unit takes in turn
+    // (divides nblk)
+    int brun = 1;
     void *Whi = nullptr, *Wlo = nullptr;
     float *colscale = nullptr;
     int *bmap = nullptr;        // per block: X half, Y half, output column, kind (TC_*)

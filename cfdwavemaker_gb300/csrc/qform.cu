@@ -308,7 +308,7 @@ struct QPrep {
     long row0;
 };
 
-constexpr int PREP_ROWS = 8;      // rows per block of the operand preparation
+constexpr int PREP_ROWS = 8;       // rows per block of the operand preparation
 
 // The arithmetic of the two components is packed (ff_mul, ff_add of
 // ffmath.cuh with the error terms carried negated).
@@ -329,11 +329,15 @@ __device__ __forceinline__ f32x2 qp_ld(const float2 &v) { return *reinterpret_ca
 // PREP_ROWS rows.  Per (row, component): the float-float phase, its cos and
 // sin (Y), and r cos, r sin split into hi and lo 16-bit parts (X).  X rows are
 // written as 16-bit pairs; Y is staged in shared memory and written
-// column-major, each column's 16 rows (64 B) by 16 adjacent threads (rows
-// past the last are zero).
+// column-major, each column's 8 rows (32 B, a sector) by 8 adjacent threads
+// (rows past the last are zero).  Bound by latency at the occupancy that the
+// staging leaves: 21342 points, 336 components 46.1 us with scalar arithmetic
+// and 16 rows a block, 44.1 packed, 41.0 with 8 rows, 72 with 4; 1096 points,
+// 688 components 10.6, 10.8, 7.4, 7.4; slots without bank conflicts, whose
+// columns lie further apart, 45.7 (16 rows) and 41.9 (8).
 // GRID: the rows are the columns of a grid, and a phasor is the product of two
 // table entries (firstorder.cu) instead of a float-float phase and its sine:
-// 65536 columns, 1024 components 350 us then, 264 now.
+// 65536 columns, 1024 components 350 us then, 206 now.
 template <bool GRID>
 __global__ void __launch_bounds__(128) k_qform_prep(QPrep a) {
     __shared__ float s_y[512][PREP_ROWS + 1];     // [cos 256 | sin 256][row]
@@ -680,6 +684,7 @@ struct QTC {
     int ntn;                 // column tiles per block (npad / N)
     int group_m;             // row blocks per tile group
     int nblk;                // coefficient blocks of W
+    int brun;                // blocks that a column unit takes in turn (tile_of)
     int nout;                // outputs per row
     const int *bmap;         // per block: X half, Y half, output column, kind
     const float *wt;         // [3][npad] column weights of the weighted blocks
@@ -731,7 +736,12 @@ struct TileInfo {
     int bn;                  // columns
 };
 
-// grouped tile order: a group of group_m row units sweeps all column tiles.
+// grouped tile order: a group of group_m row units sweeps all column units, and
+// brun consecutive blocks with the same X half take a column unit in turn, so
+// that they share its rows of X and most of them its columns of Y (the
+// precision form's four fields; a 65536-row chunk of 4096 components read
+// 51.3 GB from DRAM block by block, 46.7 now; under the power cap 1e6 points
+// 291.5 ms then, 286.3 now; groups of 4, 16 and 32 row blocks 298, 289, 293).
 // A row unit is CS consecutive row blocks, one per CTA of a cluster (CTA rank
 // r takes block CS u + r; a block past the last row reads zeros through TMA
 // and stores nothing), so that the CTAs of a cluster share every W tile.
@@ -750,8 +760,9 @@ __device__ __forceinline__ bool tile_of(const QTC &a, long nru, long t, int cran
     int ct = (int)(in / gsz);
     if (ru >= nru || ct >= ncol) return false;
     ti.rb = ru * CS + crank;
-    ti.blk = ct / a.ncu;
-    const int cu = ct % a.ncu;
+    const int run = a.brun * a.ncu, inr = ct % run;
+    ti.blk = ct / run * a.brun + inr % a.brun;
+    const int cu = inr / a.brun;
     if (a.seg) {
         ti.tn = a.cu_tn[cu];
         ti.kb0 = a.cu_kb0[cu];
@@ -793,6 +804,9 @@ __device__ __forceinline__ bool tile_of(const QTC &a, long nru, long t, int cran
 constexpr int TC_THREADS = 320;            // producer, MMA and 8 epilogue warps
 constexpr int TC_EPI_WARPS = 8;
 
+// WT: blocks with column weights (the s-grid forms); in the kernel of the forms
+// without them the weighted epilogue cost registers (52 bytes spilled, none
+// without; 21342 points, 336 components 103 us a launch then, 89 now).
 template <int BN, bool TWO, bool PAIR, bool WT>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constant__ CUtensorMap mXh,
                                                      const __grid_constant__ CUtensorMap mXl,
@@ -1420,7 +1434,7 @@ int tcform_eval(TcForm &f, const DevSea &sea, long n, const double *x, const dou
             make_map(&mWl, f.Wlo, (long)f.nblk * npad, npad, BN / CSZ, f.fp16))
             return E_CUDA;
         QTC q;
-        q.rows = mm; q.npad = npad; q.ncomp = sea.n; q.ntn = npad / BN; q.group_m = tc_group_m(); q.nblk = f.nblk; q.nout = f.nout;
+        q.rows = mm; q.npad = npad; q.ncomp = sea.n; q.ntn = npad / BN; q.group_m = tc_group_m(); q.nblk = f.nblk; q.brun = f.brun; q.nout = f.nout;
         q.bmap = f.bmap; q.wt = f.wt; q.Y = Y; q.ldy = mpad; q.colscale = f.colscale;
         q.out = out + (long)f.nout * b; q.fp16 = f.fp16 ? 1 : 0; q.err = f.err;
         // column units: each column tile's upper-triangle K range, cut into
@@ -1538,6 +1552,7 @@ int qform_build(const Config &cfg, const DevSea &sea, bool fp16, void *stream_) 
     const char *e2 = std::getenv("CFDWM_QFORM_TWO_ACC");
     const bool one_acc = fp16 && !(e2 && e2[0] == '1');
     int rc = tcform_split(g_q.tc, coef, bmap, 8, 4, npad, fp16, stream, one_acc);
+    g_q.tc.brun = 4;
     if (one_acc) {
         const char *ek = std::getenv("CFDWM_QFORM_KSEG");
         g_q.tc.kseg = ek ? std::atoi(ek) : 8;
