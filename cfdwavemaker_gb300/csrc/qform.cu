@@ -462,8 +462,7 @@ struct QPlain {
     int ntile;
     const float *tab;        // plain tiles
     const float2 *ph;        // [npad][rows] (c, s)
-    const float *rr;         // ramps, row stride rs (0 where every component has the same ramp)
-    long rs;
+    const float *rr;         // [npad][rows] ramps, or [rows] where every component has the same
     int nseg;                // segments of the tile walk (units per row block)
     int mb[QPL_MAXSEG + 1];  // segment g walks the column tiles M in [mb[g], mb[g + 1])
     float *part;             // [nseg][rows][4]: each segment's sums
@@ -487,6 +486,10 @@ __device__ __forceinline__ void qpl_kahan(float &S, float &C, float y) {
     S = t;
 }
 
+// RAMPS: the components have ramps of their own; else a row's is loaded once
+// (65536 points, 4096 components 180 ms; 186 with a load per component, 215 with a
+// row stride that is zero for one ramp).
+template <bool RAMPS>
 __global__ void __launch_bounds__(128, 2) k_qform_plain(QPlain a) {
     extern __shared__ float4 q_smem[];
     const int tid = threadIdx.x;
@@ -502,6 +505,7 @@ __global__ void __launch_bounds__(128, 2) k_qform_plain(QPlain a) {
     const long ntiles = ((long)mhi * (mhi + 1) - (long)mlo * (mlo + 1)) / 2;
     const float4 *tab4 = reinterpret_cast<const float4 *>(a.tab);
     float S0[4] = {0, 0, 0, 0}, C0[4] = {0, 0, 0, 0}, S1[4] = {0, 0, 0, 0}, C1[4] = {0, 0, 0, 0};
+    const float r0 = RAMPS ? 0.f : a.rr[q0], r1 = RAMPS ? 0.f : a.rr[q1];
     float2 pm0[QT], pm1[QT];     // (c, s) of the 32 components of tile M, rows p and p + 128
 
     // stage k of the walk: tile (I, M) with M outer, M in [mlo, mhi)
@@ -535,15 +539,13 @@ __global__ void __launch_bounds__(128, 2) k_qform_plain(QPlain a) {
         // ones past the tile re-read its last component)
         const long rbase = (long)(I * QT) * a.rows;
         float2 pa0 = a.ph[rbase + q0], pa1 = a.ph[rbase + q1];
-        const long rr0 = (long)(I * QT) * a.rs;
-        float ra0 = a.rr[rr0 + q0], ra1 = a.rr[rr0 + q1];
+        float ra0 = RAMPS ? a.rr[rbase + q0] : r0, ra1 = RAMPS ? a.rr[rbase + q1] : r1;
         float2 pb0 = a.ph[rbase + a.rows + q0], pb1 = a.ph[rbase + a.rows + q1];
-        float rb0 = a.rr[rr0 + a.rs + q0], rb1 = a.rr[rr0 + a.rs + q1];
+        float rb0 = RAMPS ? a.rr[rbase + a.rows + q0] : r0, rb1 = RAMPS ? a.rr[rbase + a.rows + q1] : r1;
         for (int ii = 0; ii < QT; ii++) {
             const long rn = rbase + (long)(ii + 2 < QT ? ii + 2 : QT - 1) * a.rows;
             const float2 n0 = a.ph[rn + q0], n1 = a.ph[rn + q1];
-            const long rrn = rr0 + (long)(ii + 2 < QT ? ii + 2 : QT - 1) * a.rs;
-            const float nr0 = a.rr[rrn + q0], nr1 = a.rr[rrn + q1];
+            const float nr0 = RAMPS ? a.rr[rn + q0] : r0, nr1 = RAMPS ? a.rr[rn + q1] : r1;
             // (A_cos, A_sin) of each field times (c_m, s_m): the record's
             // float pairs and the phasor are the two lanes of each FFMA2
             float2 e0 = {0, 0}, u0 = {0, 0}, v0 = {0, 0}, w0 = {0, 0};
@@ -806,7 +808,7 @@ constexpr int TC_EPI_WARPS = 8;
 
 // WT: blocks with column weights (the s-grid forms); in the kernel of the forms
 // without them the weighted epilogue cost registers (52 bytes spilled, none
-// without; 21342 points, 336 components 103 us a launch then, 89 now).
+// without; 21342 points, 336 components 101 us a launch then, 89 now).
 template <int BN, bool TWO, bool PAIR, bool WT>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constant__ CUtensorMap mXh,
                                                      const __grid_constant__ CUtensorMap mXl,
@@ -1595,7 +1597,8 @@ int qform_eval(const DevSea &sea, long n, const double *x, const double *y, cons
     const long chunk = 1L << 16;
     // one-time, thread-safe (static initialisation)
     static const cudaError_t pattr =
-        cudaFuncSetAttribute(k_qform_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, QPLAIN_SMEM);
+        cudaFuncSetAttribute(k_qform_plain<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, QPLAIN_SMEM);
+        cudaFuncSetAttribute(k_qform_plain<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, QPLAIN_SMEM);
     CK(pattr);
     // two blocks of the kernel fit an SM (registers, shared memory)
     static const int slots = [] {
@@ -1635,7 +1638,7 @@ int qform_eval(const DevSea &sea, long n, const double *x, const double *y, cons
             if (fill > best + 1e-9) { best = fill; nseg = g; }
         }
         QPlain q;
-        q.rows = mm; q.ntile = nt; q.tab = g_q.plain_tab; q.ph = ph; q.rr = rr; q.rs = sea.trivial_ramp ? 0 : mm; q.part = part;
+        q.rows = mm; q.ntile = nt; q.tab = g_q.plain_tab; q.ph = ph; q.rr = rr; q.part = part;
         q.nseg = nseg;
         const long total = (long)nt * (nt + 1) / 2;
         q.mb[0] = 0;
@@ -1648,7 +1651,8 @@ int qform_eval(const DevSea &sea, long n, const double *x, const double *y, cons
         }
         q.mb[nseg] = nt;
         prof_begin(PK_QFORM, stream);
-        k_qform_plain<<<(unsigned)(nrb * nseg), 128, QPLAIN_SMEM, stream>>>(q);
+        if (sea.trivial_ramp) k_qform_plain<false><<<(unsigned)(nrb * nseg), 128, QPLAIN_SMEM, stream>>>(q);
+        else k_qform_plain<true><<<(unsigned)(nrb * nseg), 128, QPLAIN_SMEM, stream>>>(q);
         note_launch();
         k_qform_plain_sum<<<(unsigned)((mm * 4 + 255) / 256), 256, 0, stream>>>(mm, nseg, part, out + 4 * b);
         note_launch();
