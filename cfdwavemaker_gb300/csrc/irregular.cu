@@ -1552,7 +1552,7 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
     float2 *s_ph = s_few;                                   // phasors [npad]
     float2 *s_px = s_ph + a.npad;                           // kin: profiles px, pz [npad]
     float *s_r = reinterpret_cast<float *>(s_px + (a.kin ? a.npad : 0));   // ramps [npad] (individual ramps)
-    __shared__ float s_red[FEW_T / 32][FEW_Q];
+    __shared__ float s_red[FEW_T / 32][FEW_Q], s_err[FEW_T / 32][FEW_Q];
     __shared__ float s_sum[FEW_Q];
     __shared__ float s_ramp;
     __shared__ int s_last;
@@ -1703,17 +1703,33 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
             kahan(S[0], C[0], ramp(i) * fmaf(pi.x, s2.x, pi.y * s2.y));
         }
     }
-    // the block's sums
+    // the block's sums; the elevation's with their rounding errors, since at one
+    // or a few terms a thread the tree is most of the summation
 #pragma unroll
     for (int q = 0; q < FEW_Q; q++) {
-        float v = S[q] - C[q];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if ((tid & 31) == 0) s_red[tid >> 5][q] = v;
+        float v = S[q] - C[q], e = 0.f;
+        for (int o = 16; o > 0; o >>= 1) {
+            const float w = __shfl_down_sync(0xffffffffu, v, o);
+            if (q == 0 || q == 5) {
+                e += __shfl_down_sync(0xffffffffu, e, o);
+                const float t = v + w, bb = t - v;
+                e += (v - (t - bb)) + (w - bb);
+                v = t;
+            } else {
+                v += w;
+            }
+        }
+        if ((tid & 31) == 0) {
+            s_red[tid >> 5][q] = v;
+            s_err[tid >> 5][q] = e;
+        }
     }
     __syncthreads();
     if (tid < FEW_Q) {
-        float v = 0.f;
-        for (int w = 0; w < FEW_T / 32; w++) v += s_red[w][tid];
+        float v = 0.f, c = 0.f;
+        for (int w = 0; w < FEW_T / 32; w++) kahan(v, c, s_red[w][tid]);
+        for (int w = 0; w < FEW_T / 32; w++) c -= s_err[w][tid];
+        v -= c;
         s_sum[tid] = v;
         if (ns > 1) __stcg(&a.part[((long)slice * FEW_Q + tid) * a.n + p], v);
     }
