@@ -1027,7 +1027,8 @@ def roofline(args, r, pk, src):
     f_mhz = r["clocks"].get("sm_mhz") or pk.get("sm_max_mhz", 2070.0)
     if args.workload == "sgrid" and r.get("depth_rank") and "qform" in prof:
         # depth-separable form: eta2 and 3R quadratic forms per column, each
-        # 2 flop per nonzero coefficient of two N x N upper triangles
+        # 2 flop per nonzero coefficient of two N x N upper triangles (or, with one
+        # ramp for all components, of one full N x N block)
         kp = prof["qform"]
         N = r["ncomp"]
         nout = 1 + 3 * r["depth_rank"]
