@@ -1238,14 +1238,19 @@ int tcform_split(TcForm &f, const double *coef64, const int *bmap_host, int nblk
 // CTAs (or CTA pairs) of this form that fit on the device at once; set and
 // queried once per process (thread-safe static initialisation); <= 0: none.
 // Row blocks per tile group of the tile walk (the group sweeps every column
-// tile while its rows of X and Y stay in L2); CFDWM_TC_GROUP overrides it.
-static int tc_group_m() {
+// tile while its rows of X and Y stay in L2).  8; where the blocks are walked one
+// by one (the s-grid's potential form), about 50 MB of X and Y, 2 KB a component
+// and row block: with 1024 components, a ring update of 65536 columns, groups of
+// 8 10.65 ms, 16 10.36, 24 10.14, 32 10.26.  With the precision form's four fields
+// in turn larger groups gain nothing (4096 components, 8 to 32 alike) or lose (100
+// to 1000 components by 50 MB 1-4 % slower).  CFDWM_TC_GROUP overrides it.
+static int tc_group_m(const TcForm &f) {
     static const int g = [] {
         const char *e = std::getenv("CFDWM_TC_GROUP");
-        int v = e ? std::atoi(e) : 8;
-        return v >= 2 && v <= 512 ? v : 8;
+        int v = e ? std::atoi(e) : 0;
+        return v >= 2 && v <= 512 ? v : 0;
     }();
-    return g;
+    return g ? g : f.wt ? std::max(8, 24576 / f.npad & ~1) : 8;
 }
 
 template <int BN, bool TWO, bool PAIR, bool WT>
@@ -1436,7 +1441,7 @@ int tcform_eval(TcForm &f, const DevSea &sea, long n, const double *x, const dou
             make_map(&mWl, f.Wlo, (long)f.nblk * npad, npad, BN / CSZ, f.fp16))
             return E_CUDA;
         QTC q;
-        q.rows = mm; q.npad = npad; q.ncomp = sea.n; q.ntn = npad / BN; q.group_m = tc_group_m(); q.nblk = f.nblk; q.brun = f.brun; q.nout = f.nout;
+        q.rows = mm; q.npad = npad; q.ncomp = sea.n; q.ntn = npad / BN; q.group_m = tc_group_m(f); q.nblk = f.nblk; q.brun = f.brun; q.nout = f.nout;
         q.bmap = f.bmap; q.wt = f.wt; q.Y = Y; q.ldy = mpad; q.colscale = f.colscale;
         q.out = out + (long)f.nout * b; q.fp16 = f.fp16 ? 1 : 0; q.err = f.err;
         // column units: each column tile's upper-triangle K range, cut into
