@@ -148,6 +148,7 @@ struct DevSea {
     // FP64 phase data, length npad_g: kx, ky, omega, phase0, ramptime, starttime, duration
     double *d_phase = nullptr;   // [7][npad_g]
     float *d_cf = nullptr;       // [NCF][npad_g]
+    float2 *d_cfp = nullptr;     // [NCF][npad_g] the same as float pairs (the short batches' first order)
     float *d_tab_eta = nullptr;  // grid-mask pair tiles of eta2 (A, B per pair)
     float *d_tab_grid = nullptr; // grid-mask pair tiles of uvw2
     float *d_tab_point = nullptr;// point-API pair tiles (built on demand): velocity records, then

@@ -108,6 +108,54 @@ __device__ __forceinline__ void ff_sincos_poly(float x, float &s, float &c) {
     c = qi == 0 ? cr : qi == 1 ? -sr : qi == 2 ? -cr : sr;
 }
 
+// a + b as a float pair, exactly
+__device__ __forceinline__ float2 ff_two_sum(float a, float b) {
+    const float s = a + b, bb = s - a;
+    return make_float2(s, (a - (s - bb)) + (b - bb));
+}
+__device__ __forceinline__ float2 ff_mul(float2 a, float2 b) { return ff_mul(a.x, a.y, b.x, b.y); }
+
+// sin and cos of the phase ph as float pairs, within 1.4e-8: the Cody-Waite
+// reduction and the Taylor series of ff_sincos_poly with the low parts kept (the
+// first two steps of the reduction are exact for |n| < 2^18).
+__device__ __forceinline__ void ff_sincos(float2 ph, float2 &s, float2 &c) {
+    const float n = rintf(ph.x * 0.636619772f), C = 7.549789948768648e-8f;
+    const float a = fmaf(-n, 4.837512969970703125e-4f, fmaf(-n, 1.5703125f, ph.x));
+    const float p = n * C;
+    float2 r = ff_two_sum(a, -p);
+    r = ff_two_sum(r.x, (r.y - fmaf(n, C, -p)) + ph.y);
+    const float h = r.x * r.x, he = fmaf(2.f * r.x, r.y, fmaf(r.x, r.x, -h));
+    const float ps = fmaf(h, fmaf(h, fmaf(h, 2.7557319e-6f, -1.98412698e-4f), 8.33333333e-3f), -0.166666667f);
+    const float pc = fmaf(h, fmaf(h, fmaf(h, -2.75573192e-7f, 2.48015873e-5f), -1.38888889e-3f), 4.16666667e-2f);
+    float2 sr = ff_two_sum(r.x, r.x * h * ps), cr = ff_two_sum(1.f, -0.5f * h);
+    sr = ff_two_sum(sr.x, fmaf(r.y, fmaf(-0.5f, h, 1.f), sr.y));
+    cr = ff_two_sum(cr.x, cr.y + fmaf(h * h, pc, -0.5f * he));
+    const int q = (int)n & 3;
+    const float2 u = (q & 1) ? cr : sr, v = (q & 1) ? sr : cr;
+    const float us = (q & 2) ? -1.f : 1.f, vs = ((q + 1) & 2) ? -1.f : 1.f;
+    s = make_float2(us * u.x, us * u.y);
+    c = make_float2(vs * v.x, vs * v.y);
+}
+
+// e^x = T (1 + p) of a pair x, T a power of two and p a pair within 1e-8,
+// |p| < 0.42: Cody-Waite reduction by ln 2, Taylor series to r^8.
+__device__ __forceinline__ float ff_exp(float2 x, float2 &p) {
+    // (comparisons, not fmin and fmax: a NaN stays one)
+    const float xh = x.x < -120.f ? -120.f : x.x > 89.f ? 89.f : x.x;
+    const float n = rintf(xh * 1.44269504f), L = -2.12194440e-4f;
+    const float a = fmaf(-n, 0.693359375f, xh), b = n * L;
+    float2 r = ff_two_sum(a, -b);
+    r = ff_two_sum(r.x, (r.y - fmaf(n, L, -b)) + x.y);
+    float t = fmaf(r.x, 2.48015873e-5f, 1.98412698e-4f);
+    t = fmaf(r.x, fmaf(r.x, fmaf(r.x, t, 1.38888889e-3f), 8.33333333e-3f), 4.16666667e-2f);
+    t = fmaf(r.x, fmaf(r.x, t, 0.166666667f), 0.5f);
+    const float h = r.x * r.x;
+    p = ff_two_sum(r.x, h * t);
+    p.y += fmaf(r.x, r.y, r.y);
+    const int k = (int)n, k2 = k / 2;
+    return __int_as_float((k2 + 127) << 23) * __int_as_float((k - k2 + 127) << 23);
+}
+
 // Irregular::freq_ramp (Irregular.cpp:200-204), FP64
 __device__ __forceinline__ double ff_freq_ramp(double t, double rt, double ts, double du) {
     const double small = 1.e-12;   // Irregular.h:8

@@ -285,7 +285,7 @@ __global__ void k_count_pairs(CompIn c, unsigned long long *cnt) {
 
 __global__ void k_component_coefs(CompIn c, int npad, double fx, double fy, double tofmax,
                                   const double *phase, const double *rt, const double *st,
-                                  const double *du, double *ph_out, float *cf) {
+                                  const double *du, double *ph_out, float *cf, float2 *cfp) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npad) return;
     double v[NCF];
@@ -318,7 +318,12 @@ __global__ void k_component_coefs(CompIn c, int npad, double fx, double fy, doub
     ph_out[4 * npad + i] = r0;
     ph_out[5 * npad + i] = r1;
     ph_out[6 * npad + i] = r2;
-    for (int q = 0; q < NCF; q++) cf[q * npad + i] = (float)v[q];
+    for (int q = 0; q < NCF; q++) {
+        float2 f;
+        ff_split(v[q], f.x, f.y);
+        cf[q * npad + i] = f.x;
+        cfp[q * npad + i] = f;
+    }
 }
 
 // floats of a phasor record: kx, ky, -omega, phase0 as float pairs, then A, GX,
@@ -390,13 +395,14 @@ int sea_build(const Config &cfg, DevSea &sea, bool point_table, void *stream_) {
 
     CK(cudaMalloc(&sea.d_phase, sizeof(double) * 7 * sea.npad_g));
     CK(cudaMalloc(&sea.d_cf, sizeof(float) * NCF * sea.npad_g));
+    CK(cudaMalloc(&sea.d_cfp, sizeof(float2) * NCF * sea.npad_g));
     // records for up to the next multiple of 256 components (the plain
     // precision form pads to 256), zero past the last component
     const int nrec_cap = ((sea.npad_g + 255) / 256) * 256;
     CK(cudaMalloc(&sea.d_phrec, sizeof(float) * PH_REC * nrec_cap));
     k_component_coefs<<<(sea.npad_g + 127) / 128, 128, 0, stream>>>(
         ci, sea.npad_g, cfg.x_pos, cfg.y_pos, cfg.tofmax, d_in + 4 * nn, d_in + 5 * nn,
-        d_in + 6 * nn, d_in + 7 * nn, sea.d_phase, sea.d_cf);
+        d_in + 6 * nn, d_in + 7 * nn, sea.d_phase, sea.d_cf, sea.d_cfp);
     note_launch();
     CK(cudaGetLastError());
     k_phasor_records<<<(nrec_cap + 127) / 128, 128, 0, stream>>>(n, nrec_cap, sea.d_phase, sea.d_cf,
@@ -476,6 +482,8 @@ int sea_build(const Config &cfg, DevSea &sea, bool point_table, void *stream_) {
 void sea_free(DevSea &sea) {
     if (sea.d_phase) cudaFree(sea.d_phase);
     if (sea.d_cf) cudaFree(sea.d_cf);
+    if (sea.d_cfp) cudaFree(sea.d_cfp);
+    sea.d_cfp = nullptr;
     if (sea.d_tab_eta) cudaFree(sea.d_tab_eta);
     if (sea.d_tab_grid) cudaFree(sea.d_tab_grid);
     if (sea.d_tab_point) cudaFree(sea.d_tab_point);
@@ -1518,6 +1526,15 @@ __global__ void k_combine(long n, long ldo, int order, double swl, const double 
 // was five dependent kernels, 26 us; 17 us now (a launch and a synchronisation are
 // 8 of these).
 // ---------------------------------------------------------------------------
+// Accuracy.  A single value is held to its own size, not to that of the largest
+// of a batch, and the first order is nearly all of it.  Its terms are formed in
+// float pairs (phase, sine, profiles, coefficients; 1e-8), as is every sum over
+// the threads and slices: 40 x 3 components, u 1.2e-7 RMS of the field with FP32
+// terms.  Heights above the bed, z + h, are taken in FP64: of an FP32 z = -50
+// little is left of them, and w = sinh(k(z + h)) lives on that difference.  For
+// the same reason the pairs' profiles are e1 (1 +- e2), e2 = e^{-2k(z+h)}, not E +-
+// Y with Y = e^{-k(z+2h)}, whose exponents, of up to 40, round apart: w within
+// 3 m of the bed, 128 components at 50 m, 3.1e-7 RMS of its maximum with E - Y.
 constexpr int FEW_T = 128;           // threads of a block
 constexpr int FEW_Q = 10;            // sums: eta2, u, v, w, dp, then eta1, gx, gy, gz, gp
 constexpr int FEW_E = 8;             // terms of an item
@@ -1527,16 +1544,31 @@ struct FewArgs {
     double fx, fy, swl, depth;
     int ncomp, npad, cstride, trivial_ramp, order, clamp, kin, mask;
     const float *rec, *cf;
+    const float2 *cfp;
     const double *phase;
     int ntp, ntg;                    // point and grid table tiles per side
     const float *tabv, *tpp, *tpk, *tabe;
     long nv, np, ne;                 // items of the velocity, pressure and elevation sums
-    float *part;                     // [slices][FEW_Q][n]
+    float2 *part;                    // [slices][FEW_Q][n] sums and their rounding errors
     unsigned *cnt;                   // [n], zero before and after
     double *out;
     ApiRows api;
     KinTab kt;
 };
+
+// whether a call of this mask needs sum q
+__device__ __forceinline__ bool few_needs(int mask, int q) { return mask >> (q < 5 ? q : q - 5) & 1; }
+
+// s + e += v, the rounding errors of s in e
+__device__ __forceinline__ void few_add(float2 &s, float v) {
+    const float2 t = ff_two_sum(s.x, v);
+    s.x = t.x;
+    s.y += t.y;
+}
+__device__ __forceinline__ void few_add(float2 &s, float2 v) {
+    few_add(s, v.x);
+    s.y += v.y;
+}
 
 // (I, M) of tile t of an upper triangle of nt x nt tiles
 __device__ __forceinline__ void tile_at(long t, int nt, int &I, int &M) {
@@ -1547,13 +1579,57 @@ __device__ __forceinline__ void tile_at(long t, int nt, int &I, int &M) {
     M = I + (int)(t - tile_index(I, I, nt));
 }
 
+// The first-order terms of component i (Irregular.cpp:178-198, 394-447, 1107-1192)
+// at offsets dx, dy and time t, heights z and zeta = -2 (z + h), ramp r.
+__device__ __forceinline__ void few_first(const FewArgs &a, int i, float2 dx, float2 dy, float2 t, float2 z, float2 zeta,
+                                          float r, float2 S[FEW_Q]) {
+    const float *R = a.rec;
+    auto rec = [&](int q) { return R[rec_at(i, q)]; };
+    auto cf = [&](int q) { return a.cfp[q * a.cstride + i]; };
+    float2 ph = ff_add(ff_mul(rec(0), rec(1), dx.x, dx.y), ff_mul(rec(2), rec(3), dy.x, dy.y));
+    ph = ff_add(ph, ff_mul(rec(4), rec(5), t.x, t.y));
+    ph = ff_add(ph, make_float2(rec(6), rec(7)));
+    float2 s, c;
+    ff_sincos(ph, s, c);
+    c = ff_mul(r, 0.f, c.x, c.y);
+    s = ff_mul(r, 0.f, s.x, s.y);
+    if (a.mask & 1) few_add(S[5], ff_mul(cf(CF_A), c));
+    if (!(a.mask & 30)) return;
+    // q E (1 +- e2), E = e^{kz}, e2 = e^{k zeta}
+    const float2 k = cf(CF_K);
+    float2 p, p2;
+    const float T = ff_exp(ff_mul(k, z), p), T2 = ff_exp(ff_mul(k, zeta), p2);
+    float2 E = ff_two_sum(1.f, p.x), up = ff_two_sum(1.f + T2, T2 * p2.x), um = ff_two_sum(1.f - T2, -T2 * p2.x);
+    E.y += p.y;
+    up.y += T2 * p2.y;
+    um.y -= T2 * p2.y;
+    E = ff_mul(cf(CF_Q), make_float2(T * E.x, T * E.y));
+    const float2 F = ff_mul(E, up), G = ff_mul(E, um);
+    if (a.mask & 6) {
+        const float2 u = ff_mul(ff_mul(cf(CF_AU), F), c);
+        few_add(S[1], ff_mul(u, cf(CF_CT)));
+        few_add(S[2], ff_mul(u, cf(CF_ST)));
+        few_add(S[6], ff_mul(cf(CF_GX), c));
+        few_add(S[7], ff_mul(cf(CF_GY), c));
+    }
+    if (a.mask & 8) {
+        few_add(S[3], ff_mul(ff_mul(cf(CF_AU), G), s));
+        few_add(S[8], ff_mul(cf(CF_GZ), s));
+    }
+    if (a.mask & 16) {
+        few_add(S[4], ff_mul(ff_mul(cf(CF_AP), F), c));
+        if (a.kin) few_add(S[4], r * fmaf(cf(CF_X1).x, F.x, cf(CF_Z1).x * G.x));
+        few_add(S[9], ff_mul(cf(CF_GP), c));
+    }
+}
+
 __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
     extern __shared__ float2 s_few[];
     float2 *s_ph = s_few;                                   // phasors [npad]
     float2 *s_px = s_ph + a.npad;                           // kin: profiles px, pz [npad]
     float *s_r = reinterpret_cast<float *>(s_px + (a.kin ? a.npad : 0));   // ramps [npad] (individual ramps)
-    __shared__ float s_red[FEW_T / 32][FEW_Q], s_err[FEW_T / 32][FEW_Q];
-    __shared__ float s_sum[FEW_Q];
+    __shared__ float2 s_red[FEW_T / 32][FEW_Q];
+    __shared__ double s_sum[FEW_Q];
     __shared__ float s_ramp;
     __shared__ int s_last;
     const int tid = threadIdx.x;
@@ -1562,26 +1638,23 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
     const double xp = a.x[p], yp = a.y[p], zp = a.z[p], tp = a.t[p];
     const double *P = a.phase;
     const int cs = a.cstride;
-    const double zz = (a.clamp ? fmax(-a.depth, zp) : zp) - a.swl;
-    const float z = (float)(a.order == 0 ? zz : fmin(0.0, zz)), h = (float)a.depth;
-    const float zk = z * LOG2E_F, yk = -(z + 2.f * h) * LOG2E_F;
-    // cosh(k(z+h))/cosh(kh), sinh(k(z+h))/cosh(kh) of component i
-    auto profile = [&](int i) {
-        const float k = a.cf[CF_K * cs + i], q = a.cf[CF_Q * cs + i];
-        const float E = ex2(k * zk), Y = ex2(k * yk);
-        return make_float2(q * (E + Y), q * (E - Y));
-    };
+    const double zz = (a.clamp ? fmax(-a.depth, zp) : zp) - a.swl, z0 = a.order == 0 ? zz : fmin(0.0, zz);
+    const double zeta0 = -2.0 * (z0 + a.depth);
+    const float zk = (float)z0 * LOG2E_F, zetak = (float)zeta0 * LOG2E_F;
     if (a.trivial_ramp) {
         if (tid == FEW_T - 1) s_ramp = (float)d_freq_ramp(tp, P[4 * cs], P[5 * cs], P[6 * cs]);
     } else {
         for (int i = tid; i < a.npad; i += FEW_T)
             s_r[i] = i < a.ncomp ? (float)d_freq_ramp(tp, P[4 * cs + i], P[5 * cs + i], P[6 * cs + i]) : 0.f;
     }
+    float2 dx, dy, tt = ff_from_double(tp);
     {
         float2 ox, oy;
         ff_split(-a.fx, ox.x, ox.y);
         ff_split(-a.fy, oy.x, oy.y);
-        const PhPoint pt(ff_add(ff_from_double(xp), ox), ff_add(ff_from_double(yp), oy), ff_from_double(tp));
+        dx = ff_add(ff_from_double(xp), ox);
+        dy = ff_add(ff_from_double(yp), oy);
+        const PhPoint pt(dx, dy, tt);
         for (int i = 2 * tid; i < a.npad; i += 2 * FEW_T) {
             f32x2 hi, lo, s2, c2;
             ph_phase(reinterpret_cast<const ulonglong2 *>(a.rec + (long)i * PH_REC), pt, hi, lo);
@@ -1592,35 +1665,27 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
         }
     }
     if (a.kin)
-        for (int i = tid; i < a.npad; i += FEW_T) s_px[i] = profile(i);
+        for (int i = tid; i < a.npad; i += FEW_T) {
+            // cosh(k(z+h))/cosh(kh), sinh(k(z+h))/cosh(kh)
+            const float q = a.cf[CF_Q * cs + i];
+            float F, G;
+            depth_fg(a.cf[CF_K * cs + i], zk, zetak, F, G);
+            s_px[i] = make_float2(q * F, q * G);
+        }
     __syncthreads();
     auto ramp = [&](int i) { return a.trivial_ramp ? s_ramp : s_r[i]; };
-    float S[FEW_Q], C[FEW_Q];
+    float2 S[FEW_Q];
 #pragma unroll
-    for (int q = 0; q < FEW_Q; q++) S[q] = C[q] = 0.f;
-    // first order (Irregular.cpp:178-198, 394-447, 1107-1192)
-    for (int i = slice * FEW_T + tid; i < a.ncomp; i += ns * FEW_T) {
-        const float2 ph = s_ph[i];
-        const float r = ramp(i), rc = r * ph.x, rs = r * ph.y;
-        kahan(S[5], C[5], rc * a.cf[CF_A * cs + i]);
-        if (a.mask & 30) {
-            const float2 px = profile(i);
-            kahan(S[6], C[6], rc * a.cf[CF_GX * cs + i]);
-            kahan(S[7], C[7], rc * a.cf[CF_GY * cs + i]);
-            kahan(S[8], C[8], rs * a.cf[CF_GZ * cs + i]);
-            kahan(S[9], C[9], rc * a.cf[CF_GP * cs + i]);
-            const float au = a.cf[CF_AU * cs + i] * r;
-            kahan(S[1], C[1], au * px.x * a.cf[CF_CT * cs + i] * ph.x);
-            kahan(S[2], C[2], au * px.x * a.cf[CF_ST * cs + i] * ph.x);
-            kahan(S[3], C[3], au * px.y * ph.y);
-            float pp = a.cf[CF_AP * cs + i] * px.x * ph.x;
-            if (a.kin) pp += a.cf[CF_X1 * cs + i] * px.x + a.cf[CF_Z1 * cs + i] * px.y;
-            kahan(S[4], C[4], r * pp);
-        }
+    for (int q = 0; q < FEW_Q; q++) S[q] = make_float2(0.f, 0.f);
+    if (slice * FEW_T + tid < a.ncomp) {
+        float2 z, zeta;
+        ff_split(z0, z.x, z.y);
+        ff_split(zeta0, zeta.x, zeta.y);
+        for (int i = slice * FEW_T + tid; i < a.ncomp; i += ns * FEW_T) few_first(a, i, dx, dy, tt, z, zeta, ramp(i), S);
     }
     // pair items, eight terms each; the records of two neighbouring terms are
     // interleaved (velocity, pressure) or adjacent (elevation)
-    const f32x2 zk2 = p_pack(zk, zk), yk2 = p_pack(yk, yk), neg1 = p_pack(-1.f, -1.f);
+    const f32x2 zk2 = p_pack(zk, zk), zetak2 = p_pack(zetak, zetak), neg1 = p_pack(-1.f, -1.f);
     const long total = a.nv + a.np + a.ne;
     for (long item = (long)slice * FEW_T + tid; item < total; item += (long)ns * FEW_T) {
         int I, M, i, m0;
@@ -1649,14 +1714,15 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
                 const f32x2 cc = p_mul(px2, mc);
                 const f32x2 cp = p_fma(ny2, ms, cc), cm = p_fma(py2, ms, cc);
                 const ulonglong2 rk = vel ? RV[4 * k + 3] : RP[2 * k + 1];
-                const f32x2 Ep = p_ex2(p_mul(rk.x, zk2)), Yp = p_ex2(p_mul(rk.x, yk2));
-                const f32x2 Em = p_ex2(p_mul(rk.y, zk2)), Ym = p_ex2(p_mul(rk.y, yk2));
-                const f32x2 A = p_mul(cp, p_add(Ep, Yp)), B = p_mul(cm, p_add(Em, Ym));
+                const f32x2 Ep = p_ex2(p_mul(rk.x, zk2)), ep = p_ex2(p_mul(rk.x, zetak2));
+                const f32x2 Em = p_ex2(p_mul(rk.y, zk2)), em = p_ex2(p_mul(rk.y, zetak2));
+                const f32x2 A = p_mul(cp, p_fma(Ep, ep, Ep)), B = p_mul(cm, p_fma(Em, em, Em));
                 if (vel) {
                     const ulonglong2 r0 = RV[4 * k], r1 = RV[4 * k + 1], r2 = RV[4 * k + 2];
                     const f32x2 sc = p_mul(py2, mc);
                     const f32x2 sp = p_fma(px2, ms, sc), sm = p_fma(nx2, ms, sc);
-                    const f32x2 Cc = p_mul(sp, p_fma(Yp, neg1, Ep)), D = p_mul(sm, p_fma(Ym, neg1, Em));
+                    const f32x2 Cc = p_mul(sp, p_fma(Ep, p_mul(ep, neg1), Ep));
+                    const f32x2 D = p_mul(sm, p_fma(Em, p_mul(em, neg1), Em));
                     au = p_fma(r0.x, A, p_fma(r0.y, B, au));
                     av = p_fma(r1.x, A, p_fma(r1.y, B, av));
                     aw = p_fma(r2.x, Cc, p_fma(r2.y, D, aw));
@@ -1673,13 +1739,13 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
             }
             const float ri = ramp(i);
             if (vel) {
-                kahan(S[1], C[1], ri * p_hsum(au));
-                kahan(S[2], C[2], ri * p_hsum(av));
-                kahan(S[3], C[3], ri * p_hsum(aw));
+                few_add(S[1], ri * p_hsum(au));
+                few_add(S[2], ri * p_hsum(av));
+                few_add(S[3], ri * p_hsum(aw));
             } else {
                 float row = p_hsum(ap);
                 if (a.kin) row = fmaf(s_px[i].x, p_hsum(ax), fmaf(s_px[i].y, p_hsum(az), row));
-                kahan(S[4], C[4], ri * row);
+                few_add(S[4], ri * row);
             }
         } else {
             const long it = item - a.nv - a.np;
@@ -1700,38 +1766,25 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
                 acc = p_fma(c.y, p_pack(q1.x, q1.y), p_fma(c.x, p_pack(q0.x, q0.y), acc));
             }
             const float2 s2 = p_un(acc), pi = s_ph[i];
-            kahan(S[0], C[0], ramp(i) * fmaf(pi.x, s2.x, pi.y * s2.y));
+            few_add(S[0], ramp(i) * fmaf(pi.x, s2.x, pi.y * s2.y));
         }
     }
-    // the block's sums; the elevation's with their rounding errors, since at one
-    // or a few terms a thread the tree is most of the summation
+    // the block's sums with their rounding errors: at one or a few terms a thread
+    // the tree is most of the summation
 #pragma unroll
     for (int q = 0; q < FEW_Q; q++) {
-        float v = S[q] - C[q], e = 0.f;
-        for (int o = 16; o > 0; o >>= 1) {
-            const float w = __shfl_down_sync(0xffffffffu, v, o);
-            if (q == 0 || q == 5) {
-                e += __shfl_down_sync(0xffffffffu, e, o);
-                const float t = v + w, bb = t - v;
-                e += (v - (t - bb)) + (w - bb);
-                v = t;
-            } else {
-                v += w;
-            }
-        }
-        if ((tid & 31) == 0) {
-            s_red[tid >> 5][q] = v;
-            s_err[tid >> 5][q] = e;
-        }
+        if (!few_needs(a.mask, q)) continue;
+        float2 v = S[q];
+        for (int o = 16; o > 0; o >>= 1)
+            few_add(v, make_float2(__shfl_down_sync(0xffffffffu, v.x, o), __shfl_down_sync(0xffffffffu, v.y, o)));
+        if ((tid & 31) == 0) s_red[tid >> 5][q] = v;
     }
     __syncthreads();
-    if (tid < FEW_Q) {
-        float v = 0.f, c = 0.f;
-        for (int w = 0; w < FEW_T / 32; w++) kahan(v, c, s_red[w][tid]);
-        for (int w = 0; w < FEW_T / 32; w++) c -= s_err[w][tid];
-        v -= c;
-        s_sum[tid] = v;
+    if (tid < FEW_Q && few_needs(a.mask, tid)) {
+        float2 v = s_red[0][tid];
+        for (int w = 1; w < FEW_T / 32; w++) few_add(v, s_red[w][tid]);
         if (ns > 1) __stcg(&a.part[((long)slice * FEW_Q + tid) * a.n + p], v);
+        else s_sum[tid] = (double)v.x + (double)v.y;
     }
     if (ns > 1) {
         __threadfence();
@@ -1742,9 +1795,12 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
         __threadfence();
         // a warp a sum in turn, its lanes over the slices
         for (int q = tid >> 5; q < FEW_Q; q += FEW_T / 32) {
-            float v = 0.f, c = 0.f;
-            for (int k = tid & 31; k < ns; k += 32) kahan(v, c, __ldcg(&a.part[((long)k * FEW_Q + q) * a.n + p]));
-            v -= c;
+            if (!few_needs(a.mask, q)) continue;
+            double v = 0.0;
+            for (int k = tid & 31; k < ns; k += 32) {
+                const float2 f = __ldcg(&a.part[((long)k * FEW_Q + q) * a.n + p]);
+                v += (double)f.x + (double)f.y;
+            }
             for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
             if ((tid & 31) == 0) s_sum[q] = v;
         }
@@ -1754,9 +1810,9 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
     // Irregular::eta/u/v/w/dp from the pieces (Irregular.cpp:9-157)
     const double za = a.order == 2 ? fmax(0.0, zp - a.swl) : 0.0;
     double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    if (a.mask & 1) v[0] = a.swl + (double)s_sum[5] + (double)s_sum[0];
+    if (a.mask & 1) v[0] = a.swl + s_sum[5] + s_sum[0];
     for (int q = 1; q < 5; q++)
-        if (a.mask & (1 << q)) v[q] = (double)s_sum[q] + (double)s_sum[5 + q] * za;
+        if (a.mask & (1 << q)) v[q] = s_sum[q] + s_sum[5 + q] * za;
     if ((a.mask & 16) && a.kt.kin)
         v[4] += (double)s_ramp * kin_at(a.kt.kin, a.kt.nz, a.kt.h, fmin(0.0, zz));
     if (!a.api.any()) {
@@ -2122,7 +2178,7 @@ static int launch_point_few(const DevSea &sea, long n, const double *x, const do
     a.fx = sea.fx; a.fy = sea.fy; a.swl = sea.swl; a.depth = sea.depth;
     a.ncomp = sea.n; a.npad = sea.npad_g; a.cstride = sea.npad_g; a.trivial_ramp = sea.trivial_ramp ? 1 : 0;
     a.order = sea.order; a.clamp = api ? 1 : 0; a.mask = mask;
-    a.rec = sea.d_phrec; a.cf = sea.d_cf; a.phase = sea.d_phase;
+    a.rec = sea.d_phrec; a.cf = sea.d_cf; a.cfp = sea.d_cfp; a.phase = sea.d_phase;
     a.ntp = sea.ntile_p; a.ntg = sea.ntile_g;
     a.tabv = sea.d_tab_point; a.tpp = sea.d_tab_pp; a.tpk = sea.d_tab_pk; a.tabe = sea.d_tab_eta;
     const bool pairs = sea.order == 2;
@@ -2132,13 +2188,13 @@ static int launch_point_few(const DevSea &sea, long n, const double *x, const do
     a.nv = pairs && (mask & 14) ? ip : 0;
     a.np = pairs && (mask & 16) ? ip : 0;
     a.ne = pairs && (mask & 1) ? tg * GRID_TILE * GRID_TILE / FEW_E : 0;
-    a.part = L.split; a.cnt = L.cnt; a.out = out;
+    a.part = reinterpret_cast<float2 *>(L.split); a.cnt = L.cnt; a.out = out;
     if (api) a.api = *api;
     if (table) a.kt = KinTab{sea.d_kin, sea.kin_nz, sea.kin_h, sea.depth, nullptr};
     // as many slices as give every thread one item, up to about eight blocks an SM in all
     const long want = std::max<long>(1, (a.nv + a.np + a.ne + FEW_T - 1) / FEW_T);
     const long cap = std::max<long>(1, 2 * SPLIT_TARGET_BLOCKS / n);
-    const long ns = std::min(std::min(want, cap), std::max<long>(1, L.split_cap / (FEW_Q * n)));
+    const long ns = std::min(std::min(want, cap), std::max<long>(1, L.split_cap / (2 * FEW_Q * n)));
     const size_t smem = sizeof(float2) * (size_t)a.npad * (a.kin ? 2 : 1) + (sea.trivial_ramp ? 0 : sizeof(float) * a.npad);
     // set once per process (thread-safe static initialisation)
     static const cudaError_t attr = cudaFuncSetAttribute(k_point_few, cudaFuncAttributeMaxDynamicSharedMemorySize,
