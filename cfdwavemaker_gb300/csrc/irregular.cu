@@ -65,7 +65,7 @@ constexpr int POINTV_NC = 8, POINTP_NC = 4, POINTK_NC = 2;
 __host__ __device__ inline long point_at(long entry, int nc, int q) { return ((entry / 2) * nc + q) * 2 + (entry & 1); }
 constexpr float LOG2E_F = 1.4426950408889634f;
 constexpr long SPLIT_TARGET_BLOCKS = 4 * 152;   // blocks a column-pair launch aims for
-// Batches that the one-kernel evaluation (k_point_few) takes: 20 points, where
+// Batches that the evaluation by points (k_point_few) takes: 20 points, where
 // the per-thread kernels' blocks of 128 are nearly empty, and as many more as
 // 4e6 (pair, point) terms are, where its terms, read per point, cost less than
 // the per-thread path's eight dependent kernels.  Measured, a wave_Kinematics
@@ -75,7 +75,6 @@ constexpr long SPLIT_TARGET_BLOCKS = 4 * 152;   // blocks a column-pair launch a
 // points 140 and 130; 384 components, 64 points 144 and 149; 4096 components,
 // 16 points 1.9 and 2.2 ms, 64 points 7.3 and 2.2.
 constexpr long FEW_MAX_POINTS = 4096;
-constexpr size_t CNT_BYTES = sizeof(unsigned) * FEW_MAX_POINTS;
 constexpr int FEW_MAX_NPAD = 4096;   // components whose phasors, profiles and ramps fit shared memory
 static bool few_points(long n, int npad) {
     return npad <= FEW_MAX_NPAD && n <= FEW_MAX_POINTS &&
@@ -1401,7 +1400,6 @@ struct WsLayout {
     double *first;
     float *z0;
     float *sec;
-    unsigned *cnt;        // the few-point kernel's counters: first, so that every layout has them there
     float *split;         // partial sums of a split point-pair launch
     long split_cap;       // its floats
     size_t bytes;
@@ -1433,7 +1431,6 @@ WsLayout layout(long n, int npad, void *base) {
     WsLayout L;
     size_t off = 0;
     auto take = [&](size_t b) { size_t o = off; off += (b + 255) & ~size_t(255); return o; };
-    const size_t o_cnt = take(CNT_BYTES);
     size_t o_ph = take(sizeof(float2) * (size_t)npad * n);
     size_t o_rr = take(sizeof(float) * (size_t)npad * n);
     size_t o_first = take(sizeof(double) * 5 * (size_t)n);
@@ -1442,7 +1439,6 @@ WsLayout layout(long n, int npad, void *base) {
     const long scap = point_split_floats(n);
     size_t o_split = take(sizeof(float) * (size_t)std::max<long>(scap, 1));
     char *b = (char *)base;
-    L.cnt = (unsigned *)(b + o_cnt);
     L.ph = (float2 *)(b + o_ph);
     L.rr = (float *)(b + o_rr);
     L.first = (double *)(b + o_first);
@@ -1513,28 +1509,31 @@ __global__ void k_combine(long n, long ldo, int order, double swl, const double 
 }
 
 // ---------------------------------------------------------------------------
-// Few points (a scalar call, a short batch): the whole evaluation in one
-// kernel.  Block (point, slice): every block forms the point's phasors in
-// shared memory (two components a thread at once), then its threads take items
-// of the sums in turn -- eight terms of a row of a tile pair of the velocity,
-// pressure or elevation tables, and the first-order terms of a component --
-// and the block's sums go to its slice's partial sums.  The last block of a
-// point to finish (a counter per point that wraps to 0) adds the slices in a
-// fixed order, assembles eta, u, v, w, dp and writes the rows.  What bounds a
-// call is latency: as separate kernels (phasors, heights, elevation and point
-// pairs, slice sums, combining pass) a wave_VeloX call of the 128-component sea
-// was five dependent kernels, 26 us; 17 us now (a launch and a synchronisation are
-// 8 of these).
-// ---------------------------------------------------------------------------
+// Few points (a scalar call, a short batch).  Block (point, slice): every block
+// forms the point's phasors in shared memory (two components a thread at once),
+// then its threads take items of the sums in turn -- eight terms of a row of a
+// tile pair of the velocity, pressure or elevation tables, and the first-order
+// terms of a component -- and the block's sums go to its slice's partial sums.
+// k_few_finish, launched so that it is there when they are written, adds the
+// slices in a fixed order, assembles eta, u, v, w, dp and writes the rows (with one
+// slice k_point_few does).  What bounds a call is latency: as separate kernels
+// (phasors, heights, elevation and point pairs, slice sums, combining pass) a
+// wave_VeloX call of the 128-component sea was five dependent kernels, 26 us; 18 us
+// now (a launch and a synchronisation are 8 of these).  The blocks of a point could
+// also find out the last of them by a counter (four scalar calls 75 us, 73 so), but
+// so nothing carries over from one call to the next, whatever the workspace held
+// and whichever streams share it.
+//
 // Accuracy.  A single value is held to its own size, not to that of the largest
 // of a batch, and the first order is nearly all of it.  Its terms are formed in
 // float pairs (phase, sine, profiles, coefficients; 1e-8), as is every sum over
-// the threads and slices: 40 x 3 components, u 1.2e-7 RMS of the field with FP32
-// terms.  Heights above the bed, z + h, are taken in FP64: of an FP32 z = -50
+// the threads and slices: 40 x 3 components, u 9e-9 RMS of the field, 1.1e-7 with
+// FP32 terms.  Heights above the bed, z + h, are taken in FP64: of an FP32 z = -50
 // little is left of them, and w = sinh(k(z + h)) lives on that difference.  For
 // the same reason the pairs' profiles are e1 (1 +- e2), e2 = e^{-2k(z+h)}, not E +-
 // Y with Y = e^{-k(z+2h)}, whose exponents, of up to 40, round apart: w within
 // 3 m of the bed, 128 components at 50 m, 3.1e-7 RMS of its maximum with E - Y.
+// ---------------------------------------------------------------------------
 constexpr int FEW_T = 128;           // threads of a block
 constexpr int FEW_Q = 10;            // sums: eta2, u, v, w, dp, then eta1, gx, gy, gz, gp
 constexpr int FEW_E = 8;             // terms of an item
@@ -1550,7 +1549,6 @@ struct FewArgs {
     const float *tabv, *tpp, *tpk, *tabe;
     long nv, np, ne;                 // items of the velocity, pressure and elevation sums
     float2 *part;                    // [slices][FEW_Q][n] sums and their rounding errors
-    unsigned *cnt;                   // [n], zero before and after
     double *out;
     ApiRows api;
     KinTab kt;
@@ -1623,6 +1621,24 @@ __device__ __forceinline__ void few_first(const FewArgs &a, int i, float2 dx, fl
     }
 }
 
+// Irregular::eta/u/v/w/dp of point p from its sums (Irregular.cpp:9-157); kin: the
+// pressure's phase-free part from the height table.
+__device__ __forceinline__ void few_rows(const FewArgs &a, long p, const double *sum, double kin) {
+    const double za = a.order == 2 ? fmax(0.0, a.z[p] - a.swl) : 0.0;
+    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (a.mask & 1) v[0] = a.swl + sum[5] + sum[0];
+    for (int q = 1; q < 5; q++)
+        if (a.mask & (1 << q)) v[q] = sum[q] + sum[5 + q] * za;
+    v[4] += kin;
+    if (!a.api.any()) {
+        for (int q = 0; q < 5; q++)
+            if (a.mask & (1 << q)) a.out[q * a.ldo + p] = v[q];
+        return;
+    }
+    v[5] = v[4] - a.api.rho * a.api.g * v[0];
+    api_store(a.api, p, v);
+}
+
 __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
     extern __shared__ float2 s_few[];
     float2 *s_ph = s_few;                                   // phasors [npad]
@@ -1631,7 +1647,7 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
     __shared__ float2 s_red[FEW_T / 32][FEW_Q];
     __shared__ double s_sum[FEW_Q];
     __shared__ float s_ramp;
-    __shared__ int s_last;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int tid = threadIdx.x;
     const long p = blockIdx.x;
     const int ns = gridDim.y, slice = blockIdx.y;
@@ -1783,45 +1799,38 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
     if (tid < FEW_Q && few_needs(a.mask, tid)) {
         float2 v = s_red[0][tid];
         for (int w = 1; w < FEW_T / 32; w++) few_add(v, s_red[w][tid]);
-        if (ns > 1) __stcg(&a.part[((long)slice * FEW_Q + tid) * a.n + p], v);
+        if (ns > 1) a.part[((long)slice * FEW_Q + tid) * a.n + p] = v;
         else s_sum[tid] = (double)v.x + (double)v.y;
     }
-    if (ns > 1) {
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) s_last = atomicInc(&a.cnt[p], (unsigned)ns - 1) == (unsigned)ns - 1;
-        __syncthreads();
-        if (!s_last) return;
-        __threadfence();
-        // a warp a sum in turn, its lanes over the slices
-        for (int q = tid >> 5; q < FEW_Q; q += FEW_T / 32) {
-            if (!few_needs(a.mask, q)) continue;
-            double v = 0.0;
-            for (int k = tid & 31; k < ns; k += 32) {
-                const float2 f = __ldcg(&a.part[((long)k * FEW_Q + q) * a.n + p]);
-                v += (double)f.x + (double)f.y;
-            }
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if ((tid & 31) == 0) s_sum[q] = v;
+    if (ns > 1) return;
+    __syncthreads();
+    if (tid == 0) few_rows(a, p, s_sum, (a.mask & 16) && a.kt.kin ? s_ramp * kin_at(a.kt.kin, a.kt.nz, a.kt.h, z0) : 0.0);
+}
+
+// The slices of a point's sums, a warp a sum in turn, its lanes over the slices.
+__global__ void __launch_bounds__(FEW_T) k_few_finish(FewArgs a, int ns) {
+    __shared__ double s_sum[FEW_Q];
+    const int lane = threadIdx.x & 31;
+    const long p = blockIdx.x;
+    double kin = 0.0;
+    if (threadIdx.x == 0 && (a.mask & 16) && a.kt.kin) {
+        const double *P = a.phase + 4 * a.cstride;
+        const double z0 = fmin(0.0, (a.clamp ? fmax(-a.depth, a.z[p]) : a.z[p]) - a.swl);
+        kin = (float)d_freq_ramp(a.t[p], P[0], P[a.cstride], P[2 * a.cstride]) * kin_at(a.kt.kin, a.kt.nz, a.kt.h, z0);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");       // k_point_few's sums; what is above only reads inputs
+    for (int q = threadIdx.x >> 5; q < FEW_Q; q += FEW_T / 32) {
+        if (!few_needs(a.mask, q)) continue;
+        double v = 0.0;
+        for (int k = lane; k < ns; k += 32) {
+            const float2 f = a.part[((long)k * FEW_Q + q) * a.n + p];
+            v += (double)f.x + (double)f.y;
         }
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) s_sum[q] = v;
     }
     __syncthreads();
-    if (tid != 0) return;
-    // Irregular::eta/u/v/w/dp from the pieces (Irregular.cpp:9-157)
-    const double za = a.order == 2 ? fmax(0.0, zp - a.swl) : 0.0;
-    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    if (a.mask & 1) v[0] = a.swl + s_sum[5] + s_sum[0];
-    for (int q = 1; q < 5; q++)
-        if (a.mask & (1 << q)) v[q] = s_sum[q] + s_sum[5 + q] * za;
-    if ((a.mask & 16) && a.kt.kin)
-        v[4] += (double)s_ramp * kin_at(a.kt.kin, a.kt.nz, a.kt.h, fmin(0.0, zz));
-    if (!a.api.any()) {
-        for (int q = 0; q < 5; q++)
-            if (a.mask & (1 << q)) a.out[q * a.ldo + p] = v[q];
-        return;
-    }
-    v[5] = v[4] - a.api.rho * a.api.g * v[0];
-    api_store(a.api, p, v);
+    if (threadIdx.x == 0) few_rows(a, p, s_sum, kin);
 }
 
 }  // namespace
@@ -2169,7 +2178,7 @@ static int launch_point_pairs(const DevSea &sea, long n, const float2 *ph, const
     return rc;
 }
 
-// The whole evaluation of a few_points() batch in one kernel.
+// The whole evaluation of a few_points() batch.
 static int launch_point_few(const DevSea &sea, long n, const double *x, const double *y, const double *z,
                             const double *t, int mask, double *out, bool table, const WsLayout &L,
                             cudaStream_t stream, const ApiRows *api) {
@@ -2188,7 +2197,7 @@ static int launch_point_few(const DevSea &sea, long n, const double *x, const do
     a.nv = pairs && (mask & 14) ? ip : 0;
     a.np = pairs && (mask & 16) ? ip : 0;
     a.ne = pairs && (mask & 1) ? tg * GRID_TILE * GRID_TILE / FEW_E : 0;
-    a.part = reinterpret_cast<float2 *>(L.split); a.cnt = L.cnt; a.out = out;
+    a.part = reinterpret_cast<float2 *>(L.split); a.out = out;
     if (api) a.api = *api;
     if (table) a.kt = KinTab{sea.d_kin, sea.kin_nz, sea.kin_h, sea.depth, nullptr};
     // as many slices as give every thread one item, up to about eight blocks an SM in all
@@ -2203,8 +2212,21 @@ static int launch_point_few(const DevSea &sea, long n, const double *x, const do
     prof_begin(PK_POINT_PAIRS, stream);
     k_point_few<<<dim3((unsigned)n, (unsigned)ns), FEW_T, smem, stream>>>(a);
     note_launch();
-    prof_end(PK_POINT_PAIRS, stream);
     CK(cudaGetLastError());
+    if (ns > 1) {
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t c = {};
+        c.gridDim = dim3((unsigned)n);
+        c.blockDim = dim3(FEW_T);
+        c.stream = stream;
+        c.attrs = &at;
+        c.numAttrs = 1;
+        CK(cudaLaunchKernelEx(&c, k_few_finish, a, (int)ns));
+        note_launch();
+    }
+    prof_end(PK_POINT_PAIRS, stream);
     return OK;
 }
 
@@ -2221,10 +2243,8 @@ int irregular_eval(const DevSea &sea, long n, const double *x, const double *y, 
     // calls clamp z to the range it covers
     const bool table = api && sea.d_kin && sea.order == 2;
     WsLayout L0 = layout(std::min(n, chunk), npad, nullptr);
-    const void *held = ws.base;
     int rc = workspace_reserve(ws, L0.bytes);
     if (rc) return rc;
-    if (ws.base != held) CK(cudaMemsetAsync(ws.base, 0, CNT_BYTES, stream));    // the few-point counters
     if (few_points(n, npad) && !(sea.smit && (mask & 30)))
         return launch_point_few(sea, n, x, y, z, t, mask, out, table, layout(n, npad, ws.base), stream, api);
     for (long b = 0; b < n; b += chunk) {
