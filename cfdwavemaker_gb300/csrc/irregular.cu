@@ -805,8 +805,11 @@ struct PairArgs {
     long rs;
     const float *cf;     // [NCF][cstride]
     int cstride;
-    const float *z0;     // [ncol*nl] evaluation heights (z0 <= 0 below the surface)
+    const float *z0;     // column kernel: [ncol*nl] evaluation heights (z0 <= 0 below the surface)
     float depth;
+    const double *z;     // point kernel: the points' heights
+    double swl, h;
+    int order, clamp;    // clamp: the seabed clamp of the wave_* calls (z below -h evaluated at -h)
     float *out;          // [nf][ncol*nl]
     int pairs;           // 0: first-order z-dependent sums only
     int first;           // 1: add first-order z-dependent sums
@@ -1016,6 +1019,19 @@ __device__ __forceinline__ void pr_cp16(void *smem, const void *gmem) {
 __device__ __forceinline__ void pr_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void pr_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
+// The height of a point's profiles, z0 = min(0, z - swl) (order 2 and 1) or z -
+// swl (order 0): z0 and -2 (z0 + h), times log2(e).  In FP64, as an FP32
+// z0 = -50 keeps little of z0 + h, on which the first-order vertical velocity near
+// the seabed, e^{kz0} (1 - e^{-2k(z0+h)}), lives: RMS error of w over its own RMS within
+// 5 m of the bed at 50 m 4.4e-7 with z0 + h in FP32, 2.1e-7 so (within 1 m 2.2e-6 and
+// 1.1e-6; at 12 m depth, within 0.2 m, 2.9e-6 and 2.3e-6).
+__device__ __forceinline__ void point_height(double z, double swl, double h, int order, int clamp, float &zk,
+                                             float &zetak) {
+    const double zz = (clamp ? fmax(-h, z) : z) - swl, z0 = order == 0 ? zz : fmin(0.0, zz);
+    zk = (float)z0 * LOG2E_F;
+    zetak = (float)(-2.0 * (z0 + h)) * LOG2E_F;
+}
+
 // Point mode: u, v, w, dp at one height per thread, point-API mask
 // (u2/v2/w2/dp2 of the reference, with rho folded into the p records).
 // VEL: the velocity sums, PR: the pressure sums (a call that asks for one of
@@ -1033,7 +1049,11 @@ __device__ __forceinline__ void pr_wait1() { asm volatile("cp.async.wait_group 1
 // pressure sums 1331 us together then, 894 now; 5003 points, 256 components 491
 // and 264 (tiles of 32 instead of 16 components: 1043 and 383; five blocks an
 // SM instead of six: 882 and 307).  In a tile of the diagonal the records below
-// it are zero; whole groups of four are skipped.
+// it are zero; whole groups of four are skipped.  The pairs' profiles are E + Y and
+// E - Y, Y = e^{-k(z+2h)}; as E (1 +- e), e = e^{-2k(z+h)}, which k_point_few takes, they
+// cost a packed operation more each (65536 points 1171 us against 1134, with the
+// velocity's sign by the integer pipe) for at most 5 % of w's error near the bed (8 and
+// 12 m depth; none from 20 m on).
 // KIN: the phase-free products of the first-order profiles in the pressure,
 // summed here (otherwise the caller adds them from the height table).
 template <bool VEL, bool PR, bool KIN>
@@ -1057,9 +1077,9 @@ __global__ void __launch_bounds__(128, KIN ? 2 : 6) k_pairs_points(PairArgs a) {
     const long p = (long)blockIdx.x * 128 + tid;
     const bool valid = p < a.ncol;
     const long pc = valid ? p : a.ncol - 1;
-    const float z = a.z0[pc];
-    const float zk = z * LOG2E_F, zetak = -2.f * (z + a.depth) * LOG2E_F;
-    const float yk = -(z + 2.f * a.depth) * LOG2E_F;
+    float zk, zetak;
+    point_height(a.z[pc], a.swl, a.h, a.order, a.clamp, zk, zetak);
+    const float yk = zk + zetak;         // -(z + 2h)
     const f32x2 zk2 = p_pack(zk, zk), yk2 = p_pack(yk, yk), neg1 = p_pack(-1.f, -1.f);
     float su = 0, cu = 0, sv = 0, cv = 0, sw = 0, cw = 0, sq = 0, cq = 0;
     // slice of the tile-pair loop owned by this blockIdx.y (block-uniform);
@@ -1398,7 +1418,6 @@ struct WsLayout {
     float2 *ph;
     float *rr;
     double *first;
-    float *z0;
     float *sec;
     float *split;         // partial sums of a split point-pair launch
     long split_cap;       // its floats
@@ -1434,7 +1453,6 @@ WsLayout layout(long n, int npad, void *base) {
     size_t o_ph = take(sizeof(float2) * (size_t)npad * n);
     size_t o_rr = take(sizeof(float) * (size_t)npad * n);
     size_t o_first = take(sizeof(double) * 5 * (size_t)n);
-    size_t o_z = take(sizeof(float) * (size_t)n);
     size_t o_sec = take(sizeof(float) * 5 * (size_t)n);
     const long scap = point_split_floats(n);
     size_t o_split = take(sizeof(float) * (size_t)std::max<long>(scap, 1));
@@ -1442,7 +1460,6 @@ WsLayout layout(long n, int npad, void *base) {
     L.ph = (float2 *)(b + o_ph);
     L.rr = (float *)(b + o_rr);
     L.first = (double *)(b + o_first);
-    L.z0 = (float *)(b + o_z);
     L.sec = (float *)(b + o_sec);
     L.split = (float *)(b + o_split);
     L.split_cap = scap;
@@ -1459,16 +1476,6 @@ __device__ __forceinline__ double kin_at(const double *kin, int nz, double h, do
     const double f0 = kin[2 * i], f1 = kin[2 * i + 2], d0 = kin[2 * i + 1], d1 = kin[2 * i + 3];
     const double a = dz * d0 - (f1 - f0), b = -dz * d1 + (f1 - f0);
     return f0 * (1.0 - r) + f1 * r + r * (1.0 - r) * (a * (1.0 - r) + b * r);
-}
-
-// z0 = min(0, z - swl) (order 2/1) or z - swl (order 0), as float
-// clamp: the seabed clamp of the wave_* calls (z below -depth evaluated at
-// -depth), or 0 for the unclamped sums of cfdwm_irregular_fields
-__global__ void k_prep_z(long n, const double *z, double swl, int order, int clamp, double depth, float *z0) {
-    long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    double zz = (clamp ? fmax(-depth, z[p]) : z[p]) - swl;
-    z0[p] = (float)(order == 0 ? zz : fmin(0.0, zz));
 }
 
 // Irregular::eta/u/v/w/dp assembled from the pieces (Irregular.cpp:9-157).
@@ -2161,14 +2168,15 @@ static int point_pairs_t(PairArgs a, long n, int ntp, float *out, float *split_b
 // Rows u, v, w (mask bits 2, 4, 8) and p (16) of out [4][n]; rows not asked
 // for are not written.  kin: the pressure's phase-free products summed here.
 static int launch_point_pairs(const DevSea &sea, long n, const float2 *ph, const float *rr,
-                              const float *z0, float *out, int pairs, int mask, bool kin, cudaStream_t stream,
+                              const double *z, bool clamp, float *out, int pairs, int mask, bool kin, cudaStream_t stream,
                               float *split_buf, long split_cap) {
     PairArgs a{};
     a.ncol = n; a.nl = 1; a.nlg = 1; a.ntile = sea.ntile_p; a.tab = sea.d_tab_point;
     a.tpp = reinterpret_cast<const float4 *>(sea.d_tab_pp);
     a.tpk = reinterpret_cast<const float4 *>(sea.d_tab_pk);
-    a.ph = ph; a.rr = rr; a.rs = sea.trivial_ramp ? 0 : n; a.cf = sea.d_cf; a.cstride = sea.npad_g; a.z0 = z0;
-    a.depth = (float)sea.depth; a.pairs = pairs; a.first = 1; a.one = 1.f;
+    a.ph = ph; a.rr = rr; a.rs = sea.trivial_ramp ? 0 : n; a.cf = sea.d_cf; a.cstride = sea.npad_g;
+    a.z = z; a.swl = sea.swl; a.h = sea.depth; a.order = sea.order; a.clamp = clamp ? 1 : 0;
+    a.pairs = pairs; a.first = 1; a.one = 1.f;
     const int ntp = pairs ? sea.ntile_p * (sea.ntile_p + 1) / 2 : sea.ntile_p;
     int rc = OK;
     if (mask & 14) rc = point_pairs_t<true, false, false>(a, n, ntp, out, split_buf, split_cap, stream);
@@ -2268,13 +2276,9 @@ int irregular_eval(const DevSea &sea, long n, const double *x, const double *y, 
                            mask, stream);
             if (rc) return rc;
         } else if (mask & 30) {
-            k_prep_z<<<(unsigned)((m + 255) / 256), 256, 0, stream>>>(m, z + b, sea.swl, sea.order, api ? 1 : 0,
-                                                                  sea.depth, L.z0);
-            note_launch();
-            CK(cudaGetLastError());
             // the point table is padded to POINT_TILE; the phasor rows beyond
             // npad_p are never read by the point kernel
-            rc = launch_point_pairs(sea, m, L.ph, L.rr, L.z0, L.sec, sea.order != 0 ? 1 : 0, mask, !table, stream,
+            rc = launch_point_pairs(sea, m, L.ph, L.rr, z + b, api != nullptr, L.sec, sea.order != 0 ? 1 : 0, mask, !table, stream,
                                     L.split, L.split_cap);
             if (rc) return rc;
         }

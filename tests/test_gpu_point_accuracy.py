@@ -1,6 +1,6 @@
 """Accuracy of the point API's vertical velocity near the seabed, where
 w = sum q sinh(k (z + h)) ... is what is left of two nearly equal exponentials:
-one point at a time and in a short batch."""
+one point at a time, short batches and a batch for the per-thread kernels."""
 import numpy as np
 import pytest
 
@@ -40,7 +40,9 @@ def test_vertical_velocity_near_the_bed(wm, individual):
     ref = oracle.Model(oracle.waveinput.read_text(txt)).api(x, y, z, t)[:, 3]
     top = np.max(np.abs(ref))
     one = np.array([wm.velocity(*p)[2] for p in zip(x, y, z, t)])
-    got = {"one by one": one, "short batch": wm.velocity_batch(x, y, z, t)[2]}
+    reps = 17                                    # 5100 points: the kernels of 128 points a block
+    got = {"one by one": one, "short batch": wm.velocity_batch(x, y, z, t)[2],
+           "batch": wm.velocity_batch(*(np.tile(a, reps) for a in (x, y, z, t)))[2][:m]}
     for what, w in got.items():
         e = np.sqrt(np.mean((w - ref) ** 2)) / top
         assert e <= TOL, (what, e)
