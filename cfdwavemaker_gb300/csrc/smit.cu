@@ -236,16 +236,16 @@ __device__ __forceinline__ void smit_pair(const ulonglong2 *r, f32x2 px, f32x2 p
     const ulonglong2 rk = r[0], r1 = r[1], r2 = r[2];
     const f32x2 cc = p_mul(px, mc);
     const f32x2 cp = p_fma(ny, ms, cc), cm = p_fma(py, ms, cc);
-    // F = e1 (1 + e2), G = e1 (1 - e2), e1 = e^{kz}, e2 = e^{-2k(z+h)}
+    // F = e1 (1 + e2), G = e1 (1 - e2), one rounding each, e1 = e^{kz}, e2 = e^{-2k(z+h)}
     const f32x2 e1p = p_ex2(p_mul(rk.x, zk)), e2p = p_ex2(p_mul(rk.x, zetak));
     const f32x2 e1m = p_ex2(p_mul(rk.y, zk)), e2m = p_ex2(p_mul(rk.y, zetak));
     if (VEL) {
         const ulonglong2 r3 = r[3], r4 = r[4], r5 = r[5];
-        const f32x2 tp = p_mul(e1p, e2p), tm = p_mul(e1m, e2m);
         const f32x2 sc = p_mul(py, mc);
         const f32x2 sp = p_fma(px, ms, sc), sm = p_fma(nx, ms, sc);
-        const f32x2 X = p_mul(cp, p_add(e1p, tp)), Y = p_mul(cm, p_add(e1m, tm));
-        const f32x2 P = p_mul(sp, p_fma(tp, neg1, e1p)), Q = p_mul(sm, p_fma(tm, neg1, e1m));
+        const f32x2 X = p_mul(cp, p_fma(e1p, e2p, e1p)), Y = p_mul(cm, p_fma(e1m, e2m, e1m));
+        const f32x2 P = p_mul(sp, p_fma(e1p, p_mul(e2p, neg1), e1p));
+        const f32x2 Q = p_mul(sm, p_fma(e1m, p_mul(e2m, neg1), e1m));
         s.u = p_fma(r1.x, X, p_fma(r1.y, Y, s.u));
         s.v = p_fma(r2.x, X, p_fma(r2.y, Y, s.v));
         s.w = p_fma(r3.x, P, p_fma(r3.y, Q, s.w));
