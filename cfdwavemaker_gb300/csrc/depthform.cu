@@ -22,12 +22,11 @@
 //
 // With individual ramps (r_i weights the first component of a pair) a basis
 // function takes six triangular blocks (eight with the pressure); with one ramp
-// for all components three full ones (k_depth_coef_pot).  Full blocks have no
-// zero half, whose MMAs cost time but little power: 1024 components, 65536
-// columns 10.0 ms triangular, 8.5 to 8.9 as potentials (at the rate the power
-// allows); 320 components, 1786 columns with pressure 84 and 48 us.  Largest
-// errors of the fields against FP64 over 24 to 640 components: 1.8e-7 to 6.6e-7
-// triangular, 1.8e-7 to 8.1e-7.
+// for all components three full ones (k_depth_coef_pot) where the sea's spectrum
+// lets them keep the precision (pot_holds).  Full blocks have no zero half, whose
+// MMAs cost time but little power: 1024 components, 65536 columns 10.0 ms
+// triangular, 8.5 to 8.9 as potentials (at the rate the power allows); 320
+// components, 1786 columns with pressure 84 and 48 us.
 //
 // Set-up (host, FP64): Gauss-Legendre nodes on [-h, 0], the weighted kernel
 // matrix, its eigenvectors by cyclic Jacobi rotations, b_r on a fine z table
@@ -398,6 +397,49 @@ __global__ void k_depth_coef_pot(DfCoefArgs a) {
     }
 }
 
+// Whether the potential form keeps the sums' precision.  Its column terms are kx_m
+// P and kx_m M; their rounding errors (16-bit split, FP32 sums) are those of terms of
+// that size, while the pair's coefficients are P (kx_i + kx_m) and M (kx_i - kx_m),
+// and M grows as 1 / (omega_i - omega_m): for close frequencies a factor
+// k / |k_i - k_m| cancels.  The measure is
+//   rho = ||k_m (P, M)|| / ||(Pu, Mu, Pv, Mv)||
+// (Frobenius norms over the pairs), alike for the pressure with rho omega.  FP32
+// emulation of both forms at z = 0, RMS error of u2 over its RMS, triangular and
+// potential: 64 x 16 components at 100 m rho 1.3, 2.8e-7 and 4.9e-7; 96 x 3 1.8, 2.0e-7
+// and 3.5e-7; 96 x 1 at 50 m 2.2, 1.2e-7 and 3.2e-7; 257 x 1 at 45 m 3.9, 1.9e-7 and
+// 9.0e-7; 64 x 16 at 10 m 4.9, 1.9e-7 and 1.3e-6; 256 x 1 at 12 m 18, 1.8e-7 and 5.0e-6;
+// 1024 x 1 at 12 m 36, 2.0e-7 and 8.9e-6; two components 1e-6 apart in frequency
+// lose the term they make.  So the errors' ratio is about 1.2 rho, and 1.8 keeps it
+// to two.  The pressure's rho is twice that of the velocities (k = omega^2 / g), its
+// second-order part smaller beside the first order: 4.5 (64 x 5 components at 100 m
+// 2.6, 48 x 1 at 50 m 4.1; per level against FP64 its errors are 3e-8 to 1.6e-7 in either
+// form).
+constexpr double POT_RHO = 1.8, POT_RHO_P = 4.5;
+__global__ void __launch_bounds__(256) k_pot_norms(DfCoefArgs a, double *sums) {
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    const long tot = (long)a.n * a.n;
+    for (long e = blockIdx.x * 256L + threadIdx.x; e < tot; e += gridDim.x * 256L) {
+        const int m = (int)(e / a.n), i = (int)(e % a.n);
+        if (i > m) continue;
+        const long rec = df_tile_index(i / DF_TT, m / DF_TT, a.ntile) * DF_TT * DF_TT + i % DF_TT * DF_TT + m % DF_TT;
+        const float *g = a.tab_grid + rec * GRIDV_NC_DF;
+        auto sq = [](double v) { return v * v; };
+        const double k2i = sq(a.phase[i]) + sq(a.phase[a.cstride + i]), k2m = sq(a.phase[m]) + sq(a.phase[a.cstride + m]);
+        const double P = g[6] > 0.f ? (double)g[4] / g[6] : 0.0, M = g[7] > 0.f ? (double)g[5] / g[7] : 0.0;
+        const double pm = (i == m ? 2.0 : 1.0) * (sq(P) + sq(M));    // twice P on the diagonal, once a column
+        s[0] += (k2i + k2m) * pm;
+        s[1] += sq(g[0]) + sq(g[1]) + sq(g[2]) + sq(g[3]);
+        if (a.nf == 4) {
+            s[2] += sq(a.rho) * (sq(a.phase[2 * a.cstride + i]) + sq(a.phase[2 * a.cstride + m])) * pm;
+            s[3] += sq(a.tab_gp[rec * 2]) + sq(a.tab_gp[rec * 2 + 1]);
+        }
+    }
+    for (int q = 0; q < 4; q++) {
+        for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_down_sync(0xffffffffu, s[q], o);
+        if ((threadIdx.x & 31) == 0) atomicAdd(sums + q, s[q]);
+    }
+}
+
 // eta2 of the columns from output column 0
 __global__ void k_df_take(long n, int nout, const float *out, float *eta2) {
     long q = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -438,6 +480,25 @@ __global__ void k_df_combine(long nact, int nl, int R, int nf, int nout, const f
 // ---------------------------------------------------------------------------
 // Host
 // ---------------------------------------------------------------------------
+static int pot_holds(const DfCoefArgs &a, bool *holds, cudaStream_t stream) {
+    double *d = nullptr, h[4];
+    CK(cudaMalloc(&d, sizeof(h)));
+    cudaError_t e = cudaMemsetAsync(d, 0, sizeof(h), stream);
+    if (e == cudaSuccess) {
+        const long blocks = ((long)a.n * a.n + 255) / 256;
+        k_pot_norms<<<(unsigned)std::min<long>(blocks, 4096), 256, 0, stream>>>(a, d);
+        note_launch();
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    cudaFree(d);
+    CK(e);
+    // (a NaN anywhere: not the potential form)
+    *holds = h[0] <= POT_RHO * POT_RHO * h[1] && (a.nf != 4 || h[2] <= POT_RHO_P * POT_RHO_P * h[3]);
+    return OK;
+}
+
 int depthform_build(const Config &cfg, const DevSea &sea, DepthForm &df, int nf, void *stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
     depthform_free(df);
@@ -492,14 +553,16 @@ int depthform_build(const Config &cfg, const DevSea &sea, DepthForm &df, int nf,
     CK(cudaMemcpyAsync(d_fk, fk.data(), sizeof(double) * fk.size(), cudaMemcpyHostToDevice, stream));
     CK(cudaMemcpyAsync(d_gk, gk.data(), sizeof(double) * gk.size(), cudaMemcpyHostToDevice, stream));
     const int npad = ((sea.n + TC_NPAD - 1) / TC_NPAD) * TC_NPAD;
-    const bool pot = sea.trivial_ramp && df_one_acc();
-    const int nblk = 2 + (pot ? 3 : 2 * nf) * R;
-    CK(cudaMalloc(&coef, sizeof(double) * (size_t)nblk * npad * npad));
     DfCoefArgs a = {};
     a.n = sea.n; a.npad = npad; a.ntile = sea.ntile_g; a.R = R; a.nf = nf;
     a.tab_grid = sea.d_tab_grid; a.tab_eta = sea.d_tab_eta; a.tab_gp = sea.d_tab_gp; a.fk = d_fk; a.gk = d_gk;
-    a.inv_dk = 1.0 / dk; a.coef = coef;
+    a.inv_dk = 1.0 / dk;
     a.cstride = sea.npad_g; a.phase = sea.d_phase; a.rho = sea.rho;
+    bool pot = sea.trivial_ramp && df_one_acc();
+    if (pot && (rc = pot_holds(a, &pot, stream)) != OK) return rc;
+    const int nblk = 2 + (pot ? 3 : 2 * nf) * R;
+    CK(cudaMalloc(&coef, sizeof(double) * (size_t)nblk * npad * npad));
+    a.coef = coef;
     if (pot) CK(cudaMalloc(&a.wt, sizeof(float) * 3 * npad));
     long tot = (long)npad * npad;
     if (pot) k_depth_coef_pot<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(a);
