@@ -332,33 +332,46 @@ static void host_copy(double *dst, const double *src, long n) {
     for (auto &t : th) t.join();
 }
 
+// Whether a kernel may write FP64 values at p: aligned for it, in this
+// device's memory or host memory it addresses.
+bool writable_here(const double *p) {
+    int dev = -1;
+    cudaPointerAttributes at;
+    if (((uintptr_t)p & 7) != 0 || cudaGetDevice(&dev) != cudaSuccess) return false;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type != cudaMemoryTypeDevice || at.device == dev;
+}
+bool apart(const double *a, long na, const double *b, long nb) {
+    return (const char *)a + sizeof(double) * na <= (const char *)b ||
+           (const char *)b + sizeof(double) * nb <= (const char *)a;
+}
 // Whether the evaluation's last kernel may write the caller's rows itself
 // with the result that a scratch block and a copy per row would give: every
-// row aligned for FP64 stores, in this device's memory (or host memory it
-// addresses), and overlapping no input and no other row except where it is
-// that same array (each thread reads its point's inputs before it writes that
-// point's rows, in row order, and no other thread reads them).
+// row overlapping no input and no other row except where it is that same array
+// (each thread reads its point's inputs before it writes that point's rows, in
+// row order, and no other thread reads them).
 bool rows_in_place(double *const outs[6], const double *const ins[4], long n) {
-    int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess) return false;
-    auto apart = [n](const double *a, const double *b) {
-        return a == b || (const char *)a + sizeof(double) * n <= (const char *)b ||
-               (const char *)b + sizeof(double) * n <= (const char *)a;
-    };
     for (int q = 0; q < 6; q++) {
         if (!outs[q]) continue;
-        if (((uintptr_t)outs[q] & 7) != 0) return false;
-        cudaPointerAttributes at;
-        if (cudaPointerGetAttributes(&at, outs[q]) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        if (at.type == cudaMemoryTypeDevice && at.device != dev) return false;
+        if (!writable_here(outs[q])) return false;
         for (int i = 0; i < 4; i++)
-            if (!apart(outs[q], ins[i])) return false;
+            if (outs[q] != ins[i] && !apart(outs[q], n, ins[i], n)) return false;
         for (int r = 0; r < q; r++)
-            if (outs[r] && !apart(outs[q], outs[r])) return false;
+            if (outs[r] && outs[q] != outs[r] && !apart(outs[q], n, outs[r], n)) return false;
     }
+    return true;
+}
+// The same of the wave_Kinematics records: a point's record lies where other
+// points' inputs do as soon as the arrays overlap.
+bool records_in_place(double *kin, double *const outs[6], const double *const ins[4], long n) {
+    if (!writable_here(kin)) return false;
+    for (int i = 0; i < 4; i++)
+        if (!apart(kin, 4 * n, ins[i], n)) return false;
+    for (int q = 0; q < 6; q++)
+        if (outs[q] && !apart(kin, 4 * n, outs[q], n)) return false;
     return true;
 }
 
@@ -391,27 +404,31 @@ int run_batch(const double *x, const double *y, const double *z, const double *t
         // where that could give another result (rows_in_place), through a
         // scratch block and a copy per row
         const bool place = rows_in_place(outs, ins, n);
+        const bool kin_place = !kin_out || records_in_place(kin_out, outs, ins, n);
         OutRows o;
-        o.kin = kin_out;
-        double *scratch = nullptr;
+        double *scratch = nullptr, *kin = kin_out;
         static thread_local Workspace dev_out;
-        if (vf_out || !place) {
-            int rc = workspace_reserve(dev_out, sizeof(double) * 6 * (size_t)n);
+        if (vf_out || !place || !kin_place) {
+            int rc = workspace_reserve(dev_out, sizeof(double) * (kin_place ? 6 : 10) * (size_t)n);
             if (rc) return rc;
             scratch = (double *)dev_out.base;
+            if (!kin_place) kin = scratch + 6 * n;
         }
+        o.kin = kin;
         for (int q = 0; q < 6; q++) o.row[q] = !outs[q] ? nullptr : place ? outs[q] : scratch + (long)q * n;
         if (vf_out) o.row[0] = scratch;
         int rc = eval_api(n, x, y, zz, t, want, o, s);
         if (rc) return rc;
-        for (int q = 0; q < 6 && !place; q++) {
-            if (!outs[q]) continue;
-            if (direct) {
-                k_copy_row<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, scratch + (long)q * n, outs[q]);
+        for (int q = 0; q < 7; q++) {            // 6: the records
+            double *to = q < 6 ? outs[q] : kin_out;
+            if (!to || (q < 6 ? place : kin_place)) continue;
+            const long m = q < 6 ? n : 4 * n;
+            if (direct && ((uintptr_t)to & 7) == 0) {
+                k_copy_row<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(m, scratch + (long)q * n, to);
                 note_launch();
                 CKR(cudaGetLastError());
             } else {
-                CKR(cudaMemcpyAsync(outs[q], scratch + (long)q * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+                CKR(cudaMemcpyAsync(to, scratch + (long)q * n, sizeof(double) * m, cudaMemcpyDefault, s));
             }
         }
         if (vf_out) {
