@@ -12,7 +12,7 @@
 //
 // Sums (FP32):
 //   surface   eta1 and the Taylor gradients phi1_dxdz, phi1_dydz, phi1_dzdz,
-//             dp1_dz (Irregular.cpp:178-198, 1107-1192), 16 terms in FP32, then Kahan
+//             dp1_dz (Irregular.cpp:178-198, 1107-1192), every term compensated (Kahan)
 //   levels    u1, v1, w1 (and dp1) at the level heights (Irregular.cpp:394-447,
 //             1107-1120), 32 terms in FP32, then Kahan
 //   features  u, v, w and the pressure head at the levels placed under eta1,
@@ -145,14 +145,18 @@ __device__ __forceinline__ void col_rows(const GridTab &T, const GridCols &c, lo
 // TILE: block (blockIdx.x, blockIdx.y) holds SR rows of 32 columns of the whole
 // grid, and a thread SR columns, whose y entries are one load; else blockIdx.x
 // holds SR x 32 listed columns.  Warp w sums the components w, w + nw, ...  Loads
-// of table entries bound it: one column a thread, 65536 columns of 1024
-// components took 144 us, 79 with four; with the phase formed per (column,
-// component) and five Kahan sums it was issue-bound, 256 us.  A short list gets
+// of table entries bound it where a term is added plainly (one column a thread,
+// 65536 columns of 1024 components 144 us, 79 with four), but every
+// term's rounding error is kept: 14 packed operations a component for two columns
+// instead of 9, eight components' loads in flight at two blocks an SM (a learned
+// update 583 us with 16 plain terms a Kahan step, 597 so; four blocks, two
+// components 615, three and four 615, one and eight 610).  With the phase
+// formed per (column, component) it was issue-bound, 256 us.  A short list gets
 // 32 warps a block (64 columns: 8 warps 54 us, 23; one thread per column
 // 180).
 constexpr int SR = 4;
 template <bool TILE, int NW>
-__global__ void __launch_bounds__(32 * NW, TILE ? 4 : 1) k_first_surface(GridTab T, GridCols c, double *first) {
+__global__ void __launch_bounds__(32 * NW, TILE ? 2 : 1) k_first_surface(GridTab T, GridCols c, double *first) {
     __shared__ float2 part[NW][5][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     constexpr int NR = TILE ? SR : 1;
@@ -172,43 +176,55 @@ __global__ void __launch_bounds__(32 * NW, TILE ? 4 : 1) k_first_surface(GridTab
         valid[0] = p[0] < c.n;
         col_rows(T, c, valid[0] ? p[0] : c.n - 1, i, j);
     }
+    // sums s with their carries k, every term compensated; TILE: two rows to a
+    // packed operand
+    constexpr int NP = TILE ? NR / 2 : 1;
     float s[NR][5] = {}, k[NR][5] = {};
+    f32x2 ps[NP][5] = {}, pk[NP][5] = {};
+    const f32x2 neg1 = p_pack(-1.f, -1.f);
     for (int q0 = w; q0 < T.ncp; q0 += 128) {
-        float v[NR][5] = {};
-#pragma unroll(TILE ? 2 : 128 / NW < 8 ? 128 / NW : 8)
+#pragma unroll(128 / NW < 8 ? 128 / NW : 8)
         for (int u = 0; u < 128 / NW; u++) {
             const int q = q0 + NW * u;
             const float2 y = T.Y[(long)q * T.sy + j];
-            float2 x[NR];
             const float2 *xp = T.X + (long)q * T.sx + i;
-            if (TILE) {
-#pragma unroll
-                for (int r = 0; r < NR; r += 2) {
-                    const float4 f = *reinterpret_cast<const float4 *>(xp + r);
-                    x[r] = make_float2(f.x, f.y);
-                    x[(r + 1) % NR] = make_float2(f.z, f.w);
-                }
-            } else {
-                x[0] = *xp;
-            }
             const float *rec = T.rec + (long)q * REC + REC_S;
             const float4 f = *reinterpret_cast<const float4 *>(rec);
-            const float gp = rec[4];
+            const float cf[5] = {f.x, f.y, f.z, f.w, rec[4]};
+            if (TILE) {
 #pragma unroll
-            for (int r = 0; r < NR; r++) {
-                const float2 e = cmul(x[r], y);
-                v[r][0] = fmaf(f.x, e.x, v[r][0]);
-                v[r][1] = fmaf(f.y, e.x, v[r][1]);
-                v[r][2] = fmaf(f.z, e.x, v[r][2]);
-                v[r][3] = fmaf(f.w, e.y, v[r][3]);
-                v[r][4] = fmaf(gp, e.x, v[r][4]);
+                for (int r = 0; r < NP; r++) {
+                    const float4 x = *reinterpret_cast<const float4 *>(xp + 2 * r);
+                    const float2 e0 = cmul(make_float2(x.x, x.y), y), e1 = cmul(make_float2(x.z, x.w), y);
+                    const f32x2 ec = p_pack(e0.x, e1.x), es = p_pack(e0.y, e1.y);
+#pragma unroll
+                    for (int v = 0; v < 5; v++) {
+                        const f32x2 a = p_fma(p_pack(cf[v], cf[v]), v == 3 ? es : ec, pk[r][v]);
+                        const f32x2 t = p_add(ps[r][v], a);
+                        pk[r][v] = p_add(p_fma(t, neg1, ps[r][v]), a);
+                        ps[r][v] = t;
+                    }
+                }
+            } else {
+                const float2 e = cmul(*xp, y);
+#pragma unroll
+                for (int v = 0; v < 5; v++) {
+                    const float a = fmaf(cf[v], v == 3 ? e.y : e.x, k[0][v]), t = s[0][v] + a;
+                    k[0][v] = (s[0][v] - t) + a;
+                    s[0][v] = t;
+                }
             }
         }
-#pragma unroll
-        for (int r = 0; r < NR; r++)
-#pragma unroll
-            for (int f = 0; f < 5; f++) kahan_add(s[r][f], k[r][f], v[r][f]);
     }
+    if (TILE)
+#pragma unroll
+        for (int r = 0; r < NP; r++)
+#pragma unroll
+            for (int v = 0; v < 5; v++) {
+                const float2 a = p_un(ps[r][v]), b = p_un(pk[r][v]);
+                s[2 * r][v] = a.x; k[2 * r][v] = b.x;
+                s[(2 * r + 1) % NR][v] = a.y; k[(2 * r + 1) % NR][v] = b.y;
+            }
 #pragma unroll
     for (int r = 0; r < NR; r++) {
         if (r) __syncthreads();
@@ -220,7 +236,7 @@ __global__ void __launch_bounds__(32 * NW, TILE ? 4 : 1) k_first_surface(GridTab
             for (int u = 0; u < NW; u++) {
                 const float2 v = part[u][w][lane];
                 kahan_add(S, K, v.x);
-                kahan_add(S, K, -v.y);
+                kahan_add(S, K, v.y);
             }
             first[w * c.n + p[r]] = (double)S - (double)K;
         }
