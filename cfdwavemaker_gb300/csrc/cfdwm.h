@@ -135,6 +135,7 @@ enum CompCoef {
 constexpr int GRID_TILE = 32;
 constexpr int POINT_TILE = 16;
 constexpr int SMIT_TILE = 16;
+constexpr int KGRP = 64;              // components of a wave-number group at most
 
 struct DevSea {
     int n = 0;              // components
@@ -170,7 +171,7 @@ struct DevSea {
     // kx, ky, -omega, phase0 as float pairs, then A, GX, GY, GZ, GP
     float *d_phrec = nullptr;
     // the components by wave number: their indices, and where each group of
-    // one (FP32) wave number begins (ngrp + 1 entries)
+    // one (FP32) wave number, of KGRP components at most, begins (ngrp + 1 entries)
     int *d_kperm = nullptr, *d_kgrp = nullptr;
     int ngrp = 0;
 };

@@ -14,7 +14,8 @@
 //   surface   eta1 and the Taylor gradients phi1_dxdz, phi1_dydz, phi1_dzdz,
 //             dp1_dz (Irregular.cpp:178-198, 1107-1192), every term compensated (Kahan)
 //   levels    u1, v1, w1 (and dp1) at the level heights (Irregular.cpp:394-447,
-//             1107-1120), 32 terms in FP32, then Kahan
+//             1107-1120): the components of a wave-number group, at most KGRP = 64, in
+//             FP32, then 32 groups, then Kahan
 //   features  u, v, w and the pressure head at the levels placed under eta1,
 //             each in phase and in quadrature
 #include "cfdwm.h"
@@ -46,7 +47,7 @@ constexpr float LOG2E_F = 1.4426950408889634f;
 constexpr int REC = 16;          // floats of a component's record:
 constexpr int REC_S = 0;         //   surface coefficients A, gx, gy, gz, gp
 constexpr int REC_L = 8;         //   level coefficients cu, cv, cw, dp1's, head's (all times the ramp)
-constexpr int REC_K = 13;        //   k, -2 k h log2(e)
+constexpr int REC_K = 13;        //   k
 
 struct TabArgs {
     GridCols c;
@@ -85,7 +86,6 @@ __global__ void __launch_bounds__(128) k_grid_tab(TabArgs a) {
             r[REC_L + 3] = rp * (f[CF_AP * cs] * qn);
             r[REC_L + 4] = rp * (f[CF_A * cs] * qn);
             r[REC_K] = k;
-            r[REC_K + 1] = -2.f * a.depth * k * LOG2E_F;
         }
         a.ramp[c] = rp;
     }
@@ -274,7 +274,7 @@ template <int MODE, bool FEW> struct LvCfg {
     static constexpr int NQ = MODE == LV_FEAT ? 2 : 1;                         // float4 of a group's sums
     // groups' wave numbers and sums, twice; FEATURES: the heights above swl, else sums and carries
     static constexpr int smem(int rows, int threads) {
-        return 2 * LGC * (16 + rows * NQ * 32 * 16) + (MODE == LV_FEAT ? 8 : 16 * NC) * LP * threads;
+        return 2 * LGC * (8 + rows * NQ * 32 * 16) + (MODE == LV_FEAT ? 8 : 16 * NC) * LP * threads;
     }
 };
 
@@ -290,9 +290,15 @@ __device__ __forceinline__ void lv_prefetch(const void *p) { asm volatile("prefe
 // (coefficient, phasor) products of its groups' components into shared memory
 // (a complex product and 3 to 8 multiply-adds each, loads of table entries),
 // then each warp adds all the groups' sums times the profiles to its levels, two
-// levels to a packed operation (12 and 4 exponentials a pair of levels).  The
-// sums of one pass are made while the warps that are done with them use those
-// of the pass before.  With the profiles per component the second half was
+// levels to a packed operation (12 and 4 exponentials a pair of levels).  Groups
+// end at 64 components: chains of 64 terms and of 32 groups round less than the one
+// chain of 128 components before them, a group of any length would not.  The
+// exponents are products of k and the level's z or -(z + 2h); -kz - 2kh, of the
+// rounded kz and 2kh, was the larger error near the bed.  1000 directions of one
+// frequency in phase, u at the bed: 6.5e-7 of its RMS without the limit and with
+// that exponent, 3.6e-7 with the limit, 1.8e-7 now (4.1e-7 with phases by the SFU and
+// chains of 128).  The sums of one pass are made while the warps that are done
+// with them use those of the pass before.  With the profiles per component the second half was
 // bound by the FMA and SFU pipes (58 % and 30 % busy).  16 levels, 1024 components
 // in 64 groups, features of 69696 columns: one level at a time with float-float
 // phases 1263 us, packed 805, by groups 169; levels of 65536 columns: 675, 660
@@ -305,8 +311,8 @@ __global__ void __launch_bounds__(512, 1) k_first_levels(LevelArgs a, int rows) 
     extern __shared__ __align__(16) uint8_t lv_raw[];
     __shared__ int2 s_ij[8][32];                                 // not TILE: the columns' table rows
     const GridCols &c = a.c;
-    float4 *s_k = reinterpret_cast<float4 *>(lv_raw);            // [2][LGC]: k, k, and the same of -2 k h
-    float4 *s_q = s_k + 2 * LGC;                                 // [2][LGC][rows][NQ][32]: the groups' sums
+    f32x2 *s_k = reinterpret_cast<f32x2 *>(lv_raw);              // [2][LGC]: k, k
+    float4 *s_q = reinterpret_cast<float4 *>(s_k + 2 * LGC);     // [2][LGC][rows][NQ][32]: the groups' sums
     f32x2 *keep = reinterpret_cast<f32x2 *>(s_q + 2 * LGC * rows * NQ * 32) + threadIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nt = blockDim.x, nw = nt >> 5;
     const int ng = min((a.nl + 2 * LP - 1) / (2 * LP), LGRP), g = w % ng;
@@ -331,7 +337,7 @@ __global__ void __launch_bounds__(512, 1) k_first_levels(LevelArgs a, int rows) 
         cj = s_ij[row][lane].y;
     }
     const f32x2 one = p_pack(a.one2.x, a.one2.y), one2 = p_mul(one, one), neg1 = p_hold(-1.f, -1.f, one);
-    f32x2 zk[LP];
+    f32x2 zk[LP], yk[LP];                                        // z and -(z + 2h), times log2(e)
 #pragma unroll
     for (int l = 0; l < LP; l++) {
         float z[2], za[2] = {0.f, 0.f};
@@ -347,6 +353,7 @@ __global__ void __launch_bounds__(512, 1) k_first_levels(LevelArgs a, int rows) 
             }
         }
         zk[l] = p_hold(z[0] * LOG2E_F, z[1] * LOG2E_F, one2);
+        yk[l] = p_hold(-(z[0] + 2.f * a.depth) * LOG2E_F, -(z[1] + 2.f * a.depth) * LOG2E_F, one2);
         if (MODE == LV_FEAT) keep[l * nt] = p_pack(za[0], za[1]);
     }
     f32x2 acc[NC][LP];
@@ -419,7 +426,7 @@ __global__ void __launch_bounds__(512, 1) k_first_levels(LevelArgs a, int rows) 
             }
             if (lane == 0) {
                 const float *rc = a.T.rec + (long)qb * REC + REC_K;
-                s_k[buf * LGC + gi] = make_float4(rc[0], rc[0], rc[1], rc[1]);
+                s_k[buf * LGC + gi] = p_pack(rc[0], rc[0]);
             }
         }
     };
@@ -440,7 +447,7 @@ __global__ void __launch_bounds__(512, 1) k_first_levels(LevelArgs a, int rows) 
         }
         const int ngc = min(LGC, a.T.ngrp - g0);
         for (int gi = 0; gi < (worker ? ngc : 0); gi++) {
-            const ulonglong2 rk = *reinterpret_cast<const ulonglong2 *>(s_k + buf * LGC + gi);
+            const f32x2 rk = s_k[buf * LGC + gi];
             const float4 *sq = s_q + (((buf * LGC + gi) * rows + row) * NQ) * 32 + lane;
             const float4 sc = sq[0];
             f32x2 q2[NC];
@@ -457,9 +464,8 @@ __global__ void __launch_bounds__(512, 1) k_first_levels(LevelArgs a, int rows) 
             f32x2 E[LP], D[LP];
 #pragma unroll
             for (int l = 0; l < LP; l++) {
-                const f32x2 x = p_mul(rk.x, zk[l]);
-                E[l] = p_ex2(x);
-                D[l] = p_ex2(p_fma(x, neg1, rk.y));
+                E[l] = p_ex2(p_mul(rk, zk[l]));
+                D[l] = p_ex2(p_mul(rk, yk[l]));
             }
 #pragma unroll
             for (int l = 0; l < LP; l++) {

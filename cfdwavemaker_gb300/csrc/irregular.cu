@@ -418,8 +418,9 @@ int sea_build(const Config &cfg, DevSea &sea, bool point_table, void *stream_) {
             perm[i] = i;
         }
         std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) { return key[a] < key[b]; });
+        // at most KGRP components to a group, whose first stage of summation is plain
         for (int i = 1; i <= n; i++)
-            if (i == n || key[perm[i]] != key[perm[i - 1]]) grp.push_back(i);
+            if (i == n || key[perm[i]] != key[perm[i - 1]] || i - grp.back() == KGRP) grp.push_back(i);
         sea.ngrp = (int)grp.size() - 1;
         CK(cudaMalloc(&sea.d_kperm, sizeof(int) * nn));
         CK(cudaMalloc(&sea.d_kgrp, sizeof(int) * grp.size()));
