@@ -1359,6 +1359,7 @@ int tcform_eval(TcForm &f, const DevSea &sea, long n, const double *x, const dou
     const int npad = f.npad;
     if (npad < sea.n) return E_BAD_ARGUMENT;
     CK(cudaMemsetAsync(out, 0, sizeof(float) * f.nout * n, stream));
+    if (sea.n == 0) return OK;                   // no components: the forms are zero (and no tile has a K block)
     const long chunk = 1L << 16;
     long m = std::min(n, chunk);
     long mpad = ((m + TBM - 1) / TBM) * TBM;
