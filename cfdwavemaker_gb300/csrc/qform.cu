@@ -1602,9 +1602,13 @@ int qform_eval(const DevSea &sea, long n, const double *x, const double *y, cons
     CK(cudaMemsetAsync(out, 0, sizeof(float) * 4 * n, stream));
     const long chunk = 1L << 16;
     // one-time, thread-safe (static initialisation)
-    static const cudaError_t pattr =
-        cudaFuncSetAttribute(k_qform_plain<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, QPLAIN_SMEM);
-        cudaFuncSetAttribute(k_qform_plain<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, QPLAIN_SMEM);
+    static const cudaError_t pattr = [] {
+        const cudaError_t e =
+            cudaFuncSetAttribute(k_qform_plain<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, QPLAIN_SMEM);
+        return e != cudaSuccess ? e
+                                : cudaFuncSetAttribute(k_qform_plain<true>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, QPLAIN_SMEM);
+    }();
     CK(pattr);
     // two blocks of the kernel fit an SM (registers, shared memory)
     static const int slots = [] {
