@@ -549,9 +549,11 @@ __global__ void k_sigma(GridGeom g, double *sig) {
     for (int m = threadIdx.x; m < g.nl; m += blockDim.x) sig[m] = d_sigma_level(g, m);
 }
 
-// Tiles of whole rows where at least two thirds of the lanes have a column.
+// Tiles of whole rows where at least two thirds of the lanes have a column (and
+// the rows, two a block at least, fit the grid's y dimension; the columns of more
+// are taken as a list, whose blocks are in x).
 bool tiled(const GridCols &c) {
-    return !c.act && c.n == (long)c.nx * c.ny && 3 * c.ny >= 2 * ((c.ny + 31) / 32 * 32);
+    return !c.act && c.n == (long)c.nx * c.ny && c.nx <= 2 * 65535 && 3 * c.ny >= 2 * ((c.ny + 31) / 32 * 32);
 }
 
 template <int MODE, bool TILE, bool FEW>
