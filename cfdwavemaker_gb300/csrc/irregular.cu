@@ -812,7 +812,7 @@ struct PairArgs {
     double swl, h;
     int order, clamp;    // clamp: the seabed clamp of the wave_* calls (z below -h evaluated at -h)
     float *out;          // [nf][ncol*nl]
-    int pairs;           // 0: first-order z-dependent sums only
+    int pairs;           // point kernel; 0: first-order z-dependent sums only
     int first;           // 1: add first-order z-dependent sums
     int tp_per;          // tile pairs per blockIdx.y (split of the pair loop; partial sums
                          // of slice y go to out + y * nf * ncol * nl)
@@ -868,19 +868,16 @@ __global__ void __launch_bounds__(128) k_pairs_columns(PairArgs a) {
     int tp = -1;
     for (int I = 0; I < a.ntile; I++) {
         for (int M = I; M < a.ntile; M++) {
-            if (!a.pairs && M != I) continue;
             tp++;
             if (tp < tp_lo || tp >= tp_hi) continue;
             __syncthreads();
-            if (a.pairs) {
-                const float4 *src = reinterpret_cast<const float4 *>(
-                    a.tab + tile_index(I, M, a.ntile) * (long)TT * TT * GRIDV_NC);
-                float4 *dst = reinterpret_cast<float4 *>(s_tab);
-                for (int e = threadIdx.x; e < TT * TT * GRIDV_NC / 4; e += blockDim.x) dst[e] = src[e];
-                if (PR) {
-                    const float2 *srp = a.tabp + tile_index(I, M, a.ntile) * (long)TT * TT;
-                    for (int e = threadIdx.x; e < TT * TT; e += blockDim.x) s_tp[e] = srp[e];
-                }
+            const float4 *src = reinterpret_cast<const float4 *>(
+                a.tab + tile_index(I, M, a.ntile) * (long)TT * TT * GRIDV_NC);
+            float4 *dst = reinterpret_cast<float4 *>(s_tab);
+            for (int e = threadIdx.x; e < TT * TT * GRIDV_NC / 4; e += blockDim.x) dst[e] = src[e];
+            if (PR) {
+                const float2 *srp = a.tabp + tile_index(I, M, a.ntile) * (long)TT * TT;
+                for (int e = threadIdx.x; e < TT * TT; e += blockDim.x) s_tp[e] = srp[e];
             }
             for (int e = threadIdx.x; e < TT * cols; e += blockDim.x) {
                 int mm = e / cols, c2 = e % cols;
@@ -889,69 +886,67 @@ __global__ void __launch_bounds__(128) k_pairs_columns(PairArgs a) {
             }
             __syncthreads();
             if (!valid) continue;
-            if (a.pairs) {
-                for (int ii = 0; ii < TT; ii++) {
-                    const int i = I * TT + ii;
-                    const float2 pi = a.ph[(long)i * a.ncol + col];
-                    const float ri = a.rr[(long)i * a.rs + col];
-                    // packed FP32x2 over level pairs: per pair and level,
-                    // E = exp(k z), Y = exp(-k(z + 2h)) = E exp(-2k(z+h)),
-                    // F = E + Y, G = E - Y (the normaliser is in the record)
-                    float2 au[LP], av[LP], aw[LP], apr[PR ? LP : 1];
+            for (int ii = 0; ii < TT; ii++) {
+                const int i = I * TT + ii;
+                const float2 pi = a.ph[(long)i * a.ncol + col];
+                const float ri = a.rr[(long)i * a.rs + col];
+                // packed FP32x2 over level pairs: per pair and level,
+                // E = exp(k z), Y = exp(-k(z + 2h)) = E exp(-2k(z+h)),
+                // F = E + Y, G = E - Y (the normaliser is in the record)
+                float2 au[LP], av[LP], aw[LP], apr[PR ? LP : 1];
 #pragma unroll
-                    for (int j = 0; j < LP; j++) au[j] = av[j] = aw[j] = make_float2(0.f, 0.f);
+                for (int j = 0; j < LP; j++) au[j] = av[j] = aw[j] = make_float2(0.f, 0.f);
 #pragma unroll
-                    for (int j = 0; j < (PR ? LP : 1); j++) apr[j] = make_float2(0.f, 0.f);
-                    const float2 neg1 = make_float2(-1.f, -1.f);
-                    const int m0 = (M == I) ? ii : 0;
-                    for (int mm = m0; mm < TT; mm++) {
-                        const float4 c0 = *reinterpret_cast<const float4 *>(s_tab + (ii * TT + mm) * GRIDV_NC);
-                        const float4 c1 = *reinterpret_cast<const float4 *>(s_tab + (ii * TT + mm) * GRIDV_NC + 4);
-                        const float2 pm = s_ph[mm * cols + cl];
-                        const float cc = pi.x * pm.x, ss = pi.y * pm.y;
-                        const float sc = pi.y * pm.x, cs = pi.x * pm.y;
-                        const float cp = cc - ss, cmn = cc + ss, sp = sc + cs, smn = sc - cs;
-                        const float up = c0.x * cp, um = c0.y * cmn, vp = c0.z * cp, vm = c0.w * cmn;
-                        const float wp = c1.x * sp, wm = c1.y * smn;
-                        const float2 up2 = make_float2(up, up), um2 = make_float2(um, um);
-                        const float2 vp2 = make_float2(vp, vp), vm2 = make_float2(vm, vm);
-                        const float2 wp2 = make_float2(wp, wp), wm2 = make_float2(wm, wm);
-                        const float2 kp2 = make_float2(c1.z, c1.z), km2 = make_float2(c1.w, c1.w);
-                        float2 pp2 = make_float2(0.f, 0.f), pm2 = pp2;
-                        if (PR) {
-                            const float2 tp = s_tp[ii * TT + mm];
-                            const float pp = tp.x * cp, pm_ = tp.y * cmn;
-                            pp2 = make_float2(pp, pp);
-                            pm2 = make_float2(pm_, pm_);
-                        }
-#pragma unroll
-                        for (int j = 0; j < LP; j++) {
-                            const float2 ap = __fmul2_rn(kp2, zk2[j]), bp = __fmul2_rn(kp2, yk2[j]);
-                            const float2 am = __fmul2_rn(km2, zk2[j]), bm = __fmul2_rn(km2, yk2[j]);
-                            const float2 Ep = make_float2(ex2(ap.x), ex2(ap.y));
-                            const float2 Yp = make_float2(ex2(bp.x), ex2(bp.y));
-                            const float2 Em = make_float2(ex2(am.x), ex2(am.y));
-                            const float2 Ym = make_float2(ex2(bm.x), ex2(bm.y));
-                            const float2 Fp = __fadd2_rn(Ep, Yp), Gp = __ffma2_rn(Yp, neg1, Ep);
-                            const float2 Fm = __fadd2_rn(Em, Ym), Gm = __ffma2_rn(Ym, neg1, Em);
-                            au[j] = __ffma2_rn(up2, Fp, __ffma2_rn(um2, Fm, au[j]));
-                            av[j] = __ffma2_rn(vp2, Fp, __ffma2_rn(vm2, Fm, av[j]));
-                            aw[j] = __ffma2_rn(wp2, Gp, __ffma2_rn(wm2, Gm, aw[j]));
-                            if (PR) apr[j] = __ffma2_rn(pp2, Fp, __ffma2_rn(pm2, Fm, apr[j]));
-                        }
+                for (int j = 0; j < (PR ? LP : 1); j++) apr[j] = make_float2(0.f, 0.f);
+                const float2 neg1 = make_float2(-1.f, -1.f);
+                const int m0 = (M == I) ? ii : 0;
+                for (int mm = m0; mm < TT; mm++) {
+                    const float4 c0 = *reinterpret_cast<const float4 *>(s_tab + (ii * TT + mm) * GRIDV_NC);
+                    const float4 c1 = *reinterpret_cast<const float4 *>(s_tab + (ii * TT + mm) * GRIDV_NC + 4);
+                    const float2 pm = s_ph[mm * cols + cl];
+                    const float cc = pi.x * pm.x, ss = pi.y * pm.y;
+                    const float sc = pi.y * pm.x, cs = pi.x * pm.y;
+                    const float cp = cc - ss, cmn = cc + ss, sp = sc + cs, smn = sc - cs;
+                    const float up = c0.x * cp, um = c0.y * cmn, vp = c0.z * cp, vm = c0.w * cmn;
+                    const float wp = c1.x * sp, wm = c1.y * smn;
+                    const float2 up2 = make_float2(up, up), um2 = make_float2(um, um);
+                    const float2 vp2 = make_float2(vp, vp), vm2 = make_float2(vm, vm);
+                    const float2 wp2 = make_float2(wp, wp), wm2 = make_float2(wm, wm);
+                    const float2 kp2 = make_float2(c1.z, c1.z), km2 = make_float2(c1.w, c1.w);
+                    float2 pp2 = make_float2(0.f, 0.f), pm2 = pp2;
+                    if (PR) {
+                        const float2 tp = s_tp[ii * TT + mm];
+                        const float pp = tp.x * cp, pm_ = tp.y * cmn;
+                        pp2 = make_float2(pp, pp);
+                        pm2 = make_float2(pm_, pm_);
                     }
 #pragma unroll
                     for (int j = 0; j < LP; j++) {
-                        kahan(su[2 * j], cu[2 * j], ri * au[j].x);
-                        kahan(su[2 * j + 1], cu[2 * j + 1], ri * au[j].y);
-                        kahan(sv[2 * j], cv[2 * j], ri * av[j].x);
-                        kahan(sv[2 * j + 1], cv[2 * j + 1], ri * av[j].y);
-                        kahan(sw[2 * j], cw[2 * j], ri * aw[j].x);
-                        kahan(sw[2 * j + 1], cw[2 * j + 1], ri * aw[j].y);
-                        if (PR) {
-                            kahan(sp[2 * j], cq[2 * j], ri * apr[j].x);
-                            kahan(sp[2 * j + 1], cq[2 * j + 1], ri * apr[j].y);
-                        }
+                        const float2 ap = __fmul2_rn(kp2, zk2[j]), bp = __fmul2_rn(kp2, yk2[j]);
+                        const float2 am = __fmul2_rn(km2, zk2[j]), bm = __fmul2_rn(km2, yk2[j]);
+                        const float2 Ep = make_float2(ex2(ap.x), ex2(ap.y));
+                        const float2 Yp = make_float2(ex2(bp.x), ex2(bp.y));
+                        const float2 Em = make_float2(ex2(am.x), ex2(am.y));
+                        const float2 Ym = make_float2(ex2(bm.x), ex2(bm.y));
+                        const float2 Fp = __fadd2_rn(Ep, Yp), Gp = __ffma2_rn(Yp, neg1, Ep);
+                        const float2 Fm = __fadd2_rn(Em, Ym), Gm = __ffma2_rn(Ym, neg1, Em);
+                        au[j] = __ffma2_rn(up2, Fp, __ffma2_rn(um2, Fm, au[j]));
+                        av[j] = __ffma2_rn(vp2, Fp, __ffma2_rn(vm2, Fm, av[j]));
+                        aw[j] = __ffma2_rn(wp2, Gp, __ffma2_rn(wm2, Gm, aw[j]));
+                        if (PR) apr[j] = __ffma2_rn(pp2, Fp, __ffma2_rn(pm2, Fm, apr[j]));
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < LP; j++) {
+                    kahan(su[2 * j], cu[2 * j], ri * au[j].x);
+                    kahan(su[2 * j + 1], cu[2 * j + 1], ri * au[j].y);
+                    kahan(sv[2 * j], cv[2 * j], ri * av[j].x);
+                    kahan(sv[2 * j + 1], cv[2 * j + 1], ri * av[j].y);
+                    kahan(sw[2 * j], cw[2 * j], ri * aw[j].x);
+                    kahan(sw[2 * j + 1], cw[2 * j + 1], ri * aw[j].y);
+                    if (PR) {
+                        kahan(sp[2 * j], cq[2 * j], ri * apr[j].x);
+                        kahan(sp[2 * j + 1], cq[2 * j + 1], ri * apr[j].y);
                     }
                 }
             }
@@ -1876,7 +1871,7 @@ int launch_eta_pairs(const DevSea &sea, long n, const float2 *ph, const float *r
     PairArgs a{};
     a.ncol = n; a.nl = 1; a.nlg = 1; a.ntile = sea.ntile_g; a.tab = sea.d_tab_eta;
     a.ph = ph; a.rr = rr; a.rs = sea.trivial_ramp ? 0 : n; a.cf = sea.d_cf; a.cstride = sea.npad_g; a.out = out;
-    a.pairs = 1; a.first = 0; a.one = 1.f;
+    a.first = 0; a.one = 1.f;
     const long nblk = (n + 128 * ETA_P - 1) / (128 * ETA_P);
     const int ntp = sea.ntile_g * (sea.ntile_g + 1) / 2 * ETA_H;   // steps of the walk
     constexpr size_t smem = ETA_SMEM;
@@ -1932,8 +1927,8 @@ static int column_pairs_t(const PairArgs &a, long nblk, int nslice, int cols, cu
 
 // u, v, w (pressure: and p) sums of the columns at their levels, out [nf][ncol nl]
 int launch_column_pairs(const DevSea &sea, long ncol, int nl, const float2 *ph, const float *rr,
-                        const float *z0, float *out, int pairs, cudaStream_t stream, float *split_buf,
-                        long split_cap, bool pressure) {
+                        const float *z0, float *out, cudaStream_t stream, float *split_buf, long split_cap,
+                        bool pressure) {
     constexpr int LV = 8;
     int nlg = 1;
     while (nlg * LV < nl) nlg *= 2;
@@ -1944,16 +1939,16 @@ int launch_column_pairs(const DevSea &sea, long ncol, int nl, const float2 *ph, 
     a.ncol = ncol; a.nl = nl; a.nlg = nlg; a.ntile = sea.ntile_g; a.tab = sea.d_tab_grid;
     a.tabp = reinterpret_cast<const float2 *>(sea.d_tab_gp);
     a.ph = ph; a.rr = rr; a.rs = sea.trivial_ramp ? 0 : ncol; a.cf = sea.d_cf; a.cstride = sea.npad_g; a.z0 = z0;
-    a.depth = (float)sea.depth; a.out = out; a.pairs = pairs; a.first = 1;
+    a.depth = (float)sea.depth; a.out = out; a.first = 1;
     int cols = 128 / nlg;
     // Few columns (a small grid, a column sample): split the tile-pair loop
     // over blockIdx.y so that the launch still fills the GPU, and sum the
     // slices in a fixed order afterwards.
     const long nblk = (ncol + cols - 1) / cols;
-    const int ntp = pairs ? sea.ntile_g * (sea.ntile_g + 1) / 2 : sea.ntile_g;
+    const int ntp = sea.ntile_g * (sea.ntile_g + 1) / 2;
     int nslice = 1;
     a.tp_per = ntp;
-    if (pairs && split_buf && nblk < SPLIT_TARGET_BLOCKS) {
+    if (split_buf && nblk < SPLIT_TARGET_BLOCKS) {
         int want = (int)std::min<long>(ntp, (SPLIT_TARGET_BLOCKS + nblk - 1) / nblk);
         int per = (ntp + want - 1) / want;
         int ns = (ntp + per - 1) / per;

@@ -1103,15 +1103,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_qform_tc(const __grid_constan
                                          fmaf(v[jj + 1], w.y, fmaf(v[jj + 2], w.z, fmaf(v[jj + 3], w.w, part2))));
                         }
                 }
-                if (TWO) {
-                    // cross products: lo parts carry a factor 2^11
-                    float w[32];
-                    tmem_ld32(acc + BN + c * 32, w);
-                    float pw = 0.f;
-#pragma unroll
-                    for (int jj = 0; jj < 32; jj++) pw = fmaf(w[jj], ys[sl][jj], pw);
-                    part = fmaf(pw, 1.0f / 2048.0f, part);
-                }
                 if (c + NSL < NCH) {
 #pragma unroll
                     for (int jj = 0; jj < 32; jj++)

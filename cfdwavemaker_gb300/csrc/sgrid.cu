@@ -43,8 +43,8 @@ namespace cfdwm {
 int launch_eta_pairs(const DevSea &sea, long n, const float2 *ph, const float *rr, float *out,
                      cudaStream_t stream, float *split_buf, long split_cap);
 int launch_column_pairs(const DevSea &sea, long ncol, int nl, const float2 *ph, const float *rr,
-                        const float *z0, float *out, int pairs, cudaStream_t stream, float *split_buf,
-                        long split_cap, bool pressure);
+                        const float *z0, float *out, cudaStream_t stream, float *split_buf, long split_cap,
+                        bool pressure);
 long column_pairs_split_floats(int nl);
 int launch_pressure_kin(const DevSea &sea, double t, int nz, double *kin, cudaStream_t stream);
 
@@ -608,8 +608,8 @@ static int fill_cols(DevGrid &g, const DevSea &sea, Workspace &ws, const int *ac
         if (!rc) rc = depthform_combine(x->df, nact, g.nl, x->zmin, x->sec, stream);
     } else {
         // first and second order per (pair, level)
-        rc = launch_column_pairs(sea, nact, g.nl, (float2 *)b, (float *)(b + fb.ph), x->zmin, x->sec, 1, stream, x->split, x->split_cap,
-                                 pres);
+        rc = launch_column_pairs(sea, nact, g.nl, (float2 *)b, (float *)(b + fb.ph), x->zmin, x->sec, stream, x->split,
+                                 x->split_cap, pres);
     }
     if (rc) return rc;
     if (pres) {

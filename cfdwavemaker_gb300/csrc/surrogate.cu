@@ -206,7 +206,7 @@ struct Surrogate {
     const float *g_eta = nullptr;      // identity of the attached grid
     double g_dx = 0, g_dy = 0, g_dom[4] = {0, 0, 0, 0}, g_ign[4] = {0, 0, 0, 0};
     void *xs = nullptr;        // first-order channels, split (convtc.h)
-    float *base = nullptr, *eta1 = nullptr, *pred = nullptr, *hbuf = nullptr;
+    float *base = nullptr, *eta1 = nullptr, *pred = nullptr;
     float *R = nullptr;        // residual (plain - network) of the last plain slot, [cout][nx ny]
     float *Rtmp = nullptr;
     bool have_res = false;
@@ -226,10 +226,10 @@ struct Surrogate {
 static Surrogate g_s;
 
 static void free_grid_side(Surrogate &s) {
-    void *q[] = {s.xs, s.base, s.eta1, s.pred, s.hbuf, s.rETA, s.rU[0], s.rU[1], s.rU[2],
+    void *q[] = {s.xs, s.base, s.eta1, s.pred, s.rETA, s.rU[0], s.rU[1], s.rU[2],
                  s.d_sample, s.d_err, s.R, s.Rtmp};
     for (void *p : q) if (p) cudaFree(p);
-    s.xs = nullptr; s.base = s.eta1 = s.pred = s.hbuf = s.rETA = s.R = nullptr;
+    s.xs = nullptr; s.base = s.eta1 = s.pred = s.rETA = s.R = nullptr;
     s.Rtmp = nullptr;
     s.have_res = false;
     s.rU[0] = s.rU[1] = s.rU[2] = nullptr;
