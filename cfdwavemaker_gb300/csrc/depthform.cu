@@ -494,8 +494,9 @@ static int pot_holds(const DfCoefArgs &a, bool *holds, cudaStream_t stream) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     cudaFree(d);
     CK(e);
-    // (a NaN anywhere: not the potential form)
-    *holds = h[0] <= POT_RHO * POT_RHO * h[1] && (a.nf != 4 || h[2] <= POT_RHO_P * POT_RHO_P * h[3]);
+    // (not the potential form with a NaN anywhere, nor where the pressure's tables, of
+    // which it takes P and M then, are zero: a density of 0)
+    *holds = h[0] <= POT_RHO * POT_RHO * h[1] && (a.nf != 4 || h[2] < POT_RHO_P * POT_RHO_P * h[3]);
     return OK;
 }
 

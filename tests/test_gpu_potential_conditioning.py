@@ -74,3 +74,23 @@ def test_close_frequencies(wm, kind, pressure):
     for f, (a, b) in enumerate(zip(got, ref)):
         e = np.max(np.abs(a - b)) / np.max(np.abs(b))
         assert np.isfinite(b).all() and e <= TOL, (kind, f, e)
+
+
+def test_no_density(wm):
+    """The pressure of a sea without density is zero, and its velocities are those of
+    the same sea without the pressure."""
+    comps = ss.irregular_components(3.0, 9.0, 2.0, 24, 0.4, 1.8, 45.0, 3, ndir=4, spreading_s=6.0)
+    grid = {"bounds": (-40.0, 20.0, 10.0, 80.0), "nx": NX, "ny": NY, "nl": NL, "t0": 17.5, "dt": 0.5,
+            "stretch": (0.7, 1.5)}
+    txt = ss.write_irregular(None, comps, 45.0, extrap=2, mtheta=20.0, rho=0.0, lsgrid=grid)
+    assert wm.initialize_text(txt) == 0, cw.last_error()
+    wm.sgrid_method(1)
+    ref = np.zeros((2, 3, NX, NY, NL), np.float32)
+    p = np.ones((NX, NY, NL), np.float32)
+    for on in (0, 1):
+        wm.sgrid_pressure(bool(on))
+        for f in range(3):
+            assert wm.lib.cfdwm_sgrid_block_export(1 + f, 0, NX, cw._ptr(ref[on, f])) == 0, cw.last_error()
+    assert wm.lib.cfdwm_sgrid_block_export(4, 0, NX, cw._ptr(p)) == 0, cw.last_error()
+    assert not p.any()
+    assert np.max(np.abs(ref[1] - ref[0])) <= TOL * np.max(np.abs(ref[0]))
