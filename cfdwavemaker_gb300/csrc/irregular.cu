@@ -68,12 +68,12 @@ constexpr long SPLIT_TARGET_BLOCKS = 4 * 152;   // blocks a column-pair launch a
 // Batches that the evaluation by points (k_point_few) takes: 20 points, where
 // the per-thread kernels' blocks of 128 are nearly empty, and as many more as
 // 4e6 (pair, point) terms are, where its terms, read per point, cost less than
-// the per-thread path's eight dependent kernels.  Measured, a wave_Kinematics
+// the per-thread path's seven dependent kernels.  Measured, a wave_Kinematics
 // and a pressure batch from host arrays, this kernel against the per-thread
-// ones: 24 components, 1024 points 82 and 150 us; 128 components, 256 points 100
-// and 127, 512 points 144 and 130; 256 components, 64 points 105 and 129, 128
-// points 140 and 130; 384 components, 64 points 144 and 149; 4096 components,
-// 16 points 1.9 and 2.2 ms, 64 points 7.3 and 2.2.
+// ones: 24 components, 1024 points 75 and 111 us; 128 components, 256 points 105
+// and 122, 512 points 145 and 123; 256 components, 64 points 99 and 126, 128
+// points 129 and 129; 384 components, 64 points 137 and 147; 4096 components,
+// 16 points 1.9 and 2.3 ms, 64 points 7.2 and 2.2.
 constexpr long FEW_MAX_POINTS = 4096;
 constexpr int FEW_MAX_NPAD = 4096;   // components whose phasors, profiles and ramps fit shared memory
 static bool few_points(long n, int npad) {
@@ -1543,7 +1543,8 @@ constexpr int FEW_E = 8;             // terms of an item
 struct FewArgs {
     long n, ldo;
     const double *x, *y, *z, *t;
-    double fx, fy, swl, depth;
+    double swl, depth;
+    float2 ox, oy;                   // -fx, -fy
     int ncomp, npad, cstride, trivial_ramp, order, clamp, kin, mask;
     const float *rec, *cf;
     const float2 *cfp;
@@ -1648,31 +1649,32 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
     float2 *s_px = s_ph + a.npad;                           // kin: profiles px, pz [npad]
     float *s_r = reinterpret_cast<float *>(s_px + (a.kin ? a.npad : 0));   // ramps [npad] (individual ramps)
     __shared__ float2 s_red[FEW_T / 32][FEW_Q];
-    __shared__ double s_sum[FEW_Q];
+    __shared__ double s_sum[FEW_Q], s_z0;
+    __shared__ float2 s_z, s_zeta;                          // z0, -2 (z0 + h)
     __shared__ float s_ramp;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int tid = threadIdx.x;
     const long p = blockIdx.x;
     const int ns = gridDim.y, slice = blockIdx.y;
-    const double xp = a.x[p], yp = a.y[p], zp = a.z[p], tp = a.t[p];
+    const double xp = a.x[p], yp = a.y[p], tp = a.t[p];
     const double *P = a.phase;
     const int cs = a.cstride;
-    const double zz = (a.clamp ? fmax(-a.depth, zp) : zp) - a.swl, z0 = a.order == 0 ? zz : fmin(0.0, zz);
-    const double zeta0 = -2.0 * (z0 + a.depth);
-    const float zk = (float)z0 * LOG2E_F, zetak = (float)zeta0 * LOG2E_F;
+    // FP64 by one thread (an instruction holds the pipe for 16 cycles a warp; by every
+    // thread, 24 components, 4096 points: 178 us a call, 148 so)
+    if (tid == 0) {
+        const double zz = (a.clamp ? fmax(-a.depth, a.z[p]) : a.z[p]) - a.swl, z0 = a.order == 0 ? zz : fmin(0.0, zz);
+        s_z0 = z0;
+        s_z = ff_from_double(z0);
+        s_zeta = ff_from_double(-2.0 * (z0 + a.depth));
+    }
     if (a.trivial_ramp) {
         if (tid == FEW_T - 1) s_ramp = (float)d_freq_ramp(tp, P[4 * cs], P[5 * cs], P[6 * cs]);
     } else {
         for (int i = tid; i < a.npad; i += FEW_T)
             s_r[i] = i < a.ncomp ? (float)d_freq_ramp(tp, P[4 * cs + i], P[5 * cs + i], P[6 * cs + i]) : 0.f;
     }
-    float2 dx, dy, tt = ff_from_double(tp);
+    const float2 dx = ff_add(ff_from_double(xp), a.ox), dy = ff_add(ff_from_double(yp), a.oy), tt = ff_from_double(tp);
     {
-        float2 ox, oy;
-        ff_split(-a.fx, ox.x, ox.y);
-        ff_split(-a.fy, oy.x, oy.y);
-        dx = ff_add(ff_from_double(xp), ox);
-        dy = ff_add(ff_from_double(yp), oy);
         const PhPoint pt(dx, dy, tt);
         for (int i = 2 * tid; i < a.npad; i += 2 * FEW_T) {
             f32x2 hi, lo, s2, c2;
@@ -1683,7 +1685,9 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
             s_ph[i + 1] = make_float2(c.y, s.y);
         }
     }
-    if (a.kin)
+    __syncthreads();
+    const float zk = s_z.x * LOG2E_F, zetak = s_zeta.x * LOG2E_F;
+    if (a.kin) {
         for (int i = tid; i < a.npad; i += FEW_T) {
             // cosh(k(z+h))/cosh(kh), sinh(k(z+h))/cosh(kh)
             const float q = a.cf[CF_Q * cs + i];
@@ -1691,22 +1695,23 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
             depth_fg(a.cf[CF_K * cs + i], zk, zetak, F, G);
             s_px[i] = make_float2(q * F, q * G);
         }
-    __syncthreads();
+        __syncthreads();
+    }
     auto ramp = [&](int i) { return a.trivial_ramp ? s_ramp : s_r[i]; };
     float2 S[FEW_Q];
 #pragma unroll
     for (int q = 0; q < FEW_Q; q++) S[q] = make_float2(0.f, 0.f);
-    if (slice * FEW_T + tid < a.ncomp) {
-        float2 z, zeta;
-        ff_split(z0, z.x, z.y);
-        ff_split(zeta0, zeta.x, zeta.y);
-        for (int i = slice * FEW_T + tid; i < a.ncomp; i += ns * FEW_T) few_first(a, i, dx, dy, tt, z, zeta, ramp(i), S);
-    }
-    // pair items, eight terms each; the records of two neighbouring terms are
-    // interleaved (velocity, pressure) or adjacent (elevation)
+    // pair items, eight terms each, then the components' first order; the records of
+    // two neighbouring terms are interleaved (velocity, pressure) or adjacent
+    // (elevation)
     const f32x2 zk2 = p_pack(zk, zk), zetak2 = p_pack(zetak, zetak), neg1 = p_pack(-1.f, -1.f);
     const long total = a.nv + a.np + a.ne;
-    for (long item = (long)slice * FEW_T + tid; item < total; item += (long)ns * FEW_T) {
+    for (long item = (long)slice * FEW_T + tid; item < total + a.ncomp; item += (long)ns * FEW_T) {
+        if (item >= total) {
+            const int i = (int)(item - total);
+            few_first(a, i, dx, dy, tt, s_z, s_zeta, ramp(i), S);
+            continue;
+        }
         int I, M, i, m0;
         if (item < a.nv + a.np) {
             const bool vel = item < a.nv;
@@ -1807,7 +1812,7 @@ __global__ void __launch_bounds__(FEW_T) k_point_few(FewArgs a) {
     }
     if (ns > 1) return;
     __syncthreads();
-    if (tid == 0) few_rows(a, p, s_sum, (a.mask & 16) && a.kt.kin ? s_ramp * kin_at(a.kt.kin, a.kt.nz, a.kt.h, z0) : 0.0);
+    if (tid == 0) few_rows(a, p, s_sum, (a.mask & 16) && a.kt.kin ? s_ramp * kin_at(a.kt.kin, a.kt.nz, a.kt.h, s_z0) : 0.0);
 }
 
 // The slices of a point's sums, a warp a sum in turn, its lanes over the slices.
@@ -2188,7 +2193,9 @@ static int launch_point_few(const DevSea &sea, long n, const double *x, const do
                             cudaStream_t stream, const ApiRows *api) {
     FewArgs a{};
     a.n = n; a.ldo = n; a.x = x; a.y = y; a.z = z; a.t = t;
-    a.fx = sea.fx; a.fy = sea.fy; a.swl = sea.swl; a.depth = sea.depth;
+    a.swl = sea.swl; a.depth = sea.depth;
+    ff_split(-sea.fx, a.ox.x, a.ox.y);
+    ff_split(-sea.fy, a.oy.x, a.oy.y);
     a.ncomp = sea.n; a.npad = sea.npad_g; a.cstride = sea.npad_g; a.trivial_ramp = sea.trivial_ramp ? 1 : 0;
     a.order = sea.order; a.clamp = api ? 1 : 0; a.mask = mask;
     a.rec = sea.d_phrec; a.cf = sea.d_cf; a.cfp = sea.d_cfp; a.phase = sea.d_phase;
@@ -2204,8 +2211,8 @@ static int launch_point_few(const DevSea &sea, long n, const double *x, const do
     a.part = reinterpret_cast<float2 *>(L.split); a.out = out;
     if (api) a.api = *api;
     if (table) a.kt = KinTab{sea.d_kin, sea.kin_nz, sea.kin_h, sea.depth, nullptr};
-    // as many slices as give every thread one item, up to about eight blocks an SM in all
-    const long want = std::max<long>(1, (a.nv + a.np + a.ne + FEW_T - 1) / FEW_T);
+    // as many slices as give every thread one item or component, up to about eight blocks an SM in all
+    const long want = std::max<long>(1, (a.nv + a.np + a.ne + a.ncomp + FEW_T - 1) / FEW_T);
     const long cap = std::max<long>(1, 2 * SPLIT_TARGET_BLOCKS / n);
     const long ns = std::min(std::min(want, cap), std::max<long>(1, L.split_cap / (2 * FEW_Q * n)));
     const size_t smem = sizeof(float2) * (size_t)a.npad * (a.kin ? 2 : 1) + (sea.trivial_ramp ? 0 : sizeof(float) * a.npad);
