@@ -145,12 +145,13 @@ __device__ __forceinline__ void col_rows(const GridTab &T, const GridCols &c, lo
 // TILE: block (blockIdx.x, blockIdx.y) holds SR rows of 32 columns of the whole
 // grid, and a thread SR columns, whose y entries are one load; else blockIdx.x
 // holds SR x 32 listed columns.  Warp w sums the components w, w + nw, ...  Loads
-// of table entries bound it where a term is added plainly (one column a thread,
-// 65536 columns of 1024 components 144 us, 79 with four), but every
+// of table entries bound it where terms are added plainly (one column a thread,
+// 65536 columns of 1024 components 144 us, 79 with four, FMA pipe 42 %); here every
 // term's rounding error is kept: 14 packed operations a component for two columns
-// instead of 9, eight components' loads in flight at two blocks an SM (a learned
-// update 583 us with 16 plain terms a Kahan step, 597 so; four blocks, two
-// components 615, three and four 615, one and eight 610).  With the phase
+// instead of 9, eight components' loads in flight at two blocks an SM, 76 us with
+// the FMA pipe at 75 %.  In a learned update, beside the checked columns' kernels,
+// 583 us with 16 plain terms a Kahan step, 597 so (four blocks of two components in
+// flight 615, three of four 615, one of eight 610).  With the phase
 // formed per (column, component) it was issue-bound, 256 us.  A short list gets
 // 32 warps a block (64 columns: 8 warps 54 us, 23; one thread per column
 // 180).

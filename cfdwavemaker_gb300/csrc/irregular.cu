@@ -1523,9 +1523,10 @@ __global__ void k_combine(long n, long ldo, int order, double swl, const double 
 // (phasors, heights, elevation and point pairs, slice sums, combining pass) a
 // wave_VeloX call of the 128-component sea was five dependent kernels, 26 us; 18 us
 // now (a launch and a synchronisation are 8 of these).  The blocks of a point could
-// also find out the last of them by a counter (four scalar calls 75 us, 73 so), but
-// so nothing carries over from one call to the next, whatever the workspace held
-// and whichever streams share it.
+// also find out the last of them by a counter, no faster (four scalar calls 75 us with
+// the counter, 73 so, 69 with the first order as items of its own), but this way
+// nothing carries over from one call to the next, whatever the workspace held and
+// whichever streams share it.
 //
 // Accuracy.  A single value is held to its own size, not to that of the largest
 // of a batch, and the first order is nearly all of it.  Its terms are formed in
