@@ -11,9 +11,10 @@ from cfdwavemaker_gb300 import seastate as ss
 
 pytestmark = pytest.mark.gpu
 
-# of a field's maximum: the FP32 rounding of the field (6e-8) and of the second-order
-# sums, a third of it at most, good to 3e-7 of their own maximum in either form
-TOL = 2e-7
+# of a field's maximum: two units in the last place of the stored FP32 values (up to
+# 1.2e-7 each; the forms' sums are atomic, in no fixed order) and of the second-order
+# sums, a fifth of it at most, 3e-7 of their own maximum in either form
+TOL = 3e-7
 NX, NY, NL = 13, 17, 10
 
 
